@@ -1,14 +1,75 @@
 // GEMM entry points: argument validation and engine choice.
 // Reference counterparts: CUDAMath::apply_normal_gemm / apply_batched_gemm (backend/cuda/kernels_math.cu:725-779),
 // whose NMMMeta / BMMMeta fields (core/types.hpp:118-158) map one to one onto the arguments here.
+#include <algorithm>
+
 #include "gemm.cuh"
 
 using namespace gcb;
 
+static constexpr int64_t kPackWork = int64_t(1) << 24;  // multiply-adds from which unaligned operands are packed for the tensor cores
+
+namespace gcb {
+
+// out[b][r][c] = in[b][r][c] for c < cols, rows `pitch` floats apart (a multiple of four; what lies beyond cols is never read as
+// an operand: the tensor maps end at cols).  Bound by memory; a block copies 1024 columns of one row per step, neighbouring
+// threads neighbouring elements, because neither side's rows need start on a 16-byte boundary.
+__global__ void __launch_bounds__(256) pack_rows_kernel(float* __restrict__ out, const float* __restrict__ in, int64_t rows, int64_t cols, int64_t ld, int64_t so, int64_t si, int64_t n_inner,
+                                                        int64_t total_rows, int64_t pitch) {
+    const int64_t c0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+    for (int64_t r = blockIdx.y; r < total_rows; r += gridDim.y) {
+        const int64_t item = r / rows, row = r - item * rows, bo = item / n_inner, bi = item - bo * n_inner;
+        const float* src = in + bo * so + bi * si + row * ld;
+        float* dst = out + r * pitch;
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = c0 + 256 * u < cols ? __ldcs(src + c0 + 256 * u) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) if (c0 + 256 * u < cols) dst[c0 + 256 * u] = v[u];
+    }
+}
+
+// An operand TMA cannot address (base off a 16-byte boundary, row or batch strides no multiple of four floats) is copied into
+// rows that it can address.  rows x cols as stored.
+struct PackedOperand {
+    Scratch sc;
+    explicit PackedOperand(gcb_ctx* ctx) : sc(ctx) {}
+    int pack(gcb_ctx* ctx, const float** p, int64_t* ld, int64_t* so, int64_t* si, int64_t rows, int64_t cols, int64_t n_outer, int64_t n_inner) {
+        auto ok4 = [](int64_t v) { return v % 4 == 0; };
+        if (aligned16(*p) && ok4(*ld) && (n_inner == 1 || ok4(*si)) && (n_outer == 1 || ok4(*so))) return GCB_OK;
+        const int64_t pitch = (cols + 3) / 4 * 4, total_rows = rows * n_outer * n_inner;
+        int rc = sc.get(sizeof(float) * (size_t)(total_rows * pitch));
+        if (rc) return rc;
+        dim3 grid((unsigned)((cols + 1023) / 1024), (unsigned)std::min<int64_t>(total_rows, 65535), 1);
+        pack_rows_kernel<<<grid, 256, 0, ctx->stream>>>(sc.as<float>(), *p, rows, cols, *ld, *so, *si, n_inner, total_rows, pitch);
+        *p = sc.as<float>();
+        *ld = pitch;
+        *si = rows * pitch;
+        *so = n_inner * rows * pitch;
+        return after_launch(ctx, "gemm_pack");
+    }
+};
+
+}  // namespace gcb
+
 // Engine choice for one validated problem; no timing here, so the GELU fallback below may call it again freely.
 static int dispatch_gemm(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g, const char* who) {
     int rc = GCB_UNSUPPORTED;
-    if (ctx->gemm_engine != 1 && gemm_tc_eligible(ta, tb, g)) rc = gemm_tc_launch(ctx, ta, tb, g);
+    if (ctx->gemm_engine != 1 && gemm_tc_eligible(g)) rc = gemm_tc_launch(ctx, ta, tb, g);
+    // Operands that only their addresses keep from the tensor cores are copied into rows that suit them, once the product is
+    // large enough to pay for the passes: a copy costs ~3 us, the FMA engine takes about that long per 2^25 multiply-adds.
+    if (rc == GCB_UNSUPPORTED && ctx->gemm_engine == 0 && g.M * g.N * g.K * g.batch_outer * g.batch_inner >= kPackWork && g.batch_outer * g.batch_inner <= 65535) {
+        GemmArgs packed = g;
+        PackedOperand pa(ctx), pb(ctx);
+        rc = pa.pack(ctx, &packed.A, &packed.lda, &packed.a_so, &packed.a_si, ta ? g.K : g.M, ta ? g.M : g.K, g.batch_outer, g.batch_inner);
+        if (rc == GCB_OK) rc = pb.pack(ctx, &packed.B, &packed.ldb, &packed.b_so, &packed.b_si, tb ? g.N : g.K, tb ? g.K : g.N, g.batch_outer, g.batch_inner);
+        if (rc) return rc;
+        rc = GCB_UNSUPPORTED;
+        if (packed.A != g.A || packed.B != g.B) {
+            if (gemm_tc_eligible(packed)) rc = gemm_tc_launch(ctx, ta, tb, packed);
+            if (rc == GCB_UNSUPPORTED && gemm_tc_eligible(packed)) return dispatch_gemm(ctx, ta, tb, packed, who);  // an epilogue that this kernel lacks runs as a second pass, on the packed operands
+        }
+    }
     if (rc == GCB_UNSUPPORTED && (g.gelu_pre || g.gelu_act)) {
         // no kernel with the fused GELU epilogues takes this problem: the same product, then the elementwise pass over C
         GemmArgs plain = g;

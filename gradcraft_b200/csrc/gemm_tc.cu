@@ -54,7 +54,8 @@ struct TcParams {
     int split_mode;      // 2 (default): one TF32 product of the truncated parts + two BF16 cross products (split_hybrid below);
                          // 1: three TF32 products; big stays as loaded — the tensor core ignores the 13 low mantissa bits — and small = rna_tf32(x - trunc(x));
                          // 0: as 1 with big = rna_tf32(x) written back, small = x - big (does not rely on the hardware's truncation)
-    float* partial;      // [splits][M][N] when splits > 1
+    float* partial;      // [splits][M][partial_ld] when splits > 1
+    int64_t partial_ld;  // N rounded up to a multiple of four: whole vectors whatever N is
     int b_twin;              // pair kernel: the BF16 companions of B come pre-split from global memory (map_t), the B-splitter warps idle
     int c_tma;               // 256-wide single-CTA kernel: C leaves (and the probabilities arrive) through TMA on swizzled 32 x 32 blocks in shared memory
     float* colsum;           // column sums of op(B) (see GemmArgs), or NULL: pair kernel with B stored K x N only
@@ -674,8 +675,7 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
         float* stg = reinterpret_cast<float*>(gen_base + TC_STAGES * S::STAGE_BYTES) + ew * 32 * S::EPI_PITCH;
         const bool to_partial = p.splits > 1;
         // the float4 fast path needs every array the epilogue touches with vector accesses on 16-byte boundaries: C and, laid out like C, the probabilities
-        const bool vec_ok = to_partial ? (p.N % 4 == 0)
-                                       : (p.ldc % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.sm_probs) | (uintptr_t)(p.c_so * 4) | (uintptr_t)(p.c_si * 4)) & 15) == 0);
+        const bool vec_ok = to_partial || (p.ldc % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.sm_probs) | (uintptr_t)(p.c_so * 4) | (uintptr_t)(p.c_si * 4)) & 15) == 0);
         const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
         const int sub_r = lane >> 3, sub_c = (lane & 7) * 4;  // store phase: 4 rows x 8 float4 per instruction (128 B per row)
         uint32_t lt = 0;
@@ -685,8 +685,8 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
             const TileCoord tc = tile_coord(p, w, BN);
             if (tc.skip) continue;
             const uint32_t buf = lt % S::NACC;
-            float* cbase = to_partial ? p.partial + (int64_t)tc.split * p.M * p.N : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
-            const int64_t ld = to_partial ? p.N : p.ldc;
+            float* cbase = to_partial ? p.partial + (int64_t)tc.split * p.M * p.partial_ld : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
+            const int64_t ld = to_partial ? p.partial_ld : p.ldc;
             const float alpha = to_partial ? 1.0f : p.alpha, beta = to_partial ? 0.0f : p.beta;
             const float* bias = to_partial ? nullptr : p.bias;
             const float* sm_probs = (BN == 256 && !to_partial) ? p.sm_probs : nullptr;  // only the 256-wide instantiation carries this epilogue (the launcher sees to it)
@@ -749,20 +749,30 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
                             }
                             st4(dst, o);
                         }
-                    } else {
-                        for (int r4 = 0; r4 < 8; ++r4) {
-                            const int64_t m = m_first + 4 * r4;
-                            if (m >= p.M) break;
-                            float* d = cbase + m * ld + n;
-                            const float* sp = src + r4 * 4 * S::EPI_PITCH;
-                            for (int u = 0; u < 4; ++u) {
-                                if (n + u < p.N) {
-                                    float r = sp[u] * alpha;
-                                    if (bias) r += bias[n + u];
-                                    if (beta != 0.0f) r += beta * d[u];
-                                    if (sm_probs) r = n + u <= m ? p.sm_scale * sm_probs[(d - p.C) + u] * (r - sm_rd[m]) : 0.0f;
-                                    d[u] = r;
-                                }
+                    } else {  // ragged or unaligned block: lane = column, so that a row is still stored as one contiguous run; eight rows' old values in flight
+                        const int64_t nc = nb + lane;
+                        const bool col_ok = nc < p.N;
+                        const float bc = (bias && col_ok) ? bias[nc] : 0.0f;
+                        const int64_t mb = (int64_t)tc.m0 + 32 * q;
+                        const int rows = (int)min((int64_t)32, p.M - mb);
+                        const int64_t poff = cbase - p.C;
+                        for (int r0 = 0; r0 < rows; r0 += 8) {
+                            float oldv[8], prv[8];
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) {
+                                const bool live = col_ok && r0 + u < rows;
+                                oldv[u] = (beta != 0.0f && live) ? cbase[(mb + r0 + u) * ld + nc] : 0.0f;
+                                prv[u] = (sm_probs && live && nc <= mb + r0 + u) ? sm_probs[poff + (mb + r0 + u) * ld + nc] : 0.0f;
+                            }
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) {
+                                const int64_t m = mb + r0 + u;
+                                if (!col_ok || r0 + u >= rows) continue;
+                                float r = stg[(r0 + u) * S::EPI_PITCH + lane] * alpha;
+                                if (bias) r += bc;
+                                if (beta != 0.0f) r += beta * oldv[u];
+                                if (sm_probs) r = nc <= m ? p.sm_scale * prv[u] * (r - sm_rd[m]) : 0.0f;
+                                cbase[m * ld + nc] = r;
                             }
                         }
                     }
@@ -1076,8 +1086,7 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
         float* stg = reinterpret_cast<float*>(gen_base + NST * S::STAGE_BYTES) + ew * 32 * S::EPI_PITCH;
         const bool to_partial = p.splits > 1;
         // the float4 fast path needs C and the GELU side arrays (laid out like C) on 16-byte boundaries; otherwise the scalar path runs
-        const bool vec_ok = to_partial ? (p.N % 4 == 0)
-                                       : (p.ldc % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.gelu_pre) | reinterpret_cast<uintptr_t>(p.gelu_act) | reinterpret_cast<uintptr_t>(p.resid) |
+        const bool vec_ok = to_partial || (p.ldc % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.gelu_pre) | reinterpret_cast<uintptr_t>(p.gelu_act) | reinterpret_cast<uintptr_t>(p.resid) |
                                                               (uintptr_t)(p.c_so * 4) | (uintptr_t)(p.c_si * 4)) & 15) == 0);
         const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
         const int sub_r = lane >> 3, sub_c = (lane & 7) * 4;
@@ -1087,8 +1096,8 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
             const TileCoord tc = pair_tile_coord(p, w);
             if (tc.skip) continue;
             const uint32_t buf = lt % NACC;
-            float* cbase = to_partial ? p.partial + (int64_t)tc.split * p.M * p.N : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
-            const int64_t ld = to_partial ? p.N : p.ldc;
+            float* cbase = to_partial ? p.partial + (int64_t)tc.split * p.M * p.partial_ld : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
+            const int64_t ld = to_partial ? p.partial_ld : p.ldc;
             const float alpha = to_partial ? 1.0f : p.alpha, beta = to_partial ? 0.0f : p.beta;
             const float* bias = to_partial ? nullptr : p.bias;
             const float* gelu_pre = to_partial ? nullptr : p.gelu_pre;
@@ -1144,22 +1153,32 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
                             st4(dst, o);
                             if (gelu_act) st4(gelu_act + (dst - p.C), make_float4(gelu_f(o.x), gelu_f(o.y), gelu_f(o.z), gelu_f(o.w)));
                         }
-                    } else {
-                        for (int r4 = 0; r4 < 8; ++r4) {
-                            const int64_t m = m_first + 4 * r4;
-                            if (m >= p.M) break;
-                            float* d = cbase + m * ld + n;
-                            const float* sp = src + r4 * 4 * S::EPI_PITCH;
-                            for (int u = 0; u < 4; ++u) {
-                                if (n + u < p.N) {
-                                    float r = sp[u] * alpha;
-                                    if (bias) r += bias[n + u];
-                                    if (beta != 0.0f) r += beta * d[u];
-                                    if (gelu_pre) r *= gelu_grad_f(gelu_pre[(d - p.C) + u]);
-                                    if (resid) r += resid[(d - p.C) + u];
-                                    d[u] = r;
-                                    if (gelu_act) gelu_act[(d - p.C) + u] = gelu_f(r);
-                                }
+                    } else {  // ragged or unaligned block: lane = column, as in the single-CTA kernel
+                        const int64_t nc = nb + lane;
+                        const bool col_ok = nc < p.N;
+                        const float bc = (bias && col_ok) ? bias[nc] : 0.0f;
+                        const int rows = (int)max((int64_t)0, min((int64_t)32, p.M - mrow0));
+                        const int64_t soff = cbase - p.C;
+                        for (int r0 = 0; r0 < rows; r0 += 8) {
+                            float oldv[8], sv[8];
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) {
+                                const bool live = col_ok && r0 + u < rows;
+                                const int64_t at = (mrow0 + r0 + u) * ld + nc;
+                                oldv[u] = (beta != 0.0f && live) ? cbase[at] : 0.0f;
+                                sv[u] = (side && live) ? side[soff + at] : 0.0f;
+                            }
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) {
+                                if (!col_ok || r0 + u >= rows) continue;
+                                const int64_t at = (mrow0 + r0 + u) * ld + nc;
+                                float r = stg[(r0 + u) * S::EPI_PITCH + lane] * alpha;
+                                if (bias) r += bc;
+                                if (beta != 0.0f) r += beta * oldv[u];
+                                if (gelu_pre) r *= gelu_grad_f(sv[u]);
+                                if (resid) r += sv[u];
+                                cbase[at] = r;
+                                if (gelu_act) gelu_act[soff + at] = gelu_f(r);
                             }
                         }
                     }
@@ -1183,12 +1202,12 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
 
 // C = alpha * sum_s partial[s] + beta * C + bias, slices added in ascending order.  Launched with programmatic stream
 // serialisation behind the GEMM that wrote the partial tiles: its blocks may be scheduled while that grid drains, and
-// nothing is read before the grid has completed.  `vec` = every row of C and of the partial tiles starts on a 16-byte
-// boundary and N % 4 == 0 (four columns per thread, same order of additions per element as the scalar form).
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ C, const float* __restrict__ partial, const float* __restrict__ bias, int64_t M, int64_t N, int64_t ldc, int splits,
-                                                            float alpha, float beta, float* __restrict__ colsum, const float* __restrict__ colsum_partial, int colsum_accumulate, int vec) {
+// nothing is read before the grid has completed.  A thread takes four columns of one row (the partial rows are padded to whole
+// vectors); `vec` = C can be accessed as float4 too, otherwise its elements are touched one by one.
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ C, const float* __restrict__ partial, int64_t partial_ld, const float* __restrict__ bias, int64_t M, int64_t N,
+                                                            int64_t ldc, int splits, float alpha, float beta, float* __restrict__ colsum, const float* __restrict__ colsum_partial,
+                                                            int colsum_accumulate, int vec) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int64_t total = M * N;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
     if (colsum != nullptr) {  // the column sums of op(B), one partial per K slice
         for (int64_t n = tid; n < N; n += nthreads) {
@@ -1197,33 +1216,31 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ 
             colsum[n] = colsum_accumulate ? colsum[n] + s : s;
         }
     }
-    if (vec) {
-        const int64_t n4 = N >> 2, total4 = total >> 2;
-        for (int64_t i = tid; i < total4; i += nthreads) {
-            const int64_t m = i / n4, n = (i - m * n4) << 2;
-            const float4* src = reinterpret_cast<const float4*>(partial) + i;
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int64_t n4 = partial_ld >> 2, total4 = M * n4;
+    for (int64_t i = tid; i < total4; i += nthreads) {
+        const int64_t m = i / n4, n = (i - m * n4) << 2;
+        const float4* src = reinterpret_cast<const float4*>(partial) + i;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-            for (int k = 0; k < splits; ++k) {
-                const float4 v = __ldcg(src + (int64_t)k * total4);
-                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-            }
-            float4 o = make_float4(alpha * s.x, alpha * s.y, alpha * s.z, alpha * s.w);
-            if (bias) { o.x += bias[n]; o.y += bias[n + 1]; o.z += bias[n + 2]; o.w += bias[n + 3]; }
-            float4* dst = reinterpret_cast<float4*>(C + m * ldc + n);
-            if (beta != 0.0f) { const float4 old = *dst; o.x += beta * old.x; o.y += beta * old.y; o.z += beta * old.z; o.w += beta * old.w; }
-            *dst = o;
+        for (int k = 0; k < splits; ++k) {
+            const float4 v = __ldcg(src + (int64_t)k * total4);
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
-        return;
-    }
-    for (int64_t i = tid; i < total; i += nthreads) {
-        const int64_t m = i / N, n = i - m * N;
-        float s = 0.0f;
-        for (int k = 0; k < splits; ++k) s += partial[(int64_t)k * total + i];
-        float o = alpha * s;
-        if (bias) o += bias[n];
-        if (beta != 0.0f) o += beta * C[m * ldc + n];
-        C[m * ldc + n] = o;
+        float o[4] = {alpha * s.x, alpha * s.y, alpha * s.z, alpha * s.w};
+        float* dst = C + m * ldc + n;
+        if (vec) {
+            if (bias) { o[0] += bias[n]; o[1] += bias[n + 1]; o[2] += bias[n + 2]; o[3] += bias[n + 3]; }
+            if (beta != 0.0f) { const float4 old = ld4(dst); o[0] += beta * old.x; o[1] += beta * old.y; o[2] += beta * old.z; o[3] += beta * old.w; }
+            st4(dst, make_float4(o[0], o[1], o[2], o[3]));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (n + e >= N) break;
+                if (bias) o[e] += bias[n + e];
+                if (beta != 0.0f) o[e] += beta * dst[e];
+                dst[e] = o[e];
+            }
+        }
     }
 }
 
@@ -1284,7 +1301,7 @@ static bool encode_output(EncodeTiledFn enc, CUtensorMap* map, const float* ptr,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool gemm_tc_eligible(bool ta, bool tb, const GemmArgs& g) {
+bool gemm_tc_eligible(const GemmArgs& g) {
     auto ok4 = [](int64_t v) { return v % 4 == 0; };
     if (g.K < 1 || g.M < 1 || g.N < 1) return false;
     if (!aligned16(g.A) || !aligned16(g.B)) return false;
@@ -1294,9 +1311,7 @@ bool gemm_tc_eligible(bool ta, bool tb, const GemmArgs& g) {
     if (g.M > (int64_t(1) << 30) || g.N > (int64_t(1) << 30) || g.K > (int64_t(1) << 30)) return false;
     if (g.batch_outer * g.batch_inner > 65535) return false;
     // tiny problems are launch-bound either way; the FMA engine avoids the descriptor set-up
-    if (g.M * g.N * g.K < (int64_t)64 * 64 * 64) return false;
-    (void)ta; (void)tb;
-    return true;
+    return g.M * g.N * g.K >= (int64_t)64 * 64 * 64;
 }
 
 template <int BN, bool A_TM>
@@ -1415,11 +1430,12 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     p.splits = splits = (p.k_blocks_total + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
     Scratch sc(ctx);
     p.partial = nullptr;
+    p.partial_ld = (g.N + 3) / 4 * 4;
     if (splits > 1) {
-        int rc = sc.get(sizeof(float) * ((size_t)splits * g.M * g.N + (g.colsum ? (size_t)splits * g.N : 0)));
+        int rc = sc.get(sizeof(float) * ((size_t)splits * g.M * p.partial_ld + (g.colsum ? (size_t)splits * g.N : 0)));
         if (rc) return rc;
         p.partial = sc.as<float>();
-        if (g.colsum) p.colsum_partial = p.partial + (size_t)splits * g.M * g.N;
+        if (g.colsum) p.colsum_partial = p.partial + (size_t)splits * g.M * p.partial_ld;
     }
     p.batches = (int)batches;
     p.causal = g.causal;
@@ -1476,9 +1492,8 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     rc = after_launch(ctx, family);
     if (rc) return rc;
     if (splits > 1) {
-        const int64_t total = g.M * g.N;
-        const int vec = (g.N % 4 == 0 && g.ldc % 4 == 0 && aligned16(g.C) && aligned16(p.partial)) ? 1 : 0;
-        const int64_t units = vec ? total / 4 : total;
+        const int vec = (g.N % 4 == 0 && g.ldc % 4 == 0 && aligned16(g.C)) ? 1 : 0;
+        const int64_t units = g.M * p.partial_ld / 4;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)std::min<int64_t>((units + 255) / 256, (int64_t)kSMs * 8), 1, 1);
         cfg.blockDim = dim3(256, 1, 1);
@@ -1488,7 +1503,7 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        GCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, splitk_reduce_kernel, g.C, (const float*)p.partial, g.bias, g.M, g.N, g.ldc, splits, g.alpha, g.beta, g.colsum, (const float*)p.colsum_partial,
+        GCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, splitk_reduce_kernel, g.C, (const float*)p.partial, p.partial_ld, g.bias, g.M, g.N, g.ldc, splits, g.alpha, g.beta, g.colsum, (const float*)p.colsum_partial,
                                           g.colsum_accumulate, vec));
         rc = after_launch(ctx, "splitk_reduce");
         if (rc) return rc;

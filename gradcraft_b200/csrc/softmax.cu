@@ -17,13 +17,13 @@ int launch_sum_partials(gcb_ctx* ctx, float* out, const float* partial, int coun
 constexpr int kSmWarps = 8;
 
 template <int NCHUNK>
-__global__ void __launch_bounds__(kSmWarps * 32) causal_softmax_fwd_warp(float* __restrict__ probs, const float* __restrict__ scores, float scale, int64_t rows, int T, int band) {
+__global__ void __launch_bounds__(kSmWarps * 32) causal_softmax_fwd_warp(float* __restrict__ probs, const float* __restrict__ scores, float scale, int64_t rows, int T, int64_t ld, int band) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * kSmWarps + (threadIdx.x >> 5);
     const int64_t nwarps = (int64_t)gridDim.x * kSmWarps;
     for (int64_t r = warp; r < rows; r += nwarps) {
         const int i = (int)(r % T);
-        const float* sr = scores + r * T;
+        const float* sr = scores + r * ld;
         float4 v[NCHUNK];
         float m = -INFINITY;
 #pragma unroll
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kSmWarps * 32) causal_softmax_fwd_warp(float* 
         }
         sum = warp_sum(sum);
         const float inv = 1.0f / sum;
-        float* pr = probs + r * T;
+        float* pr = probs + r * ld;
         const int limit = band ? min(T, (i / band + 1) * band) : T;  // zeros are written up to the end of the diagonal block only
 #pragma unroll
         for (int k = 0; k < NCHUNK; ++k) {
@@ -107,11 +107,11 @@ __global__ void __launch_bounds__(kSmWarps * 32, (NCHUNK == 8 ? 3 : 4)) causal_s
 }
 
 // generic sequence lengths: CTA per row, scalar accesses
-__global__ void __launch_bounds__(256) causal_softmax_fwd_block(float* __restrict__ probs, const float* __restrict__ scores, float scale, int64_t rows, int64_t T) {
+__global__ void __launch_bounds__(256) causal_softmax_fwd_block(float* __restrict__ probs, const float* __restrict__ scores, float scale, int64_t rows, int64_t T, int64_t ld) {
     __shared__ float red[33];
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const int64_t i = r % T;
-        const float* sr = scores + r * T;
+        const float* sr = scores + r * ld;
         float m = -INFINITY;
         for (int64_t j = threadIdx.x; j <= i; j += blockDim.x) m = fmaxf(m, sr[j] * scale);
         m = block_reduce<true>(m, red);
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) causal_softmax_fwd_block(float* __restric
         for (int64_t j = threadIdx.x; j <= i; j += blockDim.x) s += __expf(sr[j] * scale - m);
         s = block_reduce<false>(s, red);
         const float inv = 1.0f / s;
-        for (int64_t j = threadIdx.x; j < T; j += blockDim.x) probs[r * T + j] = (j <= i) ? __expf(sr[j] * scale - m) * inv : 0.0f;
+        for (int64_t j = threadIdx.x; j < T; j += blockDim.x) probs[r * ld + j] = (j <= i) ? __expf(sr[j] * scale - m) * inv : 0.0f;
     }
 }
 __global__ void __launch_bounds__(256) causal_softmax_bwd_block(float* __restrict__ ds, const float* __restrict__ dp, const float* __restrict__ probs, float scale, int64_t rows, int64_t T, int accumulate) {
@@ -275,27 +275,32 @@ int softmax_bwd_apply_launch(gcb_ctx* ctx, const GemmArgs& g) {
 
 extern "C" {
 
-static int csm_fwd(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t T, int band) {
+static int csm_fwd(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t T, int64_t ld, int band) {
     GCB_REQUIRE(ctx && rows >= 0 && T >= 0 && (rows * T == 0 || (probs && scores)), "gcb_causal_softmax_fwd_f32: bad arguments");
     GCB_REQUIRE(T == 0 || rows % T == 0, "gcb_causal_softmax_fwd_f32: rows (%lld) must be a multiple of seq_len (%lld)", (long long)rows, (long long)T);
+    GCB_REQUIRE(ld >= T, "gcb_causal_softmax_fwd_f32: rows (%lld apart) overlap", (long long)ld);
     if (rows * T == 0) return GCB_OK;
     cudaSetDevice(ctx->device);
-    if (T % 4 == 0 && T <= 1024 && aligned16(probs) && aligned16(scores)) {
+    if (ld % 4 == 0 && T <= 1024 && aligned16(probs) && aligned16(scores)) {  // the last chunk of a row may reach into the padding between T and ld, never beyond
         int64_t blocks = std::min<int64_t>((rows + kSmWarps - 1) / kSmWarps, (int64_t)kSMs * 8);
         const int n = chunks_for(T);
-#define GCB_L(N) causal_softmax_fwd_warp<N><<<(unsigned)blocks, kSmWarps * 32, 0, ctx->stream>>>(probs, scores, scale, rows, (int)T, band)
+#define GCB_L(N) causal_softmax_fwd_warp<N><<<(unsigned)blocks, kSmWarps * 32, 0, ctx->stream>>>(probs, scores, scale, rows, (int)T, ld, band)
         if (n == 1) GCB_L(1); else if (n == 2) GCB_L(2); else if (n == 4) GCB_L(4); else GCB_L(8);
 #undef GCB_L
     } else {
-        causal_softmax_fwd_block<<<(unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 8), 256, 0, ctx->stream>>>(probs, scores, scale, rows, T);
+        causal_softmax_fwd_block<<<(unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 8), 256, 0, ctx->stream>>>(probs, scores, scale, rows, T, ld);
     }
     return after_launch(ctx, "causal_softmax_fwd");
 }
 
-int gcb_causal_softmax_fwd_f32(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t T) { return csm_fwd(ctx, probs, scores, scale, rows, T, 0); }
+int gcb_causal_softmax_fwd_f32(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t T) { return csm_fwd(ctx, probs, scores, scale, rows, T, T, 0); }
 int gcb_causal_softmax_fwd_band_f32(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t T, int band) {
     GCB_REQUIRE(band >= 0 && band % 4 == 0, "gcb_causal_softmax_fwd_band_f32: band must be a non-negative multiple of 4");
-    return csm_fwd(ctx, probs, scores, scale, rows, T, band);
+    return csm_fwd(ctx, probs, scores, scale, rows, T, T, band);
+}
+int gcb_causal_softmax_fwd_band_ld_f32(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t T, int64_t ld, int band) {
+    GCB_REQUIRE(band >= 0 && band % 4 == 0, "gcb_causal_softmax_fwd_band_ld_f32: band must be a non-negative multiple of 4");
+    return csm_fwd(ctx, probs, scores, scale, rows, T, ld, band);
 }
 
 static int csm_bwd(gcb_ctx* ctx, float* ds, const float* dp, const float* probs, float scale, int64_t rows, int64_t T, int accumulate, int band) {

@@ -668,7 +668,8 @@ class SDPANode : public Node<float> {
     Tensor<float> m_q, m_k, m_v;
     float m_scale;
     int64_t m_B, m_H, m_T, m_D;
-    Tensor<float> m_probs;  // kept for backward
+    Tensor<float> m_probs;  // kept for backward; (B * H, T, m_ld)
+    int64_t m_ld;           // rows of the T x T matrices lie a multiple of four floats apart, so that TMA can address them for every T
     std::shared_ptr<Storage<float>> m_out_storage;  // O, for the row term dO . O of the softmax backward: the storage object of the tensor this node creates (realize() hands it the data)
 
     static void strides4(const Tensor<float>& t, int64_t& so, int64_t& si, int64_t& ld) { so = t.strides()[0]; si = t.strides()[1]; ld = t.strides()[2]; }
@@ -676,19 +677,20 @@ class SDPANode : public Node<float> {
 public:
     SDPANode(Tensor<float> q, Tensor<float> k, Tensor<float> v, float scale) : m_q(std::move(q)), m_k(std::move(k)), m_v(std::move(v)), m_scale(scale) {
         m_B = m_q.shape()[0]; m_H = m_q.shape()[1]; m_T = m_q.shape()[2]; m_D = m_q.shape()[3];
+        m_ld = (m_T + 3) / 4 * 4;
     }
     static std::vector<int64_t> out_strides(int64_t H, int64_t T, int64_t D) { return {T * H * D, D, H * D, 1}; }
     Tensor<float> realize() override {
         m_q.realize(); m_k.realize(); m_v.realize();
         gcb_ctx* c = ctx_of(m_q);
         const int64_t B = m_B, H = m_H, T = m_T, D = m_D;
-        m_probs = Tensor<float>({B * H, T, T}, m_q.device(), uninitialized);
+        m_probs = Tensor<float>({B * H, T, m_ld}, m_q.device(), uninitialized);
         int64_t qo, qi, ql, ko, ki, kl, vo, vi, vl;
         strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl); strides4(m_v, vo, vi, vl);
-        gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_T, T, T, D, 1.0f, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, 0.0f, m_probs.data_ptr(), T, H * T * T, T * T, B, H, 1), "attention scores");
-        gcb_check(gcb_causal_softmax_fwd_band_f32(c, m_probs.data_ptr(), m_probs.data_ptr(), m_scale, B * H * T, T, kCausalBand), "causal softmax");
+        gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_T, T, T, D, 1.0f, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, 0.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, B, H, 1), "attention scores");
+        gcb_check(gcb_causal_softmax_fwd_band_ld_f32(c, m_probs.data_ptr(), m_probs.data_ptr(), m_scale, B * H * T, T, m_ld, kCausalBand), "causal softmax");
         Tensor<float> mem({B, T, H, D}, m_q.device(), uninitialized);
-        gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_N, T, D, T, 1.0f, m_probs.data_ptr(), T, H * T * T, T * T, m_v.data_ptr(), vl, vo, vi, 0.0f, mem.data_ptr(), H * D, T * H * D, D, B, H, 2), "attention output");
+        gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_N, T, D, T, 1.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, m_v.data_ptr(), vl, vo, vi, 0.0f, mem.data_ptr(), H * D, T * H * D, D, B, H, 2), "attention output");
         return Tensor<float>({B, H, T, D}, out_strides(H, T, D), 0, mem._get_storage(), false);
     }
     void backward(const Tensor<float>& g_in, bool retain_graph) override {
@@ -704,24 +706,24 @@ public:
         };
         if (m_v.requires_grad()) {  // dV = P^T . dO
             Tensor<float> dv = fresh();
-            gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_T, GCB_OP_N, T, D, T, 1.0f, m_probs.data_ptr(), T, H * T * T, T * T, g.data_ptr(), gl, go, gi, 0.0f, dv.data_ptr(), H * D, T * H * D, D, B, H, 3), "attention dV");
+            gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_T, GCB_OP_N, T, D, T, 1.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, g.data_ptr(), gl, go, gi, 0.0f, dv.data_ptr(), H * D, T * H * D, D, B, H, 3), "attention dV");
             push_grad(m_v, dv);
         }
         if (m_q.requires_grad() || m_k.requires_grad()) {
             // dS = scale * P * (dO . V^T - rowdot), rowdot = sum_j dP_ij P_ij = dO_i . O_i: the softmax backward runs in the epilogue of the dP GEMM
-            Tensor<float> ds({B * H, T, T}, g.device(), uninitialized);
+            Tensor<float> ds({B * H, T, m_ld}, g.device(), uninitialized);
             Tensor<float> rowdot({B * H * T}, g.device(), uninitialized);
             gcb_check(gcb_rowdot_batched_f32(c, rowdot.data_ptr(), g.data_ptr(), gl, go, gi, m_out_storage->data(), H * D, T * H * D, D, T, D, B, H), "attention dO . O");
-            gcb_check(gcb_gemm_batched_softmax_bwd_f32(c, GCB_OP_N, GCB_OP_T, T, D, 1.0f, g.data_ptr(), gl, go, gi, m_v.data_ptr(), vl, vo, vi, ds.data_ptr(), T, H * T * T, T * T, B, H, m_probs.data_ptr(),
+            gcb_check(gcb_gemm_batched_softmax_bwd_f32(c, GCB_OP_N, GCB_OP_T, T, D, 1.0f, g.data_ptr(), gl, go, gi, m_v.data_ptr(), vl, vo, vi, ds.data_ptr(), m_ld, H * T * m_ld, T * m_ld, B, H, m_probs.data_ptr(),
                                                        rowdot.data_ptr(), m_scale), "attention dS");
             if (m_q.requires_grad()) {  // dQ = dS . K
                 Tensor<float> dq = fresh();
-                gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_N, T, D, T, 1.0f, ds.data_ptr(), T, H * T * T, T * T, m_k.data_ptr(), kl, ko, ki, 0.0f, dq.data_ptr(), H * D, T * H * D, D, B, H, 2), "attention dQ");
+                gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_N, T, D, T, 1.0f, ds.data_ptr(), m_ld, H * T * m_ld, T * m_ld, m_k.data_ptr(), kl, ko, ki, 0.0f, dq.data_ptr(), H * D, T * H * D, D, B, H, 2), "attention dQ");
                 push_grad(m_q, dq);
             }
             if (m_k.requires_grad()) {  // dK = dS^T . Q
                 Tensor<float> dk = fresh();
-                gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_T, GCB_OP_N, T, D, T, 1.0f, ds.data_ptr(), T, H * T * T, T * T, m_q.data_ptr(), ql, qo, qi, 0.0f, dk.data_ptr(), H * D, T * H * D, D, B, H, 3), "attention dK");
+                gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_T, GCB_OP_N, T, D, T, 1.0f, ds.data_ptr(), m_ld, H * T * m_ld, T * m_ld, m_q.data_ptr(), ql, qo, qi, 0.0f, dk.data_ptr(), H * D, T * H * D, D, B, H, 3), "attention dK");
                 push_grad(m_k, dk);
             }
         }

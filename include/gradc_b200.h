@@ -283,6 +283,10 @@ GCB_API int gcb_causal_softmax_bwd_f32(gcb_ctx* ctx, float* dscores, const float
  * band > 0 a row is written only up to the end of its band-wide diagonal block (columns < (i / band + 1) * band); what lies
  * beyond is never read by such a consumer and is left untouched.  band = 0 is the full-row form above. */
 GCB_API int gcb_causal_softmax_fwd_band_f32(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t seq_len, int band);
+/* The forward on rows that lie ld >= seq_len floats apart: with ld a multiple of four every row starts on a 16-byte boundary
+ * and the tensor-core GEMMs can address the matrix, whatever the sequence length is.  Columns between seq_len and the next
+ * multiple of four may be overwritten. */
+GCB_API int gcb_causal_softmax_fwd_band_ld_f32(gcb_ctx* ctx, float* probs, const float* scores, float scale, int64_t rows, int64_t seq_len, int64_t ld, int band);
 GCB_API int gcb_causal_softmax_bwd_band_f32(gcb_ctx* ctx, float* dscores, const float* dprobs, const float* probs, float scale, int64_t rows, int64_t seq_len, int accumulate, int band);
 
 /* ---- loss: apply_sparse_softmax_crossentropy_{forward,backward}, cuda_math.hpp:45-50 ------------ */

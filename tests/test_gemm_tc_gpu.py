@@ -552,3 +552,30 @@ def test_registered_weights_use_presplit_companions_with_identical_results(env, 
     finally:
         ctx.weight_twins_drop(W_reg, w.nbytes)
     assert ctx.weight_twins_count() == n0
+
+
+@pytest.mark.parametrize("opa,opb,M,N,K", [(0, 0, 301, 259, 517), (0, 1, 256, 131, 1031), (1, 0, 517, 301, 2051), (1, 1, 130, 515, 263), (0, 0, 300, 259, 512)])
+def test_unaligned_operands_are_packed_for_the_tensor_cores(env, opa, opb, M, N, K):
+    """Row lengths that are no multiple of four floats, and bases off a 16-byte boundary: operands are copied into rows TMA can
+    address (only those that need it), ragged results are stored row by row, with and without K slices, beta and bias."""
+    ctx, torch, capi = env
+    A, B = rnd(130, *((K, M) if opa else (M, K))), rnd(131, *((N, K) if opb else (K, N)))
+    C0, bias = rnd(132, M, N), rnd(133, N)
+    dA, dB = torch.from_numpy(A).cuda(), torch.empty(B.size + 1, device="cuda")[1:]
+    dB.copy_(torch.from_numpy(B.reshape(-1)))
+    ref = (A.T if opa else A).astype(np.float64) @ (B.T if opb else B).astype(np.float64)
+    ctx.ctx_set_gemm_engine(0)
+    try:
+        before = ctx.ctx_launch_count_named(b"gemm_pack")
+        C = torch.full((M, N), float("nan"), device="cuda")
+        ctx.gemm_f32(opa, opb, M, N, K, 1.0, dA, A.shape[1], dB, B.shape[1], 0.0, C, N, None)
+        ctx.sync()
+        assert ctx.ctx_last_gemm_engine() == 2
+        assert ctx.ctx_launch_count_named(b"gemm_pack") == before + (1 if A.shape[1] % 4 == 0 else 2)
+        assert max_abs_rel(C.cpu().numpy(), ref) < TOL
+        C = torch.from_numpy(C0).cuda()
+        ctx.gemm_f32(opa, opb, M, N, K, 0.5, dA, A.shape[1], dB, B.shape[1], 1.0, C, N, torch.from_numpy(bias).cuda())
+        ctx.sync()
+        assert max_abs_rel(C.cpu().numpy(), 0.5 * ref + C0 + bias) < TOL
+    finally:
+        ctx.ctx_set_gemm_engine(2)

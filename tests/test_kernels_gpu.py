@@ -564,3 +564,21 @@ def test_bounded_wait_that_runs_out_is_reported_and_the_context_survives(env):
     ctx.fill_f32(x, 2.5, 1000)
     ctx.sync()  # the status word was cleared
     assert float(x.sum()) == 2500.0
+
+
+@pytest.mark.parametrize("T,band", [(5, 0), (127, 128), (129, 128), (1023, 128), (1030, 0)])
+def test_causal_softmax_on_padded_rows(env, T, band):
+    """Rows that lie a multiple of four floats apart, for sequence lengths that are no such multiple, against the dense form."""
+    ctx, torch, capi = env
+    BH, ld = 3, (T + 3) // 4 * 4
+    z = dev(torch, rnd(90, BH * T, T))
+    dense = torch.empty_like(z)
+    ctx.causal_softmax_fwd_f32(dense, z, 0.25, BH * T, T)
+    padded = torch.full((BH * T, ld), float("nan"), device="cuda")
+    padded[:, :T] = z
+    ctx.causal_softmax_fwd_band_ld_f32(padded, padded, 0.25, BH * T, T, ld, band)
+    i = torch.arange(T, device="cuda").repeat(BH)[:, None]
+    j = torch.arange(T, device="cuda")[None, :]
+    seen = torch.ones_like(j < 0).expand(BH * T, T) if band == 0 else j < (i // band + 1) * band
+    ctx.sync()
+    assert max_abs_rel(torch.where(seen, padded[:, :T], dense).cpu().numpy(), dense.cpu().numpy()) < 1e-6
