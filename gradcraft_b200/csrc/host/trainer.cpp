@@ -16,6 +16,7 @@ struct gct_trainer {
     Device gpu{DeviceType::CUDA, 0};
     std::unique_ptr<Module<float>> model;
     std::function<Tensor<float>(Tensor<int64_t>)> forward;
+    std::function<std::vector<int64_t>(const std::vector<int64_t>&, int64_t, int64_t, int64_t, std::optional<float>, int64_t)> generate;
     std::unique_ptr<AdamW<float>> opt;
     std::unique_ptr<GlobalNormClipper<float>> clipper;
     std::vector<std::pair<std::string, Parameter<float>*>> ordered;  // arena order
@@ -43,6 +44,14 @@ static Tensor<int64_t> wrap_i64(const int64_t* p, int64_t B, int64_t T, Device d
     return t;
 }
 
+template <class Model>
+static void use_model(gct_trainer& tr, Model* model) {
+    tr.forward = [model](Tensor<int64_t> x) { return model->forward(std::move(x)); };
+    tr.generate = [model, gpu = tr.gpu](const std::vector<int64_t>& start, int64_t context_length, int64_t max_tokens, int64_t num_sequences, std::optional<float> temperature, int64_t top_k) {
+        return generate_tokens_incremental(*model, start, context_length, max_tokens, num_sequences, gpu, temperature, top_k);
+    };
+}
+
 extern "C" {
 
 const char* gct_last_error(void) { return g_err.c_str(); }
@@ -60,12 +69,12 @@ int gct_create(const char* arch, int64_t V, int64_t T, int64_t C, int64_t H, int
         if (a == "lngelu") {
             auto m = std::make_unique<LayerNormGPT<float>>(V, T, C, H, L, F, z, z, norm_eps);
             auto* raw = m.get();
-            tr->forward = [raw](Tensor<int64_t> x) { return raw->forward(std::move(x)); };
+            use_model(*tr, raw);
             tr->model = std::move(m);
         } else if (a == "rmsswiglu") {
             auto m = std::make_unique<GPT<float>>(V, T, C, H, L, z, z, norm_eps);
             auto* raw = m.get();
-            tr->forward = [raw](Tensor<int64_t> x) { return raw->forward(std::move(x)); };
+            use_model(*tr, raw);
             tr->model = std::move(m);
         } else {
             throw std::runtime_error("gct_create: arch must be 'lngelu' or 'rmsswiglu'");
@@ -196,7 +205,7 @@ int gct_generate(gct_trainer* tr, const int64_t* start_tokens, int64_t n_start, 
         if (!tr || !start_tokens || !out_tokens || n_start < 1) throw std::runtime_error("gct_generate: bad arguments");
         std::vector<int64_t> start(start_tokens, start_tokens + n_start);
         std::optional<float> temp = temperature > 0.0f ? std::optional<float>(temperature) : std::nullopt;
-        std::vector<int64_t> toks = generate_tokens(tr->forward, start, context_length, max_tokens, num_sequences, tr->gpu, temp, top_k);
+        std::vector<int64_t> toks = tr->generate(start, context_length, max_tokens, num_sequences, temp, top_k);
         std::copy(toks.begin(), toks.end(), out_tokens);
     });
 }

@@ -307,6 +307,8 @@ public:
         this->register_parameter("W", &m_weight);
         this->register_parameter("b", &m_bias);
     }
+    const Tensor<T>& weight() const { return m_weight.tensor(); }
+    const Tensor<T>& bias() const { return m_bias.tensor(); }
     // matmul + bias in one GEMM whose epilogue adds the bias row
     Tensor<T> forward(Tensor<T> x) { return linear(std::move(x), m_weight.tensor(), m_bias.tensor()); }
 };
@@ -329,6 +331,14 @@ public:
         this->register_module("k_proj", &m_k_proj);
         this->register_module("v_proj", &m_v_proj);
         this->register_module("out_proj", &m_out_proj);
+    }
+    int64_t num_heads() const { return m_num_heads; }
+    bool is_causal() const { return m_is_causal; }
+    void describe(gcb_gpt_layer& d) const {
+        d.wq = m_q_proj.weight().data_ptr(); d.bq = m_q_proj.bias().data_ptr();
+        d.wk = m_k_proj.weight().data_ptr(); d.bk = m_k_proj.bias().data_ptr();
+        d.wv = m_v_proj.weight().data_ptr(); d.bv = m_v_proj.bias().data_ptr();
+        d.wo = m_out_proj.weight().data_ptr(); d.bo = m_out_proj.bias().data_ptr();
     }
     Tensor<T> forward(Tensor<T> x) {  // (B, T, C)
         const int64_t B = x.shape()[0], S = x.shape()[1];
@@ -357,6 +367,9 @@ public:
         this->register_parameter("gamma", &m_gamma);
         this->register_parameter("beta", &m_beta);
     }
+    const T* gamma() const { return m_gamma.tensor().data_ptr(); }
+    const T* beta() const { return m_beta.tensor().data_ptr(); }
+    T eps() const { return m_eps; }
     Tensor<T> forward(Tensor<T> x) { return layernorm(std::move(x), m_gamma.tensor(), m_beta.tensor(), m_axes, m_eps); }
 };
 
@@ -373,6 +386,9 @@ public:
         m_gamma.set_no_decay(true);
         this->register_parameter("gamma", &m_gamma);
     }
+    const T* gamma() const { return m_gamma.tensor().data_ptr(); }
+    const T* beta() const { return nullptr; }
+    T eps() const { return m_eps; }
     Tensor<T> forward(Tensor<T> x) { return rmsnorm(std::move(x), m_gamma.tensor(), m_axes, m_eps, true); }
 };
 
@@ -406,6 +422,7 @@ public:
         m_token_range = Tensor<int64_t>::arange(0, max_seq_len, 1);
         this->register_parameter("pos_embeds", &m_pos_embeds);
     }
+    const Tensor<T>& weight() const { return m_pos_embeds.tensor(); }
     Tensor<T> forward(int64_t seq_len) {
         if (m_token_range.device() != m_pos_embeds.device()) m_token_range = Tensor<int64_t>::arange(0, m_token_range.volume(), 1, m_pos_embeds.device());
         return embed(m_token_range[Slice(0, seq_len)], m_pos_embeds.tensor());
@@ -424,6 +441,12 @@ public:
         this->register_module("w2", &m_w2);
         this->register_module("w3", &m_w3);
     }
+    int64_t hidden() const { return m_w1.weight().shape()[1]; }
+    void describe(gcb_gpt_layer& d) const {
+        d.w1 = m_w1.weight().data_ptr(); d.b1 = m_w1.bias().data_ptr();
+        d.w2 = m_w2.weight().data_ptr(); d.b2 = m_w2.bias().data_ptr();
+        d.w3 = m_w3.weight().data_ptr(); d.b3 = m_w3.bias().data_ptr();
+    }
     Tensor<T> forward(Tensor<T> x) { return m_w3.forward(swiglu_fast(m_w1.forward(x), m_w2.forward(x))); }
 };
 
@@ -437,6 +460,12 @@ public:
         : m_fc1(embed_dim, hidden_dim, base_init, ZerosInit<T>()), m_fc2(hidden_dim, embed_dim, residual_init, ZerosInit<T>()) {
         this->register_module("fc1", &m_fc1);
         this->register_module("fc2", &m_fc2);
+    }
+    int64_t hidden() const { return m_fc1.weight().shape()[1]; }
+    void describe(gcb_gpt_layer& d) const {
+        d.w1 = m_fc1.weight().data_ptr(); d.b1 = m_fc1.bias().data_ptr();
+        d.w2 = m_fc2.weight().data_ptr(); d.b2 = m_fc2.bias().data_ptr();
+        d.w3 = nullptr; d.b3 = nullptr;
     }
     Tensor<T> forward(Tensor<T> x) { return m_fc2.forward(m_fc1.forward(x).gelu()); }
 };
@@ -457,6 +486,14 @@ public:
         this->register_module("attn", &m_attn);
         this->register_module("norm2", &m_norm2);
         this->register_module("mlp", &m_mlp);
+    }
+    const MultiHeadAttention<T>& attn() const { return m_attn; }
+    const MLP& mlp() const { return m_mlp; }
+    void describe(gcb_gpt_layer& d) const {
+        d.norm1_gamma = m_norm1.gamma(); d.norm1_beta = m_norm1.beta();
+        d.norm2_gamma = m_norm2.gamma(); d.norm2_beta = m_norm2.beta();
+        m_attn.describe(d);
+        m_mlp.describe(d);
     }
     Tensor<T> forward(Tensor<T> x) {
         x = x + m_attn.forward(m_norm1.forward(x));
@@ -490,6 +527,21 @@ protected:
     void finish_registration() { this->register_module("final_norm", &m_final_norm); }
 
 public:
+    // The weights as the decoding kernel takes them; valid while the parameters stay where they are.
+    gcb_gpt_model describe(std::vector<gcb_gpt_layer>& layers) const {
+        layers.assign(m_blocks.size(), gcb_gpt_layer{});
+        for (size_t i = 0; i < m_blocks.size(); ++i) m_blocks[i]->describe(layers[i]);
+        const auto& e = m_token_embed.weight();
+        gcb_gpt_model m{};
+        m.V = e.shape()[0]; m.C = e.shape()[1]; m.T = m_pos_embed.weight().shape()[0]; m.L = (int64_t)layers.size();
+        m.H = m_blocks.empty() ? 0 : m_blocks[0]->attn().num_heads();
+        m.F = m_blocks.empty() ? 0 : m_blocks[0]->mlp().hidden();
+        m.eps = m_final_norm.eps();
+        m.token_embed = e.data_ptr(); m.pos_embed = m_pos_embed.weight().data_ptr();
+        m.final_gamma = m_final_norm.gamma(); m.final_beta = m_final_norm.beta();
+        m.layers = layers.data();
+        return m;
+    }
     Tensor<T> forward(Tensor<int64_t> indices) {  // (B, T) -> logits (B, T, V)
         const int64_t S = indices.shape()[1];
         Tensor<T> x = m_token_embed.forward(indices) + m_pos_embed.forward(S);
@@ -802,15 +854,43 @@ public:
 // (std::mt19937(67), std::nth_element, std::discrete_distribution; gpt_generator.hpp:23-25, 71-95).
 // `forward` maps (B, L) int64 tokens on the device to (B, L, V) logits: any of the GPT modules of this file.
 // Returns num_sequences x max_tokens token ids, every sequence starting with start_tokens.
+class TokenPicker {
+    std::optional<float> m_temperature;
+    int64_t m_top_k;
+    std::mt19937 m_rng;
+    std::vector<std::pair<float, int64_t>> m_cand;
+    std::vector<float> m_weights;
+
+public:
+    TokenPicker(std::optional<float> temperature, int64_t top_k) : m_temperature(temperature), m_top_k(top_k) {
+        if (temperature.has_value()) m_rng = std::mt19937(67);
+    }
+    int64_t pick(float* row, int64_t V) {  // overwrites the logits
+        if (!m_temperature.has_value()) return (int64_t)(std::max_element(row, row + V) - row);  // first maximum, as argmax does
+        const float mx = *std::max_element(row, row + V);
+        double sum = 0.0;
+        for (int64_t i = 0; i < V; ++i) { row[i] = std::exp((row[i] - mx) / m_temperature.value()); sum += row[i]; }
+        m_cand.resize((size_t)V);
+        for (int64_t i = 0; i < V; ++i) m_cand[(size_t)i] = {(float)(row[i] / sum), i};
+        const int64_t k = std::min(m_top_k, V);
+        std::nth_element(m_cand.begin(), m_cand.begin() + k - 1, m_cand.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+        m_weights.resize((size_t)k);
+        for (int64_t i = 0; i < k; ++i) m_weights[(size_t)i] = m_cand[(size_t)i].first;
+        std::discrete_distribution<int64_t> dist(m_weights.begin(), m_weights.end());
+        return m_cand[(size_t)dist(m_rng)].second;
+    }
+};
+inline void check_generation(int64_t start, int64_t max_tokens, Device device) {
+    if (start < 1) throw std::runtime_error("generate_tokens: at least one start token is needed.");
+    if (start >= max_tokens) throw std::runtime_error("Tokenized start_text is >= max_tokens in GPT inference.");
+    if (!device.is_cuda()) throw std::runtime_error("generate_tokens: the inference device must be a CUDA device.");
+}
 template <class Forward>
 std::vector<int64_t> generate_tokens(Forward&& forward, const std::vector<int64_t>& start_tokens, int64_t context_length, int64_t max_tokens, int64_t num_sequences, Device infer_device,
                                      std::optional<float> temperature = std::nullopt, int64_t top_k = 30) {
     const int64_t start = (int64_t)start_tokens.size();
-    if (start < 1) throw std::runtime_error("generate_tokens: at least one start token is needed.");
-    if (start >= max_tokens) throw std::runtime_error("Tokenized start_text is >= max_tokens in GPT inference.");
-    if (!infer_device.is_cuda()) throw std::runtime_error("generate_tokens: the inference device must be a CUDA device.");
-    std::mt19937 rng;
-    if (temperature.has_value()) rng = std::mt19937(67);
+    check_generation(start, max_tokens, infer_device);
+    TokenPicker picker(temperature, top_k);
     std::vector<int64_t> tokens((size_t)(num_sequences * max_tokens), 0);
     for (int64_t b = 0; b < num_sequences; ++b) std::copy(start_tokens.begin(), start_tokens.end(), tokens.begin() + b * max_tokens);
     gcb_ctx* c = Backend::get().ctx(infer_device);
@@ -828,26 +908,171 @@ std::vector<int64_t> generate_tokens(Forward&& forward, const std::vector<int64_
         row.resize((size_t)V);
         for (int64_t b = 0; b < num_sequences; ++b) {
             gcb_check(gcb_copy_d2h(c, row.data(), dense.data_ptr() + (b * L + (L - 1)) * V, sizeof(float) * (size_t)V), "logits download");
-            int64_t next;
-            if (!temperature.has_value()) {
-                next = (int64_t)(std::max_element(row.begin(), row.end()) - row.begin());  // first maximum, as argmax does
-            } else {
-                float mx = *std::max_element(row.begin(), row.end());
-                double sum = 0.0;
-                for (float& z : row) { z = std::exp((z - mx) / temperature.value()); sum += z; }
-                std::vector<std::pair<float, int64_t>> cand((size_t)V);
-                for (int64_t i = 0; i < V; ++i) cand[(size_t)i] = {(float)(row[(size_t)i] / sum), i};
-                const int64_t k = std::min(top_k, V);
-                std::nth_element(cand.begin(), cand.begin() + k - 1, cand.end(), [](const auto& a, const auto& b2) { return a.first > b2.first; });
-                std::vector<float> weights((size_t)k);
-                for (int64_t i = 0; i < k; ++i) weights[(size_t)i] = cand[(size_t)i].first;
-                std::discrete_distribution<int64_t> dist(weights.begin(), weights.end());
-                next = cand[(size_t)dist(rng)].second;
-            }
-            tokens[(size_t)(b * max_tokens + step)] = next;
+            tokens[(size_t)(b * max_tokens + step)] = picker.pick(row.data(), V);
         }
     }
     return tokens;
+}
+
+// The same tokens for the GPT modules of this file without forwarding the context again for every one of them.  While the text
+// fits the context window no position ever changes its index, so the keys and values of every layer are kept and a new token
+// costs one position (gcb_gpt_decode_f32): argmax decoding runs all of them in one launch.  Once the window slides, every token
+// sits at another (learned) position and the window is forwarded again, but only as far as the next token needs it: the last
+// layer computes keys and values alone, and head and final norm see one position.
+// With argmax every sequence continues the same start tokens the same way, so one of them is computed.
+class IncrementalGPT {
+    // Up to this many given positions are stepped through by the decoding kernel instead of being forwarded as one matrix: a step
+    // takes about as long as four of a layer's eleven launches.
+    static constexpr int64_t kStepInstead = 4;
+    gcb_ctx* m_ctx;
+    Device m_device;
+    std::vector<gcb_gpt_layer> m_layers;
+    gcb_gpt_model m_model;
+    int64_t m_cap = 0, m_seqs = 0;  // positions per sequence and sequences the cache holds
+    Tensor<float> m_cache, m_x, m_a, m_q, m_o, m_scores, m_h0, m_h1;
+    Tensor<int64_t> m_ids;
+
+    float* cache(int64_t layer, int which) { return m_cache.data_ptr() + (2 * layer + which) * m_seqs * m_cap * m_model.C; }
+    static void at_least(Tensor<float>& t, int64_t n, Device d) {
+        if (t._get_state() == nullptr || t.volume() < n) t = Tensor<float>({n}, d, uninitialized);
+    }
+    void norm(float* y, const float* x, const float* gamma, const float* beta, int64_t rows) {
+        if (beta != nullptr) gcb_check(gcb_layernorm_fwd_f32(m_ctx, y, nullptr, nullptr, x, gamma, beta, rows, m_model.C, m_model.eps), "layernorm");
+        else gcb_check(gcb_rmsnorm_fwd_f32(m_ctx, y, nullptr, x, gamma, rows, m_model.C, m_model.eps), "rmsnorm");
+    }
+    void project(float* y, const float* x, const float* w, const float* b, int64_t rows, int64_t K, int64_t N) {
+        gcb_check(gcb_gemm_f32(m_ctx, GCB_OP_N, GCB_OP_N, rows, N, K, 1.0f, x, K, w, N, 0.0f, y, N, b), "projection");
+    }
+    // Keys and values of the positions 0 .. n - 1 of `seqs` sequences, token ids on the device (seqs x n, dense).
+    void forward_window(const int64_t* ids, int64_t seqs, int64_t n) {
+        const gcb_gpt_model& m = m_model;
+        const int64_t C = m.C, F = m.F, H = m.H, D = C / H, rows = seqs * n, ld = (n + 3) / 4 * 4;
+        if (seqs > 1 && n != m_cap) throw std::runtime_error("IncrementalGPT: several sequences fill the whole cache");
+        const float scale = static_cast<float>(1.0 / std::sqrt((double)D));
+        for (Tensor<float>* t : {&m_x, &m_a, &m_q, &m_o}) at_least(*t, rows * C, m_device);
+        at_least(m_scores, seqs * H * n * ld, m_device);
+        at_least(m_h0, rows * F, m_device);
+        at_least(m_h1, rows * F, m_device);
+        float *x = m_x.data_ptr(), *a = m_a.data_ptr(), *q = m_q.data_ptr(), *o = m_o.data_ptr(), *s = m_scores.data_ptr(), *h0 = m_h0.data_ptr(), *h1 = m_h1.data_ptr();
+        gcb_check(gcb_embed_f32(m_ctx, x, ids, GCB_IDX_I64, m.token_embed, rows, C, m.V), "embedding gather");
+        gcb_check(gcb_binary_rowvec_f32(m_ctx, GCB_B_ADD, x, x, m.pos_embed, seqs, n * C), "positions");
+        for (int64_t l = 0; l < m.L; ++l) {
+            const gcb_gpt_layer& w = m_layers[(size_t)l];
+            float *k = cache(l, 0), *v = cache(l, 1);
+            norm(a, x, w.norm1_gamma, w.norm1_beta, rows);
+            project(k, a, w.wk, w.bk, rows, C, C);
+            project(v, a, w.wv, w.bv, rows, C, C);
+            if (l + 1 == m.L) break;
+            project(q, a, w.wq, w.bq, rows, C, C);
+            gcb_check(gcb_gemm_batched_causal_f32(m_ctx, GCB_OP_N, GCB_OP_T, n, n, D, 1.0f, q, C, n * C, D, k, C, m_cap * C, D, 0.0f, s, ld, H * n * ld, n * ld, seqs, H, 1), "attention scores");
+            gcb_check(gcb_causal_softmax_fwd_band_ld_f32(m_ctx, s, s, scale, seqs * H * n, n, ld, 128), "causal softmax");
+            gcb_check(gcb_gemm_batched_causal_f32(m_ctx, GCB_OP_N, GCB_OP_N, n, D, n, 1.0f, s, ld, H * n * ld, n * ld, v, C, m_cap * C, D, 0.0f, o, C, n * C, D, seqs, H, 2), "attention output");
+            gcb_check(gcb_linear_residual_f32(m_ctx, GCB_OP_N, rows, C, C, o, C, w.wo, C, w.bo, x, a), "linear + residual");
+            std::swap(x, a);
+            norm(a, x, w.norm2_gamma, w.norm2_beta, rows);
+            const float *w_out, *b_out;
+            if (w.w3 != nullptr) {
+                project(h0, a, w.w1, w.b1, rows, C, F);
+                project(h1, a, w.w2, w.b2, rows, C, F);
+                gcb_check(gcb_swiglu_fwd_f32(m_ctx, h1, h0, h1, rows * F), "swiglu");
+                w_out = w.w3; b_out = w.b3;
+            } else {
+                gcb_check(gcb_linear_gelu_fwd_f32(m_ctx, GCB_OP_N, rows, F, C, a, C, w.w1, F, w.b1, h0, h1), "linear + gelu");
+                w_out = w.w2; b_out = w.b2;
+            }
+            gcb_check(gcb_linear_residual_f32(m_ctx, GCB_OP_N, rows, C, F, h1, F, w_out, C, b_out, x, a), "linear + residual");
+            std::swap(x, a);
+        }
+    }
+    void decode(int64_t* ids, int64_t ids_ld, int64_t pos0, int64_t n_pos, int64_t n_known, float* logits) {
+        gcb_check(gcb_gpt_decode_f32(m_ctx, &m_model, m_seqs, m_cache.data_ptr(), m_cap, ids, ids_ld, pos0, n_pos, n_known, logits), "decoding");
+    }
+
+public:
+    template <class Model>
+    IncrementalGPT(const Model& model, Device device) : m_ctx(Backend::get().ctx(device)), m_device(device), m_model(model.describe(m_layers)) {}
+    bool takes(int64_t positions) const { return positions <= m_model.T && gcb_gpt_decode_supported(m_ctx, &m_model) == 1; }
+
+    std::vector<int64_t> generate(const std::vector<int64_t>& start_tokens, int64_t context_length, int64_t max_tokens, int64_t num_sequences, std::optional<float> temperature, int64_t top_k) {
+        const int64_t start = (int64_t)start_tokens.size(), C = m_model.C, V = m_model.V;
+        const bool greedy = !temperature.has_value();
+        m_seqs = greedy ? 1 : num_sequences;
+        m_cap = std::min(context_length, max_tokens - 1);
+        m_cache = Tensor<float>({2 * m_model.L * m_seqs * m_cap * C}, m_device, uninitialized);
+        std::vector<int64_t> tokens((size_t)(m_seqs * max_tokens), 0);
+        for (int64_t b = 0; b < m_seqs; ++b) std::copy(start_tokens.begin(), start_tokens.end(), tokens.begin() + b * max_tokens);
+        m_ids = Tensor<int64_t>({m_seqs, max_tokens}, m_device, uninitialized);
+        int64_t* ids = m_ids.data_ptr();
+        gcb_check(gcb_copy_h2d(m_ctx, ids, tokens.data(), sizeof(int64_t) * tokens.size()), "token upload");
+        TokenPicker picker(temperature, top_k);
+        Tensor<float> logits;
+        std::vector<float> host;
+        if (!greedy) {
+            logits = Tensor<float>({m_seqs, V}, m_device, uninitialized);
+            host.resize((size_t)(m_seqs * V));
+        }
+        // picks token `step` of every sequence from the logits of the call before, and hands it to the device
+        auto choose = [&](int64_t step) {
+            gcb_check(gcb_copy_d2h(m_ctx, host.data(), logits.data_ptr(), sizeof(float) * host.size()), "logits download");
+            for (int64_t b = 0; b < m_seqs; ++b) tokens[(size_t)(b * max_tokens + step)] = picker.pick(host.data() + b * V, V);
+            gcb_check(gcb_copy_h2d(m_ctx, ids, tokens.data(), sizeof(int64_t) * tokens.size()), "token upload");
+        };
+        int64_t step = start;
+        if (step <= context_length) {  // the window still holds the whole text
+            int64_t done = 0;          // positions whose keys and values are in the cache
+            if (start - 1 > kStepInstead) {
+                done = start - 1;
+                forward_window(ids, 1, done);
+                if (m_seqs > 1) {  // every sequence has the same start
+                    const int64_t shape[3] = {2 * m_model.L, m_seqs - 1, done * C}, to[3] = {m_seqs * m_cap * C, m_cap * C, 1}, from[3] = {m_seqs * m_cap * C, 0, 1};
+                    gcb_check(gcb_copy_strided_f32(m_ctx, 3, shape, m_cache.data_ptr() + m_cap * C, to, m_cache.data_ptr(), from, 0), "cache of the start tokens");
+                }
+            }
+            const int64_t last = std::min(max_tokens - 1, context_length);  // the last token whose window does not slide
+            if (greedy) {
+                decode(ids, max_tokens, done, last - done, start, nullptr);
+                step = last + 1;
+            } else {
+                for (; step <= last; ++step) {
+                    decode(ids, max_tokens, done, step - done, step, logits.data_ptr());
+                    done = step;
+                    choose(step);
+                }
+            }
+        }
+        Tensor<int64_t> window;
+        if (step < max_tokens && m_seqs > 1) window = Tensor<int64_t>({m_seqs, m_cap}, m_device, uninitialized);
+        for (; step < max_tokens; ++step) {  // the window slides: positions 0 .. context_length - 1 anew
+            const int64_t lo = step - context_length;
+            if (m_seqs == 1) {
+                if (m_cap > 1) forward_window(ids + lo, 1, m_cap - 1);
+            } else {
+                const int64_t shape[2] = {m_seqs, m_cap};
+                std::vector<int64_t> w((size_t)(m_seqs * m_cap));
+                for (int64_t b = 0; b < shape[0]; ++b) std::copy(tokens.begin() + b * max_tokens + lo, tokens.begin() + b * max_tokens + step, w.begin() + b * m_cap);
+                gcb_check(gcb_copy_h2d(m_ctx, window.data_ptr(), w.data(), sizeof(int64_t) * w.size()), "token upload");
+                forward_window(window.data_ptr(), m_seqs, m_cap);
+            }
+            decode(ids + lo, max_tokens, m_cap - 1, 1, m_cap, greedy ? nullptr : logits.data_ptr());
+            if (!greedy) choose(step);
+        }
+        if (greedy) gcb_check(gcb_copy_d2h(m_ctx, tokens.data(), ids, sizeof(int64_t) * tokens.size()), "token download");
+        std::vector<int64_t> out((size_t)(num_sequences * max_tokens));
+        for (int64_t b = 0; b < num_sequences; ++b) std::copy_n(tokens.begin() + (greedy ? 0 : b * max_tokens), max_tokens, out.begin() + b * max_tokens);
+        return out;
+    }
+};
+
+// Generation with one of the GPT modules of this file; models beyond what the decoding kernel takes forward their context again.
+template <class Model>
+std::vector<int64_t> generate_tokens_incremental(Model& model, const std::vector<int64_t>& start_tokens, int64_t context_length, int64_t max_tokens, int64_t num_sequences, Device infer_device,
+                                                 std::optional<float> temperature = std::nullopt, int64_t top_k = 30) {
+    check_generation((int64_t)start_tokens.size(), max_tokens, infer_device);
+    if (num_sequences > 0 && context_length > 0) {
+        IncrementalGPT inc(model, infer_device);
+        if (inc.takes(std::min(context_length, max_tokens - 1))) return inc.generate(start_tokens, context_length, max_tokens, num_sequences, temperature, top_k);
+    }
+    return generate_tokens([&](Tensor<int64_t> x) { return model.forward(std::move(x)); }, start_tokens, context_length, max_tokens, num_sequences, infer_device, temperature, top_k);
 }
 
 // ---- data loader (nn/utils/data_loader.hpp:13-92) ------------------------------------------------------------------------

@@ -306,6 +306,28 @@ GCB_API int gcb_adamw_step_f32(gcb_ctx* ctx, float* w, float* m, float* v, const
 GCB_API int gcb_adamw_arena_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float* grad, const uint8_t* decay_mask, int64_t n, float lr, float beta1,
                         float beta2, float beta1_pow, float beta2_pow, float weight_decay, float eps, float grad_scale);
 
+/* ---- generation: GPTGenerator::run_inference, nn/generators/gpt_generator.hpp:12-132 -------------- */
+/* Device pointers of one pre-norm block; all matrices K x N row-major as the linear layers store them.  norm*_beta NULL:
+ * RMSNorm, otherwise LayerNorm.  w3 NULL: w2(gelu(w1 x)); otherwise w3(silu(w1 x) * (w2 x)), the same for every layer. */
+typedef struct gcb_gpt_layer {
+    const float *norm1_gamma, *norm1_beta, *wq, *bq, *wk, *bk, *wv, *bv, *wo, *bo, *norm2_gamma, *norm2_beta, *w1, *b1, *w2, *b2, *w3, *b3;
+} gcb_gpt_layer;
+typedef struct gcb_gpt_model {
+    int64_t V, T, C, H, L, F;  /* vocabulary, rows of pos_embed, width, heads, layers, hidden width */
+    float eps;                 /* of every normalisation */
+    const float *token_embed, *pos_embed, *final_gamma, *final_beta;  /* token_embed (V x C) is the head as well */
+    const gcb_gpt_layer* layers;                                      /* host array of L */
+} gcb_gpt_model;
+/* 1 when gcb_gpt_decode_f32 takes this model (layer count, head width, activations that fit into shared memory), else 0. */
+GCB_API int gcb_gpt_decode_supported(gcb_ctx* ctx, const gcb_gpt_model* model);
+/* Takes n_seq sequences through the positions pos0 .. pos0 + n_pos - 1.  cache: [L][keys, values][n_seq][cache_len][C], filled for the
+ * positions before pos0 (by earlier calls, or with the k / v projections of a full forward); this call fills in its own.
+ * tokens: device, n_seq rows of tokens_ld ids, the first n_known of each given; where position p + 1 is not, the arg-max of
+ * the logits at p (the first one, as std::max_element) is stored there and used.  logits (optional, n_seq x V): those of the last
+ * position instead; then every token of the call has to be given. */
+GCB_API int gcb_gpt_decode_f32(gcb_ctx* ctx, const gcb_gpt_model* model, int64_t n_seq, float* cache, int64_t cache_len, int64_t* tokens, int64_t tokens_ld, int64_t pos0, int64_t n_pos,
+                               int64_t n_known, float* logits);
+
 /* ---- data parallel (no counterpart in the reference, which is single-GPU) ----------------------- */
 #define GCB_DP_ID_BYTES 128
 GCB_API int gcb_dp_unique_id(uint8_t id[GCB_DP_ID_BYTES]);
