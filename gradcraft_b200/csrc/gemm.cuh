@@ -1,5 +1,7 @@
 // Shared argument block and engine entry points of the two GEMM engines.
 #pragma once
+#include <cuda.h>
+
 #include "common.cuh"
 
 namespace gcb {
@@ -39,5 +41,10 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g);
 bool gemm_tc_eligible(const GemmArgs& g);
 // C <- sm_scale * sm_probs * (C - sm_rowdot[row]) on/below the diagonal, 0 above: the softmax-backward epilogue as a pass of its own
 int softmax_bwd_apply_launch(gcb_ctx* ctx, const GemmArgs& g);
+
+// cuTensorMapEncodeTiled, looked up once per context (NULL: not there).
+typedef CUresult (*TmaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+TmaEncodeFn tma_encode(gcb_ctx* ctx);
 
 }  // namespace gcb

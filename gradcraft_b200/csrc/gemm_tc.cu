@@ -1245,11 +1245,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ 
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode(gcb_ctx* ctx) {
-    if (ctx->tma_encode) return (EncodeTiledFn)ctx->tma_encode;
+TmaEncodeFn tma_encode(gcb_ctx* ctx) {
+    if (ctx->tma_encode) return (TmaEncodeFn)ctx->tma_encode;
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult qres;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess) {
@@ -1257,13 +1254,13 @@ static EncodeTiledFn get_encode(gcb_ctx* ctx) {
         return nullptr;
     }
     ctx->tma_encode = fn;
-    return (EncodeTiledFn)fn;
+    return (TmaEncodeFn)fn;
 }
 
 // Tensor map over one GEMM operand.  K-major: (k, row, batch inner, batch outer), box 16 x tile_rows.  MN-major: when the
 // row count is a multiple of 32, a 5-D view (32 floats, k, chunk of 32, batches) whose box 32 x 16 x tile_rows/32 fills every
 // 32-float chunk of the tile with one copy (*chunked = 1); otherwise the 4-D (row, k, batches) view, one copy per chunk.
-static bool encode_operand(EncodeTiledFn enc, CUtensorMap* map, const float* ptr, bool mn_major, int64_t rows_mn, int64_t K, int64_t ld, int64_t s_in, int64_t s_out, int64_t n_in, int64_t n_out, int tile_rows,
+static bool encode_operand(TmaEncodeFn enc, CUtensorMap* map, const float* ptr, bool mn_major, int64_t rows_mn, int64_t K, int64_t ld, int64_t s_in, int64_t s_out, int64_t n_in, int64_t n_out, int tile_rows,
                            int* chunked) {
     const cuuint64_t row_bytes = (cuuint64_t)ld * 4;
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
@@ -1292,7 +1289,7 @@ static bool encode_operand(EncodeTiledFn enc, CUtensorMap* map, const float* ptr
 }
 
 // Tensor map over the output (or an array laid out like it) in 32 x 32 blocks with the 128-byte swizzle: (column, row, batch inner, batch outer).
-static bool encode_output(EncodeTiledFn enc, CUtensorMap* map, const float* ptr, int64_t M, int64_t N, int64_t ld, int64_t s_in, int64_t s_out, int64_t n_in, int64_t n_out) {
+static bool encode_output(TmaEncodeFn enc, CUtensorMap* map, const float* ptr, int64_t M, int64_t N, int64_t ld, int64_t s_in, int64_t s_out, int64_t n_in, int64_t n_out) {
     const cuuint64_t row_bytes = (cuuint64_t)ld * 4;
     cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)n_in, (cuuint64_t)n_out};
     cuuint64_t strides[3] = {row_bytes, n_in > 1 ? (cuuint64_t)s_in * 4 : row_bytes * (cuuint64_t)M, n_out > 1 ? (cuuint64_t)s_out * 4 : row_bytes * (cuuint64_t)M};
@@ -1380,7 +1377,7 @@ static int launch_pair(gcb_ctx* ctx, bool ta, bool tb, const CUtensorMap& ma, co
 }
 
 int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
-    EncodeTiledFn enc = get_encode(ctx);
+    TmaEncodeFn enc = tma_encode(ctx);
     if (!enc) return GCB_UNSUPPORTED;
     cudaSetDevice(ctx->device);
     const int64_t batches = g.batch_outer * g.batch_inner;

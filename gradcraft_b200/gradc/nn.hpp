@@ -928,6 +928,7 @@ class IncrementalGPT {
     Device m_device;
     std::vector<gcb_gpt_layer> m_layers;
     gcb_gpt_model m_model;
+    std::unique_ptr<gcb_gpt_decoder, int (*)(gcb_gpt_decoder*)> m_decoder{nullptr, gcb_gpt_decoder_destroy};
     int64_t m_cap = 0, m_seqs = 0;  // positions per sequence and sequences the cache holds
     Tensor<float> m_cache, m_x, m_a, m_q, m_o, m_scores, m_h0, m_h1;
     Tensor<int64_t> m_ids;
@@ -985,7 +986,7 @@ class IncrementalGPT {
         }
     }
     void decode(int64_t* ids, int64_t ids_ld, int64_t pos0, int64_t n_pos, int64_t n_known, float* logits) {
-        gcb_check(gcb_gpt_decode_f32(m_ctx, &m_model, m_seqs, m_cache.data_ptr(), m_cap, ids, ids_ld, pos0, n_pos, n_known, logits), "decoding");
+        gcb_check(gcb_gpt_decode_f32(m_decoder.get(), m_seqs, m_cache.data_ptr(), m_cap, ids, ids_ld, pos0, n_pos, n_known, logits), "decoding");
     }
 
 public:
@@ -996,6 +997,9 @@ public:
     std::vector<int64_t> generate(const std::vector<int64_t>& start_tokens, int64_t context_length, int64_t max_tokens, int64_t num_sequences, std::optional<float> temperature, int64_t top_k) {
         const int64_t start = (int64_t)start_tokens.size(), C = m_model.C, V = m_model.V;
         const bool greedy = !temperature.has_value();
+        gcb_gpt_decoder* decoder = nullptr;
+        gcb_check(gcb_gpt_decoder_create(m_ctx, &m_model, &decoder), "decoder");
+        m_decoder.reset(decoder);
         m_seqs = greedy ? 1 : num_sequences;
         m_cap = std::min(context_length, max_tokens - 1);
         m_cache = Tensor<float>({2 * m_model.L * m_seqs * m_cap * C}, m_device, uninitialized);

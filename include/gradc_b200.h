@@ -318,15 +318,21 @@ typedef struct gcb_gpt_model {
     const float *token_embed, *pos_embed, *final_gamma, *final_beta;  /* token_embed (V x C) is the head as well */
     const gcb_gpt_layer* layers;                                      /* host array of L */
 } gcb_gpt_model;
-/* 1 when gcb_gpt_decode_f32 takes this model (layer count, head width, activations that fit into shared memory), else 0. */
+/* 1 when a decoder takes this model (layer count, head width, widths that are multiples of four, activations that fit into shared
+ * memory), else 0. */
 GCB_API int gcb_gpt_decode_supported(gcb_ctx* ctx, const gcb_gpt_model* model);
+/* What a decoder keeps of a model: the addresses of its weights, described for TMA.  Valid while the weights stay where they
+ * are; their values may change between calls. */
+typedef struct gcb_gpt_decoder gcb_gpt_decoder;
+GCB_API int gcb_gpt_decoder_create(gcb_ctx* ctx, const gcb_gpt_model* model, gcb_gpt_decoder** out);
+GCB_API int gcb_gpt_decoder_destroy(gcb_gpt_decoder* decoder);
 /* Takes n_seq sequences through the positions pos0 .. pos0 + n_pos - 1.  cache: [L][keys, values][n_seq][cache_len][C], filled for the
  * positions before pos0 (by earlier calls, or with the k / v projections of a full forward); this call fills in its own.
  * tokens: device, n_seq rows of tokens_ld ids, the first n_known of each given; where position p + 1 is not, the arg-max of
  * the logits at p (the first one, as std::max_element) is stored there and used.  logits (optional, n_seq x V): those of the last
  * position instead; then every token of the call has to be given. */
-GCB_API int gcb_gpt_decode_f32(gcb_ctx* ctx, const gcb_gpt_model* model, int64_t n_seq, float* cache, int64_t cache_len, int64_t* tokens, int64_t tokens_ld, int64_t pos0, int64_t n_pos,
-                               int64_t n_known, float* logits);
+GCB_API int gcb_gpt_decode_f32(gcb_gpt_decoder* decoder, int64_t n_seq, float* cache, int64_t cache_len, int64_t* tokens, int64_t tokens_ld, int64_t pos0, int64_t n_pos, int64_t n_known,
+                               float* logits);
 
 /* ---- data parallel (no counterpart in the reference, which is single-GPU) ----------------------- */
 #define GCB_DP_ID_BYTES 128

@@ -215,3 +215,39 @@ def test_generation_follows_the_oracle_forward(arch):
                 assert z[row[step]] >= kth - 1e-4
     finally:
         tr.close()
+
+
+@pytest.mark.parametrize("arch,V,T,C,H,L,F,prompt,new,ctx", [
+    ("lngelu", 131, 320, 96, 4, 2, 100, 1, 300, 320),      # one given token; head width 24; a second stretch of positions per head
+    ("rmsswiglu", 97, 160, 160, 4, 1, 480, 150, 12, 155),  # a prompt that is forwarded as one matrix, a gated MLP, then a window that slides
+    ("lngelu", 1031, 24, 1044, 9, 1, 2052, 3, 16, 11),     # rows of more than one ring stage, columns beyond the last whole tile
+])
+def test_incremental_decoding_follows_the_oracle_for_any_number_of_sequences(arch, V, T, C, H, L, F, prompt, new, ctx):
+    """Greedy decoding against the oracle step by step; sampling from the single most likely token, which takes the launch for 2, 4
+    and 8 sequences (and a second one beyond) and the caller's choice of tokens, has to give the same ids in every sequence."""
+    from gradcraft_b200.trainer import Trainer
+    from oracle import numpy_oracle as O
+
+    w = synth.gpt_weights(arch, V, T, C, H, L, F, seed=5, perturb=True)
+    w = {k: (v * 12.0 if v.ndim == 2 else v) for k, v in w.items()}
+    start = synth.zipf_tokens(9, prompt, V)
+    tr = Trainer(arch, V, T, C, H, L, F)
+    try:
+        tr.load(w)
+        got = tr.generate(start, prompt + new, num_sequences=2, context_length=ctx)
+        oracle = O.GPTOracle(arch, V, T, C, H, L, F)
+        for step in range(prompt, prompt + new):
+            z = oracle.logits(w, got[:1, max(0, step - ctx):step])[0, -1].astype(np.float64)
+            assert z[got[0, step]] >= z.max() - 1e-4 * np.abs(z).max(), step
+        assert np.array_equal(got[0], got[1])
+        for seqs in (2, 3, 9):
+            one = tr.generate(start, prompt + new, num_sequences=seqs, context_length=ctx, temperature=0.7, top_k=1)
+            assert np.array_equal(one, np.repeat(got[:1], seqs, axis=0)), seqs
+        from gradcraft_b200 import capi
+
+        assert capi.lib().ctx_launch_count_named(tr.context(), b"gpt_decode") > 0
+        with pytest.raises(Exception):  # an id outside the vocabulary is reported, not dereferenced
+            tr.generate([V], 4, context_length=ctx)
+        assert np.array_equal(tr.generate(start, prompt + new, context_length=ctx), got[:1])
+    finally:
+        tr.close()
