@@ -51,13 +51,11 @@ def parse_header(path=HEADER):
 
 
 def _ptr(x):
-    if x is None:
-        return None
-    if hasattr(x, "data_ptr"):
-        return ctypes.c_void_p(x.data_ptr())
-    if hasattr(x, "ctypes"):
-        return ctypes.c_void_p(x.ctypes.data)
-    return x
+    """Address of a torch tensor or numpy array; None, integers and ctypes values as they are (the prototype converts them)."""
+    try:
+        return x.data_ptr()
+    except AttributeError:
+        return x.ctypes.data if hasattr(x, "ctypes") else x
 
 
 class Lib:
@@ -73,11 +71,17 @@ class Lib:
             fn.restype, fn.argtypes = restype, argtypes
             self.names.append(name)
             checked = restype is ctypes.c_int and name not in ("gcb_ctx_device", "gcb_ctx_last_gemm_engine", "gcb_ctx_gemm_split_mode", "gcb_gpt_decode_supported")
-            setattr(self, name[4:], self._wrap(fn, checked))
+            setattr(self, name[4:], self._wrap(fn, checked, [i for i, t in enumerate(argtypes) if t is ctypes.c_void_p]))
 
-    def _wrap(self, fn, checked):
+    def _wrap(self, fn, checked, pointers):
+        # a call costs about as much as the kernel launch behind it when the GPU waits for it: only pointer arguments are looked at
         def call(*args):
-            r = fn(*[_ptr(a) for a in args])
+            a = list(args)
+            for i in pointers:
+                x = a[i]
+                if x is not None and x.__class__ is not int:
+                    a[i] = _ptr(x)
+            r = fn(*a)
             if checked and r != OK:
                 raise GcbError(r, self.cdll.gcb_last_error_string().decode())
             return r
@@ -113,10 +117,15 @@ class Context:
         self.h = h
 
     def __getattr__(self, name):
-        fn = getattr(self.lib, name, None) or getattr(self.lib, "ctx_" + name)
-        return lambda *a: fn(self.h, *a)
+        fn, h = getattr(self.lib, name, None) or getattr(self.lib, "ctx_" + name), self.h
+
+        def method(*a):
+            return fn(h, *a)
+
+        self.__dict__[name] = method  # looked up once
+        return method
 
     def close(self):
         if self.h:
             self.lib.ctx_destroy(self.h)
-            self.h = None
+            self.__dict__ = {"lib": self.lib, "h": None}  # the looked-up methods hold the handle

@@ -7,7 +7,9 @@
 
 using namespace gcb;
 
-static constexpr int64_t kPackWork = int64_t(1) << 24;  // multiply-adds from which unaligned operands are packed for the tensor cores
+// Products of fewer multiply-adds run on the FMA engine, fused epilogues included: it takes 3 - 8 us for them, while no tensor-core
+// kernel returns in less than 12.
+static constexpr int64_t kSmallWork = int64_t(1) << 26;
 
 namespace gcb {
 
@@ -54,11 +56,12 @@ struct PackedOperand {
 
 // Engine choice for one validated problem; no timing here, so the GELU fallback below may call it again freely.
 static int dispatch_gemm(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g, const char* who) {
+    const int64_t work = g.M * g.N * g.K * g.batch_outer * g.batch_inner;
+    if (ctx->gemm_engine == 1 || (ctx->gemm_engine == 0 && work < kSmallWork)) return gemm_simt_launch(ctx, ta, tb, g);
     int rc = GCB_UNSUPPORTED;
-    if (ctx->gemm_engine != 1 && gemm_tc_eligible(g)) rc = gemm_tc_launch(ctx, ta, tb, g);
-    // Operands that only their addresses keep from the tensor cores are copied into rows that suit them, once the product is
-    // large enough to pay for the passes: a copy costs ~3 us, the FMA engine takes about that long per 2^25 multiply-adds.
-    if (rc == GCB_UNSUPPORTED && ctx->gemm_engine == 0 && g.M * g.N * g.K * g.batch_outer * g.batch_inner >= kPackWork && g.batch_outer * g.batch_inner <= 65535) {
+    if (gemm_tc_eligible(g)) rc = gemm_tc_launch(ctx, ta, tb, g);
+    // operands that only their addresses keep from the tensor cores are copied into rows that suit them (~3 us each)
+    if (rc == GCB_UNSUPPORTED && ctx->gemm_engine == 0 && g.batch_outer * g.batch_inner <= 65535) {
         GemmArgs packed = g;
         PackedOperand pa(ctx), pb(ctx);
         rc = pa.pack(ctx, &packed.A, &packed.lda, &packed.a_so, &packed.a_si, ta ? g.K : g.M, ta ? g.M : g.K, g.batch_outer, g.batch_inner);
@@ -104,7 +107,6 @@ static int dispatch_gemm(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g, cons
             return GCB_UNSUPPORTED;
         }
         rc = gemm_simt_launch(ctx, ta, tb, g);
-        if (rc == GCB_OK && g.sm_probs) rc = softmax_bwd_apply_launch(ctx, g);  // this engine has no fused epilogue: same arithmetic as a second pass
     }
     return rc;
 }

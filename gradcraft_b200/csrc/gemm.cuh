@@ -33,15 +33,12 @@ struct GemmArgs {
     int colsum_accumulate = 0;
 };
 
-// fp32 FMA engine: any shape, any leading dimension.
+// fp32 FMA engine: any shape, any leading dimension, every epilogue.
 int gemm_simt_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g);
 // tcgen05 3xTF32 engine.  Returns GCB_UNSUPPORTED (without touching C) when the operands cannot be described
 // to TMA: bases must be 16-byte aligned and every leading dimension / batch stride a multiple of 4 floats.
 int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g);
 bool gemm_tc_eligible(const GemmArgs& g);
-// C <- sm_scale * sm_probs * (C - sm_rowdot[row]) on/below the diagonal, 0 above: the softmax-backward epilogue as a pass of its own
-int softmax_bwd_apply_launch(gcb_ctx* ctx, const GemmArgs& g);
-
 // cuTensorMapEncodeTiled, looked up once per context (NULL: not there).
 typedef CUresult (*TmaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

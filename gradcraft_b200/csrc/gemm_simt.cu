@@ -1,115 +1,284 @@
-// fp32 SIMT GEMM: the engine for operands TMA cannot address (leading dimensions that are not multiples of
-// four floats, unaligned bases, tiny shapes).  True fp32 FMA, so it also serves as the on-device yardstick the
-// tensor-core engine is checked against.  Reference counterpart: cublasSgemm / cublasSgemmStridedBatched behind
-// CUDAMath::apply_normal_gemm / apply_batched_gemm (backend/cuda/kernels_math.cu:725-779).
+// fp32 FMA GEMM: the engine for small products, and for operands TMA cannot address.  True fp32 arithmetic, so it also serves as
+// the on-device yardstick the tensor-core engine is checked against.  Reference counterpart: cublasSgemm /
+// cublasSgemmStridedBatched behind CUDAMath::apply_normal_gemm / apply_batched_gemm (backend/cuda/kernels_math.cu:725-779).
+//
+// What bounds a small product is latency: one trip to memory, the K loop, one trip back.  The tensor-core kernels take 12 - 13 us
+// for 256 x 128 x 128 (tensor memory, descriptors and barriers are set up, each operand is split into three, and two CTAs work on
+// it); here the tiles are small so that many SMs share the work, and what is still short of CTAs is cut along K as well:
+//   * 32 x 32 tiles, four groups of 64 threads taking a quarter of every K block each, while 64 x 64 tiles would leave SMs idle;
+//   * up to eight CTAs of a cluster take a slice of K each and add their tiles through distributed shared memory, in rank order
+//     (deterministic, no scratch memory and no second launch);
+//   * three K blocks of 32 in flight with cp.async; operands off 16-byte boundaries are copied in 4-byte pieces.
+// An operand contiguous along K stays [row][k] in shared memory and is read four k at a time, one contiguous along M / N stays
+// [k][column] and is read four columns at a time: 8 vector loads per 64 FMAs either way, without bank conflicts.
+#include <algorithm>
+
 #include "gemm.cuh"
 
 namespace gcb {
 
+constexpr int SG_BK = 32, SG_STAGES = 3, SG_THREADS = 256, SG_KP = SG_BK + 4;
 
-constexpr int BM = 128, BN = 128, BK = 16, PAD = 4;
+template <int BM>
+struct SgSmem {
+    static constexpr int KG = BM == 32 ? 4 : 1;                       // groups of threads sharing a K block
+    static constexpr int OP = BM * SG_KP > SG_BK * (BM + 4) ? BM * SG_KP : SG_BK * (BM + 4);  // floats of one operand's block
+    static constexpr int LOOP = SG_STAGES * 2 * OP, OUT = KG * BM * BM;
+    static constexpr int FLOATS = (LOOP > OUT ? LOOP : OUT) + BM;     // + column sums
+};
 
-// Row-major C[M,N] = alpha * op(A) * op(B) + beta * C (+ bias[n]).  TA: A is stored K x M; TB: B is stored N x K.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs g) {
-    __shared__ __align__(16) float As[2][BK][BM + PAD];
-    __shared__ __align__(16) float Bs[2][BK][BN + PAD];
-    const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const int64_t bz = blockIdx.z, bo = bz / g.batch_inner, bi = bz % g.batch_inner;
+__device__ __forceinline__ void sg_copy(float* dst, const float* src, int n, bool vec, const float* safe) {  // n of four floats, the rest zero
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (vec) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(n > 0 ? src : safe), "r"(4 * n) : "memory");
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * e), "l"(e < n ? src + e : safe), "r"(e < n ? 4 : 0) : "memory");
+    }
+}
+// One K block of an operand: KC: stored rows x K (contiguous along k), otherwise K x rows.
+template <int BM, bool KC>
+__device__ __forceinline__ void sg_load(float* sm, const float* p, int64_t ld, int64_t r0, int64_t rows, int64_t k0, int64_t k_end, bool vec) {
+#pragma unroll
+    for (int i = 0; i < BM * SG_BK / 4 / SG_THREADS; ++i) {
+        const int c = threadIdx.x + i * SG_THREADS;
+        if (KC) {
+            const int r = c >> 3, k = (c & 7) * 4;
+            const int n = r0 + r < rows ? (int)max((int64_t)0, min((int64_t)4, k_end - k0 - k)) : 0;
+            sg_copy(sm + r * SG_KP + k, p + (r0 + r) * ld + k0 + k, n, vec, p);
+        } else {
+            const int k = c / (BM / 4), r = (c % (BM / 4)) * 4;
+            const int n = k0 + k < k_end ? (int)max((int64_t)0, min((int64_t)4, rows - r0 - r)) : 0;
+            sg_copy(sm + k * (BM + 4) + r, p + (k0 + k) * ld + r0 + r, n, vec, p);
+        }
+    }
+}
+// f[i][q] = element (row i of this thread, k + q): rows t + (BM / 4) i where the block is [row][k], 4 t + i where it is [k][row]
+template <int BM, bool KC>
+__device__ __forceinline__ void sg_fragment(const float* sm, int t, int k, float (&f)[4][4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = KC ? ld4(sm + (t + (BM / 4) * i) * SG_KP + k) : ld4(sm + (k + i) * (BM + 4) + 4 * t);
+        if (KC) { f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w; }
+        else { f[0][i] = v.x; f[1][i] = v.y; f[2][i] = v.z; f[3][i] = v.w; }
+    }
+}
+
+// Row-major C[M,N] = alpha * op(A) * op(B) + beta * C (+ bias[n]) and the epilogues of GemmArgs.  TA: A is stored K x M; TB: B is
+// stored N x K.  A cluster of `slices` CTAs takes one tile.
+template <int BM, bool TA, bool TB>
+__global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g, int tiles_m, int tiles_n, int slices, bool a_vec, bool b_vec, bool c_vec) {
+    using S = SgSmem<BM>;
+    constexpr int KG = S::KG, TPR = BM / 4, GT = TPR * TPR;  // threads along an edge of the tile, threads of a K group
+    extern __shared__ __align__(16) float sg[];
+    const int t = threadIdx.x, rank = (int)(blockIdx.x % (unsigned)slices);
+    int64_t w = blockIdx.x / (unsigned)slices;
+    const int64_t bz = w / ((int64_t)tiles_m * tiles_n);
+    w -= bz * tiles_m * tiles_n;
+    const int64_t m0 = (w / tiles_n) * BM, n0 = (w % tiles_n) * BM;
+    const int64_t bo = bz / g.batch_inner, bi = bz % g.batch_inner;
     const float* A = g.A + bo * g.a_so + bi * g.a_si;
     const float* B = g.B + bo * g.b_so + bi * g.b_si;
-    float* C = g.C + bo * g.c_so + bi * g.c_si;
-    const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-
-    // per-thread global->shared assignment: 8 consecutive elements along the contiguous axis of each operand
-    const int a_r = TA ? (t >> 4) : (t >> 1);          // TA: k index 0..15 ; else m index 0..127
-    const int a_c = TA ? (t & 15) * 8 : (t & 1) * 8;   // TA: m offset     ; else k offset
-    const int b_r = TB ? (t >> 1) : (t >> 4);          // TB: n index      ; else k index
-    const int b_c = TB ? (t & 1) * 8 : (t & 15) * 8;   // TB: k offset     ; else n offset
-
-    float ra[8], rb[8];
-    auto load_tiles = [&](int64_t k0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            int64_t m, k;
-            if (TA) { k = k0 + a_r; m = m0 + a_c + j; } else { m = m0 + a_r; k = k0 + a_c + j; }
-            ra[j] = (m < g.M && k < g.K) ? (TA ? A[k * g.lda + m] : A[m * g.lda + k]) : 0.0f;
-            int64_t n, kk;
-            if (TB) { n = n0 + b_r; kk = k0 + b_c + j; } else { kk = k0 + b_r; n = n0 + b_c + j; }
-            rb[j] = (n < g.N && kk < g.K) ? (TB ? B[n * g.ldb + kk] : B[kk * g.ldb + n]) : 0.0f;
-        }
-    };
-    auto store_tiles = [&](int buf) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (TA) As[buf][a_r][a_c + j] = ra[j]; else As[buf][a_c + j][a_r] = ra[j];
-            if (TB) Bs[buf][b_c + j][b_r] = rb[j]; else Bs[buf][b_r][b_c + j] = rb[j];
-        }
-    };
-
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-
-    // causal operands: skip the K range where op(A) is known to be zero (same 128-row granularity as the tensor-core engine)
-    int64_t k_begin = 0, k_end = g.K;
+    // a triangular output is read in 128-wide diagonal blocks and, as scores, at or below the diagonal only; the softmax backward
+    // writes the zeros of those blocks, which take no product
+    const bool above = g.causal == 1 && n0 > m0 + BM - 1;
+    if (above && (g.sm_probs == nullptr || n0 >= (m0 / 128 + 1) * 128)) return;  // the whole cluster
+    int64_t k_begin = 0, k_end = above ? 0 : g.K;
     if (g.causal == 2) k_end = min(g.K, m0 + BM);
-    else if (g.causal == 3) k_begin = min(g.K, m0) / BK * BK;
-    load_tiles(k_begin);
-    store_tiles(0);
+    else if (g.causal == 3) k_begin = min(g.K, m0);
+    {
+        const int64_t blocks = (k_end - k_begin + SG_BK - 1) / SG_BK, each = (blocks + slices - 1) / slices * SG_BK;
+        const int64_t b0 = k_begin + rank * each;
+        k_end = min(k_end, b0 + each);
+        k_begin = b0;
+    }
+    const int nblk = k_end > k_begin ? (int)((k_end - k_begin + SG_BK - 1) / SG_BK) : 0;
+    auto load = [&](int i) {
+        if (i < nblk) {
+            float* st = sg + (i % SG_STAGES) * 2 * S::OP;
+            const int64_t k0 = k_begin + (int64_t)i * SG_BK;
+            sg_load<BM, !TA>(st, A, g.lda, m0, g.M, k0, k_end, a_vec);
+            sg_load<BM, TB>(st + S::OP, B, g.ldb, n0, g.N, k0, k_end, b_vec);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int grp = t / GT, tt = t % GT, tx = tt % TPR, ty = tt / TPR;
+    const bool sum_cols = g.colsum != nullptr && m0 == 0;
+    float acc[4][4], csum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    load(0);
+    load(1);
+    for (int i = 0; i < nblk; ++i) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(SG_STAGES - 2) : "memory");
+        __syncthreads();  // block i has landed for everybody, and everybody is done with block i - 1
+        load(i + 2);
+        const float* as = sg + (i % SG_STAGES) * 2 * S::OP;
+        const float* bs = as + S::OP;
+#pragma unroll
+        for (int k = 0; k < SG_BK / KG; k += 4) {
+            float a[4][4], b[4][4];
+            sg_fragment<BM, !TA>(as, ty, grp * (SG_BK / KG) + k, a);
+            sg_fragment<BM, TB>(bs, tx, grp * (SG_BK / KG) + k, b);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r][q], b[c][q], acc[r][c]);
+        }
+        if (sum_cols && t < BM) {
+#pragma unroll 8
+            for (int k = 0; k < SG_BK; ++k) csum += bs[k * (BM + 4) + t];  // op(B) is stored K x N here
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    int buf = 0;
-    for (int64_t k0 = k_begin; k0 < k_end; k0 += BK) {
-        const bool more = k0 + BK < k_end;
-        if (more) load_tiles(k0 + BK);
+    // the tile, K groups side by side, in row-major order
+    float* out = sg;
+    float* cols = sg + (S::LOOP > S::OUT ? S::LOOP : S::OUT);
 #pragma unroll
-        for (int k = 0; k < BK; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][k][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][k][64 + ty * 4]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][k][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][k][64 + tx * 4]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    for (int r = 0; r < 4; ++r) {
+        const int row = TA ? 4 * ty + r : ty + TPR * r;
+        float* o = out + grp * BM * BM + row * BM;
+        if (!TB) st4(o + 4 * tx, make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]));
+        else
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int c = 0; c < 4; ++c) o[tx + TPR * c] = acc[r][c];
+    }
+    if (sum_cols && t < BM) cols[t] = csum;
+    __syncthreads();
+    constexpr int VECS = BM * BM / 4;
+    if (KG > 1) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-        if (more) {
-            store_tiles(buf ^ 1);
-            __syncthreads();
-            buf ^= 1;
+        for (int v = t; v < VECS; v += SG_THREADS) {
+            float4 s = ld4(out + 4 * v);
+#pragma unroll
+            for (int q = 1; q < KG; ++q) { const float4 x = ld4(out + q * BM * BM + 4 * v); s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w; }
+            st4(out + 4 * v, s);
         }
     }
+    if (slices > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    auto remote = [&](const float* p, int r) {  // the same place in rank r's shared memory
+        uint32_t a;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(r));
+        return a;
+    };
+    float* C = g.C + bo * g.c_so + bi * g.c_si;
+    const int64_t side_off = bo * g.c_so + bi * g.c_si;
+    const int share = VECS / slices;  // of the tile's vectors, per rank
+    for (int v = rank * share + t; v < (rank + 1) * share; v += SG_THREADS) {
+        const int row = v / (BM / 4), col = (v % (BM / 4)) * 4;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (slices == 1) {
+            s = ld4(out + 4 * v);  // KG > 1: this thread's own sum
+        } else {
+            float4 x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int64_t m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-        if (m >= g.M) continue;
+            for (int r = 0; r < 8; ++r)
+                if (r < slices) asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[r].x), "=f"(x[r].y), "=f"(x[r].z), "=f"(x[r].w) : "r"(remote(out + 4 * v, r)) : "memory");
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int64_t n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-            if (n >= g.N) continue;
-            float r = g.alpha * acc[i][j];
-            if (g.bias) r += g.bias[n];
-            if (g.beta != 0.0f) r += g.beta * C[m * g.ldc + n];
-            C[m * g.ldc + n] = r;
+            for (int r = 0; r < 8; ++r) if (r < slices) { s.x += x[r].x; s.y += x[r].y; s.z += x[r].z; s.w += x[r].w; }
+        }
+        const int64_t m = m0 + row, n = n0 + col;
+        if (m >= g.M || n >= g.N) continue;
+        float o[4] = {g.alpha * s.x, g.alpha * s.y, g.alpha * s.z, g.alpha * s.w};
+        const int64_t at = m * g.ldc + n;
+        const int live = (int)min((int64_t)4, g.N - n);
+        const bool whole = c_vec && live == 4;
+        float old[4] = {0.f, 0.f, 0.f, 0.f}, side[4] = {0.f, 0.f, 0.f, 0.f};
+        const float* sp = g.residual ? g.residual : g.gelu_pre ? g.gelu_pre : g.sm_probs;
+        if (whole) {
+            if (g.beta != 0.0f) { const float4 x = ld4(C + at); old[0] = x.x; old[1] = x.y; old[2] = x.z; old[3] = x.w; }
+            if (sp) { const float4 x = ld4(sp + side_off + at); side[0] = x.x; side[1] = x.y; side[2] = x.z; side[3] = x.w; }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) if (e < live) { if (g.beta != 0.0f) old[e] = C[at + e]; if (sp) side[e] = sp[side_off + at + e]; }
+        }
+        const float rd = g.sm_probs ? g.sm_rowdot[bz * g.M + m] : 0.0f;
+        float act[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (g.bias && e < live) o[e] += g.bias[n + e];
+            if (g.beta != 0.0f) o[e] += g.beta * old[e];
+            if (g.residual) o[e] += side[e];
+            else if (g.gelu_pre) o[e] *= gelu_grad_f(side[e]);
+            else if (g.sm_probs) o[e] = n + e <= m ? g.sm_scale * side[e] * (o[e] - rd) : 0.0f;
+            act[e] = g.gelu_act ? gelu_f(o[e]) : 0.0f;
+        }
+        if (whole) {
+            st4(C + at, make_float4(o[0], o[1], o[2], o[3]));
+            if (g.gelu_act) st4(g.gelu_act + side_off + at, make_float4(act[0], act[1], act[2], act[3]));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) if (e < live) { C[at + e] = o[e]; if (g.gelu_act) g.gelu_act[side_off + at + e] = act[e]; }
         }
     }
+    if (sum_cols && rank == 0 && t < BM && n0 + t < g.N) {
+        float s = 0.0f;
+        for (int r = 0; r < slices; ++r) {
+            float x;
+            if (slices == 1) x = cols[t];
+            else asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote(cols + t, r)) : "memory");
+            s += x;
+        }
+        float* d = g.colsum + n0 + t;
+        *d = g.colsum_accumulate ? *d + s : s;
+    }
+    if (slices > 1) {  // nobody leaves while its shared memory is still read
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+template <int BM, bool TA, bool TB>
+static int sg_launch(gcb_ctx* ctx, const GemmArgs& g, int64_t tiles_m, int64_t tiles_n, int64_t batches, int slices) {
+    auto ok4 = [](int64_t v) { return v % 4 == 0; };
+    auto vec = [&](const float* p, int64_t ld, int64_t so, int64_t si) { return aligned16(p) && ok4(ld) && (g.batch_inner == 1 || ok4(si)) && (g.batch_outer == 1 || ok4(so)); };
+    const bool c_vec = vec(g.C, g.ldc, g.c_so, g.c_si) && aligned16(g.residual) && aligned16(g.gelu_pre) && aligned16(g.gelu_act) && aligned16(g.sm_probs);
+    auto kfn = gemm_simt_kernel<BM, TA, TB>;
+    constexpr size_t smem = sizeof(float) * SgSmem<BM>::FLOATS;
+    static bool attr_done[kMaxDevices] = {};  // function attributes belong to a device
+    if (smem > 48 * 1024 && !attr_done[ctx->device]) { GCB_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr_done[ctx->device] = true; }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles_m * tiles_n * batches * slices), 1, 1);
+    cfg.blockDim = dim3(SG_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)slices;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kfn, g, (int)tiles_m, (int)tiles_n, slices, vec(g.A, g.lda, g.a_so, g.a_si), vec(g.B, g.ldb, g.b_so, g.b_si), c_vec));
+    return GCB_OK;
 }
 
 int gemm_simt_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     const int64_t batches = g.batch_outer * g.batch_inner;
     if (g.M == 0 || g.N == 0 || batches == 0) return GCB_OK;
-    const int64_t gx = (g.N + BN - 1) / BN, gy = (g.M + BM - 1) / BM;
-    GCB_REQUIRE(gy <= 65535 && batches <= 65535, "gemm (SIMT): grid too large (M tiles %lld, batches %lld)", (long long)gy, (long long)batches);
-    dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)batches);
+    if (g.colsum && tb) { set_error("gemm (FMA): column sums need op(B) stored K x N"); return GCB_UNSUPPORTED; }
+    auto tiles = [&](int64_t b) { return ((g.M + b - 1) / b) * ((g.N + b - 1) / b) * batches; };
+    // 64-wide tiles read shared memory and L2 half as often per FMA: they are taken once they fill the chip by themselves
+    const int bm = tiles(64) >= kSMs ? 64 : 32;
+    const int64_t tm = (g.M + bm - 1) / bm, tn = (g.N + bm - 1) / bm;
+    GCB_REQUIRE(tm * tn <= 0x7fffffff / 8 && tiles(bm) <= 0x7fffffff / 8, "gemm (FMA): grid too large");
+    // K is cut while CTAs are missing and every slice keeps two K blocks
+    int slices = 1;
+    while (slices < 8 && tiles(bm) * slices * 2 <= 2 * kSMs && g.K >= (int64_t)slices * 2 * 2 * SG_BK) slices *= 2;
     cudaSetDevice(ctx->device);
-    if (!ta && !tb) gemm_simt_kernel<false, false><<<grid, 256, 0, ctx->stream>>>(g);
-    else if (!ta && tb) gemm_simt_kernel<false, true><<<grid, 256, 0, ctx->stream>>>(g);
-    else if (ta && !tb) gemm_simt_kernel<true, false><<<grid, 256, 0, ctx->stream>>>(g);
-    else gemm_simt_kernel<true, true><<<grid, 256, 0, ctx->stream>>>(g);
+    int rc;
+#define GCB_SG(BMV) (!ta && !tb ? sg_launch<BMV, false, false>(ctx, g, tm, tn, batches, slices) : !ta ? sg_launch<BMV, false, true>(ctx, g, tm, tn, batches, slices) \
+                     : !tb ? sg_launch<BMV, true, false>(ctx, g, tm, tn, batches, slices) : sg_launch<BMV, true, true>(ctx, g, tm, tn, batches, slices))
+    rc = bm == 64 ? GCB_SG(64) : GCB_SG(32);
+#undef GCB_SG
+    if (rc) return rc;
     ctx->last_gemm_engine = 1;
     return after_launch(ctx, "gemm_simt");
 }

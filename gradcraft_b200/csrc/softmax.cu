@@ -8,7 +8,6 @@
 // Cross-entropy forward: a persistent CTA streams a row twice (online max/sum, then normalise); the grid is
 // sized so that all rows in flight fit in L2 and the second pass does not go back to HBM.
 #include "common.cuh"
-#include "gemm.cuh"
 
 namespace gcb {
 
@@ -252,26 +251,6 @@ __global__ void __launch_bounds__(256) rowdot_kernel(float* __restrict__ out, co
         if (live && sub == 0) out[r] = acc;
     }
 }
-
-// C <- scale * P * (C - rowdot[row]) on/below the diagonal, 0 above (the GEMM epilogue of the same name, as a pass of its own)
-__global__ void __launch_bounds__(256) softmax_bwd_apply_kernel(float* __restrict__ C, const float* __restrict__ P, const float* __restrict__ rowdot, float scale, int64_t M, int64_t N,
-                                                                int64_t ldc, int64_t c_so, int64_t c_si, int64_t n_inner, int64_t total) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t n = i % N, rm = i / N, m = rm % M, item = rm / M, bo = item / n_inner, bi = item - bo * n_inner;
-        const int64_t off = bo * c_so + bi * c_si + m * ldc + n;
-        C[off] = n <= m ? scale * P[off] * (C[off] - rowdot[item * M + m]) : 0.0f;
-    }
-}
-
-namespace gcb {
-int softmax_bwd_apply_launch(gcb_ctx* ctx, const GemmArgs& g) {
-    const int64_t total = g.M * g.N * g.batch_outer * g.batch_inner;
-    if (total == 0) return GCB_OK;
-    softmax_bwd_apply_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)kSMs * 16), 256, 0, ctx->stream>>>(g.C, g.sm_probs, g.sm_rowdot, g.sm_scale, g.M, g.N, g.ldc, g.c_so, g.c_si,
-                                                                                                                  g.batch_inner, total);
-    return after_launch(ctx, "softmax_bwd_apply");
-}
-}  // namespace gcb
 
 extern "C" {
 
