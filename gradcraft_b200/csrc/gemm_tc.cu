@@ -56,7 +56,7 @@ struct TcParams {
                          // 0: as 1 with big = rna_tf32(x) written back, small = x - big (does not rely on the hardware's truncation)
     float* partial;      // [splits][M][partial_ld] when splits > 1
     int64_t partial_ld;  // N rounded up to a multiple of four: whole vectors whatever N is
-    int b_twin;              // pair kernel: the BF16 companions of B come pre-split from global memory (map_t), the B-splitter warps idle
+    int b_twin;              // pair kernel and narrow tiles: the BF16 companions of B come pre-split from global memory (map_t), the B-splitter warps idle
     int c_tma;               // 256-wide single-CTA kernel: C leaves (and the probabilities arrive) through TMA on swizzled 32 x 32 blocks in shared memory
     float* colsum;           // column sums of op(B) (see GemmArgs), or NULL: pair kernel with B stored K x N only
     float* colsum_partial;   // [splits][N] when splits > 1
@@ -377,7 +377,7 @@ __device__ __forceinline__ TileCoord tile_coord(const TcParams& p, int64_t w, in
 // A_MN: A is stored K x M (contiguous along M); B_MN: B is stored K x N (contiguous along N).
 template <int BN, bool A_MN, bool B_MN, bool A_TM>
 __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1)) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                                                                                                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_p, TcParams p) {
+                                                                                                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_p, const __grid_constant__ TcParams p) {
     using S = TcSmem<BN, A_TM>;
     constexpr int TC_STAGES = S::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -426,8 +426,10 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
                     ok = TR_WAIT(mbar_wait(empty_bar(s), ph ^ 1u, p.status, 1));
                     if (!ok) break;
                     const uint32_t sa = base + s * S::STAGE_BYTES, sb = sa + S::B_OFF;
-                    mbar_expect_tx(full_bar(s), S::A_BYTES + S::B_BYTES);
+                    const bool twin = A_TM && p.b_twin != 0;
+                    mbar_expect_tx(full_bar(s), S::A_BYTES + S::B_BYTES + (twin ? S::B_BYTES : 0));
                     const int k0 = (tc.kb0 + i) * TC_BK;
+                    if (twin) tma_load_3d(sb + S::B_BYTES, &map_p, full_bar(s), (k0 >> 3) * 64, tc.n0 >> 3, 0);  // the weight's companions, as in the pair kernel (map_p: these kernels read no probabilities)
                     if (A_MN) {
                         if (p.a_chunked) tma_load_5d(sa, &map_a, full_bar(s), 0, k0, tc.m0 / 32, tc.b_in, tc.b_out);
                         else
@@ -553,7 +555,8 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");  // the MMAs that read this TMEM stage last round have completed (empty -> TMA -> full)
                     const int row = 32 * (warp & 3) + lane;                          // a warp reaches the TMEM lanes of its quarter only
                     split_a_to_tmem<A_MN>(st, tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + S::A_TMEM_COL0 + s * 32, row);
-                    split_hybrid<B_MN, BN>(st + S::B_OFF, st + S::B_OFF + S::B_BYTES, t);
+                    if (!p.b_twin)  // otherwise the companions arrived with the tile
+                        split_hybrid<B_MN, BN>(st + S::B_OFF, st + S::B_OFF + S::B_BYTES, t);
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 } else if (p.split_mode == 2) {
                     uint8_t* st = gen_base + s * S::STAGE_BYTES;
@@ -873,9 +876,26 @@ __device__ __forceinline__ TileCoord pair_tile_coord(const TcParams& p, int64_t 
     return t;
 }
 
+// One column of a 32-row block that cannot be stored in whole vectors.  Kept out of line: inlined it costs the epilogue of whole
+// blocks a dozen registers (spills) and the step 5 %.
+__device__ __noinline__ void pair_ragged_column(const TcParams& p, const float* staged, float* d, int64_t ld, int rows, int64_t n, bool to_partial) {
+    const float alpha = to_partial ? 1.0f : p.alpha, beta = to_partial ? 0.0f : p.beta;
+    const bool epi = !to_partial;
+    const float b = epi && p.bias ? p.bias[n] : 0.0f;
+    for (int r0 = 0; r0 < rows; ++r0, d += ld) {
+        float r = staged[r0 * PairSmemT<true>::EPI_PITCH] * alpha;
+        if (epi && p.bias) r += b;
+        if (beta != 0.0f) r += beta * *d;
+        if (epi && p.gelu_pre) r *= gelu_grad_f(p.gelu_pre[d - p.C]);
+        if (epi && p.resid) r += p.resid[d - p.C];
+        *d = r;
+        if (epi && p.gelu_act) p.gelu_act[d - p.C] = gelu_f(r);
+    }
+}
+
 template <bool A_MN, bool B_MN, bool A_TM>
 __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                                                                                    const __grid_constant__ CUtensorMap map_t, TcParams p) {
+                                                                                    const __grid_constant__ CUtensorMap map_t, const __grid_constant__ TcParams p) {
     using S = PairSmemT<A_TM>;
     constexpr int BN = S::BN, NST = S::STAGES, NACC = S::NACC;
     extern __shared__ uint8_t smem_raw[];
@@ -1155,32 +1175,7 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
                         }
                     } else {  // ragged or unaligned block: lane = column, as in the single-CTA kernel
                         const int64_t nc = nb + lane;
-                        const bool col_ok = nc < p.N;
-                        const float bc = (bias && col_ok) ? bias[nc] : 0.0f;
-                        const int rows = (int)max((int64_t)0, min((int64_t)32, p.M - mrow0));
-                        const int64_t soff = cbase - p.C;
-                        for (int r0 = 0; r0 < rows; r0 += 8) {
-                            float oldv[8], sv[8];
-#pragma unroll
-                            for (int u = 0; u < 8; ++u) {
-                                const bool live = col_ok && r0 + u < rows;
-                                const int64_t at = (mrow0 + r0 + u) * ld + nc;
-                                oldv[u] = (beta != 0.0f && live) ? cbase[at] : 0.0f;
-                                sv[u] = (side && live) ? side[soff + at] : 0.0f;
-                            }
-#pragma unroll
-                            for (int u = 0; u < 8; ++u) {
-                                if (!col_ok || r0 + u >= rows) continue;
-                                const int64_t at = (mrow0 + r0 + u) * ld + nc;
-                                float r = stg[(r0 + u) * S::EPI_PITCH + lane] * alpha;
-                                if (bias) r += bc;
-                                if (beta != 0.0f) r += beta * oldv[u];
-                                if (gelu_pre) r *= gelu_grad_f(sv[u]);
-                                if (resid) r += sv[u];
-                                cbase[at] = r;
-                                if (gelu_act) gelu_act[soff + at] = gelu_f(r);
-                            }
-                        }
+                        if (nc < p.N && mrow0 < p.M) pair_ragged_column(p, stg + lane, cbase + mrow0 * ld + nc, ld, (int)min((int64_t)32, p.M - mrow0), nc, to_partial);
                     }
                 }
                 __syncwarp();
@@ -1221,25 +1216,25 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ 
         const int64_t m = i / n4, n = (i - m * n4) << 2;
         const float4* src = reinterpret_cast<const float4*>(partial) + i;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-        for (int k = 0; k < splits; ++k) {
-            const float4 v = __ldcg(src + (int64_t)k * total4);
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-        }
-        float o[4] = {alpha * s.x, alpha * s.y, alpha * s.z, alpha * s.w};
         float* dst = C + m * ldc + n;
-        if (vec) {
-            if (bias) { o[0] += bias[n]; o[1] += bias[n + 1]; o[2] += bias[n + 2]; o[3] += bias[n + 3]; }
-            if (beta != 0.0f) { const float4 old = ld4(dst); o[0] += beta * old.x; o[1] += beta * old.y; o[2] += beta * old.z; o[3] += beta * old.w; }
-            st4(dst, make_float4(o[0], o[1], o[2], o[3]));
-        } else {
+        int k = 0;
+        for (; k + 4 <= splits; k += 4) {  // four slices' loads in flight
+            float4 v[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (n + e >= N) break;
-                if (bias) o[e] += bias[n + e];
-                if (beta != 0.0f) o[e] += beta * dst[e];
-                dst[e] = o[e];
-            }
+            for (int u = 0; u < 4; ++u) v[u] = __ldcg(src + (int64_t)(k + u) * total4);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w; }
+        }
+        for (; k < splits; ++k) { const float4 v = __ldcg(src + (int64_t)k * total4); s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+        float4 o = make_float4(alpha * s.x, alpha * s.y, alpha * s.z, alpha * s.w);
+        if (vec) {
+            if (bias) { o.x += bias[n]; o.y += bias[n + 1]; o.z += bias[n + 2]; o.w += bias[n + 3]; }
+            if (beta != 0.0f) { const float4 old = ld4(dst); o.x += beta * old.x; o.y += beta * old.y; o.z += beta * old.z; o.w += beta * old.w; }
+            st4(dst, o);
+        } else {
+            const float e[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) if (n + u < N) dst[u] = e[u] + (bias ? bias[n + u] : 0.0f) + (beta != 0.0f ? beta * dst[u] : 0.0f);
         }
     }
 }
@@ -1376,14 +1371,49 @@ static int launch_pair(gcb_ctx* ctx, bool ta, bool tb, const CUtensorMap& ma, co
     return GCB_OK;
 }
 
+// Tile and K slices of one problem: the ones with the lowest modelled time, in us.  A kernel takes start + rounds x (K blocks of an
+// item x per_block + per_item); a K block costs about the same for every tile (the splitter warps' 128 rows of A), so wide
+// tiles win once they fill the chip, and for fewer tiles the narrow kernels do: they start sooner and occupy more SMs.
+// Constants from timings at M = 512 .. 16384, N = 256 .. 2304, K = 256 .. 4096, e.g. 1656 x 384 x 384: pair 26 us, 128-wide 18, 64-wide
+// 16; 4096 x 1152 x 384: 37 / 28 / 31; 4096 x 768 x 768: 31 / 49 / 51; 512 x 768 x 768: 28 / 25 / 24, in three slices 17.
+struct TcTiling {
+    int BN;
+    bool pair;
+    int splits;
+    double us;
+};
+static void consider(TcTiling& best, const GemmArgs& g, int BN, bool pair, bool may_split) {
+    const int64_t tiles = pair ? ((g.M + 255) / 256) * ((g.N + 255) / 256) : ((g.M + TC_BM - 1) / TC_BM) * ((g.N + BN - 1) / BN);
+    const int kb = (int)((g.K + TC_BK - 1) / TC_BK);
+    for (int sp = 1; sp <= 32 && (sp == 1 || (may_split && kb >= 32 && kb / sp >= 8)); ++sp) {
+        const int kbs = (kb + sp - 1) / sp;
+        const int64_t items = tiles * sp;
+        const double per_block = pair ? 0.42 : BN == 64 && items > kSMs ? 0.5 : 0.4;  // two 64-wide CTAs of one SM share its splitters' issue slots
+        const int64_t slots = pair ? kSMs / 2 : BN == 64 ? 2 * kSMs : kSMs, rounds = (items + slots - 1) / slots;
+        const double us = (pair ? 13.0 : 5.0) + (double)rounds * (kbs * per_block + (pair ? 2.0 : 1.0)) + (sp > 1 ? 4.0 + (double)sp * (double)(g.M * g.N) * 8.0 / 5.0e6 : 0.0);
+        if (us < best.us * 0.97) best = {BN, pair, sp, us};
+    }
+}
+
 int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     TmaEncodeFn enc = tma_encode(ctx);
     if (!enc) return GCB_UNSUPPORTED;
     cudaSetDevice(ctx->device);
     const int64_t batches = g.batch_outer * g.batch_inner;
-    const int BN = (g.N > 128 || g.sm_probs) ? 256 : (g.N > 64 ? 128 : 64);
     static const int pair_env = [] { const char* e = getenv("GRADC_TC_PAIR"); return e ? atoi(e) : 1; }();
-    const bool use_pair = pair_env != 0 && BN == 256 && g.M > 128 && g.K >= 256 && !g.sm_probs;  // short K loops are epilogue-bound: nothing to gain from sharing B
+    const bool by_width = g.N > 128 || g.sm_probs;
+    const bool pair_ok = pair_env != 0 && by_width && g.M > 128 && g.K >= 256 && !g.sm_probs;  // short K loops are epilogue-bound: nothing to gain from sharing B
+    TcTiling tl{by_width ? 256 : (g.N > 64 ? 128 : 64), pair_ok, 1, 1e30};
+    if (batches == 1 && g.causal == 0 && !g.sm_probs) {
+        const bool side = g.gelu_pre || g.gelu_act || g.residual;  // these epilogues and the column sums are the pair kernel's, and an epilogue sees whole sums
+        consider(tl, g, tl.BN, tl.pair, !side);
+        if (pair_ok && !side && !g.colsum && ctx->gemm_split_mode == 2) {
+            consider(tl, g, 128, false, true);
+            consider(tl, g, 64, false, true);
+        }
+    }
+    const int BN = tl.BN;
+    const bool use_pair = tl.pair;
     CUtensorMap ma, mb;
     TcParams p;
     if (!encode_operand(enc, &ma, g.A, ta, g.M, g.K, g.lda, g.a_si, g.a_so, g.batch_inner, g.batch_outer, TC_BM, &p.a_chunked)) return GCB_UNSUPPORTED;
@@ -1409,19 +1439,7 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     p.colsum = g.colsum; p.colsum_accumulate = g.colsum_accumulate; p.colsum_partial = nullptr;
     const int64_t tiles = (int64_t)p.tiles_n * p.tiles_m * batches;
     if (tiles > 2147483647LL / 2) return GCB_UNSUPPORTED;
-    // split-K when the tiles alone would leave SMs idle: pick the slice count with the lowest modelled time
-    // (rounds of 148 persistent CTAs x K blocks per slice, plus writing and re-reading the partial tiles)
-    int splits = 1;
-    if (batches == 1 && p.k_blocks_total >= 64 && g.causal == 0 && !g.gelu_pre && !g.gelu_act && !g.residual) {
-        const int ctas = use_pair ? kSMs / 2 : kSMs * (BN == 64 ? 2 : 1);
-        double best = 1e30;
-        for (int sp = 1; sp <= 32 && p.k_blocks_total / sp >= 16; ++sp) {
-            const int kbs = (p.k_blocks_total + sp - 1) / sp;
-            const int64_t rounds = (tiles * sp + ctas - 1) / ctas;
-            const double t_us = (double)rounds * (kbs * 0.5 + 2.0) + (sp > 1 ? (double)sp * g.M * g.N * 8.0 / 5.0e6 : 0.0);
-            if (t_us < best * 0.97) { best = t_us; splits = sp; }
-        }
-    }
+    int splits = tl.splits;
     p.splits = splits;
     p.k_blocks_per_split = (p.k_blocks_total + splits - 1) / splits;
     p.splits = splits = (p.k_blocks_total + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
@@ -1454,7 +1472,7 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     CUtensorMap mt = ma;
     p.b_twin = 0;
     static const int twin_env = [] { const char* e = getenv("GRADC_TC_WEIGHT_TWINS"); return e ? atoi(e) : 1; }();
-    if (twin_env != 0 && use_pair && pair_a_tmem && batches == 1 && g.colsum == nullptr) {
+    if (twin_env != 0 && (use_pair ? pair_a_tmem : a_tmem) && batches == 1 && g.colsum == nullptr) {
         const void* tw = nullptr;
         int rc_t = twins_lookup(ctx, g.B, tb, g.N, g.K, g.ldb, &tw);
         if (rc_t) return rc_t;
@@ -1462,14 +1480,14 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
             const cuuint64_t n_groups = (cuuint64_t)((g.N + 7) / 8), k_chunks = (cuuint64_t)(((g.K + 15) / 16) * 2);
             cuuint64_t dims[3] = {k_chunks * 64, n_groups, 2};
             cuuint64_t strides[2] = {k_chunks * 128, n_groups * k_chunks * 128};
-            cuuint32_t box[3] = {128u, 16u, 2u}, estr[3] = {1, 1, 1};
+            cuuint32_t box[3] = {128u, (use_pair ? 128u : (cuuint32_t)BN) / 8u, 2u}, estr[3] = {1, 1, 1};
             if (enc(&mt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(tw), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
                 p.b_twin = 1;
         }
     }
     // the 256-wide single-CTA kernel writes C (and reads the probabilities of the dS epilogue) through TMA when their layout allows it
-    CUtensorMap mc = ma, mp = ma;  // placeholders where unused
+    CUtensorMap mc = ma, mp = mt;  // placeholders where unused
     p.c_tma = 0;
     static const int c_tma_env = [] { const char* e = getenv("GRADC_TC_EPI_TMA"); return e ? atoi(e) : 1; }();
     if (c_tma_env != 0 && !use_pair && BN == 256 && splits == 1 && g.beta == 0.0f && aligned16(g.C) && g.ldc % 4 == 0 && (g.batch_inner == 1 || (g.c_si % 4 == 0 && g.c_si > 0)) &&
