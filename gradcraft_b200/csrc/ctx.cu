@@ -127,6 +127,8 @@ void Arena::destroy() {
 
 // ---- fill kernels ------------------------------------------------------------------------------
 __global__ void fill_f32_kernel(float* __restrict__ p, float v, int64_t n, int64_t n4) {
+    pdl_trigger();
+    pdl_wait();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     float4 v4 = make_float4(v, v, v, v);
@@ -134,6 +136,8 @@ __global__ void fill_f32_kernel(float* __restrict__ p, float v, int64_t n, int64
     for (int64_t k = (n4 << 2) + i; k < n; k += stride) p[k] = v;
 }
 __global__ void fill_arange_i64_kernel(int64_t* __restrict__ p, int64_t start, int64_t step, int64_t n) {
+    pdl_trigger();
+    pdl_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = start + step * i;
 }
 
@@ -356,7 +360,7 @@ int gcb_fill_f32(gcb_ctx* ctx, float* p, float v, int64_t n) {
     int64_t blocks = ((n4 ? n4 : n) + 255) / 256;
     if (blocks > kSMs * 8) blocks = kSMs * 8;
     if (blocks < 1) blocks = 1;
-    fill_f32_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(p, v, n, n4);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, fill_f32_kernel, p, v, n, n4));
     return after_launch(ctx, "fill_f32");
 }
 int gcb_fill_arange_i64(gcb_ctx* ctx, int64_t* p, int64_t start, int64_t step, int64_t n) {
@@ -364,7 +368,7 @@ int gcb_fill_arange_i64(gcb_ctx* ctx, int64_t* p, int64_t start, int64_t step, i
     if (n == 0) return GCB_OK;
     int64_t blocks = (n + 255) / 256;
     if (blocks > kSMs * 8) blocks = kSMs * 8;
-    fill_arange_i64_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(p, start, step, n);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, fill_arange_i64_kernel, p, start, step, n));
     return after_launch(ctx, "fill_arange_i64");
 }
 int gcb_set_scalar_f32(gcb_ctx* ctx, float* p, float v) {
@@ -377,7 +381,7 @@ int gcb_set_scalar_f32(gcb_ctx* ctx, float* p, float v) {
         GCB_CHECK_CUDA(cudaMemsetAsync(p, bits & 0xff, 4, ctx->stream));
         return GCB_OK;
     }
-    fill_f32_kernel<<<1, 32, 0, ctx->stream>>>(p, v, 1, 0);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, 1, 32, 0, fill_f32_kernel, p, v, 1, 0));
     return after_launch(ctx, "set_scalar_f32");
 }
 

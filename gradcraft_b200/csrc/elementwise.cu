@@ -18,6 +18,8 @@ struct EwPtrs {
 // out[k][i] = op(in[0][i], ..., in[NIN-1][i]) for i < n; n4 = number of float4 groups handled vectorised.
 template <int NIN, int NOUT, class Op>
 __global__ void __launch_bounds__(kEwThreads) ew_kernel(EwPtrs<NIN, NOUT> p, int64_t n, int64_t n4, Op op) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t tid = (int64_t)blockIdx.x * kEwThreads + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * kEwThreads;
     for (int64_t base = tid; base < n4; base += stride * kEwUnroll) {
@@ -67,7 +69,7 @@ static int ew_launch(gcb_ctx* ctx, const char* name, EwPtrs<NIN, NOUT> p, int64_
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     cudaSetDevice(ctx->device);
-    ew_kernel<NIN, NOUT, Op><<<(unsigned)blocks, kEwThreads, 0, ctx->stream>>>(p, n, n4, op);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, kEwThreads, 0, ew_kernel<NIN, NOUT, Op>, p, n, n4, op));
     return after_launch(ctx, name);
 }
 
@@ -172,6 +174,8 @@ struct AdamWTensorOp {
 // One CTA per GCB_ADAMW_CHUNK-element chunk and loop: 256 threads x float4 = 1024 elements.
 __global__ void __launch_bounds__(256) adamw_arena_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
                                                           const uint8_t* __restrict__ mask, int64_t n, int64_t n_chunks, AdamW h) {
+    pdl_trigger();
+    pdl_wait();
     for (int64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
         const bool decay = mask[c] != 0;
         const int64_t i = c * GCB_ADAMW_CHUNK + 4 * threadIdx.x;
@@ -194,6 +198,8 @@ __global__ void __launch_bounds__(256) adamw_arena_kernel(float* __restrict__ w,
 
 // ---- broadcast / strided forms -------------------------------------------------------------------
 __global__ void __launch_bounds__(256) rowvec_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ vec, int64_t rows, int64_t cols, int op, bool v4) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t total = rows * cols;
     if (v4) {
         const int64_t n4 = total >> 2, c4 = cols >> 2;
@@ -215,6 +221,8 @@ struct StridedMeta {
 // General N-d walk (row-major over `shape`), consecutive threads on the innermost dimension.
 template <bool Binary, bool Acc>
 __global__ void __launch_bounds__(256) strided_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ b, StridedMeta m, int64_t total, int op) {
+    pdl_trigger();
+    pdl_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t rem = i, oo = 0, oa = 0, ob = 0;
 #pragma unroll 1
@@ -235,6 +243,8 @@ __global__ void __launch_bounds__(256) strided_kernel(float* __restrict__ out, c
 // Stage 1: partial[slab, c] = sum over the slab's rows of in[r, c].  Block = 32 column groups x 8 row lanes.
 template <int VEC>
 __global__ void __launch_bounds__(256) reduce_rows_stage1(float* __restrict__ partial, const float* __restrict__ in, int64_t rows, int64_t cols, int64_t rows_per_slab) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float sm[8][32 * VEC + 1];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t c0 = ((int64_t)blockIdx.x * 32 + tx) * VEC;
@@ -267,6 +277,8 @@ __global__ void __launch_bounds__(256) reduce_rows_stage1(float* __restrict__ pa
     }
 }
 __global__ void __launch_bounds__(256) reduce_rows_stage2(float* __restrict__ out, const float* __restrict__ partial, int64_t slabs, int64_t cols, int accumulate) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cols) return;
     float s = 0.0f;
@@ -275,6 +287,8 @@ __global__ void __launch_bounds__(256) reduce_rows_stage2(float* __restrict__ ou
 }
 
 __global__ void __launch_bounds__(512) sum_squares_stage1(float* __restrict__ partial, const float* __restrict__ in, int64_t n, int64_t n4) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red[33];
     float acc = 0.0f;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
@@ -287,6 +301,8 @@ __global__ void __launch_bounds__(512) sum_squares_stage1(float* __restrict__ pa
     if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 __global__ void __launch_bounds__(256) sum_partials_kernel(float* __restrict__ out, const float* __restrict__ partial, int count, int accumulate, float scale) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ double sm[256];
     double s = 0.0;
     for (int i = threadIdx.x; i < count; i += 256) s += (double)partial[i];
@@ -303,7 +319,7 @@ __global__ void __launch_bounds__(256) sum_partials_kernel(float* __restrict__ o
 }
 
 int launch_sum_partials(gcb_ctx* ctx, float* out, const float* partial, int count, int accumulate, float scale) {
-    sum_partials_kernel<<<1, 256, 0, ctx->stream>>>(out, partial, count, accumulate, scale);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, 1, 256, 0, sum_partials_kernel, out, partial, count, accumulate, scale));
     return after_launch(ctx, "sum_partials");
 }
 
@@ -343,7 +359,7 @@ int gcb_binary_rowvec_f32(gcb_ctx* ctx, int op, float* out, const float* a, cons
     int64_t work = v4 ? rows * cols / 4 : rows * cols;
     int64_t blocks = std::min<int64_t>((work + 255) / 256, kSMs * 8);
     cudaSetDevice(ctx->device);
-    rowvec_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(out, a, vec, rows, cols, op, v4);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, rowvec_kernel, out, a, vec, rows, cols, op, v4));
     return after_launch(ctx, "binary_rowvec_f32");
 }
 
@@ -367,7 +383,7 @@ int gcb_binary_strided_f32(gcb_ctx* ctx, int op, int ndim, const int64_t* shape,
     int64_t blocks = std::min<int64_t>((total + 255) / 256, kSMs * 8);
     cudaSetDevice(ctx->device);
     if (ctx->twins_lo != nullptr) ctx->twins_dirty = true;  // a strided destination has no simple range: any registered weight may be hit
-    strided_kernel<true, false><<<(unsigned)blocks, 256, 0, ctx->stream>>>(out, a, b, m, total, op);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, strided_kernel<true, false>, out, a, b, m, total, op));
     return after_launch(ctx, "binary_strided_f32");
 }
 int gcb_copy_strided_f32(gcb_ctx* ctx, int ndim, const int64_t* shape, float* out, const int64_t* so, const float* in, const int64_t* si, int accumulate) {
@@ -379,8 +395,8 @@ int gcb_copy_strided_f32(gcb_ctx* ctx, int ndim, const int64_t* shape, float* ou
     int64_t blocks = std::min<int64_t>((total + 255) / 256, kSMs * 8);
     if (ctx->twins_lo != nullptr) ctx->twins_dirty = true;  // strided destination: see gcb_binary_strided_f32
     cudaSetDevice(ctx->device);
-    if (accumulate) strided_kernel<false, true><<<(unsigned)blocks, 256, 0, ctx->stream>>>(out, in, nullptr, m, total, 0);
-    else strided_kernel<false, false><<<(unsigned)blocks, 256, 0, ctx->stream>>>(out, in, nullptr, m, total, 0);
+    if (accumulate) GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, strided_kernel<false, true>, out, in, nullptr, m, total, 0));
+    else GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, strided_kernel<false, false>, out, in, nullptr, m, total, 0));
     return after_launch(ctx, "copy_strided_f32");
 }
 
@@ -401,11 +417,11 @@ int gcb_reduce_rows_f32(gcb_ctx* ctx, float* out, const float* in, int64_t rows,
     int rc = sc.get(sizeof(float) * slabs * cols);
     if (rc) return rc;
     dim3 grid((unsigned)col_tiles, (unsigned)slabs);
-    if (v4) reduce_rows_stage1<4><<<grid, 256, 0, ctx->stream>>>(sc.as<float>(), in, rows, cols, rows_per_slab);
-    else reduce_rows_stage1<1><<<grid, 256, 0, ctx->stream>>>(sc.as<float>(), in, rows, cols, rows_per_slab);
+    if (v4) GCB_CHECK_CUDA(launch_next(ctx->stream, grid, 256, 0, reduce_rows_stage1<4>, sc.as<float>(), in, rows, cols, rows_per_slab));
+    else GCB_CHECK_CUDA(launch_next(ctx->stream, grid, 256, 0, reduce_rows_stage1<1>, sc.as<float>(), in, rows, cols, rows_per_slab));
     rc = after_launch(ctx, "reduce_rows_stage1");
     if (rc) return rc;
-    reduce_rows_stage2<<<(unsigned)((cols + 255) / 256), 256, 0, ctx->stream>>>(out, sc.as<float>(), slabs, cols, accumulate);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)((cols + 255) / 256), 256, 0, reduce_rows_stage2, out, sc.as<float>(), slabs, cols, accumulate));
     return after_launch(ctx, "reduce_rows_stage2");
 }
 
@@ -418,7 +434,7 @@ int gcb_sum_squares_f32(gcb_ctx* ctx, float* out, const float* in, int64_t n, in
     Scratch sc(ctx);
     int rc = sc.get(sizeof(float) * blocks);
     if (rc) return rc;
-    sum_squares_stage1<<<blocks, 512, 0, ctx->stream>>>(sc.as<float>(), in, n, n4);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 512, 0, sum_squares_stage1, sc.as<float>(), in, n, n4));
     rc = after_launch(ctx, "sum_squares_stage1");
     if (rc) return rc;
     return launch_sum_partials(ctx, out, sc.as<float>(), blocks, accumulate, 1.0f);
@@ -481,7 +497,7 @@ int gcb_adamw_arena_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float*
     int64_t blocks = std::min<int64_t>(chunks, kSMs * 8);
     cudaSetDevice(ctx->device);
     note_write(ctx, w, sizeof(float) * (size_t)n);
-    adamw_arena_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(w, m, v, g, mask, n, chunks, make_adamw(lr, b1, b2, b1p, b2p, wd, eps, gscale));
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, adamw_arena_kernel, w, m, v, g, mask, n, chunks, make_adamw(lr, b1, b2, b1p, b2p, wd, eps, gscale)));
     return after_launch(ctx, "adamw_arena");
 }
 

@@ -18,32 +18,14 @@
 
 namespace gcb {
 
-// The launches of a scatter-add depend on one another and are short (3 - 30 us): each kernel is launched with programmatic
-// stream serialisation, lets its successor be scheduled right away (pdl_trigger) and touches global memory only after its
-// predecessor has completed and its writes are visible (pdl_wait).
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <class... KArgs, class... Args>
-static cudaError_t launch_chained(cudaStream_t stream, unsigned grid, unsigned block, size_t smem, void (*kernel)(KArgs...), Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(block, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 constexpr int kChunk = 1024;  // positions per placement CTA
 constexpr int kSeg = 32;      // hits per accumulation segment
 
 template <class IdxT>
 __global__ void __launch_bounds__(256) embed_gather_kernel(float* __restrict__ out, const IdxT* __restrict__ idx, const float* __restrict__ table, int64_t n, int64_t width,
                                                            int64_t vocab, int vec, int* __restrict__ status) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), nwarps = (int64_t)gridDim.x * 8;
     for (int64_t i = warp; i < n; i += nwarps) {
@@ -396,7 +378,7 @@ static int build_plan(gcb_ctx* ctx, Scratch& sc, ScatterPlan& p, const IdxT* idx
     p.parked = b_park ? (float*)base : nullptr;
     GCB_CHECK_CUDA(cudaMemsetAsync(p.blk, 0, b_blk, ctx->stream));
     // the first kernel follows a memset, not a kernel: launched the ordinary way (its pdl_wait is then a no-op)
-    scatter_hist_kernel<IdxT><<<(unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)kSMs * 8), 256, 0, ctx->stream>>>(p.blk, idx, n, vocab, ctx->d_status);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)kSMs * 8), 256, 0, scatter_hist_kernel<IdxT>, p.blk, idx, n, vocab, ctx->d_status));
     rc = after_launch(ctx, "scatter_hist"); if (rc) return rc;
     GCB_CHECK_CUDA(launch_chained(ctx->stream, (unsigned)n_blocks, 256, 0, scatter_colsum_kernel, p.blk, p.counts, p.blocktot, p.n_chunks, vocab));
     rc = after_launch(ctx, "scatter_colsum"); if (rc) return rc;
@@ -443,8 +425,8 @@ int gcb_embed_f32(gcb_ctx* ctx, float* out, const void* indices, int index_type,
     cudaSetDevice(ctx->device);
     const int vec = width % 4 == 0 && aligned16(out) && aligned16(table);
     const unsigned blocks = (unsigned)std::min<int64_t>((n + 7) / 8, (int64_t)kSMs * 8);
-    if (index_type == GCB_IDX_I64) embed_gather_kernel<int64_t><<<blocks, 256, 0, ctx->stream>>>(out, (const int64_t*)indices, table, n, width, vocab, vec, ctx->d_status);
-    else embed_gather_kernel<int32_t><<<blocks, 256, 0, ctx->stream>>>(out, (const int32_t*)indices, table, n, width, vocab, vec, ctx->d_status);
+    if (index_type == GCB_IDX_I64) GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 256, 0, embed_gather_kernel<int64_t>, out, (const int64_t*)indices, table, n, width, vocab, vec, ctx->d_status));
+    else GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 256, 0, embed_gather_kernel<int32_t>, out, (const int32_t*)indices, table, n, width, vocab, vec, ctx->d_status));
     return after_launch(ctx, "embed_gather");
 }
 

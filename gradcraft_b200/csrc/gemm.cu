@@ -18,6 +18,8 @@ namespace gcb {
 // threads neighbouring elements, because neither side's rows need start on a 16-byte boundary.
 __global__ void __launch_bounds__(256) pack_rows_kernel(float* __restrict__ out, const float* __restrict__ in, int64_t rows, int64_t cols, int64_t ld, int64_t so, int64_t si, int64_t n_inner,
                                                         int64_t total_rows, int64_t pitch) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t c0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
     for (int64_t r = blockIdx.y; r < total_rows; r += gridDim.y) {
         const int64_t item = r / rows, row = r - item * rows, bo = item / n_inner, bi = item - bo * n_inner;
@@ -43,7 +45,7 @@ struct PackedOperand {
         int rc = sc.get(sizeof(float) * (size_t)(total_rows * pitch));
         if (rc) return rc;
         dim3 grid((unsigned)((cols + 1023) / 1024), (unsigned)std::min<int64_t>(total_rows, 65535), 1);
-        pack_rows_kernel<<<grid, 256, 0, ctx->stream>>>(sc.as<float>(), *p, rows, cols, *ld, *so, *si, n_inner, total_rows, pitch);
+        GCB_CHECK_CUDA(launch_chained(ctx->stream, grid, 256, 0, pack_rows_kernel, sc.as<float>(), *p, rows, cols, *ld, *so, *si, n_inner, total_rows, pitch));
         *p = sc.as<float>();
         *ld = pitch;
         *si = rows * pitch;

@@ -71,6 +71,8 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
     using S = SgSmem<BM>;
     constexpr int KG = S::KG, TPR = BM / 4, GT = TPR * TPR;  // threads along an edge of the tile, threads of a K group
     extern __shared__ __align__(16) float sg[];
+    pdl_trigger();
+    pdl_wait();
     const int t = threadIdx.x, rank = (int)(blockIdx.x % (unsigned)slices);
     int64_t w = blockIdx.x / (unsigned)slices;
     const int64_t bz = w / ((int64_t)tiles_m * tiles_n);
@@ -250,12 +252,14 @@ static int sg_launch(gcb_ctx* ctx, const GemmArgs& g, int64_t tiles_m, int64_t t
     cfg.blockDim = dim3(SG_THREADS, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)slices;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)slices;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = slices > 1 ? 2 : 1;
     GCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kfn, g, (int)tiles_m, (int)tiles_n, slices, vec(g.A, g.lda, g.a_so, g.a_si), vec(g.B, g.ldb, g.b_so, g.b_si), c_vec));
     return GCB_OK;
 }

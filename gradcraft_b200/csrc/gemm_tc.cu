@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot_gen;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // a split-K reduction behind this grid may be scheduled while it drains; it still waits for the grid to complete
+    pdl_trigger();
+    pdl_wait();  // everything above passes behind the predecessor's tail
 
     if (warp == 0) {
         // ---------------- producer ----------------
@@ -926,9 +927,10 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_sync_all();  // both CTAs' barriers are initialised before anyone arrives on a remote one
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // a split-K reduction behind this grid may be scheduled while it drains; it still waits for the grid to complete
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot_gen;
+    pdl_trigger();
+    pdl_wait();  // everything above passes behind the predecessor's tail
 
     if (warp == 0) {
         // ---------------- producer (each CTA: its 128 rows of A, its 128 columns of B) ----------------
@@ -1202,7 +1204,8 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ C, const float* __restrict__ partial, int64_t partial_ld, const float* __restrict__ bias, int64_t M, int64_t N,
                                                             int64_t ldc, int splits, float alpha, float beta, float* __restrict__ colsum, const float* __restrict__ colsum_partial,
                                                             int colsum_accumulate, int vec) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_trigger();
+    pdl_wait();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
     if (colsum != nullptr) {  // the column sums of op(B), one partial per K slice
         for (int64_t n = tid; n < N; n += nthreads) {
@@ -1314,7 +1317,7 @@ static int launch_bn(gcb_ctx* ctx, bool ta, bool tb, const CUtensorMap& ma, cons
         auto kfn = gemm_tc_kernel<BN, AM, BMN, A_TM>;                                                                     \
         static bool attr_done[kMaxDevices] = {}; /* function attributes belong to a device, not to the process */       \
         if (!attr_done[ctx->device]) { GCB_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr_done[ctx->device] = true; } \
-        kfn<<<grid, TcSmem<BN, A_TM>::THREADS, smem, ctx->stream>>>(ma, mb, mc, mp, p);                                                  \
+        GCB_CHECK_CUDA(launch_chained(ctx->stream, grid, TcSmem<BN, A_TM>::THREADS, smem, kfn, ma, mb, mc, mp, p));                                                  \
     } while (0)
     // A "transposed" (stored K x M) is MN-major; B "normal" (stored K x N) is MN-major
     if (ta && !tb) GCB_TC(true, true);
@@ -1341,13 +1344,15 @@ static int launch_pair(gcb_ctx* ctx, bool ta, bool tb, const CUtensorMap& ma, co
     cfg.blockDim = dim3(PairSmemT<A_TM>::THREADS, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
 #define GCB_PAIR(AM, BMN)                                                                                                   \
     do {                                                                                                                    \
         auto kfn = gemm_tc_pair_kernel<AM, BMN, A_TM>;                                                                            \
@@ -1509,17 +1514,8 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     if (splits > 1) {
         const int vec = (g.N % 4 == 0 && g.ldc % 4 == 0 && aligned16(g.C)) ? 1 : 0;
         const int64_t units = g.M * p.partial_ld / 4;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)std::min<int64_t>((units + 255) / 256, (int64_t)kSMs * 8), 1, 1);
-        cfg.blockDim = dim3(256, 1, 1);
-        cfg.stream = ctx->stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        GCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, splitk_reduce_kernel, g.C, (const float*)p.partial, p.partial_ld, g.bias, g.M, g.N, g.ldc, splits, g.alpha, g.beta, g.colsum, (const float*)p.colsum_partial,
-                                          g.colsum_accumulate, vec));
+        GCB_CHECK_CUDA(launch_chained(ctx->stream, (unsigned)std::min<int64_t>((units + 255) / 256, (int64_t)kSMs * 8), 256, 0, splitk_reduce_kernel, g.C, (const float*)p.partial, p.partial_ld, g.bias, g.M, g.N, g.ldc,
+                                      splits, g.alpha, g.beta, g.colsum, (const float*)p.colsum_partial, g.colsum_accumulate, vec));
         rc = after_launch(ctx, "splitk_reduce");
         if (rc) return rc;
     }

@@ -20,6 +20,8 @@ constexpr int kNormWarps = 4;  // warps per CTA on the fast path
 template <int NCHUNK, bool IS_LN>
 __global__ void __launch_bounds__(kNormWarps * 32) norm_fwd_warp(float* __restrict__ y, float* __restrict__ stat0, float* __restrict__ stat1, const float* __restrict__ x,
                                                                  const float* __restrict__ gamma, const float* __restrict__ beta, int64_t rows, int cols, float eps) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * kNormWarps + (threadIdx.x >> 5);
     const int64_t nwarps = (int64_t)gridDim.x * kNormWarps;
@@ -80,7 +82,8 @@ template <int NCHUNK, bool IS_LN>
 __global__ void __launch_bounds__(kNormWarps * 32) norm_bwd_warp(float* __restrict__ dx, float* __restrict__ partial, const float* __restrict__ dy, const float* __restrict__ x,
                                                                  const float* __restrict__ gamma, const float* __restrict__ stat0, const float* __restrict__ stat1,
                                                                  int64_t rows, int cols, int acc_dx, int want_params) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the second stage (if any) may be scheduled while this grid drains; it still waits for this grid to complete
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ float sm[];  // [kNormWarps][2][cols]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t warp = (int64_t)blockIdx.x * kNormWarps + wid;
@@ -180,7 +183,8 @@ template <int NCHUNK, bool IS_LN>
 __global__ void __launch_bounds__(kRingWarps * 32, 1) norm_bwd_ring(float* __restrict__ dx, float* __restrict__ partial, const float* __restrict__ dy, const float* __restrict__ x,
                                                                     const float* __restrict__ gamma, const float* __restrict__ stat0, const float* __restrict__ stat1, int64_t rows, int cols,
                                                                     int acc_dx, int want_params, int* __restrict__ status) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the second stage (if any) may be scheduled while this grid drains; it still waits for this grid to complete
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ __align__(128) uint8_t ring_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t row_bytes = (uint32_t)cols * 4u;
@@ -292,11 +296,10 @@ __global__ void __launch_bounds__(kRingWarps * 32, 1) norm_bwd_ring(float* __res
 // adds its own in ascending row order, and the 32 lane sums are combined by a shuffle tree — the same tree for every
 // launch, so the result is deterministic.
 __global__ void __launch_bounds__(256) norm_params_stage2(float* __restrict__ dgamma, float* __restrict__ dbeta, const float* __restrict__ partial, int nparts, int cols, int accumulate) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5);  // over 2 * cols
-    // launched with programmatic stream serialisation: this grid may start while the kernel that writes `partial` drains;
-    // nothing of it is read before that kernel has completed and its writes are visible
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (i >= 2 * cols) return;
     const float* p = partial + i;
     const size_t stride = (size_t)2 * cols;
@@ -318,25 +321,16 @@ __global__ void __launch_bounds__(256) norm_params_stage2(float* __restrict__ dg
     }
 }
 
-// Launches the second stage so that its blocks are scheduled while the first stage's last blocks finish (the gap between
-// two dependent launches is a tenth of this backward at 16k x 1k).
 static cudaError_t launch_params_stage2(cudaStream_t stream, float* dgamma, float* dbeta, const float* partial, int nparts, int cols, int accumulate) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((2 * cols + 7) / 8), 1, 1);
-    cfg.blockDim = dim3(256, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, norm_params_stage2, dgamma, dbeta, partial, nparts, cols, accumulate);
+    return launch_chained(stream, (unsigned)((2 * cols + 7) / 8), 256, 0, norm_params_stage2, dgamma, dbeta, partial, nparts, cols, accumulate);
 }
 
 // ---- generic shapes: CTA per row ---------------------------------------------------------------
 template <bool IS_LN>
 __global__ void __launch_bounds__(256) norm_fwd_block(float* __restrict__ y, float* __restrict__ stat0, float* __restrict__ stat1, const float* __restrict__ x,
                                                       const float* __restrict__ gamma, const float* __restrict__ beta, int64_t rows, int64_t cols, float eps) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red[33];
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const float* xr = x + r * cols;
@@ -364,6 +358,8 @@ __global__ void __launch_bounds__(256) norm_fwd_block(float* __restrict__ y, flo
 template <bool IS_LN>
 __global__ void __launch_bounds__(256) norm_bwd_dx_block(float* __restrict__ dx, const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ gamma,
                                                          const float* __restrict__ stat0, const float* __restrict__ stat1, int64_t rows, int64_t cols, int acc_dx) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red[33];
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const float mu = IS_LN ? stat0[r] : 0.0f, rs = IS_LN ? stat1[r] : stat0[r];
@@ -387,6 +383,8 @@ __global__ void __launch_bounds__(256) norm_bwd_dx_block(float* __restrict__ dx,
 template <bool IS_LN>
 __global__ void __launch_bounds__(256) norm_bwd_params_block(float* __restrict__ partial, const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ stat0,
                                                              const float* __restrict__ stat1, int64_t rows, int64_t cols, int64_t rows_per_slab) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float sg[8][33], sb[8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t c = (int64_t)blockIdx.x * 32 + tx;
@@ -427,12 +425,12 @@ static int norm_fwd(gcb_ctx* ctx, float* y, float* s0, float* s1, const float* x
     if (fast) {
         int64_t blocks = std::min<int64_t>((rows + kNormWarps - 1) / kNormWarps, (int64_t)kSMs * 8);
         const int n = pick_chunks(cols);
-#define GCB_FWD(N) norm_fwd_warp<N, IS_LN><<<(unsigned)blocks, kNormWarps * 32, 0, ctx->stream>>>(y, s0, s1, x, gamma, beta, rows, (int)cols, eps)
+#define GCB_FWD(N) GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, kNormWarps * 32, 0, norm_fwd_warp<N, IS_LN>, y, s0, s1, x, gamma, beta, rows, (int)cols, eps))
         if (n == 1) GCB_FWD(1); else if (n == 2) GCB_FWD(2); else if (n == 4) GCB_FWD(4); else if (n == 6) GCB_FWD(6); else GCB_FWD(8);
 #undef GCB_FWD
     } else {
         int64_t blocks = std::min<int64_t>(rows, (int64_t)kSMs * 8);
-        norm_fwd_block<IS_LN><<<(unsigned)blocks, 256, 0, ctx->stream>>>(y, s0, s1, x, gamma, beta, rows, cols, eps);
+        GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, norm_fwd_block<IS_LN>, y, s0, s1, x, gamma, beta, rows, cols, eps));
     }
     return after_launch(ctx, IS_LN ? "layernorm_fwd" : "rmsnorm_fwd");
 }
@@ -465,7 +463,7 @@ static int norm_bwd(gcb_ctx* ctx, float* dx, float* dgamma, float* dbeta, const 
             auto kfn = norm_bwd_ring<N, IS_LN>;                                                                                                          \
             static bool attr_done[kMaxDevices] = {}; /* function attributes belong to a device */                                                        \
             if (!attr_done[ctx->device]) { GCB_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); attr_done[ctx->device] = true; } \
-            kfn<<<(unsigned)blocks, kRingWarps * 32, smem, ctx->stream>>>(dx, sc.as<float>(), dy, x, gamma, s0, s1, rows, (int)cols, acc_dx, want_params ? 1 : 0, ctx->d_status); \
+            GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, kRingWarps * 32, smem, kfn, dx, sc.as<float>(), dy, x, gamma, s0, s1, rows, (int)cols, acc_dx, want_params ? 1 : 0, ctx->d_status)); \
         } while (0)
         if (n == 1) GCB_RING(1); else if (n == 2) GCB_RING(2); else if (n == 4) GCB_RING(4); else if (n == 6) GCB_RING(6); else GCB_RING(8);
 #undef GCB_RING
@@ -485,7 +483,7 @@ static int norm_bwd(gcb_ctx* ctx, float* dx, float* dgamma, float* dbeta, const 
         if (want_params) { int rc = sc.get(sizeof(float) * blocks * 2 * cols); if (rc) return rc; }
         const size_t smem = want_params ? sizeof(float) * kNormWarps * 2 * cols : 0;
         const int n = pick_chunks(cols);
-#define GCB_BWD(N) norm_bwd_warp<N, IS_LN><<<(unsigned)blocks, kNormWarps * 32, smem, ctx->stream>>>(dx, sc.as<float>(), dy, x, gamma, s0, s1, rows, (int)cols, acc_dx, want_params ? 1 : 0)
+#define GCB_BWD(N) GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, kNormWarps * 32, smem, norm_bwd_warp<N, IS_LN>, dx, sc.as<float>(), dy, x, gamma, s0, s1, rows, (int)cols, acc_dx, want_params ? 1 : 0))
         if (n == 1) GCB_BWD(1); else if (n == 2) GCB_BWD(2); else if (n == 4) GCB_BWD(4); else if (n == 6) GCB_BWD(6); else GCB_BWD(8);
 #undef GCB_BWD
         int rc = after_launch(ctx, name);
@@ -498,7 +496,7 @@ static int norm_bwd(gcb_ctx* ctx, float* dx, float* dgamma, float* dbeta, const 
     }
     if (dx) {
         int64_t blocks = std::min<int64_t>(rows, (int64_t)kSMs * 8);
-        norm_bwd_dx_block<IS_LN><<<(unsigned)blocks, 256, 0, ctx->stream>>>(dx, dy, x, gamma, s0, s1, rows, cols, acc_dx);
+        GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, norm_bwd_dx_block<IS_LN>, dx, dy, x, gamma, s0, s1, rows, cols, acc_dx));
         int rc = after_launch(ctx, name);
         if (rc) return rc;
     }
@@ -512,7 +510,7 @@ static int norm_bwd(gcb_ctx* ctx, float* dx, float* dgamma, float* dbeta, const 
         int rc = sc.get(sizeof(float) * slabs * 2 * cols);
         if (rc) return rc;
         dim3 grid((unsigned)col_tiles, (unsigned)slabs);
-        norm_bwd_params_block<IS_LN><<<grid, 256, 0, ctx->stream>>>(sc.as<float>(), dy, x, s0, s1, rows, cols, rps);
+        GCB_CHECK_CUDA(launch_next(ctx->stream, grid, 256, 0, norm_bwd_params_block<IS_LN>, sc.as<float>(), dy, x, s0, s1, rows, cols, rps));
         rc = after_launch(ctx, name);
         if (rc) return rc;
         GCB_CHECK_CUDA(launch_params_stage2(ctx->stream, dgamma, dbeta, sc.as<float>(), (int)slabs, (int)cols, acc_params));
@@ -582,7 +580,7 @@ int gcb_layernorm_bwd_noalloc_f32(gcb_ctx* ctx, float* dx, float* dgamma, float*
     const int n = pick_chunks(cols);
     // Stage 1 overwrites the first `blocks` partial rows completely before stage 2 reads exactly those rows, so nothing
     // left over from an earlier call can leak into this one and nothing has to be cleared.
-#define GCB_BWD(N) norm_bwd_warp<N, true><<<(unsigned)blocks, kNormWarps * 32, smem, ctx->stream>>>(dx, scratch, dy, x, gamma, mean, rstd, rows, (int)cols, acc_dx, want_params ? 1 : 0)
+#define GCB_BWD(N) GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, kNormWarps * 32, smem, norm_bwd_warp<N, true>, dx, scratch, dy, x, gamma, mean, rstd, rows, (int)cols, acc_dx, want_params ? 1 : 0))
     if (n == 1) GCB_BWD(1); else if (n == 2) GCB_BWD(2); else if (n == 4) GCB_BWD(4); else if (n == 6) GCB_BWD(6); else GCB_BWD(8);
 #undef GCB_BWD
     rc = after_launch(ctx, "layernorm_bwd_noalloc");

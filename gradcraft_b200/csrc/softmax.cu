@@ -17,6 +17,8 @@ constexpr int kSmWarps = 8;
 
 template <int NCHUNK>
 __global__ void __launch_bounds__(kSmWarps * 32) causal_softmax_fwd_warp(float* __restrict__ probs, const float* __restrict__ scores, float scale, int64_t rows, int T, int64_t ld, int band) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * kSmWarps + (threadIdx.x >> 5);
     const int64_t nwarps = (int64_t)gridDim.x * kSmWarps;
@@ -61,6 +63,8 @@ __global__ void __launch_bounds__(kSmWarps * 32) causal_softmax_fwd_warp(float* 
 template <int NCHUNK>
 __global__ void __launch_bounds__(kSmWarps * 32, (NCHUNK == 8 ? 3 : 4)) causal_softmax_bwd_warp(float* __restrict__ ds, const float* __restrict__ dp, const float* __restrict__ probs, float scale,
                                                                          int64_t rows, int T, int accumulate, int band) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * kSmWarps + (threadIdx.x >> 5);
     const int64_t nwarps = (int64_t)gridDim.x * kSmWarps;
@@ -107,6 +111,8 @@ __global__ void __launch_bounds__(kSmWarps * 32, (NCHUNK == 8 ? 3 : 4)) causal_s
 
 // generic sequence lengths: CTA per row, scalar accesses
 __global__ void __launch_bounds__(256) causal_softmax_fwd_block(float* __restrict__ probs, const float* __restrict__ scores, float scale, int64_t rows, int64_t T, int64_t ld) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red[33];
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const int64_t i = r % T;
@@ -122,6 +128,8 @@ __global__ void __launch_bounds__(256) causal_softmax_fwd_block(float* __restric
     }
 }
 __global__ void __launch_bounds__(256) causal_softmax_bwd_block(float* __restrict__ ds, const float* __restrict__ dp, const float* __restrict__ probs, float scale, int64_t rows, int64_t T, int accumulate) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red[33];
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const int64_t i = r % T;
@@ -139,6 +147,8 @@ __global__ void __launch_bounds__(256) causal_softmax_bwd_block(float* __restric
 template <class IdxT>
 __global__ void __launch_bounds__(512, 2) softmax_ce_fwd_kernel(float* __restrict__ row_loss, float* __restrict__ probs, const float* __restrict__ logits, const IdxT* __restrict__ targets,
                                                                int64_t rows, int64_t V, int64_t V4, float eps, int* __restrict__ status) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float red[33];
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const float* zr = logits + r * V;
@@ -176,6 +186,8 @@ __global__ void __launch_bounds__(512, 2) softmax_ce_fwd_kernel(float* __restric
 template <class IdxT>
 __global__ void __launch_bounds__(256) softmax_ce_bwd_kernel(float* __restrict__ dx, const float* __restrict__ probs, const IdxT* __restrict__ targets, float s,
                                                             int64_t rows, int64_t V, int64_t V4, int accumulate, int* __restrict__ status) {
+    pdl_trigger();
+    pdl_wait();
     constexpr int U = 4;
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
         const float* pr = probs + r * V;
@@ -227,6 +239,8 @@ using namespace gcb;
 template <int LPR>
 __global__ void __launch_bounds__(256) rowdot_kernel(float* __restrict__ out, const float* __restrict__ a, int64_t lda, int64_t a_so, int64_t a_si, const float* __restrict__ b, int64_t ldb,
                                                      int64_t b_so, int64_t b_si, int64_t rows, int cols, int64_t n_inner, int64_t total_rows, int vec_ok) {
+    pdl_trigger();
+    pdl_wait();
     const int sub = threadIdx.x % LPR;
     const int64_t groups_per_block = blockDim.x / LPR;
     for (int64_t base = (int64_t)blockIdx.x * groups_per_block; base < total_rows; base += (int64_t)gridDim.x * groups_per_block) {  // block-uniform trip count: the shuffles below need whole warps
@@ -263,11 +277,11 @@ static int csm_fwd(gcb_ctx* ctx, float* probs, const float* scores, float scale,
     if (ld % 4 == 0 && T <= 1024 && aligned16(probs) && aligned16(scores)) {  // the last chunk of a row may reach into the padding between T and ld, never beyond
         int64_t blocks = std::min<int64_t>((rows + kSmWarps - 1) / kSmWarps, (int64_t)kSMs * 8);
         const int n = chunks_for(T);
-#define GCB_L(N) causal_softmax_fwd_warp<N><<<(unsigned)blocks, kSmWarps * 32, 0, ctx->stream>>>(probs, scores, scale, rows, (int)T, ld, band)
+#define GCB_L(N) GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, kSmWarps * 32, 0, causal_softmax_fwd_warp<N>, probs, scores, scale, rows, (int)T, ld, band))
         if (n == 1) GCB_L(1); else if (n == 2) GCB_L(2); else if (n == 4) GCB_L(4); else GCB_L(8);
 #undef GCB_L
     } else {
-        causal_softmax_fwd_block<<<(unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 8), 256, 0, ctx->stream>>>(probs, scores, scale, rows, T, ld);
+        GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 8), 256, 0, causal_softmax_fwd_block, probs, scores, scale, rows, T, ld));
     }
     return after_launch(ctx, "causal_softmax_fwd");
 }
@@ -290,11 +304,11 @@ static int csm_bwd(gcb_ctx* ctx, float* ds, const float* dp, const float* probs,
     if (T % 4 == 0 && T <= 1024 && aligned16(ds) && aligned16(dp) && aligned16(probs)) {
         int64_t blocks = std::min<int64_t>((rows + kSmWarps - 1) / kSmWarps, (int64_t)kSMs * 8);
         const int n = chunks_for(T);
-#define GCB_L(N) causal_softmax_bwd_warp<N><<<(unsigned)blocks, kSmWarps * 32, 0, ctx->stream>>>(ds, dp, probs, scale, rows, (int)T, accumulate, band)
+#define GCB_L(N) GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, kSmWarps * 32, 0, causal_softmax_bwd_warp<N>, ds, dp, probs, scale, rows, (int)T, accumulate, band))
         if (n == 1) GCB_L(1); else if (n == 2) GCB_L(2); else if (n == 4) GCB_L(4); else GCB_L(8);
 #undef GCB_L
     } else {
-        causal_softmax_bwd_block<<<(unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 8), 256, 0, ctx->stream>>>(ds, dp, probs, scale, rows, T, accumulate);
+        GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 8), 256, 0, causal_softmax_bwd_block, ds, dp, probs, scale, rows, T, accumulate));
     }
     return after_launch(ctx, "causal_softmax_bwd");
 }
@@ -320,7 +334,7 @@ int gcb_rowdot_batched_f32(gcb_ctx* ctx, float* out, const float* a, int64_t lda
     const int lpr = cols <= 32 ? 8 : (cols <= 64 ? 16 : 32);
     const int64_t groups = 256 / lpr;
     const unsigned blocks = (unsigned)std::min<int64_t>((total_rows + groups - 1) / groups, (int64_t)kSMs * 16);
-#define GCB_L(L) rowdot_kernel<L><<<blocks, 256, 0, ctx->stream>>>(out, a, lda, a_so, a_si, b, ldb, b_so, b_si, rows, (int)cols, batch_inner, total_rows, vec_ok)
+#define GCB_L(L) GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 256, 0, rowdot_kernel<L>, out, a, lda, a_so, a_si, b, ldb, b_so, b_si, rows, (int)cols, batch_inner, total_rows, vec_ok))
     if (lpr == 8) GCB_L(8); else if (lpr == 16) GCB_L(16); else GCB_L(32);
 #undef GCB_L
     return after_launch(ctx, "rowdot");
@@ -337,8 +351,8 @@ int gcb_softmax_ce_fwd_f32(gcb_ctx* ctx, float* loss, float* probs, const float*
     if (rc) return rc;
     // 2 CTAs per SM: with 128 KB rows that keeps ~38 MB of rows in flight, well inside L2 for the second pass
     unsigned blocks = (unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 2);
-    if (index_type == GCB_IDX_I64) softmax_ce_fwd_kernel<int64_t><<<blocks, 512, 0, ctx->stream>>>(sc.as<float>(), probs, logits, (const int64_t*)targets, rows, V, V4, eps, ctx->d_status);
-    else softmax_ce_fwd_kernel<int32_t><<<blocks, 512, 0, ctx->stream>>>(sc.as<float>(), probs, logits, (const int32_t*)targets, rows, V, V4, eps, ctx->d_status);
+    if (index_type == GCB_IDX_I64) GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 512, 0, softmax_ce_fwd_kernel<int64_t>, sc.as<float>(), probs, logits, (const int64_t*)targets, rows, V, V4, eps, ctx->d_status));
+    else GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 512, 0, softmax_ce_fwd_kernel<int32_t>, sc.as<float>(), probs, logits, (const int32_t*)targets, rows, V, V4, eps, ctx->d_status));
     rc = after_launch(ctx, "softmax_ce_fwd");
     if (rc) return rc;
     return launch_sum_partials(ctx, loss, sc.as<float>(), (int)rows, 0, 1.0f / (float)rows);
@@ -352,8 +366,8 @@ int gcb_softmax_ce_bwd_f32(gcb_ctx* ctx, float* dx, const float* probs, const vo
     const int64_t V4 = (V % 4 == 0 && aligned16(probs) && aligned16(dx)) ? V / 4 : 0;
     const float s = upstream / (float)rows;
     unsigned blocks = (unsigned)std::min<int64_t>(rows, (int64_t)kSMs * 8);
-    if (index_type == GCB_IDX_I64) softmax_ce_bwd_kernel<int64_t><<<blocks, 256, 0, ctx->stream>>>(dx, probs, (const int64_t*)targets, s, rows, V, V4, accumulate, ctx->d_status);
-    else softmax_ce_bwd_kernel<int32_t><<<blocks, 256, 0, ctx->stream>>>(dx, probs, (const int32_t*)targets, s, rows, V, V4, accumulate, ctx->d_status);
+    if (index_type == GCB_IDX_I64) GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 256, 0, softmax_ce_bwd_kernel<int64_t>, dx, probs, (const int64_t*)targets, s, rows, V, V4, accumulate, ctx->d_status));
+    else GCB_CHECK_CUDA(launch_next(ctx->stream, blocks, 256, 0, softmax_ce_bwd_kernel<int32_t>, dx, probs, (const int32_t*)targets, s, rows, V, V4, accumulate, ctx->d_status));
     return after_launch(ctx, "softmax_ce_bwd");
 }
 

@@ -38,6 +38,8 @@ struct TwinJob {
 // out layout (bf16): [which = big, small][n_group = ceil(N / 8)][k_chunk = Kp / 8][n % 8][k % 8], Kp = K rounded up to 16.
 // kn != 0: W is stored K x N (element (k, n) at W[k * ld + n]); kn == 0: stored N x K (element (k, n) at W[n * ld + k]).
 __global__ void __launch_bounds__(256) presplit_kernel(const TwinJob* __restrict__ jobs, int n_jobs, int64_t total) {
+    pdl_trigger();
+    pdl_wait();
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
         int lo = 0, hi = n_jobs;  // last job with first <= g
         while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (jobs[mid].first <= g) lo = mid; else hi = mid; }
@@ -98,7 +100,7 @@ int twins_refresh(gcb_ctx* ctx) {
         ctx->twin_jobs_total = total;
         ctx->twin_jobs_stale = false;
     }
-    presplit_kernel<<<(unsigned)std::min<int64_t>((ctx->twin_jobs_total + 255) / 256, (int64_t)kSMs * 16), 256, 0, ctx->stream>>>((const TwinJob*)ctx->twin_jobs, n_jobs, ctx->twin_jobs_total);
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)std::min<int64_t>((ctx->twin_jobs_total + 255) / 256, (int64_t)kSMs * 16), 256, 0, presplit_kernel, (const TwinJob*)ctx->twin_jobs, n_jobs, ctx->twin_jobs_total));
     int rc = after_launch(ctx, "presplit_weight");
     if (rc) return rc;
     ctx->twins_dirty = false;
