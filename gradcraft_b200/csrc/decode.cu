@@ -35,6 +35,7 @@ constexpr int kDecBox = 256;                              // weight rows one cop
 constexpr int kDecRows = 1024, kDecStage = kDecRows * 8;  // weight rows and floats of a ring stage: waiting for a stage and handing it back costs ~200 cycles however many rows it has
 constexpr int kDecMaxStages = 6, kDecMinStages = 2;
 constexpr int kDecSplit = 128;  // positions from which a second unit pays for one head
+constexpr int kDecMeet = 4;    // tiles whose sums are finished together (even: a gated tile has two)
 constexpr int kDecMaps = 7;    // tensor maps per layer: wq, wk, wv, wo, w1, w2, w3
 
 struct DecodeParams {
@@ -91,7 +92,7 @@ __device__ __forceinline__ bool get_words(const unsigned long long* w, Index&& i
         for (int u = 0; u < B; ++u) v[u] = index(u) >= 0 ? look_word(w + index(u)) : (unsigned long long)epoch << 32;
 #pragma unroll
         for (int u = 0; u < B; ++u) { all = all && (unsigned)(v[u] >> 32) == epoch; out[u] = __uint_as_float((unsigned)v[u]); }
-        if (all) return true;
+        if (__all_sync(__activemask(), all)) return true;  // together, or what follows would be run once per straggler
     }
     atomicExch(&status[0], 1);
     atomicExch(&status[1], 120);
@@ -174,7 +175,7 @@ __device__ __forceinline__ int sum_rows(float (&v)[NV]) {
 template <int S>
 struct DecSmem {
     // floats: ring [stages][kDecStage], x [S][C], activations [max(C, F)][S] (the head: [S][C]), then the fixed part
-    static constexpr int RED = 2 * kDecWarps * S * 8;                                         // two buffers of warp sums
+    static constexpr int RED = 2 * kDecMeet * kDecWarps * S * 8;                              // two buffers of warp sums
     static constexpr int ATT = kDecWarps * (kDecMaxHead + 4) + 3 * kDecMaxHead;               // a warp's stretch: sum of values, maximum, sum of weights; q, k, v of this position
     static constexpr int FIXED = RED + ATT + 2 * kDecWarps * S + 2 * kDecWarps * S + 8 + 4 + 4 * kDecMaxStages;  // + two sets of warp sums, best logits, tokens, flag, barriers
     static size_t bytes(int stages, int64_t C, int64_t F) { return 128 + sizeof(float) * (size_t)(stages * kDecStage + (S * C + 3) / 4 * 4 + (S * std::max(C, F) + 3) / 4 * 4 + FIXED); }
@@ -233,7 +234,8 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
             bt[i] = c < C && beta ? __ldg(beta + c) : 0.0f;
         }
     };
-    // xs <- the residual stream as the other CTAs left it; thread t takes the columns t, t + 256, ...
+    // xs and xr <- the residual stream as the other CTAs left it; thread t takes the columns t, t + 256, ... (xr: the first NV of them)
+    float xr[S][NV];
     auto load_x = [&](const unsigned long long* x, unsigned epoch) {
         for (int c0 = tid; c0 < C; c0 += NV * kDecThreads)
 #pragma unroll
@@ -242,7 +244,11 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                 float v[NV * SB];
                 ok = get_words<NV * SB>(x, [&](int u) { const int c = c0 + (u % NV) * kDecThreads, s = s0 + u / NV; return c < C && s < p.n_seq ? s * C + c : -1; }, epoch, v, p.status) && ok;
 #pragma unroll
-                for (int u = 0; u < NV * SB; ++u) { const int c = c0 + (u % NV) * kDecThreads; if (c < C) xs[(s0 + u / NV) * C + c] = v[u]; }
+                for (int u = 0; u < NV * SB; ++u) {
+                    const int c = c0 + (u % NV) * kDecThreads;
+                    if (c < C) xs[(s0 + u / NV) * C + c] = v[u];
+                    if (c0 == tid) xr[s0 + u / NV][u % NV] = v[u];
+                }
             }
     };
     auto all_warps = [&](const float* w) {  // the sum of the warps' sums, in warp order
@@ -251,17 +257,20 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
         for (int j = 0; j < kDecWarps; j += 4) { const float4 v = ld4(w + j); r += v.x; r += v.y; r += v.z; r += v.w; }
         return r;
     };
-    // act <- the normalised rows of xs: [k][s] for the products, [s][k] for the head.  Two passes over what every thread itself put
-    // into xs.  False when an exchange ran out of polls.
+    // act <- the normalised rows: [k][s] for the products, [s][k] for the head.  Two passes over what every thread itself loaded.
+    // False when an exchange ran out of polls.
     auto normalise = [&](const float* gamma, const float* beta, bool by_row) {
         float mu[S], rs[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             float sum = 0.0f;
-            for (int c = tid; c < C; c += kDecThreads) { const float v = xs[s * C + c]; sum += beta ? v : v * v; }
+#pragma unroll
+            for (int i = 0; i < NV; ++i) if (tid + i * kDecThreads < C) sum += beta ? xr[s][i] : xr[s][i] * xr[s][i];
+            for (int c = tid + NV * kDecThreads; c < C; c += kDecThreads) { const float v = xs[s * C + c]; sum += beta ? v : v * v; }
             sum = warp_sum(sum);
             if (lane == 0) stat[s * kDecWarps + warp] = sum;
         }
+        __syncwarp();
         if (!(ok = dec_sync_and(ok))) return false;
 #pragma unroll
         for (int s = 0; s < S; ++s) mu[s] = all_warps(stat + s * kDecWarps) * inv_c;
@@ -269,23 +278,26 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 float q = 0.0f;
-                for (int c = tid; c < C; c += kDecThreads) { const float d = xs[s * C + c] - mu[s]; q = fmaf(d, d, q); }
+#pragma unroll
+                for (int i = 0; i < NV; ++i) if (tid + i * kDecThreads < C) { const float d = xr[s][i] - mu[s]; q = fmaf(d, d, q); }
+                for (int c = tid + NV * kDecThreads; c < C; c += kDecThreads) { const float d = xs[s * C + c] - mu[s]; q = fmaf(d, d, q); }
                 q = warp_sum(q);
                 if (lane == 0) stat[(S + s) * kDecWarps + warp] = q;
             }
+            __syncwarp();
             dec_sync();
 #pragma unroll
-            for (int s = 0; s < S; ++s) rs[s] = 1.0f / sqrtf(all_warps(stat + (S + s) * kDecWarps) * inv_c + p.eps);
+            for (int s = 0; s < S; ++s) rs[s] = __frsqrt_rn(all_warps(stat + (S + s) * kDecWarps) * inv_c + p.eps);
         } else {
 #pragma unroll
-            for (int s = 0; s < S; ++s) { rs[s] = 1.0f / sqrtf(mu[s] + p.eps); mu[s] = 0.0f; }
+            for (int s = 0; s < S; ++s) { rs[s] = __frsqrt_rn(mu[s] + p.eps); mu[s] = 0.0f; }
         }
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int c = tid + i * kDecThreads;
             if (c < C) {
 #pragma unroll
-                for (int s = 0; s < S; ++s) act[by_row ? s * C + c : c * S + s] = (xs[s * C + c] - mu[s]) * rs[s] * gm[i] + bt[i];
+                for (int s = 0; s < S; ++s) act[by_row ? s * C + c : c * S + s] = (xr[s][i] - mu[s]) * rs[s] * gm[i] + bt[i];
             }
         }
         for (int c = tid + NV * kDecThreads; c < C; c += kDecThreads) {
@@ -293,11 +305,12 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
 #pragma unroll
             for (int s = 0; s < S; ++s) act[by_row ? s * C + c : c * S + s] = (xs[s * C + c] - mu[s]) * rs[s] * g + b;
         }
+        __syncwarp();
         dec_sync();
         return true;
     };
-    // The next tile of the ring times act: thread s * 8 + j (< 8 S) gets sum_k act[k][s] * W[k][column j of the tile].
-    auto tile_sum = [&](int K) {
+    // The next tile of the ring times act: this warp's share of sum_k act[k][s] * W[k][column j of the tile] goes to out[s * 8 + j].
+    auto tile_dot = [&](int K, float* out) {
         float acc[S * 4];
 #pragma unroll
         for (int i = 0; i < S * 4; ++i) acc[i] = 0.0f;
@@ -329,20 +342,11 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
             if (++stage == p.stages) { stage = 0; stage_ph ^= 1u; }
         }
         constexpr int HELD = S * 4 / 16 > 1 ? S * 4 / 16 : 1;
-        float* rb = red + (buf & 1) * (kDecWarps * S * 8);
-        ++buf;
         const int first = sum_rows(acc);
         if (first >= 0) {
 #pragma unroll
-            for (int i = 0; i < HELD; ++i) { const int q = first + i; rb[warp * (S * 8) + (q >> 2) * 8 + 4 * (lane & 1) + (q & 3)] = acc[i]; }
+            for (int i = 0; i < HELD; ++i) { const int q = first + i; out[(q >> 2) * 8 + 4 * (lane & 1) + (q & 3)] = acc[i]; }
         }
-        dec_sync();
-        float v = 0.0f;
-        if (tid < S * 8) {
-#pragma unroll
-            for (int j = 0; j < kDecWarps; ++j) v += rb[j * (S * 8) + tid];
-        }
-        return v;
     };
     auto given_token = [&](int pos) {  // an id outside the vocabulary is reported, not dereferenced
         if (tid < S) {
@@ -377,8 +381,8 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                         // four columns per lane; a warp load takes 32 / lpr rows, four of them are in flight
                         const int lpr = D <= 32 ? 8 : D <= 64 ? 16 : 32, rpw = 32 / lpr, col = 4 * (lane % lpr), step = kDecWarps * rpw, j_first = j0 + warp * rpw + lane / lpr;
                         const bool in = col < D;
-                        float4 kk[4], vv[4];
-                        auto rows = [&](int j) {
+                        float4 kk[4], vv[4], kn[4], vn[4];  // rows in hand, and the next ones
+                        auto rows = [&](int j, float4 (&kk)[4], float4 (&vv)[4]) {
 #pragma unroll
                             for (int g = 0; g < 4; ++g) {
                                 const int jj = j + g * step;
@@ -391,7 +395,7 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                         // before this call, or before the arg-max exchange that gave this position its token.  Otherwise the words of q
                         // (from the CTA that wrote this head's earlier rows, after its fence) say so.
                         const bool early = pos == p.pos0 || pos >= p.n_known;
-                        if (early) rows(j_first);
+                        if (early) rows(j_first, kk, vv);
                         if (tid < D) {
                             float v[3];
                             ok = get_words<3>(p.qkv + s * C + h * D + tid, [&](int which) { return which * S * C; }, epoch, v, p.status) && ok;
@@ -403,7 +407,8 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                         float m = -INFINITY, sum = 0.0f;
                         if (in) { q = ld4(now + col); q.x *= p.scale; q.y *= p.scale; q.z *= p.scale; q.w *= p.scale; }
                         for (int j = j_first; j - lane / lpr < j1; j += 4 * step) {  // the same trips for every lane of a warp
-                            if (j != j_first || !early) rows(j);
+                            if (j == j_first && !early) rows(j, kk, vv);
+                            rows(j + 4 * step, kn, vn);
                             float z[4];
 #pragma unroll
                             for (int g = 0; g < 4; ++g) {
@@ -430,6 +435,8 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                                     o.x = fmaf(e, vv[g].x, o.x); o.y = fmaf(e, vv[g].y, o.y); o.z = fmaf(e, vv[g].z, o.z); o.w = fmaf(e, vv[g].w, o.w);
                                 }
                             }
+#pragma unroll
+                            for (int g = 0; g < 4; ++g) { kk[g] = kn[g]; vv[g] = vn[g]; }
                         }
                         for (int b = lpr; b < 32; b <<= 1) {  // the warp's rows of the same columns
                             const float m2 = __shfl_xor_sync(0xffffffffu, m, b), s2 = __shfl_xor_sync(0xffffffffu, sum, b), M = fmaxf(m, m2);
@@ -472,9 +479,19 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                     const float* beta = ph == QKV ? w.norm1_beta : ph == MLP1 ? w.norm2_beta : p.final_beta;
                     fetch_norm(gamma, beta);
                     if (ph == QKV && l == 0) {
-                        for (int c = tid; c < C; c += kDecThreads)
+                        for (int c0 = tid; c0 < C; c0 += NV * kDecThreads)
 #pragma unroll
-                            for (int s = 0; s < S; ++s) xs[s * C + c] = __ldg(p.token_embed + (int64_t)tok[s] * C + c) + __ldg(p.pos_embed + (int64_t)pos * C + c);
+                            for (int i = 0; i < NV; ++i) {
+                                const int c = c0 + i * kDecThreads;
+                                if (c >= C) continue;
+                                const float at = __ldg(p.pos_embed + (int64_t)pos * C + c);
+#pragma unroll
+                                for (int s = 0; s < S; ++s) {
+                                    const float v = __ldg(p.token_embed + (int64_t)tok[s] * C + c) + at;
+                                    xs[s * C + c] = v;
+                                    if (c0 == tid) xr[s][i] = v;
+                                }
+                            }
                     } else {
                         load_x(ph == MLP1 ? p.xa : p.xb, ph == QKV ? epoch - 1 : epoch);
                     }
@@ -535,36 +552,48 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                     for (int i = p.n_seq * n + tid; i < S * n; i += kDecThreads) act[(i % n) * S + i / n] = 0.0f;  // no further sequence
                     if (!(ok = dec_sync_and(ok))) break;
                 }
-                // ---- the products
-                const int K = ph == MLP2 ? F : C, N = ph == MLP1 ? F : C;
+                // ---- the products: up to kDecMeet tiles of this CTA, then one meeting of its warps for all of them
+                const int K = ph == MLP2 ? F : C, N = ph == MLP1 ? F : C, each = ph == MLP1 && p.gated ? 2 : 1;  // matrices per tile
 #pragma unroll 1
-                for (int t = cta; t < tiles; t += gridDim.x) {
-                    const int which = ph == QKV ? t / tiles_c : 0, n0 = (t - which * tiles_c) * 8, s = tid >> 3, n = n0 + (tid & 7);
-                    const bool mine = tid < S * 8 && n < N && s < p.n_seq;  // this thread finishes a column
-                    const float* bias = ph == QKV ? (which == 0 ? w.bq : which == 1 ? w.bk : w.bv) : ph == OUT ? w.bo : ph == MLP1 ? w.b1 : p.gated ? w.b3 : w.b2;
-                    const float b = mine ? __ldg(bias + n) : 0.0f, b2 = mine && ph == MLP1 && p.gated ? __ldg(w.b2 + n) : 0.0f;
-                    float v = 0.0f, gate = 0.0f;
-#pragma unroll 1
-                    for (int again = ph == MLP1 && p.gated ? 1 : 0; again >= 0; --again) {  // w1 and then w2 of a gated first half
-                        gate = v;
-                        v = tile_sum(K);
+                for (int t0 = cta; t0 < tiles; t0 += kDecMeet / each * gridDim.x) {
+                    // what this thread finishes: sequence s, column n of the group's g-th tile
+                    const int g = tid / (S * 8), s = (tid >> 3) % S, t = t0 + g * gridDim.x, which = ph == QKV ? t / tiles_c : 0, n = (t - which * tiles_c) * 8 + (tid & 7);
+                    const bool mine = g < kDecMeet / each && t < tiles && n < N && s < p.n_seq;
+                    float b = 0.0f, b2 = 0.0f;
+                    if (mine) {
+                        b = __ldg((ph == QKV ? (which == 0 ? w.bq : which == 1 ? w.bk : w.bv) : ph == OUT ? w.bo : ph == MLP1 ? w.b1 : p.gated ? w.b3 : w.b2) + n);
+                        if (each == 2) b2 = __ldg(w.b2 + n);
                     }
-                    if (!mine) continue;
-                    if (ph == QKV) {
-                        v += b;
-                        put_word(p.qkv + (which * S + s) * C + n, v, epoch);
-                        if (which > 0) __stcg((which == 1 ? kc : vc) + s * p.seq_stride + (int64_t)pos * C + n, v);
-                    } else if (ph == MLP1) {
-                        if (p.gated) {
-                            gate += b;
-                            v = gate * __fdividef(1.0f, 1.0f + __expf(-gate)) * (v + b2);
+                    float* rb = red + (buf & 1) * (kDecMeet * kDecWarps * S * 8);
+                    ++buf;
+#pragma unroll 1
+                    for (int e = 0; e < kDecMeet && t0 + e / each * (int)gridDim.x < tiles; ++e) tile_dot(K, rb + (e * kDecWarps + warp) * (S * 8));
+                    __syncwarp();
+                    dec_sync();
+                    if (mine) {
+                        const float* r = rb + g * each * (kDecWarps * S * 8) + (tid & 7) + 8 * s;
+                        float v = 0.0f, v2 = 0.0f;
+#pragma unroll
+                        for (int j = 0; j < kDecWarps; ++j) v += r[j * (S * 8)];
+                        if (ph == QKV) {
+                            v += b;
+                            put_word(p.qkv + (which * S + s) * C + n, v, epoch);
+                            if (which > 0) __stcg((which == 1 ? kc : vc) + s * p.seq_stride + (int64_t)pos * C + n, v);
+                        } else if (ph == MLP1) {
+                            v += b;
+                            if (each == 2) {
+#pragma unroll
+                                for (int j = 0; j < kDecWarps; ++j) v2 += r[(kDecWarps + j) * (S * 8)];
+                                v = v * __fdividef(1.0f, 1.0f + __expf(-v)) * (v2 + b2);
+                            } else {
+                                v = gelu_f(v);
+                            }
+                            put_word(p.h + s * F + n, v, epoch);
                         } else {
-                            v = gelu_f(v + b);
+                            put_word((ph == OUT ? p.xa : p.xb) + s * C + n, xs[s * C + n] + v + b, epoch);
                         }
-                        put_word(p.h + s * F + n, v, epoch);
-                    } else {
-                        put_word((ph == OUT ? p.xa : p.xb) + s * C + n, xs[s * C + n] + v + b, epoch);
                     }
+                    __syncwarp();
                 }
             }
         }
