@@ -17,13 +17,14 @@
 
 namespace gcb {
 
-constexpr int SG_BK = 32, SG_STAGES = 3, SG_THREADS = 256, SG_KP = SG_BK + 4;
+constexpr int SG_BK = 32, SG_THREADS = 256, SG_KP = SG_BK + 4;
 
 template <int BM>
 struct SgSmem {
+    static constexpr int STAGES = 3;                                  // K blocks in shared memory (six of them: 0.1 us slower)
     static constexpr int KG = BM == 32 ? 4 : 1;                       // groups of threads sharing a K block
     static constexpr int OP = BM * SG_KP > SG_BK * (BM + 4) ? BM * SG_KP : SG_BK * (BM + 4);  // floats of one operand's block
-    static constexpr int LOOP = SG_STAGES * 2 * OP, OUT = KG * BM * BM;
+    static constexpr int LOOP = STAGES * 2 * OP, OUT = KG * BM * BM;
     static constexpr int FLOATS = (LOOP > OUT ? LOOP : OUT) + BM;     // + column sums
 };
 
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
     const int nblk = k_end > k_begin ? (int)((k_end - k_begin + SG_BK - 1) / SG_BK) : 0;
     auto load = [&](int i) {
         if (i < nblk) {
-            float* st = sg + (i % SG_STAGES) * 2 * S::OP;
+            float* st = sg + (i % S::STAGES) * 2 * S::OP;
             const int64_t k0 = k_begin + (int64_t)i * SG_BK;
             sg_load<BM, !TA>(st, A, g.lda, m0, g.M, k0, k_end, a_vec);
             sg_load<BM, TB>(st + S::OP, B, g.ldb, n0, g.N, k0, k_end, b_vec);
@@ -111,13 +112,13 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-    load(0);
-    load(1);
+#pragma unroll
+    for (int i = 0; i < S::STAGES - 1; ++i) load(i);
     for (int i = 0; i < nblk; ++i) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(SG_STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(S::STAGES - 2) : "memory");
         __syncthreads();  // block i has landed for everybody, and everybody is done with block i - 1
-        load(i + 2);
-        const float* as = sg + (i % SG_STAGES) * 2 * S::OP;
+        load(i + S::STAGES - 1);
+        const float* as = sg + (i % S::STAGES) * 2 * S::OP;
         const float* bs = as + S::OP;
 #pragma unroll
         for (int k = 0; k < SG_BK / KG; k += 4) {
@@ -273,9 +274,10 @@ int gemm_simt_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     const int bm = tiles(64) >= kSMs ? 64 : 32;
     const int64_t tm = (g.M + bm - 1) / bm, tn = (g.N + bm - 1) / bm;
     GCB_REQUIRE(tm * tn <= 0x7fffffff / 8 && tiles(bm) <= 0x7fffffff / 8, "gemm (FMA): grid too large");
-    // K is cut while CTAs are missing and every slice keeps two K blocks
+    // K is cut while SMs are left over and every slice keeps two K blocks; beyond one CTA per SM only for slices of 96 and more
+    // (256 x 512 x 128: one slice 5.5 us, two 6.4; 256 x 256 x 512: one 10.8, two 8.3, four 7.7, eight 12.9)
     int slices = 1;
-    while (slices < 8 && tiles(bm) * slices * 2 <= 2 * kSMs && g.K >= (int64_t)slices * 2 * 2 * SG_BK) slices *= 2;
+    while (slices < 8 && g.K >= (int64_t)slices * 2 * 2 * SG_BK && tiles(bm) * slices * 2 <= (g.K >= (int64_t)slices * 2 * 96 ? 2 * kSMs : kSMs)) slices *= 2;
     cudaSetDevice(ctx->device);
     int rc;
 #define GCB_SG(BMV) (!ta && !tb ? sg_launch<BMV, false, false>(ctx, g, tm, tn, batches, slices) : !ta ? sg_launch<BMV, false, true>(ctx, g, tm, tn, batches, slices) \
