@@ -657,7 +657,8 @@ inline Tensor<float> matmul(Tensor<float> x, Tensor<float> w) { return linear(st
 
 // ---- attention ----------------------------------------------------------------------------------------------------
 // softmax_causal(q k^T / sqrt(D)) v on (B, H, T, D) operands of any batch/row strides (frontend/tensor_other.hpp:53-93).
-// The six batched GEMMs skip what causality zeroes: score / dP tiles above the diagonal are not computed, and the K loops
+// Longer sequences with heads of up to 64 columns take the fused kernels, which keep two numbers per query for the backward; otherwise
+// the probabilities are kept and the six batched GEMMs skip what causality zeroes: score / dP tiles above the diagonal are not computed, and the K loops
 // over the (transposed) probability matrices stop / start at the diagonal.
 // q, k, v are read in place through two-level batch strides — the head split reshape+permute of the attention layer
 // stays a view — and the output is laid out (B, T, H, D) in memory, so merging heads is a view as well.
@@ -669,6 +670,7 @@ class SDPANode : public Node<float> {
     float m_scale;
     int64_t m_B, m_H, m_T, m_D;
     Tensor<float> m_probs;  // kept for backward; (B * H, T, m_ld)
+    Tensor<float> m_stats;  // fused kernels: row statistics kept instead
     int64_t m_ld;           // rows of the T x T matrices lie a multiple of four floats apart, so that TMA can address them for every T
     std::shared_ptr<Storage<float>> m_out_storage;  // O, for the row term dO . O of the softmax backward: the storage object of the tensor this node creates (realize() hands it the data)
 
@@ -684,9 +686,15 @@ public:
         m_q.realize(); m_k.realize(); m_v.realize();
         gcb_ctx* c = ctx_of(m_q);
         const int64_t B = m_B, H = m_H, T = m_T, D = m_D;
-        m_probs = Tensor<float>({B * H, T, m_ld}, m_q.device(), uninitialized);
         int64_t qo, qi, ql, ko, ki, kl, vo, vi, vl;
         strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl); strides4(m_v, vo, vi, vl);
+        if (gcb_attention_supported(c, B, H, T, D, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale)) {
+            m_stats = Tensor<float>({gcb_attention_stats_floats(B, H, T)}, m_q.device(), uninitialized);
+            Tensor<float> mem({B, T, H, D}, m_q.device(), uninitialized);
+            gcb_check(gcb_attention_fwd_f32(c, B, H, T, D, mem.data_ptr(), H * D, T * H * D, D, m_stats.data_ptr(), m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale), "attention");
+            return Tensor<float>({B, H, T, D}, out_strides(H, T, D), 0, mem._get_storage(), false);
+        }
+        m_probs = Tensor<float>({B * H, T, m_ld}, m_q.device(), uninitialized);
         gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_T, T, T, D, 1.0f, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, 0.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, B, H, 1), "attention scores");
         gcb_check(gcb_causal_softmax_fwd_band_ld_f32(c, m_probs.data_ptr(), m_probs.data_ptr(), m_scale, B * H * T, T, m_ld, kCausalBand), "causal softmax");
         Tensor<float> mem({B, T, H, D}, m_q.device(), uninitialized);
@@ -704,6 +712,17 @@ public:
             Tensor<float> mem({B, T, H, D}, g.device(), uninitialized);
             return Tensor<float>({B, H, T, D}, out_strides(H, T, D), 0, mem._get_storage(), false);
         };
+        if (m_stats._get_state() != nullptr) {
+            if (reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 != 0 || gl % 4 != 0 || go % 4 != 0 || gi % 4 != 0 || gl <= 0 || go <= 0 || gi <= 0) { g = make_contiguous(g); strides4(g, go, gi, gl); }
+            Tensor<float> dq = fresh(), dk = fresh(), dv = fresh();
+            gcb_check(gcb_attention_bwd_f32(c, B, H, T, D, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), H * D, T * H * D, D, g.data_ptr(), gl, go, gi, m_out_storage->data(), H * D, T * H * D, D, m_stats.data_ptr(), m_q.data_ptr(), ql, qo,
+                                            qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale), "attention backward");
+            if (m_v.requires_grad()) push_grad(m_v, dv);
+            if (m_q.requires_grad()) push_grad(m_q, dq);
+            if (m_k.requires_grad()) push_grad(m_k, dk);
+            if (!retain_graph) { m_stats = Tensor<float>(); m_out_storage.reset(); }
+            return;
+        }
         if (m_v.requires_grad()) {  // dV = P^T . dO
             Tensor<float> dv = fresh();
             gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_T, GCB_OP_N, T, D, T, 1.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, g.data_ptr(), gl, go, gi, 0.0f, dv.data_ptr(), H * D, T * H * D, D, B, H, 3), "attention dV");

@@ -209,6 +209,22 @@ GCB_API int gcb_rowdot_batched_f32(gcb_ctx* ctx, float* out, const float* a, int
                            const float* b, int64_t ldb, int64_t b_stride_outer, int64_t b_stride_inner,
                            int64_t rows, int64_t cols, int64_t batch_outer, int64_t batch_inner);
 
+/* Causal attention softmax(scale q k^T) v over batch x heads sequences of seq_len rows and head_dim columns without the seq_len x seq_len
+ * matrices, forward and backward (frontend/tensor_other.hpp:53-93 composes both from matmul and causal_softmax).  Operands are addressed
+ * through row, sequence and head strides in elements; columns are contiguous.  gcb_attention_supported says whether the operands can be
+ * taken (otherwise both calls return GCB_UNSUPPORTED and touch nothing).  stats: gcb_attention_stats_floats floats that the forward
+ * fills and the backward reads.  dq, dk and dv share one layout and are overwritten; out is the forward's result, dout its gradient. */
+GCB_API int64_t gcb_attention_stats_floats(int64_t batch, int64_t heads, int64_t seq_len);
+GCB_API int gcb_attention_supported(gcb_ctx* ctx, int64_t batch, int64_t heads, int64_t seq_len, int64_t head_dim, const float* q, int64_t q_ld, int64_t q_so, int64_t q_si,
+                            const float* k, int64_t k_ld, int64_t k_so, int64_t k_si, const float* v, int64_t v_ld, int64_t v_so, int64_t v_si, float scale);
+GCB_API int gcb_attention_fwd_f32(gcb_ctx* ctx, int64_t batch, int64_t heads, int64_t seq_len, int64_t head_dim, float* out, int64_t o_ld, int64_t o_so, int64_t o_si, float* stats,
+                          const float* q, int64_t q_ld, int64_t q_so, int64_t q_si, const float* k, int64_t k_ld, int64_t k_so, int64_t k_si,
+                          const float* v, int64_t v_ld, int64_t v_so, int64_t v_si, float scale);
+GCB_API int gcb_attention_bwd_f32(gcb_ctx* ctx, int64_t batch, int64_t heads, int64_t seq_len, int64_t head_dim, float* dq, float* dk, float* dv, int64_t d_ld, int64_t d_so, int64_t d_si,
+                          const float* dout, int64_t g_ld, int64_t g_so, int64_t g_si, const float* out, int64_t o_ld, int64_t o_so, int64_t o_si, const float* stats,
+                          const float* q, int64_t q_ld, int64_t q_so, int64_t q_si, const float* k, int64_t k_ld, int64_t k_so, int64_t k_si,
+                          const float* v, int64_t v_ld, int64_t v_so, int64_t v_si, float scale);
+
 /* Pre-split weights (no counterpart in the reference: cuBLAS in TF32 mode rounds operands on the fly, kernels_math.cu:27-36).
  * The split-fp32 GEMM needs two BF16 companions of every operand tile; for the B operand they are normally derived inside the
  * kernel, by every CTA that uses the tile.  A dense rows x cols matrix registered here keeps them in global memory in tile
