@@ -78,6 +78,8 @@ struct gcb_ctx {
     int last_gemm_engine = 0;
     int gemm_split_mode = 2;   // see gcb_ctx_set_gemm_split_mode
     int* d_status = nullptr;   // device-side status word written by kernels that give up on a bounded wait
+    char* h_small = nullptr;   // 256 pinned bytes for values the host reads back: results in front, the status word from byte 192, a scalar on its way from byte 208
+    cudaEvent_t ev_scalar = nullptr;  // gcb_read_scalar_begin / _end
     void* nccl_comm = nullptr;
     int dp_rank = 0, dp_world = 1;
     std::atomic<int> dp_failed{0};   // 0, or the status (GCB_NCCL_ERROR / GCB_TIMEOUT) the communicator watchdog ended with

@@ -179,6 +179,8 @@ static int ctx_create_common(int device, void* stream, bool own, gcb_ctx** out) 
     GCB_CHECK_CUDA(cudaEventCreateWithFlags(&c->ev_compute, cudaEventDisableTiming));
     GCB_CHECK_CUDA(cudaEventCreateWithFlags(&c->ev_comm, cudaEventDisableTiming));
     GCB_CHECK_CUDA(cudaMalloc(&c->d_status, sizeof(int) * 4));
+    GCB_CHECK_CUDA(cudaHostAlloc((void**)&c->h_small, 256, cudaHostAllocDefault));
+    GCB_CHECK_CUDA(cudaEventCreateWithFlags(&c->ev_scalar, cudaEventDisableTiming));
     GCB_CHECK_CUDA(cudaMemset(c->d_status, 0, sizeof(int) * 4));
     if (const char* g = getenv("GRADC_GEMM_ENGINE")) c->gemm_engine = atoi(g);
     if (const char* g = getenv("GRADC_TC_SPLIT_MODE")) { const int m = atoi(g); if (m >= 0 && m <= 2) c->gemm_split_mode = m; }
@@ -198,6 +200,8 @@ int gcb_ctx_destroy(gcb_ctx* ctx) {
     gcb_dp_finalize(ctx);
     ctx->arena.destroy();
     if (ctx->d_status) cudaFree(ctx->d_status);
+    if (ctx->h_small) cudaFreeHost(ctx->h_small);
+    if (ctx->ev_scalar) cudaEventDestroy(ctx->ev_scalar);
     if (ctx->ev_compute) cudaEventDestroy(ctx->ev_compute);
     if (ctx->ev_comm) cudaEventDestroy(ctx->ev_comm);
     if (ctx->comm_stream) cudaStreamDestroy(ctx->comm_stream);
@@ -257,14 +261,15 @@ int gcb_selftest_bounded_wait(gcb_ctx* ctx, int max_polls) {
 
 // Reads the device status word after the stream has been synchronised: a kernel that gave up on a bounded wait, or an
 // index / target that was skipped because it lay outside its table, turns into an error of the call that blocked.
-static int check_status_word(gcb_ctx* ctx) {
+static int check_status_word(gcb_ctx* ctx, const int* read = nullptr) {  // read: the word as already copied, or NULL
     if (const int f = ctx->dp_failed.load()) {
         set_error(f == GCB_TIMEOUT ? "data parallel: a gradient all-reduce did not complete in time; the communicator was aborted and the gradients of this step are invalid"
                                    : "data parallel: NCCL reported an asynchronous error; the communicator was aborted and the gradients of this step are invalid");
         return f;
     }
     int st[4];
-    GCB_CHECK_CUDA(cudaMemcpy(st, ctx->d_status, sizeof(st), cudaMemcpyDeviceToHost));
+    if (read) std::memcpy(st, read, sizeof(st));
+    else GCB_CHECK_CUDA(cudaMemcpy(st, ctx->d_status, sizeof(st), cudaMemcpyDeviceToHost));
     if (st[0] != 0) {
         cudaMemset(ctx->d_status, 0, sizeof(st));
         if (st[0] == 2) {
@@ -318,11 +323,31 @@ int gcb_copy_h2d(gcb_ctx* ctx, void* dst, const void* src, size_t bytes) {
 }
 int gcb_copy_d2h(gcb_ctx* ctx, void* dst, const void* src, size_t bytes) {
     GCB_REQUIRE(ctx && (bytes == 0 || (dst && src)), "gcb_copy_d2h: NULL argument");
+    if (bytes > 0 && bytes <= 192) {  // a scalar or a few: with the status word through pinned memory, one wait instead of two
+        GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small + 192, ctx->d_status, 16, cudaMemcpyDeviceToHost, ctx->stream));
+        GCB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+        std::memcpy(dst, ctx->h_small, bytes);
+        return check_status_word(ctx, reinterpret_cast<const int*>(ctx->h_small + 192));
+    }
     GCB_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     GCB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
     // the host blocks here anyway (Tensor::item() of the loss, gradient and checkpoint reads): the one place per training step
     // where a failed launch can be reported before its results are used
     return check_status_word(ctx);
+}
+int gcb_read_scalar_begin(gcb_ctx* ctx, const float* src) {
+    GCB_REQUIRE(ctx && src, "gcb_read_scalar_begin: NULL argument");
+    GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small + 208, src, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+    GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small + 224, ctx->d_status, 16, cudaMemcpyDeviceToHost, ctx->stream));
+    GCB_CHECK_CUDA(cudaEventRecord(ctx->ev_scalar, ctx->stream));
+    return GCB_OK;
+}
+int gcb_read_scalar_end(gcb_ctx* ctx, float* out) {
+    GCB_REQUIRE(ctx && out, "gcb_read_scalar_end: NULL argument");
+    GCB_CHECK_CUDA(cudaEventSynchronize(ctx->ev_scalar));
+    std::memcpy(out, ctx->h_small + 208, sizeof(float));
+    return check_status_word(ctx, reinterpret_cast<const int*>(ctx->h_small + 224));
 }
 int gcb_copy_h2d_async(gcb_ctx* ctx, void* dst, const void* src, size_t bytes) {
     GCB_REQUIRE(ctx && (bytes == 0 || (dst && src)), "gcb_copy_h2d_async: NULL argument");

@@ -173,9 +173,13 @@ struct AdamWTensorOp {
 
 // One CTA per GCB_ADAMW_CHUNK-element chunk and loop: 256 threads x float4 = 1024 elements.
 __global__ void __launch_bounds__(256) adamw_arena_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
-                                                          const uint8_t* __restrict__ mask, int64_t n, int64_t n_chunks, AdamW h) {
+                                                          const uint8_t* __restrict__ mask, int64_t n, int64_t n_chunks, AdamW h, const float* __restrict__ sum_squares, float max_norm) {
     pdl_trigger();
     pdl_wait();
+    if (sum_squares != nullptr) {  // the clip factor without a round trip through the host (a small step waits 25 us for it)
+        const float norm = sqrtf(__ldg(sum_squares)) * fabsf(h.gscale);
+        if (norm > max_norm) h.gscale *= max_norm / (norm + 1e-6f);
+    }
     for (int64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
         const bool decay = mask[c] != 0;
         const int64_t i = c * GCB_ADAMW_CHUNK + 4 * threadIdx.x;
@@ -489,6 +493,10 @@ int gcb_adamw_step_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float* 
     return ew_launch(ctx, "adamw_step", p, n, AdamWTensorOp{make_adamw(lr, b1, b2, b1p, b2p, wd, eps, gscale), !no_decay});
 }
 int gcb_adamw_arena_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float* g, const uint8_t* mask, int64_t n, float lr, float b1, float b2, float b1p, float b2p, float wd, float eps, float gscale) {
+    return gcb_adamw_arena_clip_f32(ctx, w, m, v, g, mask, n, lr, b1, b2, b1p, b2p, wd, eps, gscale, nullptr, 0.0f);
+}
+int gcb_adamw_arena_clip_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float* g, const uint8_t* mask, int64_t n, float lr, float b1, float b2, float b1p, float b2p, float wd, float eps, float gscale,
+                             const float* sum_squares, float max_norm) {
     GCB_REQUIRE(ctx && n >= 0 && (n == 0 || (w && m && v && g && mask)), "gcb_adamw_arena_f32: bad arguments");
     GCB_REQUIRE(b1p < 1.0f && b2p < 1.0f, "gcb_adamw_arena_f32: beta powers must already be advanced (< 1)");
     if (n == 0) return GCB_OK;
@@ -497,7 +505,7 @@ int gcb_adamw_arena_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float*
     int64_t blocks = std::min<int64_t>(chunks, kSMs * 8);
     cudaSetDevice(ctx->device);
     note_write(ctx, w, sizeof(float) * (size_t)n);
-    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, adamw_arena_kernel, w, m, v, g, mask, n, chunks, make_adamw(lr, b1, b2, b1p, b2p, wd, eps, gscale)));
+    GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)blocks, 256, 0, adamw_arena_kernel, w, m, v, g, mask, n, chunks, make_adamw(lr, b1, b2, b1p, b2p, wd, eps, gscale), sum_squares, max_norm));
     return after_launch(ctx, "adamw_arena");
 }
 

@@ -344,6 +344,55 @@ __global__ void __launch_bounds__(32 * kFoldWarps) scatter_fold_kernel(float* __
     }
 }
 
+// A short index list in one launch: a warp per entry and 32 lanes' worth of columns.  The first entry with a given index adds up
+// all of them in list order; the others find an earlier one and leave.  Every warp reads the list once, so this is for lists of a
+// few rounds of 32 (256 entries of 128 columns: 3 us instead of six launches and 20 us).
+constexpr int kShortList = 1024;
+template <class IdxT, int VEC>
+__global__ void __launch_bounds__(256) scatter_short_kernel(float* __restrict__ dtable, const IdxT* __restrict__ idx, const float* __restrict__ dy, int n, int64_t width, int64_t vocab, int* __restrict__ status) {
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const int64_t mine = (int64_t)idx[i];
+    if (mine < 0 || mine >= vocab) {
+        if (lane == 0 && blockIdx.y == 0) { atomicExch(&status[0], 2); atomicExch(&status[1], i); }
+        return;
+    }
+    for (int j0 = 0; j0 < i; j0 += 32)
+        if (__any_sync(0xffffffffu, j0 + lane < i && (int64_t)idx[min(j0 + lane, n - 1)] == mine)) return;
+    const int64_t c = ((int64_t)blockIdx.y * 32 + lane) * VEC;
+    const bool valid = c < width;
+    float acc[VEC] = {};
+    for (int j0 = i & ~31; j0 < n; j0 += 32) {
+        const int j = j0 + lane;
+        unsigned hits = __ballot_sync(0xffffffffu, j >= i && j < n && (int64_t)idx[min(j, n - 1)] == mine);
+        while (hits) {  // up to four rows in flight
+            float x[4][VEC];
+            int got = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (hits == 0) break;
+                const float* src = dy + (int64_t)(j0 + __ffs(hits) - 1) * width + c;
+                hits &= hits - 1;
+                got = u + 1;
+                if (!valid) continue;
+                if (VEC == 4) { const float4 v = ld4(src); x[u][0] = v.x; x[u][1 % VEC] = v.y; x[u][2 % VEC] = v.z; x[u][3 % VEC] = v.w; }
+                else x[u][0] = *src;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (u < got)
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) acc[e] += valid ? x[u][e] : 0.0f;
+        }
+    }
+    if (!valid) return;
+    float* dst = dtable + mine * width + c;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) dst[e] += acc[e];
+}
+
 struct ScatterPlan {
     int32_t *blk, *counts, *offsets, *segbase, *pbase, *blocktot, *n_hot, *order;
     int4 *segdesc, *hotdesc;
@@ -395,11 +444,16 @@ static int build_plan(gcb_ctx* ctx, Scratch& sc, ScatterPlan& p, const IdxT* idx
 
 template <class IdxT>
 static int scatter_add_impl(gcb_ctx* ctx, float* dtable, const IdxT* idx, const float* dy, int64_t n, int64_t width, int64_t vocab) {
+    const bool vec = width % 4 == 0 && aligned16(dtable) && aligned16(dy);
+    const int64_t short_tiles = (width + (vec ? 128 : 32) - 1) / (vec ? 128 : 32);
+    if (n <= kShortList && short_tiles <= 65535) {
+        GCB_CHECK_CUDA(launch_next(ctx->stream, dim3((unsigned)((n + 7) / 8), (unsigned)short_tiles), 256, 0, vec ? scatter_short_kernel<IdxT, 4> : scatter_short_kernel<IdxT, 1>, dtable, idx, dy, (int)n, width, vocab, ctx->d_status));
+        return after_launch(ctx, "scatter_short");
+    }
     Scratch sc(ctx);
     ScatterPlan p;
     int rc = build_plan<IdxT>(ctx, sc, p, idx, n, vocab, width);
     if (rc) return rc;
-    const bool vec = width % 4 == 0 && aligned16(dtable) && aligned16(dy);
     const int64_t col_tiles = (width + (vec ? 512 : 128) - 1) / (vec ? 512 : 128);
     const unsigned blocks = (unsigned)std::min<int64_t>(((n / kSeg + std::min<int64_t>(n, vocab)) * col_tiles + 7) / 8 + 1, (int64_t)kSMs * 8);
     GCB_CHECK_CUDA(launch_chained(ctx->stream, blocks, 256, 0, vec ? scatter_accumulate_kernel<4> : scatter_accumulate_kernel<1>, dtable, p.parked, dy, p.order, p.segdesc, p.segbase + vocab, width));

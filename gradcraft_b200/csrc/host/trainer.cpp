@@ -167,15 +167,22 @@ int gct_forward_backward(gct_trainer* tr, const int64_t* tokens, const int64_t* 
         logits = Tensor<float>();  // the loss node is now the only holder: probabilities may overwrite the logits
         Tensor<float> scaled = accum > 1 ? loss / static_cast<float>(accum) : loss;
         scaled.realize();
-        if (loss_out) *loss_out = scaled.item();
+        // the loss travels while the backward sweep is being launched: waiting for it here would leave the GPU without work for as long
+        // as the next launches take
+        gcb_ctx* c = Backend::get().ctx(tr->gpu);
+        if (loss_out) gcb_check(gcb_read_scalar_begin(c, scaled.data_ptr()), "loss");
         scaled.backward();
+        if (loss_out) gcb_check(gcb_read_scalar_end(c, loss_out), "loss");
     });
 }
 
 int gct_optimizer_step(gct_trainer* tr, float* norm_out) {
     return guarded([&] {
         float n = -1.0f;
-        if (tr->clipper) n = tr->clipper->normalize(tr->model->parameters());
+        if (tr->clipper) {
+            if (norm_out) n = tr->clipper->normalize(tr->model->parameters());
+            else tr->clipper->normalize_quietly(tr->model->parameters());
+        }
         if (norm_out) *norm_out = n;
         tr->opt->step();
     });

@@ -667,9 +667,10 @@ public:
         if (m_arena) {
             m_arena->sync_gradients();
             if (m_arena->all_grads_live()) {
-                gcb_check(gcb_adamw_arena_f32(c, m_arena->w, m_arena->m, m_arena->v, m_arena->g, m_arena->decay_mask, m_arena->total, this->m_lr, m_beta1, m_beta2, m_beta1_exp, m_beta2_exp,
-                                              m_weight_decay, m_eps, m_arena->pending_grad_scale), "AdamW step");
+                gcb_check(gcb_adamw_arena_clip_f32(c, m_arena->w, m_arena->m, m_arena->v, m_arena->g, m_arena->decay_mask, m_arena->total, this->m_lr, m_beta1, m_beta2, m_beta1_exp, m_beta2_exp,
+                                                   m_weight_decay, m_eps, m_arena->pending_grad_scale, m_arena->clip_pending ? m_arena->clip_sum_squares : nullptr, m_arena->clip_max_norm), "AdamW step");
                 m_arena->pending_grad_scale = 1.0f;
+                m_arena->clip_pending = false;
                 return;
             }
         }
@@ -808,7 +809,13 @@ public:
     GlobalNormClipper(T max_norm = static_cast<T>(1.0)) : m_max_norm(max_norm) {}
     // n = sqrt(sum g^2); if n > max: g *= max / (n + 1e-6)   (norm_clip.hpp:42-55).  With arena-resident parameters the
     // scale is not applied here: it is handed to the optimizer step, which multiplies it in while it reads the gradients.
-    T normalize(const std::vector<Parameter<T>*>& params) {
+    T normalize(const std::vector<Parameter<T>*>& params) { return clip(params, true); }
+    // The same for a caller that does not ask for the norm: with arena-resident parameters the optimizer finds the factor on the
+    // device and the host does not wait.
+    void normalize_quietly(const std::vector<Parameter<T>*>& params) { clip(params, false); }
+
+private:
+    T clip(const std::vector<Parameter<T>*>& params, bool want_norm) {
         if (params.empty()) return T(0);
         Device d = params[0]->device();
         gcb_ctx* c = Backend::get().ctx(d);
@@ -816,8 +823,16 @@ public:
         bool whole = a != nullptr && a->slots.size() == params.size();
         if (whole) for (auto* p : params) whole = whole && p->tensor()._get_state()->m_slot.arena == a;
         Tensor<T> sq(std::vector<int64_t>{}, d, uninitialized);
+        if (a) a->resolve_clip();
         if (whole && a->all_grads_live()) {
             a->sync_gradients();
+            if (!want_norm) {
+                if (a->clip_sum_squares == nullptr) a->clip_sum_squares = static_cast<float*>(Backend::get().allocate(sizeof(float), a->device));
+                gcb_check(gcb_sum_squares_f32(c, a->clip_sum_squares, a->g, a->total, 0), "gradient norm");
+                a->clip_max_norm = m_max_norm;
+                a->clip_pending = true;
+                return T(0);
+            }
             gcb_check(gcb_sum_squares_f32(c, sq.data_ptr(), a->g, a->total, 0), "gradient norm");
             const T norm = std::sqrt(sq.item()) * std::abs(a->pending_grad_scale);
             if (norm > m_max_norm) a->pending_grad_scale *= m_max_norm / (norm + static_cast<T>(1e-6));

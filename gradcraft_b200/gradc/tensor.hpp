@@ -16,6 +16,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <functional>
 #include <memory>
 #include <tuple>
@@ -96,6 +97,17 @@ struct ParamArena {
     std::vector<Slot> slots;
     std::vector<Bucket> buckets;
     float pending_grad_scale = 1.0f;  // clip factor not yet folded into the gradients (consumed by AdamW)
+    float* clip_sum_squares = nullptr;  // device scalar: squares of a clip whose factor is still to be found from it (by AdamW, on the device)
+    float clip_max_norm = 0.0f;
+    bool clip_pending = false;
+    void resolve_clip() {  // somebody other than AdamW wants the factor
+        if (!clip_pending) return;
+        clip_pending = false;
+        float sq = 0.0f;
+        gcb_check(gcb_copy_d2h(Backend::get().ctx(device), &sq, clip_sum_squares, sizeof(float)), "gradient norm");
+        const float norm = std::sqrt(sq) * std::abs(pending_grad_scale);
+        if (norm > clip_max_norm) pending_grad_scale *= clip_max_norm / (norm + 1e-6f);
+    }
     // data parallel bookkeeping
     int dp_world = 1;
     int64_t accum_expected = 0;   // micro-batches per optimizer step (0 = not known yet)
@@ -135,7 +147,7 @@ struct ParamArena {
     ~ParamArena() {
         Backend& b = Backend::get();
         if (w != nullptr && !device.is_cpu()) gcb_weight_twins_drop(b.ctx(device), w, sizeof(float) * (size_t)total);  // pre-split companions of the matrices in this arena
-        b.release(w, device); b.release(g, device); b.release(m, device); b.release(v, device); b.release(decay_mask, device);
+        b.release(w, device); b.release(g, device); b.release(m, device); b.release(v, device); b.release(decay_mask, device); b.release(clip_sum_squares, device);
     }
     // GRADC_DP_OVERLAP=0: no bucket is reduced while backward still runs; the whole gradient arena is reduced by one
     // all-reduce when the first consumer asks for it (NVLink moves the 743 MB of the 180M-parameter model in about 2 ms,
@@ -186,6 +198,7 @@ struct ParamArena {
         backward_calls = 0;
         reduced_this_step = false;
         pending_grad_scale = 1.0f;
+        clip_pending = false;
     }
     bool all_grads_live() const {
         for (auto& s : slots) if (!s.grad_live) return false;
@@ -417,6 +430,7 @@ void Tensor<T>::realize() {
 template <typename T>
 std::optional<Tensor<T>> Tensor<T>::grad() const {
     if constexpr (std::is_same_v<T, float>) {
+        if (m_state->m_slot.arena) m_state->m_slot.arena->resolve_clip();
         // a clip factor that is still pending must be visible to anyone who looks at a parameter gradient
         if (m_state->m_slot.arena && m_state->m_slot.arena->pending_grad_scale != 1.0f && m_state->m_grad.has_value()) {
             ParamArena& a = *m_state->m_slot.arena;

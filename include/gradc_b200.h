@@ -102,6 +102,10 @@ GCB_API int gcb_arena_set_limit(gcb_ctx* ctx, size_t bytes);
 /* ---- copies: Storage ctor / ToNode / Tensor::item, core/storage.hpp:64-68, memory_nodes.hpp:212-317 */
 GCB_API int gcb_copy_h2d(gcb_ctx* ctx, void* dst_dev, const void* src_host, size_t bytes);        /* synchronous */
 GCB_API int gcb_copy_d2h(gcb_ctx* ctx, void* dst_host, const void* src_dev, size_t bytes);        /* synchronous; reports the status word like gcb_ctx_sync */
+/* A float on its way to the host while the stream goes on: begin enqueues the copy (one at a time per context), end waits for it
+ * alone and reports what gcb_copy_d2h would report up to that point. */
+GCB_API int gcb_read_scalar_begin(gcb_ctx* ctx, const float* src);
+GCB_API int gcb_read_scalar_end(gcb_ctx* ctx, float* out);
 GCB_API int gcb_copy_h2d_async(gcb_ctx* ctx, void* dst_dev, const void* src_pinned, size_t bytes); /* on the compute stream */
 GCB_API int gcb_copy_d2h_async(gcb_ctx* ctx, void* dst_pinned, const void* src_dev, size_t bytes);
 GCB_API int gcb_copy_d2d(gcb_ctx* ctx, void* dst, const void* src, size_t bytes);
@@ -321,6 +325,11 @@ GCB_API int gcb_adamw_step_f32(gcb_ctx* ctx, float* w, float* m, float* v, const
 #define GCB_ADAMW_CHUNK 1024
 GCB_API int gcb_adamw_arena_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float* grad, const uint8_t* decay_mask, int64_t n, float lr, float beta1,
                         float beta2, float beta1_pow, float beta2_pow, float weight_decay, float eps, float grad_scale);
+
+/* The same with the clip factor of GlobalNormClipper found on the device: n = sqrt(*sum_squares) * |grad_scale|; where n > max_norm
+ * grad_scale is multiplied by max_norm / (n + 1e-6). */
+GCB_API int gcb_adamw_arena_clip_f32(gcb_ctx* ctx, float* w, float* m, float* v, const float* grad, const uint8_t* decay_mask, int64_t n, float lr, float beta1,
+                        float beta2, float beta1_pow, float beta2_pow, float weight_decay, float eps, float grad_scale, const float* sum_squares, float max_norm);
 
 /* ---- generation: GPTGenerator::run_inference, nn/generators/gpt_generator.hpp:12-132 -------------- */
 /* Device pointers of one pre-norm block; all matrices K x N row-major as the linear layers store them.  norm*_beta NULL:
