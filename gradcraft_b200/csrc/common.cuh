@@ -137,7 +137,11 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 inline void note_write(gcb_ctx* ctx, const void* p, size_t bytes) {
     if (ctx->twins_lo == nullptr || ctx->twins_dirty) return;
     const char* b = static_cast<const char*>(p);
-    if (b < ctx->twins_hi && b + bytes > ctx->twins_lo) ctx->twins_dirty = true;
+    if (b >= ctx->twins_hi || b + bytes <= ctx->twins_lo) return;
+    for (const gcb::WeightTwin& t : ctx->twins) {  // with several models in one process activations lie between their weights
+        const char* w = reinterpret_cast<const char*>(t.base);
+        if (w != nullptr && b < w + sizeof(float) * (size_t)(t.rows * t.cols) && b + bytes > w) { ctx->twins_dirty = true; return; }
+    }
 }
 int twins_lookup(gcb_ctx* ctx, const float* base, bool stored_n_by_k, int64_t N, int64_t K, int64_t ldb, const void** out);
 size_t twin_bytes(int64_t N, int64_t K);
