@@ -179,8 +179,6 @@ static int ctx_create_common(int device, void* stream, bool own, gcb_ctx** out) 
     GCB_CHECK_CUDA(cudaEventCreateWithFlags(&c->ev_compute, cudaEventDisableTiming));
     GCB_CHECK_CUDA(cudaEventCreateWithFlags(&c->ev_comm, cudaEventDisableTiming));
     GCB_CHECK_CUDA(cudaMalloc(&c->d_status, sizeof(int) * 4));
-    GCB_CHECK_CUDA(cudaHostAlloc((void**)&c->h_small, 256, cudaHostAllocDefault));
-    GCB_CHECK_CUDA(cudaEventCreateWithFlags(&c->ev_scalar, cudaEventDisableTiming));
     GCB_CHECK_CUDA(cudaMemset(c->d_status, 0, sizeof(int) * 4));
     if (const char* g = getenv("GRADC_GEMM_ENGINE")) c->gemm_engine = atoi(g);
     if (const char* g = getenv("GRADC_TC_SPLIT_MODE")) { const int m = atoi(g); if (m >= 0 && m <= 2) c->gemm_split_mode = m; }
@@ -321,9 +319,16 @@ int gcb_copy_h2d(gcb_ctx* ctx, void* dst, const void* src, size_t bytes) {
     GCB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
     return GCB_OK;
 }
+static int small_buffer(gcb_ctx* ctx) {  // made by the first read that needs it: pinning a page takes milliseconds
+    if (ctx->h_small) return GCB_OK;
+    if (!ctx->ev_scalar) GCB_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->ev_scalar, cudaEventDisableTiming));
+    GCB_CHECK_CUDA(cudaHostAlloc((void**)&ctx->h_small, 256, cudaHostAllocDefault));
+    return GCB_OK;
+}
 int gcb_copy_d2h(gcb_ctx* ctx, void* dst, const void* src, size_t bytes) {
     GCB_REQUIRE(ctx && (bytes == 0 || (dst && src)), "gcb_copy_d2h: NULL argument");
     if (bytes > 0 && bytes <= 192) {  // a scalar or a few: with the status word through pinned memory, one wait instead of two
+        if (int rc = small_buffer(ctx)) return rc;
         GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small + 192, ctx->d_status, 16, cudaMemcpyDeviceToHost, ctx->stream));
         GCB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -338,13 +343,14 @@ int gcb_copy_d2h(gcb_ctx* ctx, void* dst, const void* src, size_t bytes) {
 }
 int gcb_read_scalar_begin(gcb_ctx* ctx, const float* src) {
     GCB_REQUIRE(ctx && src, "gcb_read_scalar_begin: NULL argument");
+    if (int rc = small_buffer(ctx)) return rc;
     GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small + 208, src, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     GCB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_small + 224, ctx->d_status, 16, cudaMemcpyDeviceToHost, ctx->stream));
     GCB_CHECK_CUDA(cudaEventRecord(ctx->ev_scalar, ctx->stream));
     return GCB_OK;
 }
 int gcb_read_scalar_end(gcb_ctx* ctx, float* out) {
-    GCB_REQUIRE(ctx && out, "gcb_read_scalar_end: NULL argument");
+    GCB_REQUIRE(ctx && out && ctx->h_small, "gcb_read_scalar_end: NULL argument, or no copy was begun");
     GCB_CHECK_CUDA(cudaEventSynchronize(ctx->ev_scalar));
     std::memcpy(out, ctx->h_small + 208, sizeof(float));
     return check_status_word(ctx, reinterpret_cast<const int*>(ctx->h_small + 224));

@@ -579,3 +579,55 @@ def test_unaligned_operands_are_packed_for_the_tensor_cores(env, opa, opb, M, N,
         assert max_abs_rel(C.cpu().numpy(), 0.5 * ref + C0 + bias) < TOL
     finally:
         ctx.ctx_set_gemm_engine(2)
+
+
+@pytest.mark.parametrize("opa,opb,M,N,K", [(0, 0, 1, 1, 1), (0, 1, 33, 31, 32), (1, 0, 64, 65, 95), (0, 0, 16, 512, 1024), (1, 1, 129, 63, 257), (0, 0, 513, 300, 64), (1, 0, 640, 640, 33)])
+def test_small_products_on_the_fma_kernel(env, opa, opb, M, N, K):
+    """Edges of the 32- and 64-wide tiles, K cut over clusters, operands on and off 16-byte boundaries, bias / beta and the column sums."""
+    ctx, torch, capi = env
+    A, B = rnd(1, *((K, M) if opa else (M, K))), rnd(2, *((N, K) if opb else (K, N)))
+    C0, bias = rnd(3, M, N), rnd(4, N)
+    ref = (A.T if opa else A).astype(np.float64) @ (B.T if opb else B).astype(np.float64)
+    ctx.ctx_set_gemm_engine(1)
+    try:
+        dA, dB, dC, dbias = (torch.from_numpy(a).cuda() for a in (A, B, C0, bias))
+        ctx.gemm_f32(opa, opb, M, N, K, 0.5, dA, A.shape[1], dB, B.shape[1], 2.0, dC, N, dbias)
+        ctx.sync()
+        assert max_abs_rel(dC.cpu().numpy(), 0.5 * ref + 2.0 * C0 + bias) < TOL
+        if not opb:
+            out, sums = torch.empty(M, N, device="cuda"), torch.ones(N, device="cuda")
+            ctx.gemm_colsum_f32(opa, M, N, K, 1.0, dA, A.shape[1], dB, 0.0, out, N, sums, 1)
+            ctx.sync()
+            assert max_abs_rel(out.cpu().numpy(), ref) < TOL
+            assert np.abs(sums.cpu().numpy() - 1.0 - B.sum(0, dtype=np.float64)).max() < 1e-4 * max(1.0, np.abs(B).sum(0).max())
+    finally:
+        ctx.ctx_set_gemm_engine(2)
+
+
+@pytest.mark.parametrize("Bn,H,T,D", [(1, 1, 257, 64), (2, 3, 384, 64), (1, 2, 511, 32), (3, 2, 300, 20), (1, 1, 1025, 4), (40, 4, 260, 48)])
+def test_fused_causal_attention(env, Bn, H, T, D):
+    """Partial and whole query tiles, one and two tiles a CTA, several items a CTA, padded head widths; scores that grow along the
+    row (the running maximum moves); out of its range the entry points decline."""
+    ctx, torch, capi = env
+    C, scale = H * D, 1.0 / np.sqrt(D)
+    q, k, v, g = (rnd(s, Bn, T, C) for s in (1, 2, 3, 4))
+    k *= (1.0 + np.arange(T, dtype=np.float32) / 64)[None, :, None]
+    dq, dk, dv, dg = (torch.from_numpy(a).cuda() for a in (q, k, v, g))
+    rows = (C, T * C, D)
+    out, gq, gk, gv = (torch.empty(Bn, T, C, device="cuda") for _ in range(4))
+    stats = torch.empty(capi.lib().attention_stats_floats(Bn, H, T), device="cuda")
+    ctx.attention_fwd_f32(Bn, H, T, D, out, *rows, stats, dq, *rows, dk, *rows, dv, *rows, scale)
+    ctx.attention_bwd_f32(Bn, H, T, D, gq, gk, gv, *rows, dg, *rows, out, *rows, stats, dq, *rows, dk, *rows, dv, *rows, scale)
+    ctx.sync()
+    heads = lambda a: a.astype(np.float64).reshape(Bn, T, H, D).transpose(0, 2, 1, 3)  # noqa: E731
+    Q, K, V, G = (heads(a) for a in (q, k, v, g))
+    S = np.where(np.tril(np.ones((T, T), bool)), np.einsum("bhid,bhjd->bhij", Q, K) * scale, -np.inf)
+    P = np.exp(S - S.max(-1, keepdims=True))
+    P /= P.sum(-1, keepdims=True)
+    O = P @ V
+    dP = G @ V.transpose(0, 1, 3, 2)
+    dS = scale * P * (dP - (G * O).sum(-1, keepdims=True))
+    for got, ref in ((out, O), (gq, dS @ K), (gk, dS.transpose(0, 1, 3, 2) @ Q), (gv, P.transpose(0, 1, 3, 2) @ G)):
+        got = heads(got.cpu().numpy())
+        assert np.linalg.norm(got - ref) < TOL * np.linalg.norm(ref)
+    assert not capi.lib().attention_supported(ctx.h, Bn, H, 256, D, dq.data_ptr(), *rows, dk.data_ptr(), *rows, dv.data_ptr(), *rows, scale)

@@ -582,3 +582,35 @@ def test_causal_softmax_on_padded_rows(env, T, band):
     seen = torch.ones_like(j < 0).expand(BH * T, T) if band == 0 else j < (i // band + 1) * band
     ctx.sync()
     assert max_abs_rel(torch.where(seen, padded[:, :T], dense).cpu().numpy(), dense.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("n,V,C,i32", [(1, 3, 4, False), (256, 50, 128, True), (1024, 7, 132, False), (33, 1000, 5, False)])
+def test_scatter_add_of_a_short_list(env, n, V, C, i32):
+    """One launch up to 1024 entries: a single entry, rows hit many times, a part of a column tile, columns that are no multiple of four."""
+    ctx, torch, capi = env
+    idx = np.random.default_rng(3).integers(0, V, n)
+    dy, table = rnd(5, n, C), rnd(6, V, C)
+    ref = table.astype(np.float64)
+    np.add.at(ref, idx, dy.astype(np.float64))
+    out = dev(torch, table)
+    ctx.scatter_add_f32(out, dev(torch, idx.astype(np.int32 if i32 else np.int64)), capi.IDX_I32 if i32 else capi.IDX_I64, dev(torch, dy), n, C, V)
+    assert max_abs_rel(host(ctx, out), ref) < 1e-5
+
+
+@pytest.mark.parametrize("scale,max_norm", [(1.0, 0.5), (1.0, 1e6), (0.25, 0.5)])
+def test_adamw_finds_the_clip_factor_on_the_device(env, scale, max_norm):
+    ctx, torch, capi = env
+    n = 3000
+    w, m, v, g = rnd(1, n), rnd(2, n, scale=0.1), np.abs(rnd(3, n, scale=0.1)), rnd(4, n)
+    mask = dev(torch, np.array([1, 0, 1], np.uint8))
+    norm = np.sqrt((g.astype(np.float64) ** 2).sum()) * scale
+    factor = scale * (max_norm / (norm + 1e-6) if norm > max_norm else 1.0)
+    got = []
+    for sq, s in ((torch.empty(1, device="cuda"), scale), (None, float(factor))):
+        t = [dev(torch, a) for a in (w, m, v, g)]
+        if sq is not None:
+            ctx.sum_squares_f32(sq, t[3], n, 0)
+        ctx.adamw_arena_clip_f32(*t, mask, n, 1e-3, 0.9, 0.95, 0.9, 0.95, 0.1, 1e-5, s, sq, max_norm)
+        got.append([host(ctx, a) for a in t[:3]])
+    for a, b in zip(*got):
+        assert max_abs_rel(a, b) < 1e-5
