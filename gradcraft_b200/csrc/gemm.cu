@@ -58,10 +58,11 @@ struct PackedOperand {
 
 // Engine choice for one validated problem; no timing here, so the GELU fallback below may call it again freely.
 static int dispatch_gemm(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g, const char* who) {
-    const int64_t work = g.M * g.N * g.K * g.batch_outer * g.batch_inner;
+    const int64_t work = g.M * g.N * g.K * g.batch_outer * g.batch_inner * g.k_groups;
     if (ctx->gemm_engine == 1 || (ctx->gemm_engine == 0 && work < kSmallWork)) return gemm_simt_launch(ctx, ta, tb, g);
     int rc = GCB_UNSUPPORTED;
     if (gemm_tc_eligible(g)) rc = gemm_tc_launch(ctx, ta, tb, g);
+    if (rc == GCB_UNSUPPORTED && g.grouped) return rc;  // the caller takes the layers one by one
     // operands that only their addresses keep from the tensor cores are copied into rows that suit them (~3 us each)
     if (rc == GCB_UNSUPPORTED && ctx->gemm_engine == 0 && g.batch_outer * g.batch_inner <= 65535) {
         GemmArgs packed = g;
@@ -134,7 +135,7 @@ static int run_gemm(gcb_ctx* ctx, int op_a, int op_b, const GemmArgs& g, const c
     GCB_CHECK_CUDA(cudaEventRecord(e1, ctx->stream));
     if (rc == GCB_OK) {  // a refused problem leaves no trace in the tally
         ctx->prof_used += 2;
-        ctx->prof_flops += 2.0 * (double)g.M * (double)g.N * (double)g.K * (double)(g.batch_outer * g.batch_inner);
+        ctx->prof_flops += 2.0 * (double)g.M * (double)g.N * (double)g.K * (double)(g.batch_outer * g.batch_inner * g.k_groups);
     }
     return rc;
 }
@@ -218,6 +219,54 @@ int gcb_linear_residual_f32(gcb_ctx* ctx, int op_b, int64_t M, int64_t N, int64_
     GemmArgs g{M, N, K, 1.0f, 0.0f, x, W, bias, out, lda, ldb, N, 0, 0, 0, 0, 0, 0, 1, 1};
     g.residual = residual;
     return run_gemm(ctx, GCB_OP_N, op_b, g, "gcb_linear_residual_f32");
+}
+
+// Linear layers of one shape over one input in one launch each way (q, k and v; the two halves of a SwiGLU).  A layer by itself leaves
+// the last round of tiles nearly empty and small ones are bound by launches: 4096 x 768 x 768 is 48 pair tiles on 74 pairs, three
+// layers are 144 on two full rounds.
+int gcb_linear_group_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* x, const float* W, int64_t w_stride, const float* bias, int64_t bias_stride, float* y, int64_t y_stride) {
+    GCB_REQUIRE(ctx && groups >= 1 && groups <= 64, "gcb_linear_group_f32: bad arguments");
+    GemmArgs g{M, N, K, 1.0f, 0.0f, x, W, bias, y, K, N, N, 0, 0, 0, w_stride, 0, y_stride, 1, groups};
+    g.grouped = true;
+    g.bias_si = bias_stride;
+    int rc = run_gemm(ctx, GCB_OP_N, GCB_OP_N, g, "gcb_linear_group_f32");
+    if (rc == GCB_UNSUPPORTED)
+        for (int64_t i = 0; i < groups; ++i) {
+            rc = gcb_gemm_f32(ctx, GCB_OP_N, GCB_OP_N, M, N, K, 1.0f, x, K, W + i * w_stride, N, 0.0f, y + i * y_stride, N, bias ? bias + i * bias_stride : nullptr);
+            if (rc) return rc;
+        }
+    return rc;
+}
+
+int gcb_linear_group_dx_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* dy, int64_t dy_stride, const float* W, int64_t w_stride, float beta, float* dx) {
+    GCB_REQUIRE(ctx && groups >= 1 && groups <= 64, "gcb_linear_group_dx_f32: bad arguments");
+    GemmArgs g{M, K, N, 1.0f, beta, dy, W, nullptr, dx, N, N, K, 0, dy_stride, 0, w_stride, 0, 0, 1, 1};
+    g.grouped = true;
+    g.k_groups = (int)groups;
+    int rc = dy_stride > 0 && dy_stride % 4 == 0 && w_stride > 0 && w_stride % 4 == 0 ? run_gemm(ctx, GCB_OP_N, GCB_OP_T, g, "gcb_linear_group_dx_f32") : GCB_UNSUPPORTED;
+    if (rc == GCB_UNSUPPORTED)
+        for (int64_t i = 0; i < groups; ++i) {
+            rc = gcb_gemm_f32(ctx, GCB_OP_N, GCB_OP_T, M, K, N, 1.0f, dy + i * dy_stride, N, W + i * w_stride, N, i ? 1.0f : beta, dx, K, nullptr);
+            if (rc) return rc;
+        }
+    return rc;
+}
+
+int gcb_linear_group_dw_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* x, const float* dy, int64_t dy_stride, float beta, float* dW, int64_t w_stride, float* dbias,
+                            int64_t bias_stride, int bias_accumulate) {
+    GCB_REQUIRE(ctx && groups >= 1 && groups <= 64 && (N == 0 || dbias), "gcb_linear_group_dw_f32: bad arguments");
+    GemmArgs g{K, N, M, 1.0f, beta, x, dy, nullptr, dW, K, N, N, 0, 0, 0, dy_stride, 0, w_stride, 1, groups};
+    g.grouped = true;
+    g.colsum = dbias;
+    g.colsum_si = bias_stride;
+    g.colsum_accumulate = bias_accumulate;
+    int rc = M > 0 && K > 0 ? run_gemm(ctx, GCB_OP_T, GCB_OP_N, g, "gcb_linear_group_dw_f32") : GCB_UNSUPPORTED;
+    if (rc == GCB_UNSUPPORTED)
+        for (int64_t i = 0; i < groups; ++i) {
+            rc = gcb_gemm_colsum_f32(ctx, GCB_OP_T, K, N, M, 1.0f, x, K, dy + i * dy_stride, beta, dW + i * w_stride, N, dbias + i * bias_stride, bias_accumulate);
+            if (rc) return rc;
+        }
+    return rc;
 }
 
 int gcb_profile_gemm_begin(gcb_ctx* ctx) {

@@ -31,6 +31,12 @@ struct GemmArgs {
     // (+ colsum[n] when colsum_accumulate).  Unbatched problems only.
     float* colsum = nullptr;
     int colsum_accumulate = 0;
+    // Several linear layers of one shape over the same input (inner batch items; batch_outer == 1, causal == 0).  grouped: bias and column
+    // sums move with the item by bias_si / colsum_si, and a_si == 0 means that A is shared.  k_groups > 1 (one item, C = sum over g):
+    // K is walked once per group, A and B moving by a_si / b_si.
+    bool grouped = false;
+    int64_t bias_si = 0, colsum_si = 0;
+    int k_groups = 1;
 };
 
 // fp32 FMA engine: any shape, any leading dimension, every epilogue.

@@ -86,7 +86,9 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
     // writes the zeros of those blocks, which take no product
     const bool above = g.causal == 1 && n0 > m0 + BM - 1;
     if (above && (g.sm_probs == nullptr || n0 >= (m0 / 128 + 1) * 128)) return;  // the whole cluster
-    int64_t k_begin = 0, k_end = above ? 0 : g.K;
+    // K over several operand pairs: walked as if every group's K were whole blocks
+    const int64_t per_group = (g.K + SG_BK - 1) / SG_BK * SG_BK;
+    int64_t k_begin = 0, k_end = above ? 0 : g.k_groups > 1 ? per_group * g.k_groups : g.K;
     if (g.causal == 2) k_end = min(g.K, m0 + BM);
     else if (g.causal == 3) k_begin = min(g.K, m0);
     {
@@ -99,9 +101,16 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
     auto load = [&](int i) {
         if (i < nblk) {
             float* st = sg + (i % S::STAGES) * 2 * S::OP;
-            const int64_t k0 = k_begin + (int64_t)i * SG_BK;
-            sg_load<BM, !TA>(st, A, g.lda, m0, g.M, k0, k_end, a_vec);
-            sg_load<BM, TB>(st + S::OP, B, g.ldb, n0, g.N, k0, k_end, b_vec);
+            int64_t k0 = k_begin + (int64_t)i * SG_BK, last = k_end;
+            const float *pa = A, *pb = B;
+            if (g.k_groups > 1) {
+                const int64_t q = k0 / per_group;
+                k0 -= q * per_group;
+                last = g.K;
+                pa += q * g.a_si; pb += q * g.b_si;
+            }
+            sg_load<BM, !TA>(st, pa, g.lda, m0, g.M, k0, last, a_vec);
+            sg_load<BM, TB>(st + S::OP, pb, g.ldb, n0, g.N, k0, last, b_vec);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -207,7 +216,7 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
         float act[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            if (g.bias && e < live) o[e] += g.bias[n + e];
+            if (g.bias && e < live) o[e] += g.bias[bi * g.bias_si + n + e];
             if (g.beta != 0.0f) o[e] += g.beta * old[e];
             if (g.residual) o[e] += side[e];
             else if (g.gelu_pre) o[e] *= gelu_grad_f(side[e]);
@@ -230,7 +239,7 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
             else asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote(cols + t, r)) : "memory");
             s += x;
         }
-        float* d = g.colsum + n0 + t;
+        float* d = g.colsum + bi * g.colsum_si + n0 + t;
         *d = g.colsum_accumulate ? *d + s : s;
     }
     if (slices > 1) {  // nobody leaves while its shared memory is still read
@@ -242,7 +251,7 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
 template <int BM, bool TA, bool TB>
 static int sg_launch(gcb_ctx* ctx, const GemmArgs& g, int64_t tiles_m, int64_t tiles_n, int64_t batches, int slices) {
     auto ok4 = [](int64_t v) { return v % 4 == 0; };
-    auto vec = [&](const float* p, int64_t ld, int64_t so, int64_t si) { return aligned16(p) && ok4(ld) && (g.batch_inner == 1 || ok4(si)) && (g.batch_outer == 1 || ok4(so)); };
+    auto vec = [&](const float* p, int64_t ld, int64_t so, int64_t si) { return aligned16(p) && ok4(ld) && ((g.batch_inner == 1 && g.k_groups == 1) || ok4(si)) && (g.batch_outer == 1 || ok4(so)); };
     const bool c_vec = vec(g.C, g.ldc, g.c_so, g.c_si) && aligned16(g.residual) && aligned16(g.gelu_pre) && aligned16(g.gelu_act) && aligned16(g.sm_probs);
     auto kfn = gemm_simt_kernel<BM, TA, TB>;
     constexpr size_t smem = sizeof(float) * SgSmem<BM>::FLOATS;
@@ -277,7 +286,8 @@ int gemm_simt_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     // K is cut while SMs are left over and every slice keeps two K blocks; beyond one CTA per SM only for slices of 96 and more
     // (256 x 512 x 128: one slice 5.5 us, two 6.4; 256 x 256 x 512: one 10.8, two 8.3, four 7.7, eight 12.9)
     int slices = 1;
-    while (slices < 8 && g.K >= (int64_t)slices * 2 * 2 * SG_BK && tiles(bm) * slices * 2 <= (g.K >= (int64_t)slices * 2 * 96 ? 2 * kSMs : kSMs)) slices *= 2;
+    const int64_t K = g.K * g.k_groups;
+    while (slices < 8 && K >= (int64_t)slices * 2 * 2 * SG_BK && tiles(bm) * slices * 2 <= (K >= (int64_t)slices * 2 * 96 ? 2 * kSMs : kSMs)) slices *= 2;
     cudaSetDevice(ctx->device);
     int rc;
 #define GCB_SG(BMV) (!ta && !tb ? sg_launch<BMV, false, false>(ctx, g, tm, tn, batches, slices) : !ta ? sg_launch<BMV, false, true>(ctx, g, tm, tn, batches, slices) \

@@ -54,12 +54,15 @@ struct TcParams {
     int split_mode;      // 2 (default): one TF32 product of the truncated parts + two BF16 cross products (split_hybrid below);
                          // 1: three TF32 products; big stays as loaded — the tensor core ignores the 13 low mantissa bits — and small = rna_tf32(x - trunc(x));
                          // 0: as 1 with big = rna_tf32(x) written back, small = x - big (does not rely on the hardware's truncation)
-    float* partial;      // [splits][M][partial_ld] when splits > 1
+    float* partial;      // [splits][batches][M][partial_ld] when splits > 1
     int64_t partial_ld;  // N rounded up to a multiple of four: whole vectors whatever N is
     int b_twin;              // pair kernel and narrow tiles: the BF16 companions of B come pre-split from global memory (map_t), the B-splitter warps idle
     int c_tma;               // 256-wide single-CTA kernel: C leaves (and the probabilities arrive) through TMA on swizzled 32 x 32 blocks in shared memory
     float* colsum;           // column sums of op(B) (see GemmArgs), or NULL: pair kernel with B stored K x N only
-    float* colsum_partial;   // [splits][N] when splits > 1
+    float* colsum_partial;   // [splits][batches][N] when splits > 1
+    int64_t bias_si, colsum_si;  // grouped linear layers: what bias and column sums move by per inner batch item
+    int a_batched;           // 0: every batch item reads the same A
+    int k_group_blocks;      // K blocks per group where K runs over several operand pairs (coordinate: the inner batch), or 0
     int colsum_accumulate;
     const float* gelu_pre;   // GELU-backward epilogue (see GemmArgs), or NULL: applied by the pair kernel only
     float* gelu_act;         // GELU-forward second output (see GemmArgs), or NULL: pair kernel only
@@ -168,6 +171,14 @@ struct TileCoord {
     int m0, n0, b_in, b_out, split, kb0, nkb;
     bool skip;
 };
+// K block kb of a tile -> first k and the inner batch coordinates of the two operands
+struct KCoord {
+    int k0, a_in, b_in;
+};
+__device__ __forceinline__ KCoord k_coord(const TcParams& p, const TileCoord& t, int kb) {
+    const int g = p.k_group_blocks ? kb / p.k_group_blocks : 0;
+    return {(kb - g * p.k_group_blocks) * TC_BK, t.b_in * p.a_batched + g, t.b_in + g};
+}
 constexpr int TC_GROUP_M = 16;  // row tiles per raster panel: the panel's A rows and the B tiles it sweeps stay hot in L2
 // Column tiles of row tile i that are not entirely above the diagonal (causal mode 1).
 __host__ __device__ __forceinline__ int causal_kept_cols(int i, int tiles_n, int BN) { return min(tiles_n, ((i + 1) * TC_BM + BN - 1) / BN); }
@@ -282,23 +293,24 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
                     const uint32_t sa = base + s * S::STAGE_BYTES, sb = sa + S::B_OFF;
                     const bool twin = A_TM && p.b_twin != 0;
                     mbar_expect_tx(full_bar(s), S::A_BYTES + S::B_BYTES + (twin ? S::B_BYTES : 0));
-                    const int k0 = (tc.kb0 + i) * TC_BK;
-                    if (twin) tma_load_3d(sb + S::B_BYTES, &map_p, full_bar(s), (k0 >> 3) * 64, tc.n0 >> 3, 0);  // the weight's companions, as in the pair kernel (map_p: these kernels read no probabilities)
+                    const KCoord kc = k_coord(p, tc, tc.kb0 + i);
+                    const int k0 = kc.k0;
+                    if (twin) tma_load_4d(sb + S::B_BYTES, &map_p, full_bar(s), (k0 >> 3) * 64, tc.n0 >> 3, 0, kc.b_in);  // the weight's companions, as in the pair kernel (map_p: these kernels read no probabilities)
                     if (A_MN) {
-                        if (p.a_chunked) tma_load_5d(sa, &map_a, full_bar(s), 0, k0, tc.m0 / 32, tc.b_in, tc.b_out);
+                        if (p.a_chunked) tma_load_5d(sa, &map_a, full_bar(s), 0, k0, tc.m0 / 32, kc.a_in, tc.b_out);
                         else
 #pragma unroll
-                        for (int c = 0; c < TC_BM / 32; ++c) tma_load_4d(sa + c * 2048, &map_a, full_bar(s), tc.m0 + 32 * c, k0, tc.b_in, tc.b_out);
+                        for (int c = 0; c < TC_BM / 32; ++c) tma_load_4d(sa + c * 2048, &map_a, full_bar(s), tc.m0 + 32 * c, k0, kc.a_in, tc.b_out);
                     } else {
-                        tma_load_4d(sa, &map_a, full_bar(s), k0, tc.m0, tc.b_in, tc.b_out);
+                        tma_load_4d(sa, &map_a, full_bar(s), k0, tc.m0, kc.a_in, tc.b_out);
                     }
                     if (B_MN) {
-                        if (p.b_chunked) tma_load_5d(sb, &map_b, full_bar(s), 0, k0, tc.n0 / 32, tc.b_in, tc.b_out);
+                        if (p.b_chunked) tma_load_5d(sb, &map_b, full_bar(s), 0, k0, tc.n0 / 32, kc.b_in, tc.b_out);
                         else
 #pragma unroll
-                        for (int c = 0; c < BN / 32; ++c) tma_load_4d(sb + c * 2048, &map_b, full_bar(s), tc.n0 + 32 * c, k0, tc.b_in, tc.b_out);
+                        for (int c = 0; c < BN / 32; ++c) tma_load_4d(sb + c * 2048, &map_b, full_bar(s), tc.n0 + 32 * c, k0, kc.b_in, tc.b_out);
                     } else {
-                        tma_load_4d(sb, &map_b, full_bar(s), k0, tc.n0, tc.b_in, tc.b_out);
+                        tma_load_4d(sb, &map_b, full_bar(s), k0, tc.n0, kc.b_in, tc.b_out);
                     }
                 }
             }
@@ -497,8 +509,9 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
                         float4 o = make_float4(v[4 * e] * p.alpha, v[4 * e + 1] * p.alpha, v[4 * e + 2] * p.alpha, v[4 * e + 3] * p.alpha);
                         const int64_t n = nb + 4 * e;
                         if (p.bias != nullptr) {
-                            o.x += n + 0 < p.N ? __ldg(p.bias + n + 0) : 0.0f; o.y += n + 1 < p.N ? __ldg(p.bias + n + 1) : 0.0f;
-                            o.z += n + 2 < p.N ? __ldg(p.bias + n + 2) : 0.0f; o.w += n + 3 < p.N ? __ldg(p.bias + n + 3) : 0.0f;
+                            const float* bias = p.bias + tc.b_in * p.bias_si;
+                            o.x += n + 0 < p.N ? __ldg(bias + n + 0) : 0.0f; o.y += n + 1 < p.N ? __ldg(bias + n + 1) : 0.0f;
+                            o.z += n + 2 < p.N ? __ldg(bias + n + 2) : 0.0f; o.w += n + 3 < p.N ? __ldg(bias + n + 3) : 0.0f;
                         }
                         if (has_p) {  // dS = scale * P * (dP - rowdot), zero above the diagonal
                             const float4 pr = *slot;
@@ -532,7 +545,7 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
         const bool to_partial = p.splits > 1;
         // the float4 fast path needs every array the epilogue touches with vector accesses on 16-byte boundaries: C and, laid out like C, the probabilities
         const bool vec_ok = to_partial || (p.ldc % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.sm_probs) | (uintptr_t)(p.c_so * 4) | (uintptr_t)(p.c_si * 4)) & 15) == 0);
-        const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+        const bool bias_vec = ((reinterpret_cast<uintptr_t>(p.bias) | (uintptr_t)(p.bias_si * 4)) & 15) == 0;
         const int sub_r = lane >> 3, sub_c = (lane & 7) * 4;  // store phase: 4 rows x 8 float4 per instruction (128 B per row)
         uint32_t lt = 0;
         bool ok = true;
@@ -541,10 +554,10 @@ __global__ void __launch_bounds__(TcSmem<BN, A_TM>::THREADS, (BN == 64 ? 2 : 1))
             const TileCoord tc = tile_coord(p, w, BN);
             if (tc.skip) continue;
             const uint32_t buf = lt % S::NACC;
-            float* cbase = to_partial ? p.partial + (int64_t)tc.split * p.M * p.partial_ld : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
+            float* cbase = to_partial ? p.partial + ((int64_t)tc.split * p.batches + tc.b_in) * p.M * p.partial_ld : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
             const int64_t ld = to_partial ? p.partial_ld : p.ldc;
             const float alpha = to_partial ? 1.0f : p.alpha, beta = to_partial ? 0.0f : p.beta;
-            const float* bias = to_partial ? nullptr : p.bias;
+            const float* bias = to_partial || p.bias == nullptr ? nullptr : p.bias + tc.b_in * p.bias_si;
             const float* sm_probs = (BN == 256 && !to_partial) ? p.sm_probs : nullptr;  // only the 256-wide instantiation carries this epilogue (the launcher sees to it)
             const float* sm_rd = p.sm_rowdot + ((int64_t)tc.b_out * p.batch_inner + tc.b_in) * p.M;
             // a triangular output is consumed in 128-wide diagonal blocks: columns right of this row tile's block are not written
@@ -731,13 +744,13 @@ __device__ __forceinline__ TileCoord pair_tile_coord(const TcParams& p, int64_t 
 
 // One column of a 32-row block that cannot be stored in whole vectors.  Kept out of line: inlined it costs the epilogue of whole
 // blocks a dozen registers (spills) and the step 5 %.
-__device__ __noinline__ void pair_ragged_column(const TcParams& p, const float* staged, float* d, int64_t ld, int rows, int64_t n, bool to_partial) {
+__device__ __noinline__ void pair_ragged_column(const TcParams& p, const float* staged, float* d, int64_t ld, int rows, int64_t n, bool to_partial, const float* bias) {
     const float alpha = to_partial ? 1.0f : p.alpha, beta = to_partial ? 0.0f : p.beta;
     const bool epi = !to_partial;
-    const float b = epi && p.bias ? p.bias[n] : 0.0f;
+    const float b = bias ? bias[n] : 0.0f;
     for (int r0 = 0; r0 < rows; ++r0, d += ld) {
         float r = staged[r0 * PairSmemT<true>::EPI_PITCH] * alpha;
-        if (epi && p.bias) r += b;
+        if (bias) r += b;
         if (beta != 0.0f) r += beta * *d;
         if (epi && p.gelu_pre) r *= gelu_grad_f(p.gelu_pre[d - p.C]);
         if (epi && p.resid) r += p.resid[d - p.C];
@@ -802,24 +815,25 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
                     const uint32_t sa = base + s * S::STAGE_BYTES, sb = sa + S::B_OFF;
                     const bool twin = A_TM && p.b_twin != 0;
                     mbar_expect_tx(full_bar(s), S::A_BYTES + S::B_BYTES + (twin ? S::B_BYTES : 0));
-                    const int k0 = (tc.kb0 + i) * TC_BK;
+                    const KCoord kc = k_coord(p, tc, tc.kb0 + i);
+                    const int k0 = kc.k0;
                     // this CTA's 128 columns of the pre-split companions: 16 groups of 8 columns x 2 chunks of 8 k, big then small
-                    if (twin) tma_load_3d(sb + S::B_BYTES, &map_t, full_bar(s), (k0 >> 3) * 64, n0 >> 3, 0);
+                    if (twin) tma_load_4d(sb + S::B_BYTES, &map_t, full_bar(s), (k0 >> 3) * 64, n0 >> 3, 0, kc.b_in);
                     if (A_MN) {
-                        if (p.a_chunked) tma_load_5d(sa, &map_a, full_bar(s), 0, k0, m0 / 32, tc.b_in, tc.b_out);
+                        if (p.a_chunked) tma_load_5d(sa, &map_a, full_bar(s), 0, k0, m0 / 32, kc.a_in, tc.b_out);
                         else
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) tma_load_4d(sa + c * 2048, &map_a, full_bar(s), m0 + 32 * c, k0, tc.b_in, tc.b_out);
+                        for (int c = 0; c < 4; ++c) tma_load_4d(sa + c * 2048, &map_a, full_bar(s), m0 + 32 * c, k0, kc.a_in, tc.b_out);
                     } else {
-                        tma_load_4d(sa, &map_a, full_bar(s), k0, m0, tc.b_in, tc.b_out);
+                        tma_load_4d(sa, &map_a, full_bar(s), k0, m0, kc.a_in, tc.b_out);
                     }
                     if (B_MN) {
-                        if (p.b_chunked) tma_load_5d(sb, &map_b, full_bar(s), 0, k0, n0 / 32, tc.b_in, tc.b_out);
+                        if (p.b_chunked) tma_load_5d(sb, &map_b, full_bar(s), 0, k0, n0 / 32, kc.b_in, tc.b_out);
                         else
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) tma_load_4d(sb + c * 2048, &map_b, full_bar(s), n0 + 32 * c, k0, tc.b_in, tc.b_out);
+                        for (int c = 0; c < 4; ++c) tma_load_4d(sb + c * 2048, &map_b, full_bar(s), n0 + 32 * c, k0, kc.b_in, tc.b_out);
                     } else {
-                        tma_load_4d(sb, &map_b, full_bar(s), k0, n0, tc.b_in, tc.b_out);
+                        tma_load_4d(sb, &map_b, full_bar(s), k0, n0, kc.b_in, tc.b_out);
                     }
                 }
             }
@@ -946,8 +960,9 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
             if (want_colsum && ok) {
                 const int64_t n = (int64_t)tc.n0 + 128 * (int)rank + t;
                 if (n < p.N) {
-                    if (p.splits > 1) p.colsum_partial[(int64_t)tc.split * p.N + n] = colsum_acc;  // summed over the K slices, in slice order, by the reduce kernel
-                    else p.colsum[n] = p.colsum_accumulate ? p.colsum[n] + colsum_acc : colsum_acc;
+                    float* sum = p.colsum + tc.b_in * p.colsum_si + n;
+                    if (p.splits > 1) p.colsum_partial[((int64_t)tc.split * p.batches + tc.b_in) * p.N + n] = colsum_acc;  // summed over the K slices, in slice order, by the reduce kernel
+                    else *sum = p.colsum_accumulate ? *sum + colsum_acc : colsum_acc;
                 }
             }
         }
@@ -962,7 +977,7 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
         // the float4 fast path needs C and the GELU side arrays (laid out like C) on 16-byte boundaries; otherwise the scalar path runs
         const bool vec_ok = to_partial || (p.ldc % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.gelu_pre) | reinterpret_cast<uintptr_t>(p.gelu_act) | reinterpret_cast<uintptr_t>(p.resid) |
                                                               (uintptr_t)(p.c_so * 4) | (uintptr_t)(p.c_si * 4)) & 15) == 0);
-        const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+        const bool bias_vec = ((reinterpret_cast<uintptr_t>(p.bias) | (uintptr_t)(p.bias_si * 4)) & 15) == 0;
         const int sub_r = lane >> 3, sub_c = (lane & 7) * 4;
         uint32_t lt = 0;
         bool ok = true;
@@ -970,10 +985,10 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
             const TileCoord tc = pair_tile_coord(p, w);
             if (tc.skip) continue;
             const uint32_t buf = lt % NACC;
-            float* cbase = to_partial ? p.partial + (int64_t)tc.split * p.M * p.partial_ld : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
+            float* cbase = to_partial ? p.partial + ((int64_t)tc.split * p.batches + tc.b_in) * p.M * p.partial_ld : p.C + (int64_t)tc.b_out * p.c_so + (int64_t)tc.b_in * p.c_si;
             const int64_t ld = to_partial ? p.partial_ld : p.ldc;
             const float alpha = to_partial ? 1.0f : p.alpha, beta = to_partial ? 0.0f : p.beta;
-            const float* bias = to_partial ? nullptr : p.bias;
+            const float* bias = to_partial || p.bias == nullptr ? nullptr : p.bias + tc.b_in * p.bias_si;
             const float* gelu_pre = to_partial ? nullptr : p.gelu_pre;
             float* gelu_act = to_partial ? nullptr : p.gelu_act;
             const float* resid = to_partial ? nullptr : p.resid;
@@ -1029,7 +1044,7 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
                         }
                     } else {  // ragged or unaligned block: lane = column, as in the single-CTA kernel
                         const int64_t nc = nb + lane;
-                        if (nc < p.N && mrow0 < p.M) pair_ragged_column(p, stg + lane, cbase + mrow0 * ld + nc, ld, (int)min((int64_t)32, p.M - mrow0), nc, to_partial);
+                        if (nc < p.N && mrow0 < p.M) pair_ragged_column(p, stg + lane, cbase + mrow0 * ld + nc, ld, (int)min((int64_t)32, p.M - mrow0), nc, to_partial, bias);
                     }
                 }
                 __syncwarp();
@@ -1053,25 +1068,28 @@ __global__ void __launch_bounds__(PairSmemT<A_TM>::THREADS, 1) gemm_tc_pair_kern
 // serialisation behind the GEMM that wrote the partial tiles: its blocks may be scheduled while that grid drains, and
 // nothing is read before the grid has completed.  A thread takes four columns of one row (the partial rows are padded to whole
 // vectors); `vec` = C can be accessed as float4 too, otherwise its elements are touched one by one.
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ C, const float* __restrict__ partial, int64_t partial_ld, const float* __restrict__ bias, int64_t M, int64_t N,
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ C, const float* __restrict__ partial, int64_t partial_ld, const float* __restrict__ bias_all, int64_t M, int64_t N,
                                                             int64_t ldc, int splits, float alpha, float beta, float* __restrict__ colsum, const float* __restrict__ colsum_partial,
-                                                            int colsum_accumulate, int vec) {
+                                                            int colsum_accumulate, int vec, int batches, int64_t c_si, int64_t bias_si, int64_t colsum_si) {
     pdl_trigger();
     pdl_wait();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
     if (colsum != nullptr) {  // the column sums of op(B), one partial per K slice
-        for (int64_t n = tid; n < N; n += nthreads) {
+        for (int64_t i = tid; i < N * batches; i += nthreads) {
             float s = 0.0f;
-            for (int k = 0; k < splits; ++k) s += colsum_partial[(int64_t)k * N + n];
-            colsum[n] = colsum_accumulate ? colsum[n] + s : s;
+            for (int k = 0; k < splits; ++k) s += colsum_partial[(int64_t)k * N * batches + i];
+            const int64_t b = i / N;
+            float* sum = colsum + b * colsum_si + (i - b * N);
+            *sum = colsum_accumulate ? *sum + s : s;
         }
     }
-    const int64_t n4 = partial_ld >> 2, total4 = M * n4;
+    const int64_t n4 = partial_ld >> 2, total4 = M * n4 * batches;
     for (int64_t i = tid; i < total4; i += nthreads) {
-        const int64_t m = i / n4, n = (i - m * n4) << 2;
+        const int64_t r = i / n4, n = (i - r * n4) << 2, b = batches > 1 ? r / M : 0, m = r - b * M;
         const float4* src = reinterpret_cast<const float4*>(partial) + i;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        float* dst = C + m * ldc + n;
+        float* dst = C + b * c_si + m * ldc + n;
+        const float* bias = bias_all ? bias_all + b * bias_si : nullptr;
         int k = 0;
         for (; k + 4 <= splits; k += 4) {  // four slices' loads in flight
             float4 v[4];
@@ -1153,7 +1171,7 @@ bool gemm_tc_eligible(const GemmArgs& g) {
     if (g.K < 1 || g.M < 1 || g.N < 1) return false;
     if (!aligned16(g.A) || !aligned16(g.B)) return false;
     if (!ok4(g.lda) || !ok4(g.ldb)) return false;
-    if (g.batch_inner > 1 && (!ok4(g.a_si) || !ok4(g.b_si) || g.a_si <= 0 || g.b_si <= 0)) return false;
+    if (g.batch_inner > 1 && (!ok4(g.a_si) || !ok4(g.b_si) || (g.a_si <= 0 && !(g.grouped && g.a_si == 0)) || g.b_si <= 0)) return false;
     if (g.batch_outer > 1 && (!ok4(g.a_so) || !ok4(g.b_so) || g.a_so <= 0 || g.b_so <= 0)) return false;
     if (g.M > (int64_t(1) << 30) || g.N > (int64_t(1) << 30) || g.K > (int64_t(1) << 30)) return false;
     if (g.batch_outer * g.batch_inner > 65535) return false;
@@ -1239,16 +1257,17 @@ struct TcTiling {
     int splits;
     double us;
 };
-static void consider(TcTiling& best, const GemmArgs& g, int BN, bool pair, bool may_split) {
-    const int64_t tiles = pair ? ((g.M + 255) / 256) * ((g.N + 255) / 256) : ((g.M + TC_BM - 1) / TC_BM) * ((g.N + BN - 1) / BN);
+static void consider(TcTiling& best, const GemmArgs& g, int BN, bool pair, bool may_split, int max_kbs) {
+    const int64_t tiles = g.batch_inner * (pair ? ((g.M + 255) / 256) * ((g.N + 255) / 256) : ((g.M + TC_BM - 1) / TC_BM) * ((g.N + BN - 1) / BN));
     const int kb = (int)((g.K + TC_BK - 1) / TC_BK);
-    for (int sp = 1; sp <= 32 && (sp == 1 || (may_split && kb >= 32 && kb / sp >= 8)); ++sp) {
-        const int kbs = (kb + sp - 1) / sp;
+    for (int s = 1; s <= 32 && (s == 1 || (may_split && kb >= 32 && kb / s >= 8)); ++s) {
+        const int kbs = (kb + s - 1) / s, sp = s * g.k_groups;
+        if (kbs > max_kbs) continue;
         const int64_t items = tiles * sp;
         const double per_block = pair ? 0.42 : BN == 64 && items > kSMs ? 0.5 : 0.4;  // two 64-wide CTAs of one SM share its splitters' issue slots
         const int64_t slots = pair ? kSMs / 2 : BN == 64 ? 2 * kSMs : kSMs, rounds = (items + slots - 1) / slots;
-        const double us = (pair ? 13.0 : 5.0) + (double)rounds * (kbs * per_block + (pair ? 2.0 : 1.0)) + (sp > 1 ? 4.0 + (double)sp * (double)(g.M * g.N) * 8.0 / 5.0e6 : 0.0);
-        if (us < best.us * 0.97) best = {BN, pair, sp, us};
+        const double us = (pair ? 13.0 : 5.0) + (double)rounds * (kbs * per_block + (pair ? 2.0 : 1.0)) + (sp > 1 ? 4.0 + (double)sp * (double)(g.M * g.N * g.batch_inner) * 8.0 / 5.0e6 : 0.0);
+        if (us < best.us * 0.97) best = {BN, pair, s, us};
     }
 }
 
@@ -1260,21 +1279,36 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     static const int pair_env = [] { const char* e = getenv("GRADC_TC_PAIR"); return e ? atoi(e) : 1; }();
     const bool by_width = g.N > 128 || g.sm_probs;
     const bool pair_ok = pair_env != 0 && by_width && g.M > 128 && g.K >= 256 && !g.sm_probs;  // short K loops are epilogue-bound: nothing to gain from sharing B
-    TcTiling tl{by_width ? 256 : (g.N > 64 ? 128 : 64), pair_ok, 1, 1e30};
-    if (batches == 1 && g.causal == 0 && !g.sm_probs) {
+    const TcTiling by_default{by_width ? 256 : (g.N > 64 ? 128 : 64), pair_ok, 1, 1e30};
+    auto choose = [&](const GemmArgs& q, int max_kbs) {
+        TcTiling t = by_default;
         const bool side = g.gelu_pre || g.gelu_act || g.residual;  // these epilogues and the column sums are the pair kernel's, and an epilogue sees whole sums
-        consider(tl, g, tl.BN, tl.pair, !side);
+        consider(t, q, t.BN, t.pair, !side, max_kbs);
         if (pair_ok && !side && !g.colsum && ctx->gemm_split_mode == 2) {
-            consider(tl, g, 128, false, true);
-            consider(tl, g, 64, false, true);
+            consider(t, q, 128, false, true, max_kbs);
+            consider(t, q, 64, false, true, max_kbs);
         }
+        return t;
+    };
+    TcTiling tl = by_default;
+    if (g.grouped) {
+        // no sum is longer than the layer's own would be (the tensor core's accumulator truncates), so a K over several operand
+        // pairs is cut between them; where that costs more than the layers one by one, the caller takes those
+        GemmArgs one = g;
+        one.batch_inner = one.k_groups = 1;
+        const TcTiling t1 = choose(one, 1 << 30);
+        const int kb = (int)((g.K + TC_BK - 1) / TC_BK);
+        tl = choose(g, (kb + t1.splits - 1) / t1.splits);
+        if (g.k_groups > 1 && t1.us * g.k_groups <= tl.us) return GCB_UNSUPPORTED;
+    } else if (batches == 1 && g.causal == 0 && !g.sm_probs) {
+        tl = choose(g, 1 << 30);
     }
     const int BN = tl.BN;
     const bool use_pair = tl.pair;
     CUtensorMap ma, mb;
     TcParams p;
-    if (!encode_operand(enc, &ma, g.A, ta, g.M, g.K, g.lda, g.a_si, g.a_so, g.batch_inner, g.batch_outer, TC_BM, &p.a_chunked)) return GCB_UNSUPPORTED;
-    if (!encode_operand(enc, &mb, g.B, !tb, g.N, g.K, g.ldb, g.b_si, g.b_so, g.batch_inner, g.batch_outer, use_pair ? 128 : BN, &p.b_chunked)) return GCB_UNSUPPORTED;
+    if (!encode_operand(enc, &ma, g.A, ta, g.M, g.K, g.lda, g.a_si, g.a_so, g.grouped ? (g.a_si == 0 ? 1 : g.batch_inner * g.k_groups) : g.batch_inner, g.batch_outer, TC_BM, &p.a_chunked)) return GCB_UNSUPPORTED;
+    if (!encode_operand(enc, &mb, g.B, !tb, g.N, g.K, g.ldb, g.b_si, g.b_so, g.batch_inner * g.k_groups, g.batch_outer, use_pair ? 128 : BN, &p.b_chunked)) return GCB_UNSUPPORTED;
     p.M = g.M; p.N = g.N; p.K = g.K;
     p.alpha = g.alpha; p.beta = g.beta; p.bias = g.bias; p.C = g.C;
     p.ldc = g.ldc; p.c_so = g.c_so; p.c_si = g.c_si;
@@ -1282,6 +1316,7 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     p.tiles_n = (int)((g.N + BN - 1) / BN);
     p.tiles_m = use_pair ? (int)((g.M + 255) / 256) : (int)((g.M + TC_BM - 1) / TC_BM);
     p.k_blocks_total = (int)((g.K + TC_BK - 1) / TC_BK);
+    p.bias_si = g.bias_si; p.colsum_si = g.colsum_si; p.a_batched = g.grouped && g.a_si == 0 ? 0 : 1;
     p.status = ctx->d_status;
 #ifdef GCB_TC_TRACE
     p.dbg = getenv("GRADC_TC_DBG") ? atoi(getenv("GRADC_TC_DBG")) : 0;
@@ -1292,7 +1327,7 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     static const int pair_tmem_env = [] { const char* e = getenv("GRADC_TC_PAIR_ATMEM"); return e ? atoi(e) : 1; }();
     const bool pair_a_tmem = pair_tmem_env != 0 && ctx->gemm_split_mode == 2;
     // column sums of op(B): gathered by the B-splitter warps of the pair kernel (A through tensor memory) from B stored K x N
-    if (g.colsum && !(use_pair && pair_a_tmem && !tb && batches == 1)) return GCB_UNSUPPORTED;
+    if (g.colsum && !(use_pair && pair_a_tmem && !tb && (batches == 1 || g.grouped))) return GCB_UNSUPPORTED;
     p.colsum = g.colsum; p.colsum_accumulate = g.colsum_accumulate; p.colsum_partial = nullptr;
     const int64_t tiles = (int64_t)p.tiles_n * p.tiles_m * batches;
     if (tiles > 2147483647LL / 2) return GCB_UNSUPPORTED;
@@ -1300,14 +1335,20 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     p.splits = splits;
     p.k_blocks_per_split = (p.k_blocks_total + splits - 1) / splits;
     p.splits = splits = (p.k_blocks_total + p.k_blocks_per_split - 1) / p.k_blocks_per_split;
+    p.k_group_blocks = 0;
+    if (g.k_groups > 1) {  // whole slices per group; blocks beyond K read zeros
+        p.k_group_blocks = splits * p.k_blocks_per_split;
+        p.k_blocks_total = p.k_group_blocks * g.k_groups;
+        p.splits = splits = splits * g.k_groups;
+    }
     Scratch sc(ctx);
     p.partial = nullptr;
     p.partial_ld = (g.N + 3) / 4 * 4;
     if (splits > 1) {
-        int rc = sc.get(sizeof(float) * ((size_t)splits * g.M * p.partial_ld + (g.colsum ? (size_t)splits * g.N : 0)));
+        int rc = sc.get(sizeof(float) * (size_t)splits * batches * (g.M * p.partial_ld + (g.colsum ? g.N : 0)));
         if (rc) return rc;
         p.partial = sc.as<float>();
-        if (g.colsum) p.colsum_partial = p.partial + (size_t)splits * g.M * p.partial_ld;
+        if (g.colsum) p.colsum_partial = p.partial + (size_t)splits * batches * g.M * p.partial_ld;
     }
     p.batches = (int)batches;
     p.causal = g.causal;
@@ -1329,16 +1370,26 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     CUtensorMap mt = ma;
     p.b_twin = 0;
     static const int twin_env = [] { const char* e = getenv("GRADC_TC_WEIGHT_TWINS"); return e ? atoi(e) : 1; }();
-    if (twin_env != 0 && (use_pair ? pair_a_tmem : a_tmem) && batches == 1 && g.colsum == nullptr) {
+    if (twin_env != 0 && (use_pair ? pair_a_tmem : a_tmem) && (batches == 1 || g.grouped) && g.colsum == nullptr) {
         const void* tw = nullptr;
         int rc_t = twins_lookup(ctx, g.B, tb, g.N, g.K, g.ldb, &tw);
         if (rc_t) return rc_t;
+        const int64_t n_w = g.batch_inner * g.k_groups;  // weights of a group: their companions have to lie evenly as well
+        int64_t step = 0;
+        for (int64_t i = 1; i < n_w && tw != nullptr; ++i) {
+            const void* t_i = nullptr;
+            rc_t = twins_lookup(ctx, g.B + i * g.b_si, tb, g.N, g.K, g.ldb, &t_i);
+            if (rc_t) return rc_t;
+            const int64_t d = t_i ? (const char*)t_i - (const char*)tw : 0;
+            if (i == 1) step = d;
+            if (d <= 0 || d % 16 != 0 || d != i * step) tw = nullptr;
+        }
         if (tw != nullptr) {
             const cuuint64_t n_groups = (cuuint64_t)((g.N + 7) / 8), k_chunks = (cuuint64_t)(((g.K + 15) / 16) * 2);
-            cuuint64_t dims[3] = {k_chunks * 64, n_groups, 2};
-            cuuint64_t strides[2] = {k_chunks * 128, n_groups * k_chunks * 128};
-            cuuint32_t box[3] = {128u, (use_pair ? 128u : (cuuint32_t)BN) / 8u, 2u}, estr[3] = {1, 1, 1};
-            if (enc(&mt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(tw), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            cuuint64_t dims[4] = {k_chunks * 64, n_groups, 2, (cuuint64_t)n_w};
+            cuuint64_t strides[3] = {k_chunks * 128, n_groups * k_chunks * 128, n_w > 1 ? (cuuint64_t)step : 2 * n_groups * k_chunks * 128};
+            cuuint32_t box[4] = {128u, (use_pair ? 128u : (cuuint32_t)BN) / 8u, 2u, 1u}, estr[4] = {1, 1, 1, 1};
+            if (enc(&mt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(tw), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
                 p.b_twin = 1;
         }
@@ -1364,10 +1415,10 @@ int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     rc = after_launch(ctx, family);
     if (rc) return rc;
     if (splits > 1) {
-        const int vec = (g.N % 4 == 0 && g.ldc % 4 == 0 && aligned16(g.C)) ? 1 : 0;
-        const int64_t units = g.M * p.partial_ld / 4;
+        const int vec = (g.N % 4 == 0 && g.ldc % 4 == 0 && aligned16(g.C) && (batches == 1 || g.c_si % 4 == 0)) ? 1 : 0;
+        const int64_t units = batches * g.M * p.partial_ld / 4;
         GCB_CHECK_CUDA(launch_chained(ctx->stream, (unsigned)std::min<int64_t>((units + 255) / 256, (int64_t)kSMs * 8), 256, 0, splitk_reduce_kernel, g.C, (const float*)p.partial, p.partial_ld, g.bias, g.M, g.N, g.ldc,
-                                      splits, g.alpha, g.beta, g.colsum, (const float*)p.colsum_partial, g.colsum_accumulate, vec));
+                                      splits, g.alpha, g.beta, g.colsum, (const float*)p.colsum_partial, g.colsum_accumulate, vec, (int)batches, g.c_si, g.bias_si, g.colsum_si));
         rc = after_launch(ctx, "splitk_reduce");
         if (rc) return rc;
     }

@@ -343,7 +343,8 @@ public:
     Tensor<T> forward(Tensor<T> x) {  // (B, T, C)
         const int64_t B = x.shape()[0], S = x.shape()[1];
         auto heads = [&](Tensor<T> t) { return t.reshape({B, S, m_num_heads, m_head_dim}).permute({0, 2, 1, 3}); };  // views only
-        Tensor<T> Q = heads(m_q_proj.forward(x)), K = heads(m_k_proj.forward(x)), V = heads(m_v_proj.forward(x));
+        std::vector<Tensor<T>> qkv = linear_group(std::move(x), {{m_q_proj.weight(), m_q_proj.bias()}, {m_k_proj.weight(), m_k_proj.bias()}, {m_v_proj.weight(), m_v_proj.bias()}});
+        Tensor<T> Q = heads(qkv[0]), K = heads(qkv[1]), V = heads(qkv[2]);
         Tensor<T> attn = sdpa(Q, K, V, m_is_causal);
         attn = attn.permute({0, 2, 1, 3}).reshape({B, S, m_num_heads * m_head_dim});  // a view: sdpa lays its output out (B, T, H, D)
         return m_out_proj.forward(attn);
@@ -447,7 +448,10 @@ public:
         d.w2 = m_w2.weight().data_ptr(); d.b2 = m_w2.bias().data_ptr();
         d.w3 = m_w3.weight().data_ptr(); d.b3 = m_w3.bias().data_ptr();
     }
-    Tensor<T> forward(Tensor<T> x) { return m_w3.forward(swiglu_fast(m_w1.forward(x), m_w2.forward(x))); }
+    Tensor<T> forward(Tensor<T> x) {
+        std::vector<Tensor<T>> h = linear_group(std::move(x), {{m_w1.weight(), m_w1.bias()}, {m_w2.weight(), m_w2.bias()}});
+        return m_w3.forward(swiglu_fast(h[0], h[1]));
+    }
 };
 
 template <typename T>

@@ -7,6 +7,7 @@
 // bias add + bias gradient by atomics, permute/contiguous copies around every batched GEMM) one fused call runs.
 #pragma once
 
+#include <utility>
 #include <cmath>
 #include <random>
 
@@ -404,6 +405,16 @@ public:
     }
     void backward(const Tensor<float>& g, bool) override {
         Tensor<float> gc = make_contiguous(g);
+        if (!m_a._get_state()->m_grad.has_value() && !m_b._get_state()->m_grad.has_value() && m_a._get_state() != m_b._get_state() && m_a.requires_grad() && m_b.requires_grad()) {
+            // both in one block, in the order of the layers' parameters in their arena, so that the layers' backward can take them together
+            const int64_t n = gc.volume(), each = (n + 3) / 4 * 4;
+            Tensor<float> block({2 * each}, gc.device(), uninitialized);
+            Tensor<float> da(m_a.shape(), dense_strides(m_a.shape()), each, block._get_storage(), false), db(m_b.shape(), dense_strides(m_b.shape()), 0, block._get_storage(), false);
+            gcb_check(gcb_swiglu_bwd_f32(ctx_of(gc), da.data_ptr(), db.data_ptr(), gc.data_ptr(), m_a.data_ptr(), m_b.data_ptr(), n, 0, 0), "swiglu backward");
+            push_grad(m_a, da);
+            push_grad(m_b, db);
+            return;
+        }
         auto [da, acc_a] = m_a.grad_target();
         auto [db, acc_b] = m_b.grad_target();
         gcb_check(gcb_swiglu_bwd_f32(ctx_of(gc), da.data_ptr(), db.data_ptr(), gc.data_ptr(), m_a.data_ptr(), m_b.data_ptr(), gc.volume(), acc_a ? 1 : 0, acc_b ? 1 : 0), "swiglu backward");
@@ -653,6 +664,137 @@ inline Tensor<float> linear(Tensor<float> x, Tensor<float> w, Tensor<float> b) {
     out._get_state()->m_creation_op = std::make_unique<MatMulNode>(std::move(x), std::move(w), std::move(b), M, K, N, out_shape);
     return out;
 }
+// Linear layers of one shape over one input whose parameters lie evenly spaced in a parameter arena (consecutive layers do): one
+// product forward, one for dX and one for all dW and bias gradients.  Every member is a tensor of its own with a node of its own; the
+// first to be realized computes all, the last to pass in the backward sweep runs the backward of all.  Each member depends on every
+// weight, so that no parameter counts as final before that.
+struct LinearGroup {
+    struct Member {
+        Tensor<float> w, b, out;
+        std::optional<Tensor<float>> grad;
+    };
+    Tensor<float> x;
+    std::vector<Member> members;  // by ascending weight address
+    int64_t M, N, K, w_stride, b_stride;
+    std::vector<int64_t> out_shape;
+    size_t passed = 0;
+
+    void forward() {
+        x.realize();
+        const int64_t n = (int64_t)members.size(), each = (M * N + 3) / 4 * 4;
+        auto block = std::make_shared<Storage<float>>(n * each, 0.0f, x.device(), true, false);
+        gcb_check(gcb_linear_group_f32(ctx_of(x), n, M, N, K, x.data_ptr(), members[0].w.data_ptr(), w_stride, members[0].b.data_ptr(), b_stride, block->data(), each), "linear layers");
+        for (int64_t i = 0; i < n; ++i) {
+            float* p = block->data() + i * each;
+            members[(size_t)i].out = Tensor<float>(out_shape, dense_strides(out_shape), 0, std::make_shared<Storage<float>>(p, M * N, x.device(), std::shared_ptr<void>(block, p)), false);
+        }
+    }
+    void backward() {
+        const int64_t n = (int64_t)members.size();
+        gcb_ctx* c = ctx_of(x);
+        std::vector<const float*> dy;
+        for (auto& m : members) {
+            if (!m.grad.has_value()) throw std::runtime_error("linear layers: a member of a group has no gradient");
+            m.grad = make_contiguous(m.grad.value());
+            dy.push_back(m.grad->data_ptr());
+        }
+        // evenly spaced runs of `stride` elements: one call; otherwise one per member
+        auto evenly = [&](auto&& at, int64_t& stride) {
+            stride = n > 1 ? at(1) - at(0) : 0;
+            bool ok = stride >= 0;
+            for (int64_t i = 1; i < n; ++i) ok = ok && at(i) - at(0) == i * stride;
+            return ok;
+        };
+        int64_t y_stride = 0;
+        const bool together = evenly([&](int64_t i) { return dy[(size_t)i]; }, y_stride) && y_stride >= M * N;
+        const int64_t runs = together ? 1 : n, per = together ? n : 1;
+        if (x.requires_grad()) {
+            auto [dx, acc] = x.grad_target();
+            for (int64_t i = 0; i < runs; ++i)
+                gcb_check(gcb_linear_group_dx_f32(c, per, M, N, K, dy[(size_t)i], y_stride, members[(size_t)i].w.data_ptr(), w_stride, acc || i > 0 ? 1.0f : 0.0f, dx.data_ptr()), "linear layers dX");
+        }
+        if (members[0].w.requires_grad()) {
+            std::vector<float*> dw, db;
+            std::vector<std::pair<bool, bool>> acc;
+            for (auto& m : members) {
+                auto [gw, aw] = m.w.grad_target();
+                auto [gb, ab] = m.b.grad_target();
+                dw.push_back(gw.data_ptr()); db.push_back(gb.data_ptr());
+                acc.emplace_back(aw, ab);
+            }
+            int64_t dw_stride = 0, db_stride = 0;
+            bool one = together && evenly([&](int64_t i) { return dw[(size_t)i]; }, dw_stride) && dw_stride >= K * N && evenly([&](int64_t i) { return db[(size_t)i]; }, db_stride) && db_stride >= N;
+            for (auto& a : acc) one = one && a == acc[0];
+            for (int64_t i = 0; i < (one ? 1 : n); ++i)
+                gcb_check(gcb_linear_group_dw_f32(c, one ? n : 1, M, N, K, x.data_ptr(), dy[(size_t)i], y_stride, acc[(size_t)i].first ? 1.0f : 0.0f, dw[(size_t)i], dw_stride, db[(size_t)i], db_stride,
+                                                  acc[(size_t)i].second ? 1 : 0), "linear layers dW + bias gradients");
+        }
+        for (auto& m : members) m.grad.reset();
+        passed = 0;
+    }
+};
+
+class LinearGroupNode : public Node<float> {
+    std::shared_ptr<LinearGroup> m_group;
+    size_t m_index;
+
+public:
+    LinearGroupNode(std::shared_ptr<LinearGroup> group, size_t index) : m_group(std::move(group)), m_index(index) {}
+    Tensor<float> realize() override {
+        Tensor<float>& out = m_group->members[m_index].out;
+        if (out._get_state() == nullptr) m_group->forward();
+        return std::exchange(out, Tensor<float>());
+    }
+    void backward(const Tensor<float>& g, bool) override {
+        m_group->members[m_index].grad = g;
+        if (++m_group->passed == m_group->members.size()) m_group->backward();
+    }
+    std::vector<TensorStateBase*> get_input_states() override {
+        std::vector<TensorStateBase*> v{m_group->x._get_state_base()};
+        for (auto& m : m_group->members) { v.push_back(m.w._get_state_base()); v.push_back(m.b._get_state_base()); }
+        return v;
+    }
+};
+
+inline std::vector<Tensor<float>> linear_group(Tensor<float> x, const std::vector<std::pair<Tensor<float>, Tensor<float>>>& layers) {
+    if (!x.is_contiguous()) x = x.contiguous();
+    const size_t n = layers.size();
+    std::vector<size_t> order(n);
+    for (size_t i = 0; i < n; ++i) order[i] = i;
+    auto in_arena = [](const Tensor<float>& t) { return t._get_state() != nullptr && t._get_state()->m_slot.arena != nullptr && t.is_dense(); };
+    bool ok = n > 1 && !x.shape().empty() && !x.device().is_cpu();
+    for (const auto& [w, b] : layers)
+        ok = ok && in_arena(w) && in_arena(b) && w._get_state()->m_slot.arena == layers[0].first._get_state()->m_slot.arena && w.shape() == layers[0].first.shape() && w.shape().size() == 2 && w.shape()[0] == x.shape().back() &&
+             b.volume() == w.shape()[1] && w.requires_grad() == layers[0].first.requires_grad() && b.requires_grad() == w.requires_grad();
+    auto group = std::make_shared<LinearGroup>();
+    if (ok) {
+        std::sort(order.begin(), order.end(), [&](size_t a, size_t b) { return layers[a].first.data_ptr() < layers[b].first.data_ptr(); });
+        const float *w0 = layers[order[0]].first.data_ptr(), *b0 = layers[order[0]].second.data_ptr();
+        group->w_stride = layers[order[1]].first.data_ptr() - w0;
+        group->b_stride = layers[order[1]].second.data_ptr() - b0;
+        for (size_t i = 1; i < n; ++i) ok = ok && layers[order[i]].first.data_ptr() - w0 == (int64_t)i * group->w_stride && layers[order[i]].second.data_ptr() - b0 == (int64_t)i * group->b_stride;
+    }
+    std::vector<Tensor<float>> outs(n);
+    if (!ok) {
+        for (size_t i = 0; i < n; ++i) outs[i] = linear(x, layers[i].first, layers[i].second);
+        return outs;
+    }
+    group->K = layers[0].first.shape()[0];
+    group->N = layers[0].first.shape()[1];
+    group->M = x.volume() / group->K;
+    group->out_shape = x.shape();
+    group->out_shape.back() = group->N;
+    for (size_t i : order) group->members.push_back({layers[i].first, layers[i].second, Tensor<float>(), std::nullopt});
+    const bool rg = x.requires_grad() || layers[0].first.requires_grad();
+    const Device d = x.device();
+    group->x = std::move(x);
+    for (size_t i = 0; i < n; ++i) {
+        Tensor<float> out(group->out_shape, rg, lazy, d);
+        out._get_state()->m_creation_op = std::make_unique<LinearGroupNode>(group, i);
+        outs[order[i]] = std::move(out);
+    }
+    return outs;
+}
 inline Tensor<float> matmul(Tensor<float> x, Tensor<float> w) { return linear(std::move(x), std::move(w), Tensor<float>()); }
 
 // ---- attention ----------------------------------------------------------------------------------------------------
@@ -708,13 +850,14 @@ public:
         const int64_t B = m_B, H = m_H, T = m_T, D = m_D;
         int64_t go, gi, gl, qo, qi, ql, ko, ki, kl, vo, vi, vl;
         strides4(g, go, gi, gl); strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl); strides4(m_v, vo, vi, vl);
-        auto fresh = [&]() {  // gradient in (B, T, H, D) memory order, seen as (B, H, T, D)
-            Tensor<float> mem({B, T, H, D}, g.device(), uninitialized);
-            return Tensor<float>({B, H, T, D}, out_strides(H, T, D), 0, mem._get_storage(), false);
-        };
+        // gradients in (B, T, H, D) memory order, seen as (B, H, T, D); one block, in the order of the projections' parameters in
+        // their arena, so that the projections' backward can take them together
+        const int64_t each = (B * T * H * D + 3) / 4 * 4;
+        Tensor<float> block({3 * each}, g.device(), uninitialized);
+        auto part = [&](int64_t i) { return Tensor<float>({B, H, T, D}, out_strides(H, T, D), i * each, block._get_storage(), false); };
         if (m_stats._get_state() != nullptr) {
             if (reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 != 0 || gl % 4 != 0 || go % 4 != 0 || gi % 4 != 0 || gl <= 0 || go <= 0 || gi <= 0) { g = make_contiguous(g); strides4(g, go, gi, gl); }
-            Tensor<float> dq = fresh(), dk = fresh(), dv = fresh();
+            Tensor<float> dq = part(2), dk = part(1), dv = part(0);
             gcb_check(gcb_attention_bwd_f32(c, B, H, T, D, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), H * D, T * H * D, D, g.data_ptr(), gl, go, gi, m_out_storage->data(), H * D, T * H * D, D, m_stats.data_ptr(), m_q.data_ptr(), ql, qo,
                                             qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale), "attention backward");
             if (m_v.requires_grad()) push_grad(m_v, dv);
@@ -724,7 +867,7 @@ public:
             return;
         }
         if (m_v.requires_grad()) {  // dV = P^T . dO
-            Tensor<float> dv = fresh();
+            Tensor<float> dv = part(0);
             gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_T, GCB_OP_N, T, D, T, 1.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, g.data_ptr(), gl, go, gi, 0.0f, dv.data_ptr(), H * D, T * H * D, D, B, H, 3), "attention dV");
             push_grad(m_v, dv);
         }
@@ -736,12 +879,12 @@ public:
             gcb_check(gcb_gemm_batched_softmax_bwd_f32(c, GCB_OP_N, GCB_OP_T, T, D, 1.0f, g.data_ptr(), gl, go, gi, m_v.data_ptr(), vl, vo, vi, ds.data_ptr(), m_ld, H * T * m_ld, T * m_ld, B, H, m_probs.data_ptr(),
                                                        rowdot.data_ptr(), m_scale), "attention dS");
             if (m_q.requires_grad()) {  // dQ = dS . K
-                Tensor<float> dq = fresh();
+                Tensor<float> dq = part(2);
                 gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_N, T, D, T, 1.0f, ds.data_ptr(), m_ld, H * T * m_ld, T * m_ld, m_k.data_ptr(), kl, ko, ki, 0.0f, dq.data_ptr(), H * D, T * H * D, D, B, H, 2), "attention dQ");
                 push_grad(m_q, dq);
             }
             if (m_k.requires_grad()) {  // dK = dS^T . Q
-                Tensor<float> dk = fresh();
+                Tensor<float> dk = part(1);
                 gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_T, GCB_OP_N, T, D, T, 1.0f, ds.data_ptr(), m_ld, H * T * m_ld, T * m_ld, m_q.data_ptr(), ql, qo, qi, 0.0f, dk.data_ptr(), H * D, T * H * D, D, B, H, 3), "attention dK");
                 push_grad(m_k, dk);
             }

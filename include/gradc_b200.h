@@ -207,6 +207,15 @@ GCB_API int gcb_linear_residual_f32(gcb_ctx* ctx, int op_b, int64_t M, int64_t N
 GCB_API int gcb_gemm_gelu_bwd_f32(gcb_ctx* ctx, int op_a, int op_b, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B, int64_t ldb,
                           const float* pre, float* dpre);
 
+/* `groups` linear layers of one shape over the same input x (M x K): W, bias and the outputs of layer i lie at i times their
+ * stride (weights K x N as stored).  Forward, input gradient dx = sum_i dy_i W_i^T + beta dx, and weight + bias gradients
+ * (dW_i = x^T dy_i + beta dW_i); each is one product where the strides are whole vectors, otherwise one per layer.  The reference
+ * runs the layers one after another (nn/layers/linear.hpp:23, math_nodes.hpp:475-535). */
+GCB_API int gcb_linear_group_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* x, const float* W, int64_t w_stride, const float* bias, int64_t bias_stride, float* y, int64_t y_stride);
+GCB_API int gcb_linear_group_dx_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* dy, int64_t dy_stride, const float* W, int64_t w_stride, float beta, float* dx);
+GCB_API int gcb_linear_group_dw_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* x, const float* dy, int64_t dy_stride, float beta, float* dW, int64_t w_stride, float* dbias,
+                            int64_t bias_stride, int bias_accumulate);
+
 /* out[(o * batch_inner + i) * rows + r] = sum_c a[o, i, r, c] * b[o, i, r, c]; rows of a and b are addressed through
  * (outer, inner, row) strides in elements, columns are contiguous. */
 GCB_API int gcb_rowdot_batched_f32(gcb_ctx* ctx, float* out, const float* a, int64_t lda, int64_t a_stride_outer, int64_t a_stride_inner,

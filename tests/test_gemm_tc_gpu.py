@@ -631,3 +631,40 @@ def test_fused_causal_attention(env, Bn, H, T, D):
         got = heads(got.cpu().numpy())
         assert np.linalg.norm(got - ref) < TOL * np.linalg.norm(ref)
     assert not capi.lib().attention_supported(ctx.h, Bn, H, 256, D, dq.data_ptr(), *rows, dk.data_ptr(), *rows, dv.data_ptr(), *rows, scale)
+
+
+@pytest.mark.parametrize("engine", [0, 1])
+@pytest.mark.parametrize("G,M,N,K,family", [(3, 70, 40, 33, None), (3, 1656, 384, 384, "gemm_tc"), (2, 1000, 1152, 264, "gemm_tc"), (2, 700, 513, 300, None), (3, 5000, 1024, 1024, "gemm_tc_pair")])
+def test_linear_layers_taken_together(env, engine, G, M, N, K, family):
+    """Forward, input gradient (one sum over all layers, cut between them) and weight + bias gradients; K ends inside a block, widths
+    that TMA cannot address, strides with gaps, accumulating forms."""
+    ctx, torch, capi = env
+    if engine == 1 and M * N * K > 1 << 29:
+        pytest.skip("the FMA kernel's branches are those of the smaller sizes")
+    ws, ys = K * N + 24, M * N + (-M * N) % 4
+    x, W, b, dy = rnd(1, M, K), rnd(2, G, ws), rnd(3, G, 2 * N + (-2 * N) % 4), rnd(4, G, ys)
+    dx0, dW0 = rnd(5, M, K), rnd(6, G, ws)
+    X, DY = x.astype(np.float64), dy[:, : M * N].reshape(G, M, N).astype(np.float64)
+    Ws = W[:, : K * N].reshape(G, K, N).astype(np.float64)
+    ctx.ctx_set_gemm_engine(engine)
+    try:
+        tx, tW, tb, tdy, tdx, tdW = (torch.from_numpy(a).cuda() for a in (x, W, b, dy, dx0, dW0))
+        ty, tdb = torch.zeros(G, ys, device="cuda"), torch.ones(G, b.shape[1], device="cuda")
+        if K >= 128 and N >= 128 and N % 4 == 0:
+            for g in range(G):
+                ctx.weight_twins_register(tW[g], K, N)
+        ctx.linear_group_f32(G, M, N, K, tx, tW, ws, tb, b.shape[1], ty, ys)
+        ctx.linear_group_dx_f32(G, M, N, K, tdy, ys, tW, ws, 1.0, tdx)
+        ctx.linear_group_dw_f32(G, M, N, K, tx, tdy, ys, 1.0, tdW, ws, tdb, b.shape[1], 1)
+        ctx.sync()
+        for g in range(G):
+            assert max_abs_rel(ty[g, : M * N].cpu().numpy().reshape(M, N), X @ Ws[g] + b[g, :N]) < TOL
+            assert max_abs_rel(tdW[g, : K * N].cpu().numpy().reshape(K, N), X.T @ DY[g] + dW0[g, : K * N].reshape(K, N)) < TOL
+            assert np.array_equal(tdW[g, K * N :].cpu().numpy(), dW0[g, K * N :])
+            assert np.abs(tdb[g, :N].cpu().numpy() - 1.0 - DY[g].sum(0)).max() < 1e-4 * np.abs(DY[g]).sum(0).max()
+        assert max_abs_rel(tdx.cpu().numpy(), sum(DY[g] @ Ws[g].T for g in range(G)) + dx0) < TOL
+        if engine == 0 and family == "gemm_tc_pair":
+            assert capi.lib().ctx_launch_count_named(ctx.h, b"gemm_tc_pair") > 0
+    finally:
+        ctx.weight_twins_drop(None, 0)
+        ctx.ctx_set_gemm_engine(2)
