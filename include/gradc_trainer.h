@@ -40,8 +40,8 @@ GCT_API int gct_optimizer_step(gct_trainer* tr, float* norm_out);
 GCT_API int gct_save_checkpoint(gct_trainer* tr, const char* model_path, const char* optim_path);
 GCT_API int gct_load_checkpoint(gct_trainer* tr, const char* model_path, const char* optim_path);
 /* Token-level generation (nn/generators/gpt_generator.hpp:12-132 without the tokenizer): num_sequences rows of max_tokens ids
- * into out_tokens, each starting with the n_start given tokens; the context (at most context_length tokens) is re-forwarded
- * for every new token.  temperature <= 0: argmax; otherwise top_k sampling with the reference's generator and seed. */
+ * into out_tokens, each starting with the n_start given tokens; the last context_length tokens are the context
+ * of every new token (keys and values are kept; the whole context is forwarded only when it slides).  temperature <= 0: argmax; otherwise top_k sampling with the reference's generator and seed. */
 GCT_API int gct_generate(gct_trainer* tr, const int64_t* start_tokens, int64_t n_start, int64_t context_length, int64_t max_tokens, int64_t num_sequences, float temperature,
                          int64_t top_k, int64_t* out_tokens);
 GCT_API int gct_sync(gct_trainer* tr);
