@@ -949,7 +949,7 @@ class IncrementalGPT {
     gcb_gpt_model m_model;
     std::unique_ptr<gcb_gpt_decoder, int (*)(gcb_gpt_decoder*)> m_decoder{nullptr, gcb_gpt_decoder_destroy};
     int64_t m_cap = 0, m_seqs = 0;  // positions per sequence and sequences the cache holds
-    Tensor<float> m_cache, m_x, m_a, m_q, m_o, m_scores, m_h0, m_h1;
+    Tensor<float> m_cache, m_x, m_a, m_q, m_o, m_scores, m_stats, m_h0, m_h1;
     Tensor<int64_t> m_ids;
 
     float* cache(int64_t layer, int which) { return m_cache.data_ptr() + (2 * layer + which) * m_seqs * m_cap * m_model.C; }
@@ -963,6 +963,15 @@ class IncrementalGPT {
     void project(float* y, const float* x, const float* w, const float* b, int64_t rows, int64_t K, int64_t N) {
         gcb_check(gcb_gemm_f32(m_ctx, GCB_OP_N, GCB_OP_N, rows, N, K, 1.0f, x, K, w, N, 0.0f, y, N, b), "projection");
     }
+    // Two layers over one input in one product where the first one's weights precede the second one's (as in a parameter arena).
+    void project_two(float* y0, float* y1, const float* x, const float* w0, const float* w1, const float* b0, const float* b1, int64_t rows, int64_t K, int64_t N) {
+        if (w1 > w0 && b1 > b0) {
+            gcb_check(gcb_linear_group_f32(m_ctx, 2, rows, N, K, x, w0, w1 - w0, b0, b1 - b0, y0, y1 - y0), "projections");
+        } else {
+            project(y0, x, w0, b0, rows, K, N);
+            project(y1, x, w1, b1, rows, K, N);
+        }
+    }
     // Keys and values of the positions 0 .. n - 1 of `seqs` sequences, token ids on the device (seqs x n, dense).
     void forward_window(const int64_t* ids, int64_t seqs, int64_t n) {
         const gcb_gpt_model& m = m_model;
@@ -970,30 +979,34 @@ class IncrementalGPT {
         if (seqs > 1 && n != m_cap) throw std::runtime_error("IncrementalGPT: several sequences fill the whole cache");
         const float scale = static_cast<float>(1.0 / std::sqrt((double)D));
         for (Tensor<float>* t : {&m_x, &m_a, &m_q, &m_o}) at_least(*t, rows * C, m_device);
-        at_least(m_scores, seqs * H * n * ld, m_device);
         at_least(m_h0, rows * F, m_device);
         at_least(m_h1, rows * F, m_device);
-        float *x = m_x.data_ptr(), *a = m_a.data_ptr(), *q = m_q.data_ptr(), *o = m_o.data_ptr(), *s = m_scores.data_ptr(), *h0 = m_h0.data_ptr(), *h1 = m_h1.data_ptr();
+        float *x = m_x.data_ptr(), *a = m_a.data_ptr(), *q = m_q.data_ptr(), *o = m_o.data_ptr(), *h0 = m_h0.data_ptr(), *h1 = m_h1.data_ptr();
         gcb_check(gcb_embed_f32(m_ctx, x, ids, GCB_IDX_I64, m.token_embed, rows, C, m.V), "embedding gather");
         gcb_check(gcb_binary_rowvec_f32(m_ctx, GCB_B_ADD, x, x, m.pos_embed, seqs, n * C), "positions");
         for (int64_t l = 0; l < m.L; ++l) {
             const gcb_gpt_layer& w = m_layers[(size_t)l];
             float *k = cache(l, 0), *v = cache(l, 1);
             norm(a, x, w.norm1_gamma, w.norm1_beta, rows);
-            project(k, a, w.wk, w.bk, rows, C, C);
-            project(v, a, w.wv, w.bv, rows, C, C);
+            project_two(v, k, a, w.wv, w.wk, w.bv, w.bk, rows, C, C);
             if (l + 1 == m.L) break;
             project(q, a, w.wq, w.bq, rows, C, C);
-            gcb_check(gcb_gemm_batched_causal_f32(m_ctx, GCB_OP_N, GCB_OP_T, n, n, D, 1.0f, q, C, n * C, D, k, C, m_cap * C, D, 0.0f, s, ld, H * n * ld, n * ld, seqs, H, 1), "attention scores");
-            gcb_check(gcb_causal_softmax_fwd_band_ld_f32(m_ctx, s, s, scale, seqs * H * n, n, ld, 128), "causal softmax");
-            gcb_check(gcb_gemm_batched_causal_f32(m_ctx, GCB_OP_N, GCB_OP_N, n, D, n, 1.0f, s, ld, H * n * ld, n * ld, v, C, m_cap * C, D, 0.0f, o, C, n * C, D, seqs, H, 2), "attention output");
+            if (gcb_attention_supported(m_ctx, seqs, H, n, D, q, C, n * C, D, k, C, m_cap * C, D, v, C, m_cap * C, D, scale)) {
+                at_least(m_stats, gcb_attention_stats_floats(seqs, H, n), m_device);
+                gcb_check(gcb_attention_fwd_f32(m_ctx, seqs, H, n, D, o, C, n * C, D, m_stats.data_ptr(), q, C, n * C, D, k, C, m_cap * C, D, v, C, m_cap * C, D, scale), "attention");
+            } else {
+                at_least(m_scores, seqs * H * n * ld, m_device);
+                float* s = m_scores.data_ptr();
+                gcb_check(gcb_gemm_batched_causal_f32(m_ctx, GCB_OP_N, GCB_OP_T, n, n, D, 1.0f, q, C, n * C, D, k, C, m_cap * C, D, 0.0f, s, ld, H * n * ld, n * ld, seqs, H, 1), "attention scores");
+                gcb_check(gcb_causal_softmax_fwd_band_ld_f32(m_ctx, s, s, scale, seqs * H * n, n, ld, 128), "causal softmax");
+                gcb_check(gcb_gemm_batched_causal_f32(m_ctx, GCB_OP_N, GCB_OP_N, n, D, n, 1.0f, s, ld, H * n * ld, n * ld, v, C, m_cap * C, D, 0.0f, o, C, n * C, D, seqs, H, 2), "attention output");
+            }
             gcb_check(gcb_linear_residual_f32(m_ctx, GCB_OP_N, rows, C, C, o, C, w.wo, C, w.bo, x, a), "linear + residual");
             std::swap(x, a);
             norm(a, x, w.norm2_gamma, w.norm2_beta, rows);
             const float *w_out, *b_out;
             if (w.w3 != nullptr) {
-                project(h0, a, w.w1, w.b1, rows, C, F);
-                project(h1, a, w.w2, w.b2, rows, C, F);
+                project_two(h1, h0, a, w.w2, w.w1, w.b2, w.b1, rows, C, F);
                 gcb_check(gcb_swiglu_fwd_f32(m_ctx, h1, h0, h1, rows * F), "swiglu");
                 w_out = w.w3; b_out = w.b3;
             } else {
