@@ -269,6 +269,28 @@ int gcb_linear_group_dw_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, 
     return rc;
 }
 
+int gcb_linear_group_bwd_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* x, const float* dy, int64_t dy_stride, const float* W, int64_t w_stride, const float* gelu_pre, float dx_beta,
+                             float* dx, float dw_beta, float* dW, int64_t dw_stride, float* dbias, int64_t bias_stride, int bias_accumulate) {
+    GCB_REQUIRE(ctx && groups >= 1 && groups <= 64 && (M == 0 || K == 0 || dx) && (N == 0 || dbias), "gcb_linear_group_bwd_f32: bad arguments");
+    GCB_REQUIRE(gelu_pre == nullptr || (groups == 1 && dx_beta == 0.0f && gelu_pre != dx), "gcb_linear_group_bwd_f32: a GELU behind the input takes one layer and overwrites its gradient");
+    const int64_t work = M * N * K * groups;
+    if (!ctx->prof_on && work > 0 && (ctx->gemm_engine == 1 || (ctx->gemm_engine == 0 && work < kSmallWork)) && x && dy && W && dW && (groups == 1 || (dy_stride >= M * N && w_stride > 0))) {
+        GemmArgs gx{M, K, N, 1.0f, dx_beta, dy, W, nullptr, dx, N, N, K, 0, dy_stride, 0, w_stride, 0, 0, 1, 1};
+        gx.gelu_pre = gelu_pre;
+        gx.k_groups = (int)groups;
+        GemmArgs gw{K, N, M, 1.0f, dw_beta, x, dy, nullptr, dW, K, N, N, 0, 0, 0, dy_stride, 0, dw_stride, 1, groups};
+        gw.grouped = gx.grouped = true;
+        gw.colsum = dbias; gw.colsum_si = bias_stride; gw.colsum_accumulate = bias_accumulate;
+        if (gemm_simt_backward_fits(gx, gw)) return gemm_simt_backward_launch(ctx, gx, gw);
+    }
+    int rc = gelu_pre ? gcb_gemm_gelu_bwd_f32(ctx, GCB_OP_N, GCB_OP_T, M, K, N, dy, N, W, N, gelu_pre, dx)
+             : groups == 1 ? gcb_gemm_f32(ctx, GCB_OP_N, GCB_OP_T, M, K, N, 1.0f, dy, N, W, N, dx_beta, dx, K, nullptr)
+                           : gcb_linear_group_dx_f32(ctx, groups, M, N, K, dy, dy_stride, W, w_stride, dx_beta, dx);
+    if (rc) return rc;
+    return groups == 1 ? gcb_gemm_colsum_f32(ctx, GCB_OP_T, K, N, M, 1.0f, x, K, dy, dw_beta, dW, N, dbias, bias_accumulate)
+                       : gcb_linear_group_dw_f32(ctx, groups, M, N, K, x, dy, dy_stride, dw_beta, dW, dw_stride, dbias, bias_stride, bias_accumulate);
+}
+
 int gcb_profile_gemm_begin(gcb_ctx* ctx) {
     GCB_REQUIRE(ctx, "gcb_profile_gemm_begin: ctx is NULL");
     ctx->prof_on = true;

@@ -41,6 +41,9 @@ struct GemmArgs {
 
 // fp32 FMA engine: any shape, any leading dimension, every epilogue.
 int gemm_simt_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g);
+// A linear layer's two gradients in one launch of the FMA engine: dx = dY W^T (op N, T), dw = X^T dY (op T, N).
+bool gemm_simt_backward_fits(const GemmArgs& dx, const GemmArgs& dw);
+int gemm_simt_backward_launch(gcb_ctx* ctx, const GemmArgs& dx, const GemmArgs& dw);
 // tcgen05 3xTF32 engine.  Returns GCB_UNSUPPORTED (without touching C) when the operands cannot be described
 // to TMA: bases must be 16-byte aligned and every leading dimension / batch stride a multiple of 4 floats.
 int gemm_tc_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g);

@@ -67,15 +67,19 @@ __device__ __forceinline__ void sg_fragment(const float* sm, int t, int k, float
 
 // Row-major C[M,N] = alpha * op(A) * op(B) + beta * C (+ bias[n]) and the epilogues of GemmArgs.  TA: A is stored K x M; TB: B is
 // stored N x K.  A cluster of `slices` CTAs takes one tile.
+struct SgShape {
+    int tiles_m, tiles_n;
+    bool a_vec, b_vec, c_vec;  // 16-byte accesses
+};
 template <int BM, bool TA, bool TB>
-__global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g, int tiles_m, int tiles_n, int slices, bool a_vec, bool b_vec, bool c_vec) {
+__device__ __forceinline__ void sg_tile(const GemmArgs& g, const SgShape& sh, int slices, unsigned block) {
     using S = SgSmem<BM>;
     constexpr int KG = S::KG, TPR = BM / 4, GT = TPR * TPR;  // threads along an edge of the tile, threads of a K group
     extern __shared__ __align__(16) float sg[];
-    pdl_trigger();
-    pdl_wait();
-    const int t = threadIdx.x, rank = (int)(blockIdx.x % (unsigned)slices);
-    int64_t w = blockIdx.x / (unsigned)slices;
+    const int tiles_m = sh.tiles_m, tiles_n = sh.tiles_n;
+    const bool a_vec = sh.a_vec, b_vec = sh.b_vec, c_vec = sh.c_vec;
+    const int t = threadIdx.x, rank = (int)(block % (unsigned)slices);
+    int64_t w = block / (unsigned)slices;
     const int64_t bz = w / ((int64_t)tiles_m * tiles_n);
     w -= bz * tiles_m * tiles_n;
     const int64_t m0 = (w / tiles_n) * BM, n0 = (w % tiles_n) * BM;
@@ -249,16 +253,42 @@ __global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g,
 }
 
 template <int BM, bool TA, bool TB>
-static int sg_launch(gcb_ctx* ctx, const GemmArgs& g, int64_t tiles_m, int64_t tiles_n, int64_t batches, int slices) {
+__global__ void __launch_bounds__(SG_THREADS) gemm_simt_kernel(const GemmArgs g, const SgShape sh, int slices) {
+    pdl_trigger();
+    pdl_wait();
+    sg_tile<BM, TA, TB>(g, sh, slices, blockIdx.x);
+}
+// A linear layer's dX = dY W^T and dW = X^T dY side by side: neither waits for the other, and in a small model each is a launch of
+// 5 - 6 us that leaves most SMs idle (two-layer step: 13 launches less).
+template <int BM>
+__global__ void __launch_bounds__(SG_THREADS) gemm_simt_backward_kernel(const GemmArgs dx, const SgShape dx_sh, const GemmArgs dw, const SgShape dw_sh, int slices, unsigned dx_blocks) {
+    pdl_trigger();
+    pdl_wait();
+    if (blockIdx.x < dx_blocks) sg_tile<BM, false, true>(dx, dx_sh, slices, blockIdx.x);
+    else sg_tile<BM, true, false>(dw, dw_sh, slices, blockIdx.x - dx_blocks);
+}
+
+static SgShape sg_shape(const GemmArgs& g, int bm) {
     auto ok4 = [](int64_t v) { return v % 4 == 0; };
     auto vec = [&](const float* p, int64_t ld, int64_t so, int64_t si) { return aligned16(p) && ok4(ld) && ((g.batch_inner == 1 && g.k_groups == 1) || ok4(si)) && (g.batch_outer == 1 || ok4(so)); };
     const bool c_vec = vec(g.C, g.ldc, g.c_so, g.c_si) && aligned16(g.residual) && aligned16(g.gelu_pre) && aligned16(g.gelu_act) && aligned16(g.sm_probs);
-    auto kfn = gemm_simt_kernel<BM, TA, TB>;
+    return {(int)((g.M + bm - 1) / bm), (int)((g.N + bm - 1) / bm), vec(g.A, g.lda, g.a_so, g.a_si), vec(g.B, g.ldb, g.b_so, g.b_si), c_vec};
+}
+static int64_t sg_tiles(const GemmArgs& g, int64_t bm) { return ((g.M + bm - 1) / bm) * ((g.N + bm - 1) / bm) * g.batch_outer * g.batch_inner; }
+// K is cut while SMs are left over and every slice keeps two K blocks; beyond one CTA per SM only for slices of 96 and more
+// (256 x 512 x 128: one slice 5.5 us, two 6.4; 256 x 256 x 512: one 10.8, two 8.3, four 7.7, eight 12.9)
+static int sg_slices(int64_t tiles, int64_t K) {
+    int slices = 1;
+    while (slices < 8 && K >= (int64_t)slices * 2 * 2 * SG_BK && tiles * slices * 2 <= (K >= (int64_t)slices * 2 * 96 ? 2 * kSMs : kSMs)) slices *= 2;
+    return slices;
+}
+template <int BM, class... P, class... Args>
+static int sg_launch(gcb_ctx* ctx, bool* attr_done, void (*kfn)(P...), int64_t tiles, int slices, Args... args) {
     constexpr size_t smem = sizeof(float) * SgSmem<BM>::FLOATS;
-    static bool attr_done[kMaxDevices] = {};  // function attributes belong to a device
+    // attr_done: function attributes belong to a device
     if (smem > 48 * 1024 && !attr_done[ctx->device]) { GCB_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr_done[ctx->device] = true; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles_m * tiles_n * batches * slices), 1, 1);
+    cfg.gridDim = dim3((unsigned)(tiles * slices), 1, 1);
     cfg.blockDim = dim3(SG_THREADS, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
@@ -270,33 +300,46 @@ static int sg_launch(gcb_ctx* ctx, const GemmArgs& g, int64_t tiles_m, int64_t t
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = slices > 1 ? 2 : 1;
-    GCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kfn, g, (int)tiles_m, (int)tiles_n, slices, vec(g.A, g.lda, g.a_so, g.a_si), vec(g.B, g.ldb, g.b_so, g.b_si), c_vec));
+    GCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kfn, args...));
     return GCB_OK;
+}
+template <int BM, bool TA, bool TB>
+static int sg_run(gcb_ctx* ctx, const GemmArgs& g, int64_t tiles, int slices) {
+    static bool done[kMaxDevices] = {};
+    return sg_launch<BM>(ctx, done, gemm_simt_kernel<BM, TA, TB>, tiles, slices, g, sg_shape(g, BM), slices);
 }
 
 int gemm_simt_launch(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g) {
     const int64_t batches = g.batch_outer * g.batch_inner;
     if (g.M == 0 || g.N == 0 || batches == 0) return GCB_OK;
     if (g.colsum && tb) { set_error("gemm (FMA): column sums need op(B) stored K x N"); return GCB_UNSUPPORTED; }
-    auto tiles = [&](int64_t b) { return ((g.M + b - 1) / b) * ((g.N + b - 1) / b) * batches; };
     // 64-wide tiles read shared memory and L2 half as often per FMA: they are taken once they fill the chip by themselves
-    const int bm = tiles(64) >= kSMs ? 64 : 32;
-    const int64_t tm = (g.M + bm - 1) / bm, tn = (g.N + bm - 1) / bm;
-    GCB_REQUIRE(tm * tn <= 0x7fffffff / 8 && tiles(bm) <= 0x7fffffff / 8, "gemm (FMA): grid too large");
-    // K is cut while SMs are left over and every slice keeps two K blocks; beyond one CTA per SM only for slices of 96 and more
-    // (256 x 512 x 128: one slice 5.5 us, two 6.4; 256 x 256 x 512: one 10.8, two 8.3, four 7.7, eight 12.9)
-    int slices = 1;
-    const int64_t K = g.K * g.k_groups;
-    while (slices < 8 && K >= (int64_t)slices * 2 * 2 * SG_BK && tiles(bm) * slices * 2 <= (K >= (int64_t)slices * 2 * 96 ? 2 * kSMs : kSMs)) slices *= 2;
+    const int bm = sg_tiles(g, 64) >= kSMs ? 64 : 32;
+    const int64_t tiles = sg_tiles(g, bm);
+    GCB_REQUIRE(tiles <= 0x7fffffff / 8, "gemm (FMA): grid too large");
+    const int slices = sg_slices(tiles, g.K * g.k_groups);
     cudaSetDevice(ctx->device);
     int rc;
-#define GCB_SG(BMV) (!ta && !tb ? sg_launch<BMV, false, false>(ctx, g, tm, tn, batches, slices) : !ta ? sg_launch<BMV, false, true>(ctx, g, tm, tn, batches, slices) \
-                     : !tb ? sg_launch<BMV, true, false>(ctx, g, tm, tn, batches, slices) : sg_launch<BMV, true, true>(ctx, g, tm, tn, batches, slices))
+#define GCB_SG(BMV) (!ta && !tb ? sg_run<BMV, false, false>(ctx, g, tiles, slices) : !ta ? sg_run<BMV, false, true>(ctx, g, tiles, slices) \
+                     : !tb ? sg_run<BMV, true, false>(ctx, g, tiles, slices) : sg_run<BMV, true, true>(ctx, g, tiles, slices))
     rc = bm == 64 ? GCB_SG(64) : GCB_SG(32);
 #undef GCB_SG
     if (rc) return rc;
     ctx->last_gemm_engine = 1;
     return after_launch(ctx, "gemm_simt");
+}
+
+// dX (op N, T) and dW (op T, N) in one launch; both with the 32-wide tiles.  False: too large for that.
+bool gemm_simt_backward_fits(const GemmArgs& dx, const GemmArgs& dw) { return sg_tiles(dx, 64) + sg_tiles(dw, 64) < kSMs; }
+int gemm_simt_backward_launch(gcb_ctx* ctx, const GemmArgs& dx, const GemmArgs& dw) {
+    const int64_t t0 = sg_tiles(dx, 32), t1 = sg_tiles(dw, 32);
+    const int slices = sg_slices(t0 + t1, std::min(dx.K * dx.k_groups, dw.K));
+    cudaSetDevice(ctx->device);
+    static bool done[kMaxDevices] = {};
+    const int rc = sg_launch<32>(ctx, done, gemm_simt_backward_kernel<32>, t0 + t1, slices, dx, sg_shape(dx, 32), dw, sg_shape(dw, 32), slices, (unsigned)(t0 * slices));
+    if (rc) return rc;
+    ctx->last_gemm_engine = 1;
+    return after_launch(ctx, "gemm_simt_backward");
 }
 
 }  // namespace gcb

@@ -558,12 +558,20 @@ public:
         return out;
     }
     int64_t out_volume() const { return m_M * m_N; }
+    void backward_together(gcb_ctx* c, const Tensor<float>& g, const float* w, const float* gelu_pre, bool acc_x, Tensor<float>& dx) {
+        auto [dw, acc_w] = m_w.grad_target();
+        auto [db, acc_b] = m_b.grad_target();
+        gcb_check(gcb_linear_group_bwd_f32(c, 1, m_M, m_N, m_K, m_x.data_ptr(), g.data_ptr(), 0, w, 0, gelu_pre, acc_x ? 1.0f : 0.0f, dx.data_ptr(), acc_w ? 1.0f : 0.0f, dw.data_ptr(), 0, db.data_ptr(), 0, acc_b ? 1 : 0),
+                  "linear backward");
+    }
     void backward(const Tensor<float>& g, bool) override {
         Tensor<float> gc = make_contiguous(g);
         gcb_ctx* c = ctx_of(gc);
         MatView w;
         as_matview(m_w, w);
         bool bias_done = false;
+        // a plain layer with a bias: dX and dW go down together
+        const bool plain = m_x.requires_grad() && m_w.requires_grad() && !w.transposed && w.ld == m_N && m_b._get_state() != nullptr && m_b.requires_grad();
         if (m_x.requires_grad()) {  // dX[M,K] = dY[M,N] . W^T
             // x = gelu(pre): the GEMM applies gelu'(pre) in its epilogue and hands the result to pre directly; x itself then
             // receives no gradient here, so the sweep skips the GELU node (any other consumer of x still goes through it)
@@ -572,6 +580,10 @@ public:
             if (gn != nullptr && gn->parent().requires_grad() && gn->parent().is_contiguous() && gn->parent().volume() == m_M * m_K && !m_x._get_state()->m_grad.has_value()) {
                 Tensor<float> pre = gn->parent();
                 auto [dpre, acc] = pre.grad_target();
+                if (!acc && plain) {
+                    backward_together(c, gc, w.p, pre.data_ptr(), false, dpre);
+                    return;
+                }
                 if (!acc) {
                     gcb_check(gcb_gemm_gelu_bwd_f32(c, GCB_OP_N, w.transposed ? GCB_OP_N : GCB_OP_T, m_M, m_K, m_N, gc.data_ptr(), m_N, w.p, w.ld, pre.data_ptr(), dpre.data_ptr()), "matmul dX with GELU backward");
                     fused = true;
@@ -579,6 +591,10 @@ public:
             }
             if (!fused) {
                 auto [dx, acc] = m_x.grad_target();
+                if (plain) {
+                    backward_together(c, gc, w.p, nullptr, acc, dx);
+                    return;
+                }
                 gcb_check(gcb_gemm_f32(c, GCB_OP_N, w.transposed ? GCB_OP_N : GCB_OP_T, m_M, m_K, m_N, 1.0f, gc.data_ptr(), m_N, w.p, w.ld, acc ? 1.0f : 0.0f, dx.data_ptr(), m_K, nullptr), "matmul dX");
             }
         }
@@ -708,11 +724,19 @@ struct LinearGroup {
         int64_t y_stride = 0;
         const bool together = evenly([&](int64_t i) { return dy[(size_t)i]; }, y_stride) && y_stride >= M * N;
         const int64_t runs = together ? 1 : n, per = together ? n : 1;
+        std::optional<Tensor<float>> dx;
+        bool acc_x = false;
         if (x.requires_grad()) {
-            auto [dx, acc] = x.grad_target();
-            for (int64_t i = 0; i < runs; ++i)
-                gcb_check(gcb_linear_group_dx_f32(c, per, M, N, K, dy[(size_t)i], y_stride, members[(size_t)i].w.data_ptr(), w_stride, acc || i > 0 ? 1.0f : 0.0f, dx.data_ptr()), "linear layers dX");
+            auto [t, acc] = x.grad_target();
+            dx = t;
+            acc_x = acc;
         }
+        auto input_gradient = [&] {
+            if (!dx.has_value()) return;
+            for (int64_t i = 0; i < runs; ++i)
+                gcb_check(gcb_linear_group_dx_f32(c, per, M, N, K, dy[(size_t)i], y_stride, members[(size_t)i].w.data_ptr(), w_stride, acc_x || i > 0 ? 1.0f : 0.0f, dx->data_ptr()), "linear layers dX");
+        };
+        if (!members[0].w.requires_grad()) input_gradient();
         if (members[0].w.requires_grad()) {
             std::vector<float*> dw, db;
             std::vector<std::pair<bool, bool>> acc;
@@ -725,7 +749,11 @@ struct LinearGroup {
             int64_t dw_stride = 0, db_stride = 0;
             bool one = together && evenly([&](int64_t i) { return dw[(size_t)i]; }, dw_stride) && dw_stride >= K * N && evenly([&](int64_t i) { return db[(size_t)i]; }, db_stride) && db_stride >= N;
             for (auto& a : acc) one = one && a == acc[0];
-            for (int64_t i = 0; i < (one ? 1 : n); ++i)
+            if (one && dx.has_value()) {
+                gcb_check(gcb_linear_group_bwd_f32(c, n, M, N, K, x.data_ptr(), dy[0], y_stride, members[0].w.data_ptr(), w_stride, nullptr, acc_x ? 1.0f : 0.0f, dx->data_ptr(), acc[0].first ? 1.0f : 0.0f, dw[0], dw_stride, db[0],
+                                                   db_stride, acc[0].second ? 1 : 0), "linear layers backward");
+            } else input_gradient();
+            for (int64_t i = 0; i < (one ? (dx.has_value() ? 0 : 1) : n); ++i)
                 gcb_check(gcb_linear_group_dw_f32(c, one ? n : 1, M, N, K, x.data_ptr(), dy[(size_t)i], y_stride, acc[(size_t)i].first ? 1.0f : 0.0f, dw[(size_t)i], dw_stride, db[(size_t)i], db_stride,
                                                   acc[(size_t)i].second ? 1 : 0), "linear layers dW + bias gradients");
         }

@@ -217,6 +217,11 @@ GCB_API int gcb_linear_group_dx_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int
 GCB_API int gcb_linear_group_dw_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* x, const float* dy, int64_t dy_stride, float beta, float* dW, int64_t w_stride, float* dbias,
                             int64_t bias_stride, int bias_accumulate);
 
+/* Both of them, in one launch where the products are small.  gelu_pre (one layer only): x = gelu(gelu_pre), dx receives
+ * (dy W^T) * gelu'(gelu_pre) as in gcb_gemm_gelu_bwd_f32. */
+GCB_API int gcb_linear_group_bwd_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N, int64_t K, const float* x, const float* dy, int64_t dy_stride, const float* W, int64_t w_stride, const float* gelu_pre, float dx_beta,
+                             float* dx, float dw_beta, float* dW, int64_t dw_stride, float* dbias, int64_t bias_stride, int bias_accumulate);
+
 /* out[(o * batch_inner + i) * rows + r] = sum_c a[o, i, r, c] * b[o, i, r, c]; rows of a and b are addressed through
  * (outer, inner, row) strides in elements, columns are contiguous. */
 GCB_API int gcb_rowdot_batched_f32(gcb_ctx* ctx, float* out, const float* a, int64_t lda, int64_t a_stride_outer, int64_t a_stride_inner,

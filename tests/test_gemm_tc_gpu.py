@@ -636,7 +636,7 @@ def test_fused_causal_attention(env, Bn, H, T, D):
 
 
 @pytest.mark.parametrize("engine", [0, 1])
-@pytest.mark.parametrize("G,M,N,K,family", [(3, 70, 40, 33, None), (3, 1656, 384, 384, "gemm_tc"), (2, 1000, 1152, 264, "gemm_tc"), (2, 700, 513, 300, None), (3, 5000, 1024, 1024, "gemm_tc_pair")])
+@pytest.mark.parametrize("G,M,N,K,family", [(3, 70, 40, 33, None), (3, 250, 96, 130, None), (3, 1656, 384, 384, "gemm_tc"), (2, 1000, 1152, 264, "gemm_tc"), (2, 700, 513, 300, None), (3, 5000, 1024, 1024, "gemm_tc_pair")])
 def test_linear_layers_taken_together(env, engine, G, M, N, K, family):
     """Forward, input gradient (one sum over all layers, cut between them) and weight + bias gradients; K ends inside a block, widths
     that TMA cannot address, strides with gaps, accumulating forms."""
@@ -665,6 +665,14 @@ def test_linear_layers_taken_together(env, engine, G, M, N, K, family):
             assert np.array_equal(tdW[g, K * N :].cpu().numpy(), dW0[g, K * N :])
             assert np.abs(tdb[g, :N].cpu().numpy() - 1.0 - DY[g].sum(0)).max() < 1e-4 * np.abs(DY[g]).sum(0).max()
         assert max_abs_rel(tdx.cpu().numpy(), sum(DY[g] @ Ws[g].T for g in range(G)) + dx0) < TOL
+        # both gradients in one call: one launch where the products are small
+        tdx2, tdW2, tdb2 = torch.empty(M, K, device="cuda"), torch.zeros(G, ws, device="cuda"), torch.empty(G, b.shape[1], device="cuda")
+        ctx.linear_group_bwd_f32(G, M, N, K, tx, tdy, ys, tW, ws, None, 0.0, tdx2, 0.0, tdW2, ws, tdb2, b.shape[1], 0)
+        ctx.sync()
+        assert max_abs_rel(tdx2.cpu().numpy(), sum(DY[g] @ Ws[g].T for g in range(G))) < TOL
+        for g in range(G):
+            assert max_abs_rel(tdW2[g, : K * N].cpu().numpy().reshape(K, N), X.T @ DY[g]) < TOL
+            assert np.abs(tdb2[g, :N].cpu().numpy() - DY[g].sum(0)).max() < 1e-4 * np.abs(DY[g]).sum(0).max()
         if engine == 0 and family == "gemm_tc_pair":
             assert capi.lib().ctx_launch_count_named(ctx.h, b"gemm_tc_pair") > 0
     finally:
