@@ -244,9 +244,9 @@ __global__ void __launch_bounds__(256) strided_kernel(float* __restrict__ out, c
 }
 
 // ---- reductions ----------------------------------------------------------------------------------
-// Stage 1: partial[slab, c] = sum over the slab's rows of in[r, c].  Block = 32 column groups x 8 row lanes.
+// Stage 1: partial[slab, c] (+)= sum over the slab's rows of in[r, c]; a single slab goes straight to the result.  Block = 32 column groups x 8 row lanes.
 template <int VEC>
-__global__ void __launch_bounds__(256) reduce_rows_stage1(float* __restrict__ partial, const float* __restrict__ in, int64_t rows, int64_t cols, int64_t rows_per_slab) {
+__global__ void __launch_bounds__(256) reduce_rows_stage1(float* __restrict__ partial, const float* __restrict__ in, int64_t rows, int64_t cols, int64_t rows_per_slab, int accumulate) {
     pdl_trigger();
     pdl_wait();
     __shared__ float sm[8][32 * VEC + 1];
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) reduce_rows_stage1(float* __restrict__ pa
             float s = 0.0f;
 #pragma unroll
             for (int j = 0; j < 8; ++j) s += sm[j][tx * VEC + k];
-            partial[(int64_t)blockIdx.y * cols + c0 + k] = s;
+            partial[(int64_t)blockIdx.y * cols + c0 + k] = accumulate ? partial[(int64_t)blockIdx.y * cols + c0 + k] + s : s;
         }
     }
 }
@@ -418,13 +418,15 @@ int gcb_reduce_rows_f32(gcb_ctx* ctx, float* out, const float* in, int64_t rows,
     const int64_t rows_per_slab = (rows + slabs - 1) / slabs;
     slabs = (rows + rows_per_slab - 1) / rows_per_slab;
     Scratch sc(ctx);
-    int rc = sc.get(sizeof(float) * slabs * cols);
+    int rc = slabs > 1 ? sc.get(sizeof(float) * slabs * cols) : GCB_OK;
     if (rc) return rc;
+    float* first = slabs > 1 ? sc.as<float>() : out;
+    const int acc1 = slabs > 1 ? 0 : accumulate;
     dim3 grid((unsigned)col_tiles, (unsigned)slabs);
-    if (v4) GCB_CHECK_CUDA(launch_next(ctx->stream, grid, 256, 0, reduce_rows_stage1<4>, sc.as<float>(), in, rows, cols, rows_per_slab));
-    else GCB_CHECK_CUDA(launch_next(ctx->stream, grid, 256, 0, reduce_rows_stage1<1>, sc.as<float>(), in, rows, cols, rows_per_slab));
+    if (v4) GCB_CHECK_CUDA(launch_next(ctx->stream, grid, 256, 0, reduce_rows_stage1<4>, first, in, rows, cols, rows_per_slab, acc1));
+    else GCB_CHECK_CUDA(launch_next(ctx->stream, grid, 256, 0, reduce_rows_stage1<1>, first, in, rows, cols, rows_per_slab, acc1));
     rc = after_launch(ctx, "reduce_rows_stage1");
-    if (rc) return rc;
+    if (rc || slabs == 1) return rc;
     GCB_CHECK_CUDA(launch_next(ctx->stream, (unsigned)((cols + 255) / 256), 256, 0, reduce_rows_stage2, out, sc.as<float>(), slabs, cols, accumulate));
     return after_launch(ctx, "reduce_rows_stage2");
 }
