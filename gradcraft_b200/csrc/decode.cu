@@ -10,8 +10,9 @@
 // without a trip to the host.
 //   * Exchange: a phase needs what all CTAs computed in the one before.  Every exchanged value is an 8-byte word, the float beside
 //     the number of the layer it belongs to; the reader polls the words themselves.  That is one store and one load latency per
-//     phase and no fence (a fence also waits for the weights in flight).  Each buffer is written again only after its readers
-//     have contributed to something the writer needs, so one copy of each is enough (candidates of the arg-max: two).
+//     phase and no fence (a fence also waits for the weights in flight); only keys and values, read a position later, are fenced,
+//     once a position.  Each buffer is written again only after its readers have contributed to something the writer needs, so
+//     one copy of each is enough (candidates of the arg-max: two).
 //   * Products: a CTA owns tiles of eight output columns, i.e. one 32-byte sector of every weight row: N = 1024 columns give 128
 //     tiles for 148 SMs, which wider tiles would not.  Two lanes take a row's sector, sixteen rows per warp load; lane and warp
 //     sums are combined by shuffles and shared memory in a fixed order.
@@ -81,6 +82,10 @@ __device__ __forceinline__ unsigned long long look_word(const unsigned long long
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
     return v;
 }
+// Keys and values travel through the cache with plain stores and loads; the words say when they are there.  Between such a store and the
+// word that announces it, and between the word as seen and the load, stands a fence: of the thread that does both, or of the one that
+// deals with the word where a barrier of the CTA lies between (the fence is cumulative).
+__device__ __forceinline__ void dec_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 constexpr unsigned kDecPolls = 1u << 21;  // of ~1 us: seconds
 // out[u] = the float of w[index(u)] (index < 0: none, 0) as soon as all of them belong to `epoch`; false when they do not in time
 template <int B, class Index>
@@ -392,13 +397,14 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                             }
                         };
                         // Earlier rows are requested before this position's q arrives, where all of them are known to be there: written
-                        // before this call, or before the arg-max exchange that gave this position its token.  Otherwise the words of q
-                        // (from the CTA that wrote this head's earlier rows, after its fence) say so.
+                        // before this call, or before the arg-max exchange that gave this position its token.  Otherwise this position's
+                        // k and v say so: the thread that wrote a column of the earlier rows has fenced them and writes the word now.
                         const bool early = pos == p.pos0 || pos >= p.n_known;
                         if (early) rows(j_first, kk, vv);
                         if (tid < D) {
                             float v[3];
                             ok = get_words<3>(p.qkv + s * C + h * D + tid, [&](int which) { return which * S * C; }, epoch, v, p.status) && ok;
+                            if (!early) dec_fence();
 #pragma unroll
                             for (int i = 0; i < 3; ++i) now[i * kDecMaxHead + tid] = v[i];
                         }
@@ -597,10 +603,9 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                 }
             }
         }
-        // later positions read this one's keys and values from the cache, having seen a word that this thread writes from here on
-        if (tid < S * 8 && cta < 3 * tiles_c) __threadfence();
         if (!ok) break;
-        if (!head) {  // the next token is given
+        if (!head) {  // the next token is given: who wrote keys and values (the threads that finish a group's tiles) writes q, k and v next
+            if (tid < kDecMeet * S * 8 && cta < 3 * tiles_c) dec_fence();
             given_token(pos + 1);
             continue;
         }
@@ -649,6 +654,7 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
             float2 b = best[tid];
 #pragma unroll
             for (int j = 1; j < kDecWarps; ++j) better(b, best[j * S + tid]);
+            dec_fence();  // for the keys and values of all of this CTA's threads, which the barrier above has gathered
             put_word(cand + 2 * (cta * S + tid), b.x, epoch);
             put_word(cand + 2 * (cta * S + tid) + 1, b.y, epoch);
         }
@@ -657,6 +663,7 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
             constexpr int B = (kSMs + 31) / 32;
             float v[2 * B];
             ok = get_words<2 * B>(cand, [&](int u) { const int j = lane + 32 * (u >> 1); return j < (int)gridDim.x ? 2 * (j * S + warp) + (u & 1) : -1; }, epoch, v, p.status) && ok;
+            dec_fence();
 #pragma unroll
             for (int u = 0; u < B; ++u) if (lane + 32 * u < (int)gridDim.x) better(b, make_float2(v[2 * u], v[2 * u + 1]));
 #pragma unroll

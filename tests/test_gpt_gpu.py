@@ -251,3 +251,80 @@ def test_incremental_decoding_follows_the_oracle_for_any_number_of_sequences(arc
         assert np.array_equal(tr.generate(start, prompt + new, context_length=ctx), got[:1])
     finally:
         tr.close()
+
+
+def _gpt_on_device(capi, torch, arch, V, T, C, H, L, F, seed):
+    """A gcb_gpt_model over seeded weights on the device, and what has to stay alive with it."""
+    import ctypes
+
+    fp = ctypes.c_void_p
+
+    class Layer(ctypes.Structure):
+        _fields_ = [(n, fp) for n in ("norm1_gamma", "norm1_beta", "wq", "bq", "wk", "bk", "wv", "bv", "wo", "bo", "norm2_gamma", "norm2_beta", "w1", "b1", "w2", "b2", "w3", "b3")]
+
+    class Model(ctypes.Structure):
+        _fields_ = [(n, ctypes.c_int64) for n in ("V", "T", "C", "H", "L", "F")] + [("eps", ctypes.c_float)] + [(n, fp) for n in ("token_embed", "pos_embed", "final_gamma", "final_beta", "layers")]
+
+    rng = np.random.default_rng(seed)
+    keep = []
+
+    def weight(*shape, std=0.08):
+        keep.append(torch.from_numpy((rng.standard_normal(shape) * std).astype(np.float32)).cuda())
+        return keep[-1].data_ptr()
+
+    gated = arch == "rmsswiglu"
+    layers = (Layer * L)()
+    for lay in layers:
+        for n, shape in dict(norm1_gamma=(C,), norm2_gamma=(C,), wq=(C, C), wk=(C, C), wv=(C, C), wo=(C, C), w1=(C, F), w2=(C, F) if gated else (F, C), bq=(C,), bk=(C,), bv=(C,), bo=(C,), b1=(F,),
+                             b2=(F if gated else C,)).items():
+            setattr(lay, n, weight(*shape, std=1.0 if "gamma" in n else 0.08))
+        if gated:
+            lay.w3, lay.b3 = weight(F, C), weight(C)
+        else:
+            lay.norm1_beta, lay.norm2_beta = weight(C), weight(C)
+    m = Model(V=V, T=T, C=C, H=H, L=L, F=F, eps=1e-5, token_embed=weight(V, C), pos_embed=weight(T, C), final_gamma=weight(C, std=1.0), final_beta=None if gated else weight(C), layers=ctypes.addressof(layers))
+    return m, (keep, layers)
+
+
+@pytest.mark.parametrize("arch,V,C,H,L,F,seqs,n", [
+    ("lngelu", 300, 1024, 16, 2, 2048, 1, 150),  # several tiles a CTA, finished in groups by more threads than a tile has; two stretches of positions
+    ("lngelu", 97, 96, 4, 2, 100, 3, 40),        # more sequences than one
+    ("rmsswiglu", 131, 160, 4, 1, 480, 8, 20),
+])
+def test_given_positions_in_one_launch_equal_one_launch_each(arch, V, C, H, L, F, seqs, n):
+    """A position reads the keys and values that the same launch has written for the earlier ones.  Cache and logits are, bit for bit,
+    those of a launch per position, where the end of each launch orders everything; and so are the tokens where none is given."""
+    import ctypes
+
+    import torch
+
+    from gradcraft_b200 import capi
+
+    T = n + 8
+    ctx = capi.Context()
+    model, alive = _gpt_on_device(capi, torch, arch, V, T, C, H, L, F, seed=11)
+    decoder = ctypes.c_void_p()
+    ctx.gpt_decoder_create(ctypes.byref(model), ctypes.byref(decoder))
+    try:
+        ids = torch.from_numpy(np.random.default_rng(2).integers(0, V, (seqs, T))).cuda()
+
+        def run(chunks, known):
+            cache, toks, logits = torch.zeros(2 * L * seqs * T * C, device="cuda"), ids.clone(), torch.zeros(seqs, V, device="cuda")
+            for i, (pos0, count) in enumerate(chunks):
+                last = logits if known > n and i + 1 == len(chunks) else None
+                capi.lib().gpt_decode_f32(decoder, seqs, cache, T, toks, T, pos0, count, max(known, pos0 + 1), last)
+            ctx.sync()
+            return cache, toks, logits
+
+        one, each = run([(0, n)], n + 1), run([(p, 1) for p in range(n)], n + 1)
+        assert float(each[2].abs().max()) > 0
+        for a, b in zip(one, each):
+            assert torch.equal(a, b)
+        one, each = run([(0, n)], 3), run([(p, 1) for p in range(n)], 3)
+        assert not torch.equal(one[1], ids)
+        for a, b in zip(one, each):
+            assert torch.equal(a, b)
+    finally:
+        capi.lib().gpt_decoder_destroy(decoder)
+        ctx.close()
+    del alive
