@@ -484,6 +484,10 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                     const float* gamma = ph == QKV ? w.norm1_gamma : ph == MLP1 ? w.norm2_gamma : p.final_gamma;
                     const float* beta = ph == QKV ? w.norm1_beta : ph == MLP1 ? w.norm2_beta : p.final_beta;
                     fetch_norm(gamma, beta);
+                    // A given token holds no CTA back, and one with tiles of q, k and v alone (hidden widths below three widths) waits for nobody
+                    // after them: it would write a position's words over the last ones while somebody still looks for those.  The
+                    // stream after the last layer says that nobody does.
+                    if (ph != QKV || l > 0 || (pos > p.pos0 && pos < p.n_known)) load_x(ph == MLP1 ? p.xa : p.xb, ph == QKV ? epoch - 1 : epoch);
                     if (ph == QKV && l == 0) {
                         for (int c0 = tid; c0 < C; c0 += NV * kDecThreads)
 #pragma unroll
@@ -498,8 +502,6 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                                     if (c0 == tid) xr[s][i] = v;
                                 }
                             }
-                    } else {
-                        load_x(ph == MLP1 ? p.xa : p.xb, ph == QKV ? epoch - 1 : epoch);
                     }
                     if (ph == QKV) for (int s = 0; s < p.n_seq; ++s) { l2_prefetch(kc + s * p.seq_stride, (int64_t)pos * C); l2_prefetch(vc + s * p.seq_stride, (int64_t)pos * C); }
                     if ((cta < tiles || ph == HEAD) && !normalise(gamma, beta, ph == HEAD)) break;

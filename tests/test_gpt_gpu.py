@@ -289,6 +289,8 @@ def _gpt_on_device(capi, torch, arch, V, T, C, H, L, F, seed):
 @pytest.mark.parametrize("arch,V,C,H,L,F,seqs,n", [
     ("lngelu", 300, 1024, 16, 2, 2048, 1, 150),  # several tiles a CTA, finished in groups by more threads than a tile has; two stretches of positions
     ("lngelu", 97, 96, 4, 2, 100, 3, 40),        # more sequences than one
+    ("lngelu", 2500, 256, 4, 2, 512, 1, 60),     # a CTA for every SM, a third of which have columns of q, k and v and no others
+    ("lngelu", 2500, 256, 4, 1, 64, 2, 60),      # the same, one layer; fewer hidden columns than columns
     ("rmsswiglu", 131, 160, 4, 1, 480, 8, 20),
 ])
 def test_given_positions_in_one_launch_equal_one_launch_each(arch, V, C, H, L, F, seqs, n):
