@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
     unsigned epoch = 1;
     int buf = 0, stage = 0;
     uint32_t stage_ph = 0;
-    bool ok = true;
+    bool ok = true;  // no wait of this thread has run out; loops are left on it only after dec_sync_and has made it the same for all
     const float inv_c = 1.0f / (float)C;
     const int kt = warp * 16 + (lane >> 1);  // this thread's weight rows: kt + 128 u
 
@@ -504,7 +504,12 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
                             }
                     }
                     if (ph == QKV) for (int s = 0; s < p.n_seq; ++s) { l2_prefetch(kc + s * p.seq_stride, (int64_t)pos * C); l2_prefetch(vc + s * p.seq_stride, (int64_t)pos * C); }
-                    if ((cta < tiles || ph == HEAD) && !normalise(gamma, beta, ph == HEAD)) break;
+                    if (cta < tiles || ph == HEAD) {
+                        if (!normalise(gamma, beta, ph == HEAD)) break;
+                    } else {  // the stream alone, for the residual of MLP2
+                        __syncwarp();
+                        if (!(ok = dec_sync_and(ok))) break;
+                    }
                 } else if (ph == OUT && nsplit > 1) {
                     // weights of the stretches of every head, then their weighted sum: at most 148 stretches in all
                     for (int i = tid; i < heads * nsplit; i += kDecThreads) {
@@ -577,7 +582,7 @@ __global__ void __launch_bounds__(kDecThreads + 32, 1) gpt_decode_kernel(const _
 #pragma unroll 1
                     for (int e = 0; e < kDecMeet && t0 + e / each * (int)gridDim.x < tiles; ++e) tile_dot(K, rb + (e * kDecWarps + warp) * (S * 8));
                     __syncwarp();
-                    dec_sync();
+                    if (!(ok = dec_sync_and(ok))) break;
                     if (mine) {
                         const float* r = rb + g * each * (kDecWarps * S * 8) + (tid & 7) + 8 * s;
                         float v = 0.0f, v2 = 0.0f;
