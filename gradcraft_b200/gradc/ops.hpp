@@ -682,8 +682,9 @@ inline Tensor<float> linear(Tensor<float> x, Tensor<float> w, Tensor<float> b) {
 }
 // Linear layers of one shape over one input whose parameters lie evenly spaced in a parameter arena (consecutive layers do): one
 // product forward, one for dX and one for all dW and bias gradients.  Every member is a tensor of its own with a node of its own; the
-// first to be realized computes all, the last to pass in the backward sweep runs the backward of all.  Each member depends on every
-// weight, so that no parameter counts as final before that.
+// first to be realized computes all.  Between the members and the input stands a state without data, the meeting point: the sweep
+// passes it after every member that it reaches, and there the backward of those that received a gradient runs.  All weights hang on
+// it, so that no parameter counts as final before that.
 struct LinearGroup {
     struct Member {
         Tensor<float> w, b, out;
@@ -693,7 +694,6 @@ struct LinearGroup {
     std::vector<Member> members;  // by ascending weight address
     int64_t M, N, K, w_stride, b_stride;
     std::vector<int64_t> out_shape;
-    size_t passed = 0;
 
     void forward() {
         x.realize();
@@ -706,13 +706,14 @@ struct LinearGroup {
         }
     }
     void backward() {
-        const int64_t n = (int64_t)members.size();
+        std::vector<Member*> live;  // a program need not use every output
+        for (auto& m : members) if (m.grad.has_value()) live.push_back(&m);
+        const int64_t n = (int64_t)live.size();
         gcb_ctx* c = ctx_of(x);
         std::vector<const float*> dy;
-        for (auto& m : members) {
-            if (!m.grad.has_value()) throw std::runtime_error("linear layers: a member of a group has no gradient");
-            m.grad = make_contiguous(m.grad.value());
-            dy.push_back(m.grad->data_ptr());
+        for (Member* m : live) {
+            m->grad = make_contiguous(m->grad.value());
+            dy.push_back(m->grad->data_ptr());
         }
         // evenly spaced runs of `stride` elements: one call; otherwise one per member
         auto evenly = [&](auto&& at, int64_t& stride) {
@@ -722,7 +723,7 @@ struct LinearGroup {
             return ok;
         };
         int64_t y_stride = 0;
-        const bool together = evenly([&](int64_t i) { return dy[(size_t)i]; }, y_stride) && y_stride >= M * N;
+        const bool together = live.size() == members.size() && evenly([&](int64_t i) { return dy[(size_t)i]; }, y_stride) && y_stride >= M * N;
         const int64_t runs = together ? 1 : n, per = together ? n : 1;
         std::optional<Tensor<float>> dx;
         bool acc_x = false;
@@ -734,15 +735,15 @@ struct LinearGroup {
         auto input_gradient = [&] {
             if (!dx.has_value()) return;
             for (int64_t i = 0; i < runs; ++i)
-                gcb_check(gcb_linear_group_dx_f32(c, per, M, N, K, dy[(size_t)i], y_stride, members[(size_t)i].w.data_ptr(), w_stride, acc_x || i > 0 ? 1.0f : 0.0f, dx->data_ptr()), "linear layers dX");
+                gcb_check(gcb_linear_group_dx_f32(c, per, M, N, K, dy[(size_t)i], y_stride, live[(size_t)i]->w.data_ptr(), w_stride, acc_x || i > 0 ? 1.0f : 0.0f, dx->data_ptr()), "linear layers dX");
         };
         if (!members[0].w.requires_grad()) input_gradient();
         if (members[0].w.requires_grad()) {
             std::vector<float*> dw, db;
             std::vector<std::pair<bool, bool>> acc;
-            for (auto& m : members) {
-                auto [gw, aw] = m.w.grad_target();
-                auto [gb, ab] = m.b.grad_target();
+            for (Member* m : live) {
+                auto [gw, aw] = m->w.grad_target();
+                auto [gb, ab] = m->b.grad_target();
                 dw.push_back(gw.data_ptr()); db.push_back(gb.data_ptr());
                 acc.emplace_back(aw, ab);
             }
@@ -758,30 +759,43 @@ struct LinearGroup {
                                                   acc[(size_t)i].second ? 1 : 0), "linear layers dW + bias gradients");
         }
         for (auto& m : members) m.grad.reset();
-        passed = 0;
     }
 };
 
-class LinearGroupNode : public Node<float> {
+class LinearGroupNode : public Node<float> {  // of the meeting point
     std::shared_ptr<LinearGroup> m_group;
+
+public:
+    explicit LinearGroupNode(std::shared_ptr<LinearGroup> group) : m_group(std::move(group)) {}
+    Tensor<float> realize() override { throw std::runtime_error("linear layers: the meeting point of a group holds no data"); }
+    void backward(const Tensor<float>&, bool) override { m_group->backward(); }
+    std::vector<TensorStateBase*> get_input_states() override {
+        std::vector<TensorStateBase*> v{m_group->x._get_state_base()};
+        for (auto& m : m_group->members) { v.push_back(m.w._get_state_base()); v.push_back(m.b._get_state_base()); }
+        return v;
+    }
+};
+
+class LinearMemberNode : public Node<float> {
+    std::shared_ptr<LinearGroup> m_group;
+    Tensor<float> m_meeting;
     size_t m_index;
 
 public:
-    LinearGroupNode(std::shared_ptr<LinearGroup> group, size_t index) : m_group(std::move(group)), m_index(index) {}
+    LinearMemberNode(std::shared_ptr<LinearGroup> group, Tensor<float> meeting, size_t index) : m_group(std::move(group)), m_meeting(std::move(meeting)), m_index(index) {}
     Tensor<float> realize() override {
         Tensor<float>& out = m_group->members[m_index].out;
         if (out._get_state() == nullptr) m_group->forward();
         return std::exchange(out, Tensor<float>());
     }
     void backward(const Tensor<float>& g, bool) override {
+        std::optional<Tensor<float>>& reached = m_meeting._get_state()->m_grad;  // set: the sweep runs the meeting point's backward
+        if (!reached.has_value())
+            for (auto& m : m_group->members) m.grad.reset();  // of a sweep that did not end
+        reached = g;
         m_group->members[m_index].grad = g;
-        if (++m_group->passed == m_group->members.size()) m_group->backward();
     }
-    std::vector<TensorStateBase*> get_input_states() override {
-        std::vector<TensorStateBase*> v{m_group->x._get_state_base()};
-        for (auto& m : m_group->members) { v.push_back(m.w._get_state_base()); v.push_back(m.b._get_state_base()); }
-        return v;
-    }
+    std::vector<TensorStateBase*> get_input_states() override { return {m_meeting._get_state_base()}; }
 };
 
 inline std::vector<Tensor<float>> linear_group(Tensor<float> x, const std::vector<std::pair<Tensor<float>, Tensor<float>>>& layers) {
@@ -816,9 +830,11 @@ inline std::vector<Tensor<float>> linear_group(Tensor<float> x, const std::vecto
     const bool rg = x.requires_grad() || layers[0].first.requires_grad();
     const Device d = x.device();
     group->x = std::move(x);
+    Tensor<float> meeting({}, rg, lazy, d);
+    meeting._get_state()->m_creation_op = std::make_unique<LinearGroupNode>(group);
     for (size_t i = 0; i < n; ++i) {
         Tensor<float> out(group->out_shape, rg, lazy, d);
-        out._get_state()->m_creation_op = std::make_unique<LinearGroupNode>(group, i);
+        out._get_state()->m_creation_op = std::make_unique<LinearMemberNode>(group, meeting, i);
         outs[order[i]] = std::move(out);
     }
     return outs;
