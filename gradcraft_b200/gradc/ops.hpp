@@ -806,7 +806,7 @@ inline std::vector<Tensor<float>> linear_group(Tensor<float> x, const std::vecto
     auto in_arena = [](const Tensor<float>& t) { return t._get_state() != nullptr && t._get_state()->m_slot.arena != nullptr && t.is_dense(); };
     bool ok = n > 1 && !x.shape().empty() && !x.device().is_cpu();
     for (const auto& [w, b] : layers)
-        ok = ok && in_arena(w) && in_arena(b) && w._get_state()->m_slot.arena == layers[0].first._get_state()->m_slot.arena && w.shape() == layers[0].first.shape() && w.shape().size() == 2 && w.shape()[0] == x.shape().back() &&
+        ok = ok && in_arena(w) && in_arena(b) && w.device() == x.device() && b.device() == x.device() && w._get_state()->m_slot.arena == layers[0].first._get_state()->m_slot.arena && w.shape() == layers[0].first.shape() && w.shape().size() == 2 && w.shape()[0] == x.shape().back() &&
              b.volume() == w.shape()[1] && w.requires_grad() == layers[0].first.requires_grad() && b.requires_grad() == w.requires_grad();
     auto group = std::make_shared<LinearGroup>();
     if (ok) {
