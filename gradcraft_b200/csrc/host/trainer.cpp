@@ -167,12 +167,26 @@ int gct_forward_backward(gct_trainer* tr, const int64_t* tokens, const int64_t* 
         logits = Tensor<float>();  // the loss node is now the only holder: probabilities may overwrite the logits
         Tensor<float> scaled = accum > 1 ? loss / static_cast<float>(accum) : loss;
         scaled.realize();
-        // the loss travels while the backward sweep is being launched: waiting for it here would leave the GPU without work for as long
-        // as the next launches take
+        // A skipped id and a wait that ran out are reported with the loss, and no gradient may then hold this batch.  Where there are no
+        // gradients yet (the first micro-batch after zero_grad) the loss travels while the sweep is being launched, as waiting for it
+        // would leave the GPU without work for as long as the next launches take, and a bad batch's gradients are dropped again.
+        // Where they would be added to, or averaged over ranks before the report, the loss comes first.
         gcb_ctx* c = Backend::get().ctx(tr->gpu);
-        if (loss_out) gcb_check(gcb_read_scalar_begin(c, scaled.data_ptr()), "loss");
-        scaled.backward();
-        if (loss_out) gcb_check(gcb_read_scalar_end(c, loss_out), "loss");
+        bool droppable = true;
+        for (auto& [name, p] : tr->ordered) droppable = droppable && !p->tensor()._get_state()->m_grad.has_value();
+        if (auto a = tr->model->arena()) droppable = droppable && a->dp_world <= 1;
+        if (!loss_out) {
+            scaled.backward();
+        } else if (droppable) {
+            gcb_check(gcb_read_scalar_begin(c, scaled.data_ptr()), "loss");
+            scaled.backward();
+            const int rc = gcb_read_scalar_end(c, loss_out);
+            if (rc != GCB_OK) tr->model->zero_grad();
+            gcb_check(rc, "loss");
+        } else {
+            *loss_out = scaled.item();
+            scaled.backward();
+        }
     });
 }
 

@@ -124,6 +124,45 @@ def test_training_step_reports_a_skipped_target_and_a_given_up_wait():
         tr.close()
 
 
+def test_a_reported_batch_leaves_no_trace_in_the_gradients():
+    """A call that fails on a skipped target leaves the gradients as they were: none after zero_grad (and an optimizer step then changes
+    no weight), the earlier micro-batch's, bit for bit, where they are accumulated."""
+    from gradcraft_b200.trainer import Trainer, TrainerError
+
+    arch, V, T, C, H, L, F, B = "rmsswiglu", 96, 16, 32, 4, 2, 96, 3
+    w = synth.gpt_weights(arch, V, T, C, H, L, F, seed=0, perturb=True)
+    (X, Y), (X2, Y2) = ((np.ascontiguousarray(a) for a in b) for b in synth.token_batches(7, 2, B, T, V))
+    bad = Y2.copy()
+    bad[2, 1] = -3
+    tr = Trainer(arch, V, T, C, H, L, F, clip=1.0)
+    try:
+        tr.load(w)
+        tr.zero_grad()
+        with pytest.raises(TrainerError, match="outside its table"):
+            tr.forward_backward(X2, bad)
+        with pytest.raises(TrainerError, match="no gradient"):
+            tr.get("grad")
+        tr.optimizer_step()
+        after = tr.get("param")
+        assert all(np.array_equal(after[k].reshape(-1), w[k].reshape(-1)) for k in w)
+        tr.zero_grad()
+        tr.forward_backward(X, Y, 2)
+        first = tr.get("grad")
+        with pytest.raises(TrainerError, match="outside its table"):
+            tr.forward_backward(X2, bad, 2)
+        now = tr.get("grad")
+        assert all(np.array_equal(now[k], first[k]) for k in first)
+        tr.forward_backward(X2, Y2, 2)  # and the step goes on from there
+        both = tr.get("grad")
+        tr.zero_grad()
+        for x, y in ((X, Y), (X2, Y2)):
+            tr.forward_backward(x, y, 2)
+        clean = tr.get("grad")
+        assert all(np.array_equal(both[k], clean[k]) for k in clean)
+    finally:
+        tr.close()
+
+
 def test_arena_order_follows_gradient_finality():
     from gradcraft_b200.trainer import Trainer
 
