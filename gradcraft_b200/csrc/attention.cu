@@ -794,13 +794,13 @@ extern "C" {
 
 // Long sequences: heads of up to 64 columns (tensor memory holds two query tiles of that width) and the split arithmetic of mode 2; TMA wants
 // every stride in whole 16 bytes.  From 129 positions on this is the faster way whatever the number of heads (8 heads of 180 x 64: 94 ->
-// 55 us, 768 of 130 x 48: 329 -> 303, 1024 of 192 x 64: 456 -> 393).  Exactly 256 stays with the separate kernels, whose score tiles it
-// fills: whole steps of that length are what those kernels, which wider heads need, are held to the reference by.
+// 55 us, 768 of 130 x 48: 329 -> 303, 1024 of 192 x 64: 456 -> 393, 80 of 256 x 64:
+// 99 -> 77, 512 of 256 x 64: 306 -> 283).
 int gcb_attention_supported(gcb_ctx* ctx, int64_t B, int64_t H, int64_t T, int64_t D, const float* q, int64_t q_ld, int64_t q_so, int64_t q_si, const float* k, int64_t k_ld, int64_t k_so, int64_t k_si, const float* v,
                             int64_t v_ld, int64_t v_so, int64_t v_si, float scale) {
-    if (!ctx || B <= 0 || H <= 0 || !rows_ok(q, q_ld, q_so, q_si, B, H) || !rows_ok(k, k_ld, k_so, k_si, B, H) || !rows_ok(v, v_ld, v_so, v_si, B, H)) return 0;
+    if (!ctx || !ctx->fused_attention || B <= 0 || H <= 0 || !rows_ok(q, q_ld, q_so, q_si, B, H) || !rows_ok(k, k_ld, k_so, k_si, B, H) || !rows_ok(v, v_ld, v_so, v_si, B, H)) return 0;
     if (takes_small(ctx, B, H, T, D)) return 1;
-    return ctx->gemm_engine != 1 && ctx->gemm_split_mode == 2 && T > kSmallT && T != 256 && T < (int64_t(1) << 24) && D > 0 && D <= 64 && D % 4 == 0 && B * H * ((T + 127) / 128) < (int64_t(1) << 30) && scale > 0.0f && tma_encode(ctx) != nullptr;
+    return ctx->gemm_engine != 1 && ctx->gemm_split_mode == 2 && T > kSmallT && T < (int64_t(1) << 24) && D > 0 && D <= 64 && D % 4 == 0 && B * H * ((T + 127) / 128) < (int64_t(1) << 30) && scale > 0.0f && tma_encode(ctx) != nullptr;
 }
 
 int gcb_attention_fwd_f32(gcb_ctx* ctx, int64_t B, int64_t H, int64_t T, int64_t D, float* out, int64_t o_ld, int64_t o_so, int64_t o_si, float* stats, const float* q, int64_t q_ld, int64_t q_so, int64_t q_si,

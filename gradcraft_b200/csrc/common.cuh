@@ -77,6 +77,7 @@ struct gcb_ctx {
     int gemm_engine = 0;       // 0 auto, 1 simt, 2 tcgen05
     int last_gemm_engine = 0;
     int gemm_split_mode = 2;   // see gcb_ctx_set_gemm_split_mode
+    bool fused_attention = true;  // see gcb_ctx_set_fused_attention
     int* d_status = nullptr;   // device-side status word written by kernels that give up on a bounded wait
     char* h_small = nullptr;   // 256 pinned bytes for values the host reads back: results in front, the status word from byte 192, a scalar on its way from byte 208
     cudaEvent_t ev_scalar = nullptr;  // gcb_read_scalar_begin / _end

@@ -230,6 +230,11 @@ int gcb_ctx_set_gemm_split_mode(gcb_ctx* ctx, int mode) {
     ctx->gemm_split_mode = mode;
     return GCB_OK;
 }
+int gcb_ctx_set_fused_attention(gcb_ctx* ctx, int on) {
+    GCB_REQUIRE(ctx && (on == 0 || on == 1), "gcb_ctx_set_fused_attention: on must be 0 or 1");
+    ctx->fused_attention = on != 0;
+    return GCB_OK;
+}
 int gcb_ctx_gemm_split_mode(gcb_ctx* ctx) { return ctx ? ctx->gemm_split_mode : -1; }
 
 // Self-test of the failure path every barrier wait in this library has: one thread waits on an mbarrier that nothing will

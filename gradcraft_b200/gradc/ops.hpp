@@ -861,6 +861,20 @@ class SDPANode : public Node<float> {
     std::shared_ptr<Storage<float>> m_out_storage;  // O, for the row term dO . O of the softmax backward: the storage object of the tensor this node creates (realize() hands it the data)
 
     static void strides4(const Tensor<float>& t, int64_t& so, int64_t& si, int64_t& ld) { so = t.strides()[0]; si = t.strides()[1]; ld = t.strides()[2]; }
+    bool fused() const {
+        int64_t qo, qi, ql, ko, ki, kl, vo, vi, vl;
+        strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl); strides4(m_v, vo, vi, vl);
+        return gcb_attention_supported(ctx_of(m_q), m_B, m_H, m_T, m_D, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale) == 1;
+    }
+    void probabilities() {
+        gcb_ctx* c = ctx_of(m_q);
+        const int64_t B = m_B, H = m_H, T = m_T, D = m_D;
+        int64_t qo, qi, ql, ko, ki, kl;
+        strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl);
+        m_probs = Tensor<float>({B * H, T, m_ld}, m_q.device(), uninitialized);
+        gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_T, T, T, D, 1.0f, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, 0.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, B, H, 1), "attention scores");
+        gcb_check(gcb_causal_softmax_fwd_band_ld_f32(c, m_probs.data_ptr(), m_probs.data_ptr(), m_scale, B * H * T, T, m_ld, kCausalBand), "causal softmax");
+    }
 
 public:
     SDPANode(Tensor<float> q, Tensor<float> k, Tensor<float> v, float scale) : m_q(std::move(q)), m_k(std::move(k)), m_v(std::move(v)), m_scale(scale) {
@@ -874,15 +888,13 @@ public:
         const int64_t B = m_B, H = m_H, T = m_T, D = m_D;
         int64_t qo, qi, ql, ko, ki, kl, vo, vi, vl;
         strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl); strides4(m_v, vo, vi, vl);
-        if (gcb_attention_supported(c, B, H, T, D, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale)) {
+        if (fused()) {
             m_stats = Tensor<float>({gcb_attention_stats_floats(B, H, T)}, m_q.device(), uninitialized);
             Tensor<float> mem({B, T, H, D}, m_q.device(), uninitialized);
             gcb_check(gcb_attention_fwd_f32(c, B, H, T, D, mem.data_ptr(), H * D, T * H * D, D, m_stats.data_ptr(), m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale), "attention");
             return Tensor<float>({B, H, T, D}, out_strides(H, T, D), 0, mem._get_storage(), false);
         }
-        m_probs = Tensor<float>({B * H, T, m_ld}, m_q.device(), uninitialized);
-        gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_T, T, T, D, 1.0f, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, 0.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, B, H, 1), "attention scores");
-        gcb_check(gcb_causal_softmax_fwd_band_ld_f32(c, m_probs.data_ptr(), m_probs.data_ptr(), m_scale, B * H * T, T, m_ld, kCausalBand), "causal softmax");
+        probabilities();
         Tensor<float> mem({B, T, H, D}, m_q.device(), uninitialized);
         gcb_check(gcb_gemm_batched_causal_f32(c, GCB_OP_N, GCB_OP_N, T, D, T, 1.0f, m_probs.data_ptr(), m_ld, H * T * m_ld, T * m_ld, m_v.data_ptr(), vl, vo, vi, 0.0f, mem.data_ptr(), H * D, T * H * D, D, B, H, 2), "attention output");
         return Tensor<float>({B, H, T, D}, out_strides(H, T, D), 0, mem._get_storage(), false);
@@ -899,6 +911,10 @@ public:
         const int64_t each = (B * T * H * D + 3) / 4 * 4;
         Tensor<float> block({3 * each}, g.device(), uninitialized);
         auto part = [&](int64_t i) { return Tensor<float>({B, H, T, D}, out_strides(H, T, D), i * each, block._get_storage(), false); };
+        if (m_stats._get_state() != nullptr && !fused()) {  // the context's settings have changed since the forward
+            probabilities();
+            m_stats = Tensor<float>();
+        }
         if (m_stats._get_state() != nullptr) {
             if (reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 != 0 || gl % 4 != 0 || go % 4 != 0 || gi % 4 != 0 || gl <= 0 || go <= 0 || gi <= 0) { g = make_contiguous(g); strides4(g, go, gi, gl); }
             Tensor<float> dq = part(2), dk = part(1), dv = part(0);

@@ -88,6 +88,9 @@ GCB_API int gcb_ctx_set_gemm_engine(gcb_ctx* ctx, int engine);
  * GRADC_TC_SPLIT_MODE sets the initial value of new contexts. */
 GCB_API int gcb_ctx_set_gemm_split_mode(gcb_ctx* ctx, int mode);
 GCB_API int gcb_ctx_gemm_split_mode(gcb_ctx* ctx);
+/* 0: gcb_attention_supported declines everything, so that attention goes through the batched products and the causal softmax (the path
+ * that heads beyond the fused kernels' range take anyway).  1 (default): the fused kernels take what they can. */
+GCB_API int gcb_ctx_set_fused_attention(gcb_ctx* ctx, int on);
 
 /* ---- arena: CUDAMemPool::{allocate,free,clear,get_hwm_gb}, memory_pool.hpp:40-102 -------------- */
 GCB_API int gcb_arena_alloc(gcb_ctx* ctx, size_t bytes, void** out);

@@ -604,10 +604,11 @@ def test_small_products_on_the_fma_kernel(env, opa, opb, M, N, K):
         ctx.ctx_set_gemm_engine(2)
 
 
-@pytest.mark.parametrize("Bn,H,T,D", [(1, 1, 257, 64), (1, 2, 129, 64), (2, 2, 255, 32), (2, 3, 384, 64), (1, 2, 511, 32), (3, 2, 300, 20), (1, 1, 1025, 4), (40, 4, 260, 48), (1, 1, 1, 4), (2, 3, 63, 32), (2, 2, 65, 64), (1, 2, 128, 128), (3, 1, 100, 68)])
+@pytest.mark.parametrize("Bn,H,T,D", [(1, 1, 257, 64), (1, 2, 129, 64), (2, 2, 255, 32), (2, 2, 256, 64), (3, 2, 256, 32), (2, 3, 384, 64), (1, 2, 511, 32), (3, 2, 300, 20), (1, 1, 1025, 4), (40, 4, 260, 48), (1, 1, 1, 4), (2, 3, 63, 32), (2, 2, 65, 64), (1, 2, 128, 128), (3, 1, 100, 68)])
 def test_fused_causal_attention(env, Bn, H, T, D):
     """Both pairs of kernels (up to 128 positions: fp32 FMA): partial and whole query tiles, one and two tiles a CTA, several items a CTA, padded head widths; scores that grow along the
-    row (the running maximum moves); out of its range the entry points decline."""
+    row (the running maximum moves).  256 positions are taken like any other length; heads beyond the range, and contexts that asked for
+    the separate kernels, are declined."""
     ctx, torch, capi = env
     ctx.ctx_set_gemm_engine(0)
     C, scale = H * D, 1.0 / np.sqrt(D)
@@ -632,7 +633,18 @@ def test_fused_causal_attention(env, Bn, H, T, D):
     for got, ref in ((out, O), (gq, dS @ K), (gk, dS.transpose(0, 1, 3, 2) @ Q), (gv, P.transpose(0, 1, 3, 2) @ G)):
         got = heads(got.cpu().numpy())
         assert np.linalg.norm(got - ref) <= TOL * np.linalg.norm(ref)
-    assert not capi.lib().attention_supported(ctx.h, Bn, H, 256, D, dq.data_ptr(), *rows, dk.data_ptr(), *rows, dv.data_ptr(), *rows, scale)
+
+    def takes(length, width):
+        return capi.lib().cdll.gcb_attention_supported(ctx.h, Bn, H, length, width, dq.data_ptr(), *rows, dk.data_ptr(), *rows, dv.data_ptr(), *rows, scale)
+
+    ctx.ctx_set_gemm_engine(0)
+    try:
+        assert takes(256, 64) == 1 and takes(256, 68) == 0 and takes(T, D) == 1
+        ctx.ctx_set_fused_attention(0)
+        assert takes(256, 64) == 0 and takes(T, D) == 0
+    finally:
+        ctx.ctx_set_fused_attention(1)
+        ctx.ctx_set_gemm_engine(2)
 
 
 @pytest.mark.parametrize("engine", [0, 1])

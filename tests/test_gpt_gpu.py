@@ -11,7 +11,7 @@ from tests.helpers import assert_grads_close, assert_matches_digest, load_golden
 pytestmark = pytest.mark.gpu
 
 
-def run_case(name, engine=None, split_mode=None, families=()):
+def run_case(name, engine=None, split_mode=None, families=(), fused_attention=True):
     from gradcraft_b200 import capi
     from gradcraft_b200.trainer import Trainer
 
@@ -25,7 +25,9 @@ def run_case(name, engine=None, split_mode=None, families=()):
         assert tr.num_params() == sum(v.size for v in w.values())
         if split_mode is not None:
             capi.lib().ctx_set_gemm_split_mode(tr.context(), split_mode)
+        capi.lib().ctx_set_fused_attention(tr.context(), int(fused_attention))
         tr.load(w)
+        launched = {fam: capi.lib().ctx_launch_count_named(tr.context(), fam.encode()) for fam in families}
         losses = []
         for step in range(1, steps + 1):
             tr.zero_grad()
@@ -59,8 +61,10 @@ def run_case(name, engine=None, split_mode=None, families=()):
                 assert float(np.abs(a.reshape(ref_w[k].shape) - ref_w[k]).max()) < 2e-5, k
         assert tr.launch_count() > 0
         for fam in families:  # the kernel families this case exists to reach
-            assert capi.lib().ctx_launch_count_named(tr.context(), fam.encode()) > 0, "no launch of kernel family " + fam
+            assert capi.lib().ctx_launch_count_named(tr.context(), fam.encode()) > launched[fam], "no launch of kernel family " + fam
     finally:
+        capi.lib().ctx_set_fused_attention(tr.context(), 1)  # the trainers of a process share a device's context
+        capi.lib().ctx_set_gemm_split_mode(tr.context(), 2)
         tr.close()
 
 
@@ -69,20 +73,28 @@ def test_training_matches_reference(name):
     run_case(name)
 
 
-def test_mid_size_training_step_runs_the_full_size_kernels_and_matches_reference():
+SEPARATE_ATTENTION, FUSED_ATTENTION = ("gemm_tc_256_softmax_bwd", "gemm_tc_64"), ("attention_fwd", "attention_delta", "attention_bwd")
+
+
+@pytest.mark.parametrize("attention", [SEPARATE_ATTENTION, FUSED_ATTENTION], ids=["separate", "fused"])
+def test_mid_size_training_step_runs_the_full_size_kernels_and_matches_reference(attention):
     """5120 rows x 256 / 1024 columns, 80 heads of 256 x 64: one step goes through the CTA-pair GEMM (plain and with both GELU
-    epilogues), split-K weight gradients, the 256-wide dS GEMM with the softmax backward in its epilogue, the 64-wide causal
-    attention GEMMs and the staged LayerNorm backward, i.e. the kernels the full-size benchmark runs, and is held to the
-    same loss / gradient / weight bar against the compiled reference (3 steps with clipping)."""
-    run_case("mid_lngelu", families=("gemm_tc_pair", "gemm_tc_pair_gelu_fwd", "gemm_tc_pair_gelu_bwd", "gemm_tc_pair_residual", "splitk_reduce", "gemm_tc_256_softmax_bwd", "gemm_tc_64",
-                                     "layernorm_bwd_ring", "adamw_arena", "scatter_accumulate", "scatter_fold", "softmax_ce_bwd"))
+    epilogues), split-K weight gradients and the staged LayerNorm backward, i.e. the kernels the full-size benchmark runs, and is
+    held to the same loss / gradient / weight bar against the compiled reference (3 steps with clipping), with either attention:
+    the fused kernels, and what heads beyond their range take (the 256-wide dS GEMM with the softmax backward in its epilogue, the
+    64-wide causal attention GEMMs)."""
+    run_case("mid_lngelu", fused_attention=attention is FUSED_ATTENTION,
+             families=("gemm_tc_pair", "gemm_tc_pair_gelu_fwd", "gemm_tc_pair_gelu_bwd", "gemm_tc_pair_residual", "splitk_reduce", "layernorm_bwd_ring", "adamw_arena", "scatter_accumulate", "scatter_fold",
+                       "softmax_ce_bwd") + attention)
 
 
-def test_mid_size_rmsnorm_swiglu_training_step_matches_reference():
+@pytest.mark.parametrize("attention", [SEPARATE_ATTENTION, FUSED_ATTENTION], ids=["separate", "fused"])
+def test_mid_size_rmsnorm_swiglu_training_step_matches_reference(attention):
     """The reference's own GPT (RMSNorm + SwiGLU) at 5120 rows: the staged RMSNorm backward, the fused SwiGLU kernels and the
-    CTA-pair GEMM on 768-wide outputs, held to the loss / gradient / weight bar against the compiled reference (3 steps, clip)."""
-    run_case("mid_rmsswiglu", families=("gemm_tc_pair", "gemm_tc_pair_residual", "splitk_reduce", "gemm_tc_256_softmax_bwd", "gemm_tc_64", "rmsnorm_bwd_ring", "swiglu_fwd", "swiglu_bwd", "adamw_arena",
-                                        "scatter_accumulate", "scatter_fold", "softmax_ce_bwd"))
+    CTA-pair GEMM on 768-wide outputs, held to the loss / gradient / weight bar against the compiled reference (3 steps, clip), with
+    either attention."""
+    run_case("mid_rmsswiglu", fused_attention=attention is FUSED_ATTENTION,
+             families=("gemm_tc_pair", "gemm_tc_pair_residual", "splitk_reduce", "rmsnorm_bwd_ring", "swiglu_fwd", "swiglu_bwd", "adamw_arena", "scatter_accumulate", "scatter_fold", "softmax_ce_bwd") + attention)
 
 
 def test_training_matches_reference_with_three_tf32_products():
