@@ -70,7 +70,7 @@ class Lib:
             fn = getattr(self.cdll, name)  # AttributeError here means the header declares a symbol the library lacks
             fn.restype, fn.argtypes = restype, argtypes
             self.names.append(name)
-            checked = restype is ctypes.c_int and name not in ("gcb_ctx_device", "gcb_ctx_last_gemm_engine", "gcb_ctx_gemm_split_mode", "gcb_gpt_decode_supported")
+            checked = restype is ctypes.c_int and name not in ("gcb_ctx_device", "gcb_ctx_last_gemm_engine", "gcb_ctx_gemm_split_mode", "gcb_gpt_decode_supported", "gcb_attention_supported", "gcb_attention_preferred")
             setattr(self, name[4:], self._wrap(fn, checked, [i for i, t in enumerate(argtypes) if t is ctypes.c_void_p]))
 
     def _wrap(self, fn, checked, pointers):

@@ -785,10 +785,10 @@ int64_t gcb_attention_stats_floats(int64_t batch, int64_t heads, int64_t seq_len
 
 }  // extern "C"
 
-// Short sequences, in any split mode, while a CTA per 32 rows leaves SMs over: 16 heads of 64 x 32 take 19 us instead of 30 in nine
-// launches, 16 heads of 96 x 64 35 instead of 36; 96 heads of 128 x 64 would take 81 instead of 60.
+// Short sequences, in any split mode, while a CTA per 32 rows leaves SMs over.
 constexpr int64_t kSmallT = 128;
-static bool takes_small(gcb_ctx* ctx, int64_t B, int64_t H, int64_t T, int64_t D) { return T <= kSmallT && T > 0 && D > 0 && D <= 128 && D % 4 == 0 && ctx->gemm_engine != 2 && B * H * ((T + AS_OWN - 1) / AS_OWN) <= kSMs; }
+static int64_t small_ctas(int64_t B, int64_t H, int64_t T) { return B * H * ((T + AS_OWN - 1) / AS_OWN); }
+static bool takes_small(gcb_ctx* ctx, int64_t B, int64_t H, int64_t T, int64_t D) { return T <= kSmallT && T > 0 && D > 0 && D <= 128 && D % 4 == 0 && ctx->gemm_engine != 2 && small_ctas(B, H, T) <= kSMs; }
 
 extern "C" {
 
@@ -798,9 +798,22 @@ extern "C" {
 // 99 -> 77, 512 of 256 x 64: 306 -> 283).
 int gcb_attention_supported(gcb_ctx* ctx, int64_t B, int64_t H, int64_t T, int64_t D, const float* q, int64_t q_ld, int64_t q_so, int64_t q_si, const float* k, int64_t k_ld, int64_t k_so, int64_t k_si, const float* v,
                             int64_t v_ld, int64_t v_so, int64_t v_si, float scale) {
-    if (!ctx || !ctx->fused_attention || B <= 0 || H <= 0 || !rows_ok(q, q_ld, q_so, q_si, B, H) || !rows_ok(k, k_ld, k_so, k_si, B, H) || !rows_ok(v, v_ld, v_so, v_si, B, H)) return 0;
+    if (!ctx || B <= 0 || H <= 0 || !rows_ok(q, q_ld, q_so, q_si, B, H) || !rows_ok(k, k_ld, k_so, k_si, B, H) || !rows_ok(v, v_ld, v_so, v_si, B, H)) return 0;
     if (takes_small(ctx, B, H, T, D)) return 1;
     return ctx->gemm_engine != 1 && ctx->gemm_split_mode == 2 && T > kSmallT && T < (int64_t(1) << 24) && D > 0 && D <= 64 && D % 4 == 0 && B * H * ((T + 127) / 128) < (int64_t(1) << 30) && scale > 0.0f && tma_encode(ctx) != nullptr;
+}
+
+// Where the short kernels pay.  A CTA's chain is as long as its tiles of 64 on the other side times their columns, and the nine launches
+// that it replaces spread theirs over more CTAs.  Forward + backward in a stream of launches, separate -> fused: a chain of 64 columns
+// wins at any number of heads (16 heads of 64 x 32 30 -> 20 us, 96 of 32 x 32 31 -> 20, 36 of 128 x 32 46 -> 44); one of 128 from about 60
+// CTAs on (32 CTAs of 128 x 64 37 -> 40, 48 of 96 x 64 40 -> 41, 96 of 128 x 64 48 -> 42, 144 53 -> 50, 144 of 64 x 128 57 -> 48; a
+// two-layer step with 12 CTAs of 96 x 64 413 -> 434 us, with 60 of 128 x 64 691 -> 685); a longer one does not (64 CTAs of 128 x 96
+// 51 -> 75, 144 of 100 x 68 55 -> 79), but where a product in between meets an unlucky tile (147 CTAs of 96 x 72: 94 -> 71).
+int gcb_attention_preferred(gcb_ctx* ctx, int64_t B, int64_t H, int64_t T, int64_t D) {
+    if (!ctx || !ctx->fused_attention || B <= 0 || H <= 0) return 0;
+    if (!takes_small(ctx, B, H, T, D)) return 1;  // whatever gcb_attention_supported takes
+    const int64_t chain = (T + AS_T - 1) / AS_T * D;
+    return chain <= 64 || (chain <= 128 && 5 * small_ctas(B, H, T) >= 2 * kSMs);
 }
 
 int gcb_attention_fwd_f32(gcb_ctx* ctx, int64_t B, int64_t H, int64_t T, int64_t D, float* out, int64_t o_ld, int64_t o_so, int64_t o_si, float* stats, const float* q, int64_t q_ld, int64_t q_so, int64_t q_si,

@@ -991,7 +991,7 @@ class IncrementalGPT {
             project_two(v, k, a, w.wv, w.wk, w.bv, w.bk, rows, C, C);
             if (l + 1 == m.L) break;
             project(q, a, w.wq, w.bq, rows, C, C);
-            if (gcb_attention_supported(m_ctx, seqs, H, n, D, q, C, n * C, D, k, C, m_cap * C, D, v, C, m_cap * C, D, scale)) {
+            if (gcb_attention_preferred(m_ctx, seqs, H, n, D) && gcb_attention_supported(m_ctx, seqs, H, n, D, q, C, n * C, D, k, C, m_cap * C, D, v, C, m_cap * C, D, scale)) {
                 at_least(m_stats, gcb_attention_stats_floats(seqs, H, n), m_device);
                 gcb_check(gcb_attention_fwd_f32(m_ctx, seqs, H, n, D, o, C, n * C, D, m_stats.data_ptr(), q, C, n * C, D, k, C, m_cap * C, D, v, C, m_cap * C, D, scale), "attention");
             } else {

@@ -861,7 +861,7 @@ class SDPANode : public Node<float> {
     std::shared_ptr<Storage<float>> m_out_storage;  // O, for the row term dO . O of the softmax backward: the storage object of the tensor this node creates (realize() hands it the data)
 
     static void strides4(const Tensor<float>& t, int64_t& so, int64_t& si, int64_t& ld) { so = t.strides()[0]; si = t.strides()[1]; ld = t.strides()[2]; }
-    bool fused() const {
+    bool supported() const {
         int64_t qo, qi, ql, ko, ki, kl, vo, vi, vl;
         strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl); strides4(m_v, vo, vi, vl);
         return gcb_attention_supported(ctx_of(m_q), m_B, m_H, m_T, m_D, m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale) == 1;
@@ -888,7 +888,7 @@ public:
         const int64_t B = m_B, H = m_H, T = m_T, D = m_D;
         int64_t qo, qi, ql, ko, ki, kl, vo, vi, vl;
         strides4(m_q, qo, qi, ql); strides4(m_k, ko, ki, kl); strides4(m_v, vo, vi, vl);
-        if (fused()) {
+        if (gcb_attention_preferred(c, B, H, T, D) && supported()) {
             m_stats = Tensor<float>({gcb_attention_stats_floats(B, H, T)}, m_q.device(), uninitialized);
             Tensor<float> mem({B, T, H, D}, m_q.device(), uninitialized);
             gcb_check(gcb_attention_fwd_f32(c, B, H, T, D, mem.data_ptr(), H * D, T * H * D, D, m_stats.data_ptr(), m_q.data_ptr(), ql, qo, qi, m_k.data_ptr(), kl, ko, ki, m_v.data_ptr(), vl, vo, vi, m_scale), "attention");
@@ -911,7 +911,7 @@ public:
         const int64_t each = (B * T * H * D + 3) / 4 * 4;
         Tensor<float> block({3 * each}, g.device(), uninitialized);
         auto part = [&](int64_t i) { return Tensor<float>({B, H, T, D}, out_strides(H, T, D), i * each, block._get_storage(), false); };
-        if (m_stats._get_state() != nullptr && !fused()) {  // the context's settings have changed since the forward
+        if (m_stats._get_state() != nullptr && !supported()) {  // the context's settings have changed since the forward
             probabilities();
             m_stats = Tensor<float>();
         }

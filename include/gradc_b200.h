@@ -88,8 +88,8 @@ GCB_API int gcb_ctx_set_gemm_engine(gcb_ctx* ctx, int engine);
  * GRADC_TC_SPLIT_MODE sets the initial value of new contexts. */
 GCB_API int gcb_ctx_set_gemm_split_mode(gcb_ctx* ctx, int mode);
 GCB_API int gcb_ctx_gemm_split_mode(gcb_ctx* ctx);
-/* 0: gcb_attention_supported declines everything, so that attention goes through the batched products and the causal softmax (the path
- * that heads beyond the fused kernels' range take anyway).  1 (default): the fused kernels take what they can. */
+/* 0: gcb_attention_preferred declines everything, so that attention goes through the batched products and the causal softmax (the path
+ * that heads beyond the fused kernels' range take anyway).  1 (default): the fused kernels are taken where they are the faster way. */
 GCB_API int gcb_ctx_set_fused_attention(gcb_ctx* ctx, int on);
 
 /* ---- arena: CUDAMemPool::{allocate,free,clear,get_hwm_gb}, memory_pool.hpp:40-102 -------------- */
@@ -234,11 +234,13 @@ GCB_API int gcb_rowdot_batched_f32(gcb_ctx* ctx, float* out, const float* a, int
 /* Causal attention softmax(scale q k^T) v over batch x heads sequences of seq_len rows and head_dim columns without the seq_len x seq_len
  * matrices, forward and backward (frontend/tensor_other.hpp:53-93 composes both from matmul and causal_softmax).  Operands are addressed
  * through row, sequence and head strides in elements; columns are contiguous.  gcb_attention_supported says whether the operands can be
- * taken (otherwise both calls return GCB_UNSUPPORTED and touch nothing).  stats: gcb_attention_stats_floats floats that the forward
+ * taken (otherwise both calls return GCB_UNSUPPORTED and touch nothing), gcb_attention_preferred whether for these sizes they are the
+ * faster way (gcb_ctx_set_fused_attention).  stats: gcb_attention_stats_floats floats that the forward
  * fills and the backward reads.  dq, dk and dv share one layout and are overwritten; out is the forward's result, dout its gradient. */
 GCB_API int64_t gcb_attention_stats_floats(int64_t batch, int64_t heads, int64_t seq_len);
 GCB_API int gcb_attention_supported(gcb_ctx* ctx, int64_t batch, int64_t heads, int64_t seq_len, int64_t head_dim, const float* q, int64_t q_ld, int64_t q_so, int64_t q_si,
                             const float* k, int64_t k_ld, int64_t k_so, int64_t k_si, const float* v, int64_t v_ld, int64_t v_so, int64_t v_si, float scale);
+GCB_API int gcb_attention_preferred(gcb_ctx* ctx, int64_t batch, int64_t heads, int64_t seq_len, int64_t head_dim);
 GCB_API int gcb_attention_fwd_f32(gcb_ctx* ctx, int64_t batch, int64_t heads, int64_t seq_len, int64_t head_dim, float* out, int64_t o_ld, int64_t o_so, int64_t o_si, float* stats,
                           const float* q, int64_t q_ld, int64_t q_so, int64_t q_si, const float* k, int64_t k_ld, int64_t k_so, int64_t k_si,
                           const float* v, int64_t v_ld, int64_t v_so, int64_t v_si, float scale);

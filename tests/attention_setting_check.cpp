@@ -26,9 +26,9 @@ int main() {
             Tensor<float> act = out.gelu();
             act.realize();
             if (gcb_ctx_launch_count_named(c, "attention_") == 0) { std::printf("not fused\n"); return 1; }
-            gcb_check(gcb_ctx_set_fused_attention(c, change ? 0 : 1), "setting");
+            if (change) gcb_check(gcb_ctx_set_gemm_split_mode(c, 1), "setting");  // which the tensor-core pair does not compute in
             act.backward();
-            gcb_check(gcb_ctx_set_fused_attention(c, 1), "setting");
+            gcb_check(gcb_ctx_set_gemm_split_mode(c, 2), "setting");
             for (int i = 0; i < 3; ++i) {
                 Tensor<float> g = make_contiguous(in[i].grad().value());
                 grads[change][i].resize((size_t)g.volume());

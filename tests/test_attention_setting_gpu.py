@@ -1,5 +1,5 @@
-"""The setting for the separate attention kernels may change between a forward and its backward: the fused forward keeps row statistics
-(not the probabilities that the reference's CausalSoftmax node keeps, frontend/tensor_other.hpp:53-93), so the backward forms them."""
+"""A context's settings may change between a forward and its backward: the fused attention forward keeps row statistics (not the
+probabilities that the reference's CausalSoftmax node keeps, frontend/tensor_other.hpp:53-93), so the backward then forms them."""
 import os
 import subprocess
 

@@ -607,8 +607,7 @@ def test_small_products_on_the_fma_kernel(env, opa, opb, M, N, K):
 @pytest.mark.parametrize("Bn,H,T,D", [(1, 1, 257, 64), (1, 2, 129, 64), (2, 2, 255, 32), (2, 2, 256, 64), (3, 2, 256, 32), (2, 3, 384, 64), (1, 2, 511, 32), (3, 2, 300, 20), (1, 1, 1025, 4), (40, 4, 260, 48), (1, 1, 1, 4), (2, 3, 63, 32), (2, 2, 65, 64), (1, 2, 128, 128), (3, 1, 100, 68)])
 def test_fused_causal_attention(env, Bn, H, T, D):
     """Both pairs of kernels (up to 128 positions: fp32 FMA): partial and whole query tiles, one and two tiles a CTA, several items a CTA, padded head widths; scores that grow along the
-    row (the running maximum moves).  256 positions are taken like any other length; heads beyond the range, and contexts that asked for
-    the separate kernels, are declined."""
+    row (the running maximum moves).  256 positions are taken like any other length; heads beyond the range are declined."""
     ctx, torch, capi = env
     ctx.ctx_set_gemm_engine(0)
     C, scale = H * D, 1.0 / np.sqrt(D)
@@ -635,13 +634,23 @@ def test_fused_causal_attention(env, Bn, H, T, D):
         assert np.linalg.norm(got - ref) <= TOL * np.linalg.norm(ref)
 
     def takes(length, width):
-        return capi.lib().cdll.gcb_attention_supported(ctx.h, Bn, H, length, width, dq.data_ptr(), *rows, dk.data_ptr(), *rows, dv.data_ptr(), *rows, scale)
+        return capi.lib().attention_supported(ctx.h, Bn, H, length, width, dq.data_ptr(), *rows, dk.data_ptr(), *rows, dv.data_ptr(), *rows, scale)
 
     ctx.ctx_set_gemm_engine(0)
     try:
         assert takes(256, 64) == 1 and takes(256, 68) == 0 and takes(T, D) == 1
+    finally:
+        ctx.ctx_set_gemm_engine(2)
+
+
+@pytest.mark.parametrize("Bn,H,T,D,preferred", [(1, 2, 64, 64, 1), (9, 4, 128, 32, 1), (1, 1, 65, 36, 0), (3, 4, 128, 64, 0), (5, 3, 128, 64, 1), (4, 4, 64, 96, 0), (8, 8, 64, 96, 1), (9, 4, 100, 68, 0), (1, 1, 129, 64, 1)])
+def test_short_attention_is_taken_where_its_chain_is_short_or_its_ctas_many(env, Bn, H, T, D, preferred):
+    ctx, torch, capi = env
+    ctx.ctx_set_gemm_engine(0)
+    try:
+        assert ctx.attention_preferred(Bn, H, T, D) == preferred
         ctx.ctx_set_fused_attention(0)
-        assert takes(256, 64) == 0 and takes(T, D) == 0
+        assert ctx.attention_preferred(Bn, H, T, D) == 0
     finally:
         ctx.ctx_set_fused_attention(1)
         ctx.ctx_set_gemm_engine(2)
