@@ -344,37 +344,50 @@ __global__ void __launch_bounds__(32 * kFoldWarps) scatter_fold_kernel(float* __
     }
 }
 
-// A short index list in one launch: a warp per entry and 32 lanes' worth of columns.  The first entry with a given index adds up
-// all of them in list order; the others find an earlier one and leave.  Every warp reads the list once, so this is for lists of a
-// few rounds of 32 (256 entries of 128 columns: 3 us instead of six launches and 20 us).
-constexpr int kShortList = 1024;
+// A short index list in one launch: a block per entry and 32 lanes' worth of columns, each of its warps looking through a stretch of the
+// list.  The block of the first entry with a given index adds up all of them, every warp its stretch in list order and then the
+// stretches in theirs; the blocks of the others find an earlier one and leave.
+// Bound by the blocks' start and one pass over the list, and for a list of one repeated index (padding) by a warp's chain of rows: 256
+// entries of 128 columns 3.1 us (tokens) and 5.1 (all equal), 1024 entries of 1024 columns 12 and 21; with one warp an entry 8.0 and 30,
+// 29 and 117; in the six launches 18.6 and 18.6, 22 and 21.  Their line lies where the slowest list takes as long either way: 1024
+// entries, and 12288 blocks (384 entries of 4096 columns 20 us, 512 24 against 21; 256 of 1537 columns, a float a lane, 17, 384 26 against 18).
+constexpr int kShortList = 1024, kShortBlocks = 12288, kShortWarps = 8, kShortRounds = kShortList / (32 * kShortWarps);
 template <class IdxT, int VEC>
-__global__ void __launch_bounds__(256) scatter_short_kernel(float* __restrict__ dtable, const IdxT* __restrict__ idx, const float* __restrict__ dy, int n, int64_t width, int64_t vocab, int* __restrict__ status) {
+__global__ void __launch_bounds__(32 * kShortWarps) scatter_short_kernel(float* __restrict__ dtable, const IdxT* __restrict__ idx, const float* __restrict__ dy, int n, int64_t width, int64_t vocab, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
-    const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (i >= n) return;
+    __shared__ float part[kShortWarps][32 * VEC];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x;
     const int64_t mine = (int64_t)idx[i];
     if (mine < 0 || mine >= vocab) {
-        if (lane == 0 && blockIdx.y == 0) { atomicExch(&status[0], 2); atomicExch(&status[1], i); }
+        if (threadIdx.x == 0 && blockIdx.y == 0) { atomicExch(&status[0], 2); atomicExch(&status[1], i); }
         return;
     }
-    for (int j0 = 0; j0 < i; j0 += 32)
-        if (__any_sync(0xffffffffu, j0 + lane < i && (int64_t)idx[min(j0 + lane, n - 1)] == mine)) return;
+    const int rounds = (n + 32 * kShortWarps - 1) / (32 * kShortWarps), first = warp * rounds * 32;
+    unsigned hits[kShortRounds];
+    bool earlier = false;
+#pragma unroll
+    for (int r = 0; r < kShortRounds; ++r) {
+        const int j = first + 32 * r + lane;
+        const bool same = r < rounds && j < n && (int64_t)idx[j] == mine;
+        hits[r] = __ballot_sync(0xffffffffu, same);
+        earlier = earlier || (same && j < i);
+    }
+    if (__syncthreads_or(earlier)) return;
     const int64_t c = ((int64_t)blockIdx.y * 32 + lane) * VEC;
     const bool valid = c < width;
     float acc[VEC] = {};
-    for (int j0 = i & ~31; j0 < n; j0 += 32) {
-        const int j = j0 + lane;
-        unsigned hits = __ballot_sync(0xffffffffu, j >= i && j < n && (int64_t)idx[min(j, n - 1)] == mine);
-        while (hits) {  // up to four rows in flight
+#pragma unroll
+    for (int r = 0; r < kShortRounds; ++r) {
+        unsigned h = hits[r];
+        while (h) {  // up to four rows in flight
             float x[4][VEC];
             int got = 0;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                if (hits == 0) break;
-                const float* src = dy + (int64_t)(j0 + __ffs(hits) - 1) * width + c;
-                hits &= hits - 1;
+                if (h == 0) break;
+                const float* src = dy + (int64_t)(first + 32 * r + __ffs(h) - 1) * width + c;
+                h &= h - 1;
                 got = u + 1;
                 if (!valid) continue;
                 if (VEC == 4) { const float4 v = ld4(src); x[u][0] = v.x; x[u][1 % VEC] = v.y; x[u][2 % VEC] = v.z; x[u][3 % VEC] = v.w; }
@@ -387,7 +400,13 @@ __global__ void __launch_bounds__(256) scatter_short_kernel(float* __restrict__ 
                     for (int e = 0; e < VEC; ++e) acc[e] += valid ? x[u][e] : 0.0f;
         }
     }
-    if (!valid) return;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) part[warp][lane * VEC + e] = acc[e];
+    __syncthreads();
+    if (warp > 0 || !valid) return;
+    for (int w = 1; w < kShortWarps && w * rounds * 32 < n; ++w)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] += part[w][lane * VEC + e];
     float* dst = dtable + mine * width + c;
 #pragma unroll
     for (int e = 0; e < VEC; ++e) dst[e] += acc[e];
@@ -446,8 +465,8 @@ template <class IdxT>
 static int scatter_add_impl(gcb_ctx* ctx, float* dtable, const IdxT* idx, const float* dy, int64_t n, int64_t width, int64_t vocab) {
     const bool vec = width % 4 == 0 && aligned16(dtable) && aligned16(dy);
     const int64_t short_tiles = (width + (vec ? 128 : 32) - 1) / (vec ? 128 : 32);
-    if (n <= kShortList && short_tiles <= 65535) {
-        GCB_CHECK_CUDA(launch_next(ctx->stream, dim3((unsigned)((n + 7) / 8), (unsigned)short_tiles), 256, 0, vec ? scatter_short_kernel<IdxT, 4> : scatter_short_kernel<IdxT, 1>, dtable, idx, dy, (int)n, width, vocab, ctx->d_status));
+    if (n <= kShortList && n * short_tiles <= kShortBlocks) {
+        GCB_CHECK_CUDA(launch_next(ctx->stream, dim3((unsigned)n, (unsigned)short_tiles), 32 * kShortWarps, 0, vec ? scatter_short_kernel<IdxT, 4> : scatter_short_kernel<IdxT, 1>, dtable, idx, dy, (int)n, width, vocab, ctx->d_status));
         return after_launch(ctx, "scatter_short");
     }
     Scratch sc(ctx);

@@ -273,8 +273,8 @@ GCB_API int gcb_profile_gemm_end(gcb_ctx* ctx, int64_t* launches, double* total_
 
 /* ---- embedding: CUDAMath::apply_embed / apply_scatter_add, cuda_math.hpp:29-32 ------------------ */
 GCB_API int gcb_embed_f32(gcb_ctx* ctx, float* out, const void* indices, int index_type, const float* table, int64_t n_indices, int64_t width, int64_t vocab);
-/* dtable[idx[i], :] += dy[i, :].  Deterministic: positions are counting-sorted by row (stable) and each
- * row is accumulated in ascending position order.  Out-of-range indices are reported, not dereferenced. */
+/* dtable[idx[i], :] += dy[i, :].  Deterministic: the positions of a row are added up in a fixed order (ascending
+ * within stretches, the stretches in order).  Out-of-range indices are reported, not dereferenced. */
 GCB_API int gcb_scatter_add_f32(gcb_ctx* ctx, float* dtable, const void* indices, int index_type, const float* dy, int64_t n_indices, int64_t width, int64_t vocab);
 /* The integer plan of the scatter alone (for bit-exact bookkeeping checks): order[n] = positions sorted
  * by row (stable), counts[vocab], offsets[vocab + 1].  All int32 device buffers. */

@@ -584,17 +584,25 @@ def test_causal_softmax_on_padded_rows(env, T, band):
     assert max_abs_rel(torch.where(seen, padded[:, :T], dense).cpu().numpy(), dense.cpu().numpy()) < 1e-6
 
 
-@pytest.mark.parametrize("n,V,C,i32", [(1, 3, 4, False), (256, 50, 128, True), (1024, 7, 132, False), (33, 1000, 5, False)])
-def test_scatter_add_of_a_short_list(env, n, V, C, i32):
-    """One launch up to 1024 entries: a single entry, rows hit many times, a part of a column tile, columns that are no multiple of four."""
+@pytest.mark.parametrize("n,V,C,i32,short", [(1, 3, 4, False, True), (256, 50, 128, True, True), (1024, 7, 132, False, True), (33, 1000, 5, False, True), (1024, 1, 128, True, True), (257, 2, 36, False, True), (1023, 900, 33, True, True),
+                                             (768, 5, 2048, False, True), (769, 1, 2048, False, False), (1025, 3, 8, False, False)])
+def test_scatter_add_of_a_short_list(env, n, V, C, i32, short):
+    """One launch up to 1024 entries and 12288 blocks: a single entry, rows hit many times, one row hit by all, a part of a column tile, columns
+    that are no multiple of four, lists that end inside a warp's stretch; beyond, the sorted way.  Bit-identical when repeated."""
     ctx, torch, capi = env
+    before = ctx.ctx_launch_count_named(b"scatter_short")
     idx = np.random.default_rng(3).integers(0, V, n)
     dy, table = rnd(5, n, C), rnd(6, V, C)
     ref = table.astype(np.float64)
     np.add.at(ref, idx, dy.astype(np.float64))
     out = dev(torch, table)
     ctx.scatter_add_f32(out, dev(torch, idx.astype(np.int32 if i32 else np.int64)), capi.IDX_I32 if i32 else capi.IDX_I64, dev(torch, dy), n, C, V)
-    assert max_abs_rel(host(ctx, out), ref) < 1e-5
+    got = host(ctx, out)
+    assert ctx.ctx_launch_count_named(b"scatter_short") == before + int(short)
+    assert max_abs_rel(got, ref) < 1e-5
+    out = dev(torch, table)
+    ctx.scatter_add_f32(out, dev(torch, idx.astype(np.int32 if i32 else np.int64)), capi.IDX_I32 if i32 else capi.IDX_I64, dev(torch, dy), n, C, V)
+    assert np.array_equal(host(ctx, out), got)
 
 
 @pytest.mark.parametrize("scale,max_norm", [(1.0, 0.5), (1.0, 1e6), (0.25, 0.5)])
