@@ -114,9 +114,25 @@ static int dispatch_gemm(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g, cons
     return rc;
 }
 
-// Validation, then the dispatch bracketed by one pair of timing events when profiling is on: a product is counted once
-// whatever path it takes, and the closing event is recorded on every exit so that gcb_profile_gemm_end never meets an
-// unrecorded event.
+// A dispatch bracketed by one pair of timing events when profiling is on: it is counted once whatever path it takes, and the closing
+// event is recorded on every exit so that gcb_profile_gemm_end never meets an unrecorded event.
+template <class F>
+static int profiled(gcb_ctx* ctx, double flops, F&& dispatch) {
+    if (!ctx->prof_on) return dispatch();
+    if (ctx->prof_used + 2 > ctx->prof_events.size()) {
+        for (int i = 0; i < 512; ++i) { cudaEvent_t e; GCB_CHECK_CUDA(cudaEventCreate(&e)); ctx->prof_events.push_back(e); }
+    }
+    cudaEvent_t e0 = ctx->prof_events[ctx->prof_used], e1 = ctx->prof_events[ctx->prof_used + 1];
+    GCB_CHECK_CUDA(cudaEventRecord(e0, ctx->stream));
+    const int rc = dispatch();
+    GCB_CHECK_CUDA(cudaEventRecord(e1, ctx->stream));
+    if (rc == GCB_OK) {  // a refused problem leaves no trace in the tally
+        ctx->prof_used += 2;
+        ctx->prof_flops += flops;
+    }
+    return rc;
+}
+
 static int run_gemm(gcb_ctx* ctx, int op_a, int op_b, const GemmArgs& g, const char* who) {
     GCB_REQUIRE((op_a == GCB_OP_N || op_a == GCB_OP_T) && (op_b == GCB_OP_N || op_b == GCB_OP_T), "%s: op must be GCB_OP_N or GCB_OP_T", who);
     GCB_REQUIRE(g.M >= 0 && g.N >= 0 && g.K >= 0, "%s: negative dimension", who);
@@ -125,19 +141,7 @@ static int run_gemm(gcb_ctx* ctx, int op_a, int op_b, const GemmArgs& g, const c
     const bool ta = op_a == GCB_OP_T, tb = op_b == GCB_OP_T;
     GCB_REQUIRE(g.lda >= (ta ? g.M : g.K) && g.ldb >= (tb ? g.K : g.N) && g.ldc >= g.N, "%s: leading dimension smaller than the row length (lda %lld ldb %lld ldc %lld)", who,
                 (long long)g.lda, (long long)g.ldb, (long long)g.ldc);
-    if (!ctx->prof_on) return dispatch_gemm(ctx, ta, tb, g, who);
-    if (ctx->prof_used + 2 > ctx->prof_events.size()) {
-        for (int i = 0; i < 512; ++i) { cudaEvent_t e; GCB_CHECK_CUDA(cudaEventCreate(&e)); ctx->prof_events.push_back(e); }
-    }
-    cudaEvent_t e0 = ctx->prof_events[ctx->prof_used], e1 = ctx->prof_events[ctx->prof_used + 1];
-    GCB_CHECK_CUDA(cudaEventRecord(e0, ctx->stream));
-    const int rc = dispatch_gemm(ctx, ta, tb, g, who);
-    GCB_CHECK_CUDA(cudaEventRecord(e1, ctx->stream));
-    if (rc == GCB_OK) {  // a refused problem leaves no trace in the tally
-        ctx->prof_used += 2;
-        ctx->prof_flops += 2.0 * (double)g.M * (double)g.N * (double)g.K * (double)(g.batch_outer * g.batch_inner * g.k_groups);
-    }
-    return rc;
+    return profiled(ctx, 2.0 * (double)g.M * (double)g.N * (double)g.K * (double)(g.batch_outer * g.batch_inner * g.k_groups), [&] { return dispatch_gemm(ctx, ta, tb, g, who); });
 }
 
 extern "C" {
@@ -274,14 +278,14 @@ int gcb_linear_group_bwd_f32(gcb_ctx* ctx, int64_t groups, int64_t M, int64_t N,
     GCB_REQUIRE(ctx && groups >= 1 && groups <= 64 && (M == 0 || K == 0 || dx) && (N == 0 || dbias), "gcb_linear_group_bwd_f32: bad arguments");
     GCB_REQUIRE(gelu_pre == nullptr || (groups == 1 && dx_beta == 0.0f && gelu_pre != dx), "gcb_linear_group_bwd_f32: a GELU behind the input takes one layer and overwrites its gradient");
     const int64_t work = M * N * K * groups;
-    if (!ctx->prof_on && work > 0 && (ctx->gemm_engine == 1 || (ctx->gemm_engine == 0 && work < kSmallWork)) && x && dy && W && dW && (groups == 1 || (dy_stride >= M * N && w_stride > 0))) {
+    if (work > 0 && (ctx->gemm_engine == 1 || (ctx->gemm_engine == 0 && work < kSmallWork)) && x && dy && W && dW && (groups == 1 || (dy_stride >= M * N && w_stride > 0))) {
         GemmArgs gx{M, K, N, 1.0f, dx_beta, dy, W, nullptr, dx, N, N, K, 0, dy_stride, 0, w_stride, 0, 0, 1, 1};
         gx.gelu_pre = gelu_pre;
         gx.k_groups = (int)groups;
         GemmArgs gw{K, N, M, 1.0f, dw_beta, x, dy, nullptr, dW, K, N, N, 0, 0, 0, dy_stride, 0, dw_stride, 1, groups};
         gw.grouped = gx.grouped = true;
         gw.colsum = dbias; gw.colsum_si = bias_stride; gw.colsum_accumulate = bias_accumulate;
-        if (gemm_simt_backward_fits(gx, gw)) return gemm_simt_backward_launch(ctx, gx, gw);
+        if (gemm_simt_backward_fits(gx, gw)) return profiled(ctx, 4.0 * (double)work, [&] { return gemm_simt_backward_launch(ctx, gx, gw); });
     }
     int rc = gelu_pre ? gcb_gemm_gelu_bwd_f32(ctx, GCB_OP_N, GCB_OP_T, M, K, N, dy, N, W, N, gelu_pre, dx)
              : groups == 1 ? gcb_gemm_f32(ctx, GCB_OP_N, GCB_OP_T, M, K, N, 1.0f, dy, N, W, N, dx_beta, dx, K, nullptr)

@@ -267,7 +267,8 @@ GCB_API int64_t gcb_weight_twins_count(gcb_ctx* ctx);
 
 /* Measurement aid (the reference times with std::chrono around whole loops, benchmarks/bench_kernels.cpp:10-27):
  * between begin and end every GEMM launch is bracketed by CUDA events on the compute stream; end synchronises and
- * returns the number of launches, their summed device time and their algorithmic FLOPs (2*M*N*K*batches). */
+ * returns the number of launches, their summed device time and their algorithmic FLOPs (2*M*N*K*batches).  Both gradients of
+ * a small layer are one launch.  The products inside the fused attention kernels are not counted. */
 GCB_API int gcb_profile_gemm_begin(gcb_ctx* ctx);
 GCB_API int gcb_profile_gemm_end(gcb_ctx* ctx, int64_t* launches, double* total_ms, double* total_flops);
 

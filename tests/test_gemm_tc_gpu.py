@@ -699,3 +699,32 @@ def test_linear_layers_taken_together(env, engine, G, M, N, K, family):
     finally:
         ctx.weight_twins_drop(None, 0)
         ctx.ctx_set_gemm_engine(2)
+
+
+def test_profiling_times_the_launches_that_run_without_it(env):
+    """The two gradients of a small layer go down in one launch whether or not products are being timed, and count with the work of both."""
+    import ctypes
+
+    ctx, torch, capi = env
+    M, N, K = 70, 48, 36
+    x, dy, W = (torch.from_numpy(rnd(s, *shape)).cuda() for s, shape in ((1, (M, K)), (2, (M, N)), (3, (K, N))))
+    ctx.ctx_set_gemm_engine(0)
+    try:
+        launched, results = [], []
+        for profile in (False, True):
+            dx, dW, db = torch.empty(M, K, device="cuda"), torch.empty(K, N, device="cuda"), torch.empty(N, device="cuda")
+            before = ctx.ctx_launch_count_named(b"gemm_simt_backward"), ctx.ctx_launch_count()
+            if profile:
+                ctx.profile_gemm_begin()
+            ctx.linear_group_bwd_f32(1, M, N, K, x, dy, 0, W, 0, None, 0.0, dx, 0.0, dW, 0, db, 0, 0)
+            if profile:
+                n, ms, flops = ctypes.c_int64(), ctypes.c_double(), ctypes.c_double()
+                ctx.profile_gemm_end(ctypes.byref(n), ctypes.byref(ms), ctypes.byref(flops))
+                assert n.value == 1 and ms.value > 0.0 and flops.value == 4.0 * M * N * K
+            ctx.sync()
+            launched.append((ctx.ctx_launch_count_named(b"gemm_simt_backward") - before[0], ctx.ctx_launch_count() - before[1]))
+            results.append((dx, dW, db))
+        assert launched == [(1, 1), (1, 1)]
+        assert all(torch.equal(a, b) for a, b in zip(*results))
+    finally:
+        ctx.ctx_set_gemm_engine(2)
