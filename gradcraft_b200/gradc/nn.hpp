@@ -1104,7 +1104,9 @@ template <class Model>
 std::vector<int64_t> generate_tokens_incremental(Model& model, const std::vector<int64_t>& start_tokens, int64_t context_length, int64_t max_tokens, int64_t num_sequences, Device infer_device,
                                                  std::optional<float> temperature = std::nullopt, int64_t top_k = 30) {
     check_generation((int64_t)start_tokens.size(), max_tokens, infer_device);
-    if (num_sequences > 0 && context_length > 0) {
+    bool here = true;  // a model elsewhere is refused by its own forward
+    for (auto* p : model.parameters()) here = here && p->device() == infer_device;
+    if (here && num_sequences > 0 && context_length > 0) {
         IncrementalGPT inc(model, infer_device);
         if (inc.takes(std::min(context_length, max_tokens - 1))) return inc.generate(start_tokens, context_length, max_tokens, num_sequences, temperature, top_k);
     }
