@@ -73,7 +73,12 @@ static int dispatch_gemm(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g, cons
         rc = GCB_UNSUPPORTED;
         if (packed.A != g.A || packed.B != g.B) {
             if (gemm_tc_eligible(packed)) rc = gemm_tc_launch(ctx, ta, tb, packed);
-            if (rc == GCB_UNSUPPORTED && gemm_tc_eligible(packed)) return dispatch_gemm(ctx, ta, tb, packed, who);  // an epilogue that this kernel lacks runs as a second pass, on the packed operands
+            if (rc == GCB_UNSUPPORTED && gemm_tc_eligible(packed)) {  // an epilogue that this kernel lacks runs as a second pass, the product on the packed operands
+                packed.colsum = nullptr;  // of the operand as it was: packed rows lie further apart
+                rc = dispatch_gemm(ctx, ta, tb, packed, who);
+                if (rc == GCB_OK && g.colsum) rc = gcb_reduce_rows_f32(ctx, g.colsum, g.B, g.K, g.N, g.colsum_accumulate);
+                return rc;
+            }
         }
     }
     if (rc == GCB_UNSUPPORTED && (g.gelu_pre || g.gelu_act)) {
@@ -100,7 +105,7 @@ static int dispatch_gemm(gcb_ctx* ctx, bool ta, bool tb, const GemmArgs& g, cons
         plain.colsum = nullptr;
         rc = dispatch_gemm(ctx, ta, tb, plain, who);
         if (rc != GCB_OK) return rc;
-        if (!tb) return gcb_reduce_rows_f32(ctx, g.colsum, g.B, g.K, g.N, g.colsum_accumulate);
+        if (!tb && g.ldb == g.N) return gcb_reduce_rows_f32(ctx, g.colsum, g.B, g.K, g.N, g.colsum_accumulate);
         set_error("%s: column sums need op(B) stored K x N with ldb == N", who);
         return GCB_UNSUPPORTED;
     }

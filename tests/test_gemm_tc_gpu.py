@@ -460,7 +460,8 @@ def test_fused_epilogues_take_the_scalar_path_for_side_arrays_off_a_16_byte_boun
     assert torch.equal(out_a, out_b)
 
 
-@pytest.mark.parametrize("Kin,Nout,Mtok,family", [(1024, 1024, 8192, "gemm_tc_pair"), (512, 768, 4096, "gemm_tc_pair"), (256, 1024, 300, "gemm_tc_pair"), (96, 80, 200, None), (1024, 100, 4096, None)])
+@pytest.mark.parametrize("Kin,Nout,Mtok,family", [(1024, 1024, 8192, "gemm_tc_pair"), (512, 768, 4096, "gemm_tc_pair"), (256, 1024, 300, "gemm_tc_pair"), (96, 80, 200, None), (1024, 100, 4096, None),
+                                                    (479, 94, 2098, None), (867, 1105, 135, None), (256, 1031, 300, "gemm_tc_pair")])  # rows that TMA cannot address: packed, with and without the pair kernel
 def test_weight_gradient_with_bias_gradient_from_one_pass(env, Kin, Nout, Mtok, family):
     """dW = x^T dy and db = column sums of dy from one call, against float64: shapes that run the CTA-pair kernel with and
     without K slices (the B-splitter warps gather the sums), and shapes that fall back to the product plus a row reduction.
