@@ -609,8 +609,10 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) attention_bwd_kernel(const 
                 if (k_major != (b <= OK)) return true;
                 if (!warp_wait(full(b), (n0 + i) & 1u, p.status, 36)) return false;
                 uint8_t* raw = gen + S::BLOCKS_OFF + b * S::BLOCK;
-                if (keeps) {  // the block before last has been used: its products preceded this block's
-                    float* slot = stats_sm + (i & 1) * 3 * AT_KEYS + t;
+                // Two slots, by the running number of the block: the one before last has been used (its products preceded the last one's, which
+                // this block's copy waited for), also where the last one belongs to the item before.
+                if (keeps) {
+                    float* slot = stats_sm + ((n0 + i) & 1u) * 3 * AT_KEYS + t;
                     const int64_t next = at + (int64_t)(i + 1) * AT_KEYS;
                     if (b == QK) {
                         slot[0] = nm; slot[AT_KEYS] = ni;
@@ -657,7 +659,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) attention_bwd_kernel(const 
             const int cnt = steps(it);
 #pragma unroll 1
             for (int i = 0; i < cnt; ++i, ++n) {
-                const float4* mp = reinterpret_cast<const float4*>(gen + S::STATS_OFF + (i & 1) * 3 * AT_KEYS * 4) + 4 * part;
+                const float4* mp = reinterpret_cast<const float4*>(gen + S::STATS_OFF + (n & 1u) * 3 * AT_KEYS * 4) + 4 * part;
                 const float4 *ip = mp + AT_KEYS / 4, *dp = ip + AT_KEYS / 4;
                 ok = warp_wait(s_full, n & 1u, p.status, 37);
                 if (!ok) break;

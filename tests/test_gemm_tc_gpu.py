@@ -605,9 +605,10 @@ def test_small_products_on_the_fma_kernel(env, opa, opb, M, N, K):
         ctx.ctx_set_gemm_engine(2)
 
 
-@pytest.mark.parametrize("Bn,H,T,D", [(1, 1, 257, 64), (1, 2, 129, 64), (2, 2, 255, 32), (2, 2, 256, 64), (3, 2, 256, 32), (2, 3, 384, 64), (1, 2, 511, 32), (3, 2, 300, 20), (1, 1, 1025, 4), (40, 4, 260, 48), (1, 1, 1, 4), (2, 3, 63, 32), (2, 2, 65, 64), (1, 2, 128, 128), (3, 1, 100, 68)])
+@pytest.mark.parametrize("Bn,H,T,D", [(1, 1, 257, 64), (1, 2, 129, 64), (2, 2, 255, 32), (2, 2, 256, 64), (3, 2, 256, 32), (2, 3, 384, 64), (1, 2, 511, 32), (3, 2, 300, 20), (6, 5, 546, 48), (6, 5, 530, 4), (5, 6, 600, 64), (1, 1, 1025, 4), (40, 4, 260, 48), (1, 1, 1, 4), (2, 3, 63, 32), (2, 2, 65, 64), (1, 2, 128, 128), (3, 1, 100, 68)])
 def test_fused_causal_attention(env, Bn, H, T, D):
-    """Both pairs of kernels (up to 128 positions: fp32 FMA): partial and whole query tiles, one and two tiles a CTA, several items a CTA, padded head widths; scores that grow along the
+    """Both pairs of kernels (up to 128 positions: fp32 FMA): partial and whole query tiles, one and two tiles a CTA, several items a CTA (also two CTAs alone with a second one, after an odd number
+    of blocks), padded head widths; scores that grow along the
     row (the running maximum moves).  256 positions are taken like any other length; heads beyond the range are declined."""
     ctx, torch, capi = env
     ctx.ctx_set_gemm_engine(0)
