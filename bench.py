@@ -13,7 +13,8 @@ Prints one JSON line (rank 0):
   e2e       the same through the public trainer call with pinned HOST token buffers, the H2D copies and a D2H read of
             the loss inside the timed region;
   roofline  the GEMM engine (dominant kernel): algorithmic FLOP/s over the launches of the timed region vs the measured
-            dense tensor peak;
+            dense tensor peak (the products inside the fused attention kernels are not among those launches: step_frac_of_split_ceiling
+            is the whole step's algorithmic FLOP/s over the same ceiling);
   kernels   (1 GPU) every bandwidth-bound backward / optimizer kernel at the microbenchmark shapes: achieved HBM GB/s over the
             measured copy peak ("bwd kernel % HBM peak", the second half of the metric);
   reference_cuda / vs_reference_cuda  (1 GPU) the reference's own CUDA path built for sm_100a, same model and batch, and
@@ -382,6 +383,8 @@ def run_ours(args, rank, world, local_rank):
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": pk["tensor_tflops"], "unit": "TFLOP/s", "frac": achieved / pk["tensor_tflops"],
                          "traffic": profile_traffic(TRAFFIC_PROFILE), "traffic_note": "dram read+write of one captured launch of the most frequent shape (M=32768, N=K=1024; algorithmic 272.6 MB), read from profiles/" + TRAFFIC_PROFILE,
                          "frac_of_split_ceiling": achieved / (pk["tensor_tflops"] / units),
+                         "step_frac_of_split_ceiling": fpt * tokens_per_step / world / (ms_dev / K / 1e3) / 1e12 / (pk["tensor_tflops"] / units),
+                         "covers": "linear layers, vocabulary head and attention's dQ; the other attention products run inside the fused attention kernels",
                          "kernel": "gemm (%d launches, %.1f ms of the timed region)" % (n_gemm, gemm_ms),
                          "peak_source": "%s dense bf16, sustained; split mode %d spends the tensor time of %d bf16 MMAs per product (a tf32 MMA counts 2), so its ceiling is 1/%d of this" % (pk["source"], split_mode, units, units),
                          "gemm_share_of_step": gemm_ms / ms_dev},

@@ -1,4 +1,4 @@
-// Causal attention without the T x T matrices: softmax(scale q k^T) v and its backward in one kernel each, on tcgen05 / TMEM with the
+// Causal attention, softmax(scale q k^T) v, in one kernel and its backward in one kernel and a GEMM, on tcgen05 / TMEM with the
 // split-fp32 arithmetic of the GEMMs (one TF32 product of truncated operands + two BF16 cross products, tcgen05.cuh).
 // Reference counterpart: matmul, causal_softmax and their backward nodes as composed by frontend/tensor_other.hpp:53-93.
 //
@@ -18,12 +18,15 @@
 // first block; the quotient is exact either way.
 // Backward: a CTA takes 128 keys and walks over the queries from the diagonal on, with everything transposed (a thread owns a
 // key): S^T = k q^T, dP^T = v dO^T, dV += P^T dO, dK += dS^T q.  P comes from the row maximum and reciprocal sum the forward kept.
-// dS^T leaves through TMA for dQ = dS k, which is a GEMM.  Products are ordered so that the tensor core has dV(i), S(i+1) to do
+// dS^T leaves through TMA for dQ = dS k, which is a GEMM: the one T x T matrix that goes through memory.  Products are ordered so that the tensor core has dV(i), S(i+1) to do
 // while dS(i) is made and dK(i), dP(i+1) while P(i+1) is.  Four threads per key, 16 of a block's queries each; one splitter group per
 // layout (one for both: 10 % slower).
-// Measured, 32 x 16 heads of 1024 x 64: forward 391 us, forward + backward 1821 us (through memory: 2373); 8 x 12 heads of 512: 185
-// (210).  Tensor pipe 34 % / 27 % active, memory under a fifth of the copy rate: bound by the threads between the products, which
-// split what they have made and store it to tensor memory.
+// Measured, 32 x 16 heads of 1024 x 64: forward 391 us, forward + backward 1812 us (through memory: 2373 - 2480); 8 x 12 heads of 512:
+// 173 (188).  2800 cycles a block forward, 7000 backward, the tensor pipe active in 37 % / 29 % of them, memory under a third of the
+// copy rate; the threads between the products, which split what they have made and store it to tensor memory, were timed at 1400 and
+// 3000, so that the rest of the time has no name yet.
+// The tiling with a running maximum, P formed again from row statistics, and two query tiles in alternation are steps of the
+// FlashAttention publications (Dao et al. 2022, Dao 2023, Shah et al. 2024).
 // Every wait is bounded, as in the GEMM kernels.
 #include <algorithm>
 

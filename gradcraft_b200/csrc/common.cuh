@@ -133,8 +133,8 @@ inline int after_launch(gcb_ctx* ctx, const char* what, int n = 1) {
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Every entry point that writes device memory a caller could also use as a registered weight reports the range here: an
-// overlap marks the pre-split companions stale (they are recomputed before the next GEMM that needs one).
+// The entry points through which weights are written (copies, fills, elementwise, AdamW; the header lists them) report the range here:
+// an overlap marks the pre-split companions stale (they are recomputed before the next GEMM that needs one).
 inline void note_write(gcb_ctx* ctx, const void* p, size_t bytes) {
     if (ctx->twins_lo == nullptr || ctx->twins_dirty) return;
     const char* b = static_cast<const char*>(p);

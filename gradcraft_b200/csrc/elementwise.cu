@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(256) strided_kernel(float* __restrict__ out, c
 }
 
 // ---- reductions ----------------------------------------------------------------------------------
-// Stage 1: partial[slab, c] (+)= sum over the slab's rows of in[r, c]; a single slab goes straight to the result.  Block = 32 column groups x 8 row lanes.
+// Stage 1: partial[slab, c] (+)= sum over the slab's rows of in[r, c]; a single slab goes straight to the result (64 x 4096: 2.9 -> 1.7 us,
+// 5 x 127104: 3.9 -> 2.3).  Block = 32 column groups x 8 row lanes.
 template <int VEC>
 __global__ void __launch_bounds__(256) reduce_rows_stage1(float* __restrict__ partial, const float* __restrict__ in, int64_t rows, int64_t cols, int64_t rows_per_slab, int accumulate) {
     pdl_trigger();

@@ -843,7 +843,7 @@ inline Tensor<float> matmul(Tensor<float> x, Tensor<float> w) { return linear(st
 
 // ---- attention ----------------------------------------------------------------------------------------------------
 // softmax_causal(q k^T / sqrt(D)) v on (B, H, T, D) operands of any batch/row strides (frontend/tensor_other.hpp:53-93).
-// Longer sequences with heads of up to 64 columns take the fused kernels, which keep two numbers per query for the backward; otherwise
+// Where the fused kernels are preferred and take the operands they keep two numbers per query for the backward; otherwise
 // the probabilities are kept and the six batched GEMMs skip what causality zeroes: score / dP tiles above the diagonal are not computed, and the K loops
 // over the (transposed) probability matrices stop / start at the diagonal.
 // q, k, v are read in place through two-level batch strides — the head split reshape+permute of the attention layer

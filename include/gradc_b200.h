@@ -231,8 +231,9 @@ GCB_API int gcb_rowdot_batched_f32(gcb_ctx* ctx, float* out, const float* a, int
                            const float* b, int64_t ldb, int64_t b_stride_outer, int64_t b_stride_inner,
                            int64_t rows, int64_t cols, int64_t batch_outer, int64_t batch_inner);
 
-/* Causal attention softmax(scale q k^T) v over batch x heads sequences of seq_len rows and head_dim columns without the seq_len x seq_len
- * matrices, forward and backward (frontend/tensor_other.hpp:53-93 composes both from matmul and causal_softmax).  Operands are addressed
+/* Causal attention softmax(scale q k^T) v over batch x heads sequences of seq_len rows and head_dim columns, forward and backward, keeping
+ * two numbers a row instead of the seq_len x seq_len probabilities (frontend/tensor_other.hpp:53-93 composes both from matmul and
+ * causal_softmax).  Beyond 128 positions the backward takes batch x heads x seq_len x seq_len floats from the arena while it runs.  Operands are addressed
  * through row, sequence and head strides in elements; columns are contiguous.  gcb_attention_supported says whether the operands can be
  * taken (otherwise both calls return GCB_UNSUPPORTED and touch nothing), gcb_attention_preferred whether for these sizes they are the
  * faster way (gcb_ctx_set_fused_attention).  stats: gcb_attention_stats_floats floats that the forward
